@@ -207,6 +207,18 @@ int32_t pplb200_i8i8_linear_fp16(pplb200_stream_t stream, const void* x, const v
                                  int32_t epilogue_mode, float requant_up_scale,
                                  void* ws, int64_t ws_bytes, void* y, void* y_q, void* y_q_scale);
 
+/* The same call with its arguments in one block, for bindings in which every argument costs a conversion. */
+typedef struct pplb200_linear_args {
+    const void *x, *W, *scale_N, *optional_bias;
+    int64_t M, N, K;
+    void* ws;
+    int64_t ws_bytes;
+    void *y, *y_q, *y_q_scale;
+    float up_scale, down_scale_M, down_scale_N, requant_up_scale;
+    int32_t epilogue_mode, reserved;
+} pplb200_linear_args;
+int32_t pplb200_i8i8_linear_fp16_args(pplb200_stream_t stream, const pplb200_linear_args* args);
+
 /*
  * The same fused linear for callers whose activations and results live in HOST memory (pinned for the copies to be
  * asynchronous): x_host fp16 [M, K] in, y_host fp16 [M, N] out (and y_q_host int8 [M, N], y_q_scale_host fp16 [M]

@@ -327,6 +327,13 @@ int32_t pplb200_i8i8_linear_fp16(pplb200_stream_t stream, const void* x, const v
                       down_scale_N, requant_up_scale, gws, gemm_ws_bytes(M, epilogue_mode), y, N, y_q, y_q_scale, true);
 }
 
+int32_t pplb200_i8i8_linear_fp16_args(pplb200_stream_t stream, const pplb200_linear_args* a) {
+    if (!a) return fail(RC_INVALID_VALUE, "null argument block");
+    return pplb200_i8i8_linear_fp16(stream, a->x, a->W, a->scale_N, a->optional_bias, a->M, a->N, a->K, a->up_scale,
+                                    a->down_scale_M, a->down_scale_N, a->epilogue_mode, a->requant_up_scale, a->ws, a->ws_bytes,
+                                    a->y, a->y_q, a->y_q_scale);
+}
+
 int32_t pplb200_i8i8_relayout(pplb200_stream_t stream, const void* src, int32_t src_layout, void* dst, int32_t dst_layout,
                               int64_t rows, int64_t cols, int32_t elem_bytes) {
     auto known = [](int32_t l) { return l == LAYOUT_ROW_MAJOR || l == LAYOUT_COL32 || l == LAYOUT_COL32_2R_4R4 || l == LAYOUT_COL4_4R2_8C; };
