@@ -56,6 +56,8 @@ activation_rows_kernel(const ActParams p) {
     const int64_t row = blockIdx.x;
     const int units = (int)(p.dim >> 4);
     const int64_t in_cols = KIND == ACT_SWIGLU ? 2 * p.dim : p.dim;
+    pdl_launch_dependents();
+    pdl_wait_prior_grid();
     const float bs = __fmul_rn(__half2float(p.scale_batch[row]), p.down_batch);
     float gs = 0.0f;
     if (KIND == ACT_SILU_GATED) gs = __fmul_rn(__half2float(p.gate_scale_batch[row]), p.down_batch);
@@ -142,13 +144,15 @@ int32_t launch_act(cudaStream_t stream, const ActParams& p) {
     threads = (threads + 31) / 32 * 32;
     if (threads > ATPB) threads = ATPB;
     const dim3 grid((unsigned)p.batch), block(threads);
+    cudaError_t e;
     switch (bucket) {
-    case 1: activation_rows_kernel<1, KIND, REQUANT><<<grid, block, 0, stream>>>(p); break;
-    case 2: activation_rows_kernel<2, KIND, REQUANT><<<grid, block, 0, stream>>>(p); break;
-    case 4: activation_rows_kernel<4, KIND, REQUANT><<<grid, block, 0, stream>>>(p); break;
-    default: activation_rows_kernel<8, KIND, REQUANT><<<grid, block, 0, stream>>>(p); break;
+    case 1: e = launch_ex(activation_rows_kernel<1, KIND, REQUANT>, grid, block, stream, /*pdl=*/true, p); break;
+    case 2: e = launch_ex(activation_rows_kernel<2, KIND, REQUANT>, grid, block, stream, /*pdl=*/true, p); break;
+    case 4: e = launch_ex(activation_rows_kernel<4, KIND, REQUANT>, grid, block, stream, /*pdl=*/true, p); break;
+    default: e = launch_ex(activation_rows_kernel<8, KIND, REQUANT>, grid, block, stream, /*pdl=*/true, p); break;
     }
-    return check_launch("activation");
+    if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "activation launch failed: %s", cudaGetErrorString(e));
+    return RC_SUCCESS;
 }
 
 // dequantize (+bias) and scatter the columns into three row-major outputs; 4 columns per thread
@@ -158,6 +162,8 @@ dequantize_split3_kernel(const int32_t* __restrict__ acc, const half* __restrict
                          float down_m, float down_n, int32_t layout, half* __restrict__ o0, half* __restrict__ o1,
                          half* __restrict__ o2) {
     const int64_t chunks = dim >> 2, total = batch * chunks;
+    pdl_launch_dependents();
+    pdl_wait_prior_grid();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t m = i / chunks, n = (i - m * chunks) << 2;
         const float bs = __fmul_rn(__half2float(scale_m[m]), down_m);
@@ -234,10 +240,11 @@ int32_t dequantize_split3(cudaStream_t stream, const void* acc, const void* bias
     if (!acc || !sm || !sn || (d0 && !o0) || (d1 && !o1) || (d2 && !o2)) return fail(RC_INVALID_VALUE, "null pointer");
     int64_t blocks = (batch * (dim >> 2) + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    dequantize_split3_kernel<<<(unsigned)blocks, 256, 0, stream>>>((const int32_t*)acc, (const half*)bias, (const half*)sm,
-                                                                   (const half*)sn, batch, dim, d0, d1, d2, down_m, down_n, layout,
-                                                                   (half*)o0, (half*)o1, (half*)o2);
-    return check_launch("dequantize_split3");
+    const cudaError_t e = launch_ex(dequantize_split3_kernel, dim3((unsigned)blocks), dim3(256), stream, /*pdl=*/true,
+                                    (const int32_t*)acc, (const half*)bias, (const half*)sm, (const half*)sn, batch, dim, d0, d1, d2,
+                                    down_m, down_n, layout, (half*)o0, (half*)o1, (half*)o2);
+    if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "dequantize_split3 launch failed: %s", cudaGetErrorString(e));
+    return RC_SUCCESS;
 }
 
 } // namespace pplb200

@@ -96,12 +96,13 @@ int32_t gemm_entry(cudaStream_t stream, const void* A, int64_t lda, const void* 
         g.sk_ws = (char*)ws + need;
         g.sk_ws_bytes = ws_bytes - need;
     }
-    g.pdl = chained;
+    g.pdl = true;
+    g.after_quantizer = chained;
     rc = launch_gemm(stream, g);
     if (rc != RC_SUCCESS) return rc;
     if (mode == EPI_DEQUANT_F16_REQUANT_I8)
         rc = launch_quantize(stream, (const half*)out, M, N, requant_up, LAYOUT_ROW_MAJOR, (int8_t*)out_q,
-                             (half*)out_q_scale, g.row_absmax_bits, nullptr, /*pdl=*/M <= 128);
+                             (half*)out_q_scale, g.row_absmax_bits, nullptr, /*pdl=*/true);
     return rc;
 }
 
@@ -127,7 +128,7 @@ int32_t pplb200_i8i8_minmax_quantize_fp16(pplb200_stream_t stream, const void* i
     if (!aligned16(in) || !aligned16(q)) return fail(RC_INVALID_VALUE, "in and q must be 16-byte aligned");
     if (batch > 0x7fffffffLL) return fail(RC_UNSUPPORTED, "batch beyond 2^31 - 1");
     return launch_quantize((cudaStream_t)stream, (const half*)in, batch, quant_dim, up_scale, to_layout, (int8_t*)q,
-                           (half*)scale, nullptr);
+                           (half*)scale, nullptr, nullptr, /*pdl=*/true);
 }
 
 int32_t pplb200_i8i8_minmax_dequantize_fp16(pplb200_stream_t stream, const void* acc, const void* optional_bias,
@@ -254,10 +255,11 @@ int32_t pplb200_i8i8_gate_up_swiglu_requant(pplb200_stream_t stream_, const void
     g.out = activated; g.ldc = D;
     g.row_absmax_bits = maxima;
     g.beta = beta;
+    g.pdl = true;
     int32_t rc = launch_gemm(stream, g);
     if (rc != RC_SUCCESS) return rc;
     return launch_quantize(stream, (const half*)activated, M, D, up_scale, LAYOUT_ROW_MAJOR, (int8_t*)out_q, (half*)out_q_scale,
-                           maxima, nullptr, false);
+                           maxima, nullptr, /*pdl=*/true);
 }
 
 int64_t pplb200_i8i8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t epilogue_mode) {
@@ -287,6 +289,7 @@ int32_t pplb200_i8i8_gemm_i32(pplb200_stream_t stream, const void* A, int64_t ld
     g.down_m = 0.f; g.down_n = 0.f;
     g.out = C; g.ldc = ldc;
     g.row_absmax_bits = nullptr;
+    g.pdl = true;
     g.raw_alpha = alpha; g.raw_beta = beta; g.raw_bias = (const int32_t*)optional_bias_i32;
     return launch_gemm((cudaStream_t)stream, g);
 }

@@ -50,6 +50,7 @@ struct DecodeParams {
     // EPI_RAW_I32 with raw_affine != 0: out = raw_alpha * acc + raw_beta * out + raw_bias[n] (wrapping int32)
     int32_t raw_affine, raw_alpha, raw_beta;
     const int32_t* raw_bias;
+    int32_t early_weights;       // the preceding kernel does not write the weights: load them before waiting for it
     int32_t w_stages;            // stages of the weight ring (tile_rows * 128 bytes each)
     unsigned long long* stamps;  // optional diagnostics: 8 x uint64 per CTA, global-timer stamps of its phases
 };
@@ -123,12 +124,6 @@ __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
-}
-__device__ __forceinline__ void pdl_wait_prior_grid() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-__device__ __forceinline__ void pdl_launch_dependents() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // Per-token maximum over the 32 lanes of a warp for NV tokens held as a[0..NV) in every lane
@@ -262,7 +257,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const uint32_t tmem_base = tmem_base_slot;
     const unsigned long long t_setup = p.stamps ? globaltimer_ns() : 0ull;
 
-    // per-thread output column (= weight row) and its constants; these belong to the weights, not to
+    // per-thread output column (= weight row) and its constants; behind the quantizer they belong to the weights, not to
     // the preceding kernel, so they are fetched now and their latency hides behind the main loop
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     const int grp = warp >> 2; // which slice of the token columns it handles
@@ -273,17 +268,27 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const bool n_ok = n < p.N && q * 32 + lane < p.tile_rows;
     float sn = 0.0f;
     half bias_h = __ushort_as_half((unsigned short)0x8000u); // x + (-0.0) == x for every x: no branch for "no bias"
-    if (p.mode != EPI_RAW_I32 && n_ok) {
-        sn = __half2float(p.scale_n[n]);
-        if (p.bias != nullptr) bias_h = p.bias[n];
-    }
+    auto load_column_constants = [&] {
+        if (p.mode != EPI_RAW_I32 && n_ok) {
+            sn = __half2float(p.scale_n[n]);
+            if (p.bias != nullptr) bias_h = p.bias[n];
+        }
+    };
+    if (p.early_weights) load_column_constants();
 
     bool ok = true;
     if (warp == 0 && lane == 0) {
-        // ---- TMA producer of the weight ring.  The first tiles do not depend on the preceding kernel: they are
-        // requested before the programmatic-dependency wait.
+        // ---- TMA producer of the weight ring.  Behind the fused linear's own quantizer, which does not write the
+        // weights, the first tiles are requested before the programmatic-dependency wait.  Behind an unknown kernel
+        // (it may be the one that writes the weights) the same tiles are only brought into L2 by then, where a later
+        // write still reaches them; the loads proper follow the wait.
         const uint32_t fw0 = ptx::smem_addr(&full_w[0]), ew0 = ptx::smem_addr(&empty_w[0]);
         const int prew = nkb < SW ? nkb : SW;
+        if (!p.early_weights) {
+            const int ahead = nkb < 2 * SW ? nkb : 2 * SW;
+            for (int i = 0; i < ahead; ++i) ptx::tma_prefetch_l2_2d(&tmap_w, PPLB200_KB(i) * BK, n_tile * p.tile_rows);
+            pdl_wait_prior_grid();
+        }
         for (int i = 0; i < prew; ++i) {
             ptx::mbar_arrive_expect_tx(fw0 + i * 8u, w_stride);
             ptx::tma_load_2d(ring + i * w_stride, &tmap_w, fw0 + i * 8u, PPLB200_KB(i) * BK, n_tile * p.tile_rows);
@@ -344,6 +349,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     (void)ok;
     __syncwarp();
     pdl_wait_prior_grid(); // every thread: scale_m / row_absmax come from the preceding kernel too
+    if (!p.early_weights) load_column_constants();
 
     if (p.mode != EPI_RAW_I32) {
         for (int m = threadIdx.x; m < BT; m += NUM_THREADS)
@@ -653,6 +659,7 @@ int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecDeviceInfo& d
     if (p.w_stages > MAX_W_STAGES) p.w_stages = MAX_W_STAGES;
     p.w_stages -= p.w_stages % DCfg<BT>::NACC; // see X_STAGES
     p.stamps = stall_counters();
+    p.early_weights = a.after_quantizer ? 1 : 0;
 
     const int n_tiles = (int)((a.N + tile_rows - 1) / tile_rows);
     if (!make_map(&tw, a.B, a.N, a.K, a.ldb, tile_rows)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (W) encode failed");

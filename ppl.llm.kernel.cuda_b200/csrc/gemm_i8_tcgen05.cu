@@ -287,6 +287,8 @@ gemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem_base = tmem_base_slot;
+    pdl_launch_dependents(); // every CTA is resident: a dependent kernel may set itself up under this one
+    pdl_wait_prior_grid();   // as a programmatic dependent: everything above ran under the tail of the preceding kernel
 
     const int num_tiles = p.num_m_tiles * p.num_n_tiles;
     const int nkb = p.num_k_blocks;
@@ -497,7 +499,8 @@ gemm_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
     // Launched as a programmatic dependent (fused linear), everything above ran under the tail of the preceding
     // kernel; its results (quantized activations, row scales, cleared scratch) are needed from here on.  Every
     // thread waits: all of them read such data.  A no-op in an ordinary launch.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_launch_dependents(); // every CTA is resident: a dependent kernel may set itself up under this one
+    pdl_wait_prior_grid();
 
     const int num_pairs = (int)(gridDim.x >> 1);
     const int pair_id = (int)(blockIdx.x >> 1);
@@ -827,17 +830,19 @@ gemm_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
     }
 }
 
-// Clears the K-slice scratch.  In the fused linear it is launched as a programmatic dependent of the quantizer: it
-// depends on nothing the quantizer writes, so it runs under the quantizer's last wave -- but it only EXITS after the
-// quantizer has completed (the wait below), because the GEMM, its own programmatic dependent, takes the completion of
-// this grid as its licence to read the quantizer's output.
-__global__ void __launch_bounds__(256) zero_fill_kernel(uint4* dst, int64_t vecs) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); // the GEMM may run its preamble meanwhile
+// Clears the K-slice scratch.  In the fused linear it is launched as a programmatic dependent of the quantizer, which is
+// an ordinary launch: nothing that came before still uses the scratch, so it is cleared under the quantizer's last wave
+// (idle) -- but the kernel only EXITS after the quantizer has completed (the wait below), because the GEMM, its own
+// programmatic dependent, takes the completion of this grid as its licence to read the quantizer's output.  Behind any
+// other kernel, which may itself have started before an earlier user of the scratch ended, it waits first.
+__global__ void __launch_bounds__(256) zero_fill_kernel(uint4* dst, int64_t vecs, bool idle) {
+    pdl_launch_dependents(); // the GEMM may run its preamble meanwhile
+    if (!idle) pdl_wait_prior_grid();
     const int64_t i0 = (int64_t)blockIdx.x * 1024 + threadIdx.x;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
         if (i0 + j * 256 < vecs) dst[i0 + j * 256] = make_uint4(0u, 0u, 0u, 0u);
-    asm volatile("griddepcontrol.wait;" ::: "memory"); // a no-op in an ordinary launch
+    pdl_wait_prior_grid(); // a no-op in an ordinary launch
 }
 
 // ---- host side ---------------------------------------------------------------------------------
@@ -956,8 +961,19 @@ int32_t launch_bn(cudaStream_t stream, const GemmArgs& a, const DeviceInfo& dev)
     p.num_n_tiles = (int32_t)((a.N + BN - 1) / BN);
     const int64_t tiles = (int64_t)p.num_m_tiles * p.num_n_tiles;
     const int grid = (int)(tiles < dev.sms ? tiles : dev.sms);
-    gemm_i8_tcgen05_kernel<BN><<<grid, NUM_THREADS, Cfg<BN>::SMEM_BYTES, stream>>>(ta, tb, tc, p);
-    return check_launch("gemm_i8_tcgen05");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid, 1, 1);
+    cfg.blockDim = dim3(NUM_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = Cfg<BN>::SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = a.pdl ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_i8_tcgen05_kernel<BN>, ta, tb, tc, p);
+    if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "GEMM launch failed: %s", cudaGetErrorString(e));
+    return RC_SUCCESS;
 }
 
 // 256 x 256 tiles on CTA pairs (clusters of two), persistent: one pair per two SMs.
@@ -1012,16 +1028,8 @@ int32_t launch_pair(cudaStream_t stream, const GemmArgs& a, const DeviceInfo& de
         if (f >= 2 && (g_slice_leftover_tiles == 2 || 4 * (f - 1) * p.num_k_blocks >= f * (52 + 5 * rest))) {
             // cleared by a kernel: a memset node between two kernels costs several times as much on the stream
             const int64_t vecs = (kSkStateBytes + rest * kSkTileBytes) / 16;
-            cudaLaunchConfig_t zc = {};
-            zc.gridDim = dim3((unsigned)((vecs + 1023) / 1024), 1, 1);
-            zc.blockDim = dim3(256, 1, 1);
-            zc.stream = stream;
-            cudaLaunchAttribute za;
-            za.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            za.val.programmaticStreamSerializationAllowed = 1;
-            zc.attrs = &za;
-            zc.numAttrs = a.pdl ? 1 : 0;
-            if (cudaLaunchKernelEx(&zc, zero_fill_kernel, static_cast<uint4*>(a.sk_ws), vecs) != cudaSuccess)
+            if (launch_ex(zero_fill_kernel, dim3((unsigned)((vecs + 1023) / 1024), 1, 1), dim3(256, 1, 1), stream, a.pdl,
+                          static_cast<uint4*>(a.sk_ws), vecs, a.after_quantizer) != cudaSuccess)
                 return fail(RC_DEVICE_RUNTIME_ERROR, "clearing the slice scratch failed: %s", cudaGetErrorString(cudaGetLastError()));
             p.sk_arrivals = static_cast<unsigned int*>(a.sk_ws);
             p.sk_scratch = reinterpret_cast<int32_t*>(static_cast<char*>(a.sk_ws) + kSkStateBytes);

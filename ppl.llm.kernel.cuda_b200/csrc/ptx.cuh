@@ -87,6 +87,12 @@ __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const CUtensorMap
         : "memory");
 }
 
+// brings the box into L2 only (nothing is tracked; L2 stays coherent with later writes of any SM)
+__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int32_t x, int32_t y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];"
+                 ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
+}
+
 // 2-D tiled store, shared -> global, tracked by the thread's bulk async-group.  The box is clipped at the
 // tensor's bounds; x * element size must be a multiple of 16 bytes and neither coordinate negative.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, uint32_t src, int32_t x, int32_t y) {

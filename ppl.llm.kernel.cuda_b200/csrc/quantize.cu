@@ -15,9 +15,6 @@ namespace {
 
 using namespace qdev;
 
-__device__ __forceinline__ void pdl_wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // One CTA per row.  A "unit" is 16 consecutive halves (two 128-bit loads, one 128-bit store).
 // Thread t owns units t, t + blockDim.x, ... (UNITS of them), kept in registers.
 template <int UNITS>
@@ -210,20 +207,6 @@ int grid_for(int64_t work_items, int tpb) {
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     return (int)blocks;
-}
-
-template <typename... Args>
-cudaError_t launch_ex(void (*kernel)(Args...), dim3 grid, dim3 block, cudaStream_t stream, bool pdl, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 } // namespace

@@ -34,6 +34,9 @@ skip_rmsnorm_quantize_kernel(const half* __restrict__ input, const half* __restr
     const int units = (int)(dim >> 4);
     const half* in_row = input + row * dim;
 
+    pdl_launch_dependents();
+    pdl_wait_prior_grid();
+
     // ---- load, skip add, statistics
     __half2 z[UNITS][8];
     float sumsq = 0.0f;
@@ -131,13 +134,15 @@ int32_t launch_skip_rmsnorm_quantize(cudaStream_t stream, const half* input, con
     threads = (threads + 31) / 32 * 32;
     if (threads > RTPB) threads = RTPB;
     const dim3 grid((unsigned)batch), block(threads);
+    cudaError_t e;
     switch (bucket) {
-    case 1: skip_rmsnorm_quantize_kernel<1><<<grid, block, 0, stream>>>(input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
-    case 2: skip_rmsnorm_quantize_kernel<2><<<grid, block, 0, stream>>>(input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
-    case 4: skip_rmsnorm_quantize_kernel<4><<<grid, block, 0, stream>>>(input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
-    default: skip_rmsnorm_quantize_kernel<8><<<grid, block, 0, stream>>>(input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
+    case 1: e = launch_ex(skip_rmsnorm_quantize_kernel<1>, grid, block, stream, /*pdl=*/true, input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
+    case 2: e = launch_ex(skip_rmsnorm_quantize_kernel<2>, grid, block, stream, /*pdl=*/true, input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
+    case 4: e = launch_ex(skip_rmsnorm_quantize_kernel<4>, grid, block, stream, /*pdl=*/true, input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
+    default: e = launch_ex(skip_rmsnorm_quantize_kernel<8>, grid, block, stream, /*pdl=*/true, input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
     }
-    return check_launch("skip_rmsnorm_quantize");
+    if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "skip_rmsnorm_quantize launch failed: %s", cudaGetErrorString(e));
+    return RC_SUCCESS;
 }
 
 } // namespace pplb200

@@ -400,3 +400,29 @@ def test_gemm_i32_alpha_beta_bias(cuda, M, N, K, alpha, beta, with_bias):
         want = want + bias.to(cuda.int64)[None, :]
     want = ((want + 2 ** 31) % (2 ** 32) - 2 ** 31).to(cuda.int32)
     assert cuda.equal(c, want)
+
+
+@pytest.mark.parametrize("M,N,K", [(8, 1024, 2048), (100, 2048, 1024), (300, 512, 1024), (2400, 2048, 512)])
+def test_back_to_back_launches_see_fresh_operands(cuda, M, N, K):
+    """Every kernel starts before its predecessor on the stream has ended.  Both operands of the GEMM are rewritten by the
+    launches right before it, round after round on the same buffers, and its result is rewritten right after."""
+    import pplb200
+    g = cuda.Generator(device="cuda").manual_seed(M + N + K)
+    xs = [cuda.randn((M, K), generator=g, device="cuda").half() for _ in range(12)]
+    wf = [cuda.randn((N, K), generator=g, device="cuda").half() for _ in range(12)]
+    xq, sm = cuda.empty((M, K), dtype=cuda.int8, device="cuda"), cuda.empty((M,), dtype=cuda.float16, device="cuda")
+    wq, sn = cuda.empty((N, K), dtype=cuda.int8, device="cuda"), cuda.empty((N,), dtype=cuda.float16, device="cuda")
+    acc = cuda.empty((M, N), dtype=cuda.int32, device="cuda")
+    ws = cuda.empty((max(256, pplb200.gemm_workspace_bytes(M, N, K, pplb200.EPI_RAW_I32)),), dtype=cuda.uint8, device="cuda")
+    got = []
+    for x, w in zip(xs, wf):
+        pplb200.minmax_quantize_fp16(x, out=xq, scale=sm)
+        pplb200.minmax_quantize_fp16(w, out=wq, scale=sn)
+        pplb200.gemm_i8i8(xq, wq, out=acc, ws=ws)
+        got.append(pplb200.minmax_dequantize_fp16(acc, sm, sn))
+    cuda.cuda.synchronize()
+    assert pplb200.gemm_status() == 0
+    for x, w, y in zip(xs, wf, got):
+        (q, s), (p, t) = pplb200.minmax_quantize_fp16(x), pplb200.minmax_quantize_fp16(w)
+        want = pplb200.minmax_dequantize_fp16((q.double() @ p.double().T).to(cuda.int32), s, t)  # int32 sums are exact in fp64
+        assert cuda.equal(y.view(cuda.int16), want.view(cuda.int16))
