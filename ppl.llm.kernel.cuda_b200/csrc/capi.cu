@@ -236,8 +236,8 @@ int32_t pplb200_i8i8_gate_up_swiglu_requant(pplb200_stream_t stream_, const void
     if ((reinterpret_cast<uintptr_t>(ws) & (WS_ALIGN - 1)) != 0) return fail(RC_INVALID_VALUE, "workspace must be 256-byte aligned");
     uint32_t* maxima = (uint32_t*)ws;
 
-    if (!swiglu_fusable(M, D)) {
-        // small problems: raw int32 GEMM, then the stand-alone SwiGLU + re-quantize kernel
+    if (M > 128 && !swiglu_fusable(M, D)) {
+        // too few tiles for the CTA pairs, too many tokens for the small-batch kernel: raw int32 GEMM, then the stand-alone SwiGLU + re-quantize kernel
         void* acc = (char*)ws + round_up(M * 4 + 4, WS_ALIGN);
         int32_t rc = gemm_entry(stream, input, lda, weight, K, M, 2 * D, K, EPI_RAW_I32, nullptr, nullptr, nullptr, 0.f, 0.f, 0.f,
                                 nullptr, 0, acc, 2 * D, nullptr, nullptr, false);
@@ -246,8 +246,12 @@ int32_t pplb200_i8i8_gate_up_swiglu_requant(pplb200_stream_t stream_, const void
                           activated, out_q, out_q_scale);
     }
 
-    if (cudaMemsetAsync(maxima, 0, (size_t)M * 4, stream) != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "memset failed");
+    // The small-batch kernel writes its CTAs' partial maxima, at most 2 D per row: the [M, 2 D] int32 that the workspace
+    // holds for such a batch.
+    int32_t parts = 1;
+    if (M > 128 && cudaMemsetAsync(maxima, 0, (size_t)M * 4, stream) != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "memset failed");
     GemmArgs g;
+    g.row_absmax_parts = &parts;
     g.A = (const int8_t*)input; g.lda = lda; g.B = (const int8_t*)weight; g.ldb = K;
     g.M = M; g.N = 2 * D; g.K = K; g.mode = EPI_SWIGLU_F16;
     g.scale_m = (const half*)scale_M; g.scale_n = (const half*)scale_N; g.bias = nullptr;
@@ -259,7 +263,7 @@ int32_t pplb200_i8i8_gate_up_swiglu_requant(pplb200_stream_t stream_, const void
     int32_t rc = launch_gemm(stream, g);
     if (rc != RC_SUCCESS) return rc;
     return launch_quantize(stream, (const half*)activated, M, D, up_scale, LAYOUT_ROW_MAJOR, (int8_t*)out_q, (half*)out_q_scale,
-                           maxima, nullptr, /*pdl=*/true);
+                           maxima, nullptr, /*pdl=*/true, parts);
 }
 
 int64_t pplb200_i8i8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t epilogue_mode) {

@@ -93,11 +93,11 @@ __host__ __device__ inline int64_t layout_offset(int32_t layout, int64_t rows, i
 // ---- kernels / launchers implemented across the translation units ----
 
 // given_absmax_bits != null: rows are quantized with that precomputed max |x| (float bits) instead of
-// scanning the row.  zero_absmax_bits != null: the kernel also clears that per-row array (for the
+// scanning the row, the maximum of given_parts values per row.  zero_absmax_bits != null: the kernel also clears that per-row array (for the
 // GEMM that follows).  pdl: launch as a programmatic dependent of the preceding kernel in the stream.
 int32_t launch_quantize(cudaStream_t stream, const half* in, int64_t batch, int64_t dim, float up_scale,
                         int32_t layout, int8_t* q, half* scale, const uint32_t* given_absmax_bits,
-                        uint32_t* zero_absmax_bits = nullptr, bool pdl = false);
+                        uint32_t* zero_absmax_bits = nullptr, bool pdl = false, int32_t given_parts = 1);
 
 int32_t launch_dequantize(cudaStream_t stream, const int32_t* acc, const half* bias, const half* scale_m,
                           const half* scale_n, int64_t batch, int64_t dim, float down_m, float down_n,
@@ -139,6 +139,9 @@ struct GemmArgs {
     // the weights, and above 128 tokens it is an ordinary launch, so nothing before it still uses the scratch.
     bool after_quantizer = false;
     float beta = 1.0f;         // EPI_SWIGLU_F16
+    // EPI_SWIGLU_F16, M <= 128: the row maxima are written as *row_absmax_parts partial maxima per row, [M][parts] (at
+    // most N values per row), instead of one cleared word; the launcher returns the number here.
+    int32_t* row_absmax_parts = nullptr;
     // EPI_RAW_I32 only: out = raw_alpha * acc + raw_beta * out + raw_bias[n] in wrapping int32 (the scaling and
     // int32 bias of the reference's gemm_i8i8i32, src/ppl/kernel/llm/cuda/cublas/gemm.cu:187-188,239-243)
     int32_t raw_alpha = 1, raw_beta = 0;

@@ -38,8 +38,12 @@ constexpr int SMEM_BUDGET = 210 * 1024; // one CTA per SM: the whole shared memo
 constexpr unsigned ST_DEC_PRODUCER = 16u, ST_DEC_MMA = 32u, ST_DEC_EPI = 64u;
 
 struct DecodeParams {
-    int32_t M, N;           // tokens, weight rows
-    int32_t tile_rows;      // weight rows per tile (a multiple of 8, <= 128), chosen so that the tiles fill the SMs
+    int32_t M, N;           // tokens, output columns (= weight rows; EPI_SWIGLU_F16: half of them)
+    int32_t tile_rows;      // weight rows per tile (a multiple of 8, <= 128; two-part tiles: per part), chosen so that the tiles fill the SMs
+    int32_t part_stride;    // two-part tiles: the second part starts this many weight rows after the first
+    int32_t w_box_bytes;    // bytes of weights that one K block brings in
+    int32_t w_slot_bytes;   // bytes between the slots of the weight ring
+    float beta;             // EPI_SWIGLU_F16
     int32_t num_k_blocks;
     int32_t mode;
     void* out; int64_t ldc; // [M, ldc] int32 or fp16
@@ -76,8 +80,8 @@ template <int BT> struct DCfg {
     // come from (measured), which capped the weight stream at two thirds of the HBM rate.  Two threads taking
     // alternate K blocks halve that; the epilogue adds the two partial tiles while it reads them.
     static constexpr int NACC = 2;
-    static constexpr int TMEM_COLS = NACC * BT < 32 ? 32 : NACC * BT;
-    static_assert(TMEM_COLS <= 512 && (TMEM_COLS & (TMEM_COLS - 1)) == 0, "tensor-memory allocation size");
+    template <bool DUAL> static constexpr int tmem_cols() { return NACC * BT * (DUAL ? 2 : 1) < 32 ? 32 : NACC * BT * (DUAL ? 2 : 1); }
+    static_assert(NACC * BT * 2 <= 512 && (BT & (BT - 1)) == 0, "tensor-memory allocation size");
     // A lone warp per scheduler runs the epilogue at a fraction of an instruction per clock, so
     // the accumulator columns are spread over GROUPS sets of four warps (one warp per TMEM lane
     // quarter in each set).
@@ -86,6 +90,9 @@ template <int BT> struct DCfg {
     static constexpr int GROUP_COLS = BT / GROUPS;
     static constexpr int LD_COLS = GROUP_COLS < 32 ? GROUP_COLS : 32; // columns per tcgen05.ld
     static constexpr int PIECES = 4 * (BT / PIECE_COLS);
+    // EPI_SWIGLU_F16: once the main loop is over, [received partials | partner accumulators | output tile] share the rings
+    static constexpr int SWIGLU_PARTNER = 72 * 1024, SWIGLU_OUT = 104 * 1024; // at most 72 KB are received (split in 7)
+    static_assert(SWIGLU_OUT + BT * 128 * 2 <= RING_BYTES, "swiglu epilogue buffers fit the rings");
     static_assert(LD_COLS == 8 || LD_COLS == 16 || LD_COLS == 32, "tcgen05.ld shape");
     static_assert(BT == 16 || BT == 32 || BT == 64 || BT == 128, "token tile");
     static_assert(X_RING_OFFSET % 1024 == 0 && X_RING_OFFSET >= 6 * BW * BK, "room for at least six full weight tiles");
@@ -176,8 +183,8 @@ template <> struct TmemLd<16> {
     }
 };
 
-// Reads N columns of each of the first `valid` accumulator tiles (BT columns apart) and returns their sum.
-template <int N, int NACC, int BT>
+// Reads N columns of each of the first `valid` accumulator tiles (STRIDE columns apart) and returns their sum.
+template <int N, int NACC, int STRIDE>
 __device__ __forceinline__ void tmem_ld_sum(uint32_t taddr, uint32_t (&acc)[N], int valid) {
     TmemLd<N>::run(taddr, acc);
     ptx::tmem_ld_wait();
@@ -185,21 +192,117 @@ __device__ __forceinline__ void tmem_ld_sum(uint32_t taddr, uint32_t (&acc)[N], 
     for (int a = 1; a < NACC; ++a) { // one partial tile at a time: two register arrays live, not NACC
         if (a >= valid) break; // warp-uniform: that issuer had no K block
         uint32_t part[N];
-        TmemLd<N>::run(taddr + a * BT, part);
+        TmemLd<N>::run(taddr + a * STRIDE, part);
         ptx::tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < N; ++j) acc[j] += part[j];
     }
 }
 
+// One activated value of the fused gate + up projection, operation by operation as the stand-alone kernel of
+// activation_requant.cu computes it.
+__device__ __forceinline__ float swiglu_value(uint32_t xi, uint32_t gi, float sx, float sg, float down_n, float ts, float beta) {
+    const float x = __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)xi, sx), down_n), ts);
+    const float g = __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)gi, sg), down_n), ts);
+    return __fmul_rn(__fdiv_rn(x, __fadd_rn(1.0f, __expf(__fmul_rn(-x, beta)))), g);
+}
+
+// SwiGLU over the accumulators this CTA owns: activated fp16 values into the output tile [token][channel] at
+// ring + SWIGLU_OUT, row maxima (of the fp32 values) into token_absmax.  Called by every thread of the CTA.
+template <int BT, bool DUAL>
+__device__ __forceinline__ void swiglu_epilogue(const DecodeParams& p, uint32_t taddr_row, uint32_t ring, uint32_t S, uint32_t rank,
+                                                uint32_t own0, uint32_t slot0, uint32_t step_div, uint32_t step_rem, uint32_t slot_carry,
+                                                uint32_t recv_pieces, bool have_acc, int nkb, int col_begin, int col_end, int nl, int n,
+                                                int q, int lane, const float (&sn)[2], const float* token_scale, uint32_t* token_absmax) {
+    using C = DCfg<BT>;
+    constexpr int NPART = DUAL ? 2 : 1;
+    const int valid = nkb < C::NACC ? nkb : C::NACC;
+    const bool ok = nl < p.tile_rows && n < p.N;
+    auto load8 = [&](int col, uint32_t slot, uint32_t (&v)[8]) { // eight tokens of this lane's row, K slices summed
+        if (have_acc) {
+            tmem_ld_sum<8, C::NACC, NPART * BT>(taddr_row + col, v, valid);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = 0u;
+        }
+        for (uint32_t r = 0; r + 1 < S; ++r) {
+            const uint32_t addr = ring + (r * recv_pieces + slot) * PIECE_BYTES + lane * 32;
+            const uint4 a = ld_shared_v4(addr), b = ld_shared_v4(addr + 16);
+            v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+            v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+        }
+    };
+    const uint32_t partner = ring + C::SWIGLU_PARTNER + (uint32_t)nl * 4u; // [token][64 rows] int32
+    const int side = q >> 1;                                              // lanes of the x rows (0) or of the gate rows (1)
+    if (!DUAL) {
+        // each half of the lanes computes every other chunk and hands the accumulators of the rest to the other half
+        uint32_t own = own0, slot = slot0;
+#pragma unroll 1
+        for (int c0 = col_begin; c0 < col_end; c0 += PIECE_COLS) {
+            if (c0 >= p.M) break;
+            if (own == rank && ((c0 / PIECE_COLS) & 1) != side) {
+                uint32_t v[8];
+                load8(c0, slot, v);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(partner + (uint32_t)(c0 + j) * 256u), "r"(v[j]) : "memory");
+            }
+            own += step_rem; slot += step_div;
+            if (own >= S) { own -= S; slot += slot_carry; }
+        }
+        __syncthreads();
+    }
+    uint32_t own = own0, slot = slot0;
+#pragma unroll 1
+    for (int c0 = col_begin; c0 < col_end; c0 += PIECE_COLS) {
+        if (c0 >= p.M) break;
+        if (DUAL || (own == rank && ((c0 / PIECE_COLS) & 1) == side)) {
+            uint32_t v[8], w[8], absbits[8];
+            load8(c0, slot, v);
+            if (DUAL) {
+                load8(BT + c0, slot, w);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[j]) : "r"(partner + (uint32_t)(c0 + j) * 256u) : "memory");
+            }
+            const float4 ts0 = *reinterpret_cast<const float4*>(&token_scale[c0]);
+            const float4 ts1 = *reinterpret_cast<const float4*>(&token_scale[c0 + 4]);
+            const float ts[8] = {ts0.x, ts0.y, ts0.z, ts0.w, ts1.x, ts1.y, ts1.z, ts1.w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const bool swap = !DUAL && side != 0; // this lane holds the gate, its partner the x value
+                const float r = swiglu_value(swap ? w[j] : v[j], swap ? v[j] : w[j], sn[0], sn[1], p.down_n, ts[j], p.beta);
+                const float a = ok ? fabsf(r) : 0.0f;
+                absbits[j] = a == a ? __float_as_uint(a) : 0u; // NaNs are dropped, as fmax does
+                if (nl < p.tile_rows)
+                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(ring + C::SWIGLU_OUT + ((uint32_t)(c0 + j) * (uint32_t)p.tile_rows + (uint32_t)nl) * 2u),
+                                 "h"(__half_as_ushort(__float2half_rn(r))) : "memory");
+            }
+            const uint32_t tok_max = warp_token_max<8>(absbits, lane);
+            if (lane < 8 && c0 + lane < p.M && tok_max != 0u) atomicMax(&token_absmax[c0 + lane], tok_max);
+        }
+        own += step_rem; slot += step_div;
+        if (own >= S) { own -= S; slot += slot_carry; }
+    }
+}
+
 // grid = (S, weight-row tiles); cluster = (S, 1, 1): the S CTAs of a cluster share one weight-row
 // tile and each takes a contiguous range of K blocks.
-template <int BT>
+//
+// DUAL: the tile has two parts of tile_rows weight rows, each with accumulators of its own, and S is 1.  The parts are
+// neighbours (more weight rows than the SMs have TMEM lanes for: 22016 rows are 138 tiles of 2 x 80 in one wave instead
+// of 172 tiles of 128 in two), or, for EPI_SWIGLU_F16, the "x" and the "gate" rows of the same output channels.
+// EPI_SWIGLU_F16 without DUAL (at most 64 channels per tile): x rows on TMEM lanes 0..63, gate rows on lanes 64..127 of
+// one accumulator -- half the MMA time, and K can be split; the epilogue exchanges the halves through shared memory.
+// With both, and no int32 product written and read back, a layer's nine launches take 62.3 us for 8 tokens of a 4096-wide
+// model, 82.0 with the raw GEMM and the stand-alone SwiGLU kernel; 96 tokens of an 8192-wide one's eighth 81.2 instead of 81.7.
+template <int BT, bool DUAL, bool SWIGLU>
 __global__ void __launch_bounds__(DCfg<BT>::NUM_THREADS, 1)
 gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                       const __grid_constant__ CUtensorMap tmap_y, const DecodeParams p) {
     using C = DCfg<BT>;
     constexpr int NUM_THREADS = C::NUM_THREADS;
+    constexpr int NPART = DUAL ? 2 : 1;
+    constexpr int TMEM_COLS = C::template tmem_cols<DUAL>();
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_w[MAX_W_STAGES], empty_w[MAX_W_STAGES];
     __shared__ __align__(8) uint64_t full_x[C::X_STAGES], empty_x[C::X_STAGES];
@@ -216,7 +319,9 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const int n_tile = blockIdx.y;
     const unsigned long long t_start = p.stamps ? globaltimer_ns() : 0ull;
     const int SW = p.w_stages;
-    const uint32_t w_stride = (uint32_t)p.tile_rows * BK;
+    const uint32_t w_stride = (uint32_t)p.w_slot_bytes;
+    constexpr bool pack = SWIGLU && !DUAL, two_parts = SWIGLU || DUAL;
+    const int tile_row0 = n_tile * p.tile_rows * (DUAL && !SWIGLU ? 2 : 1); // first weight row (= output column)
     const uint32_t x_ring = ring + C::X_RING_OFFSET;
 
     // this CTA's K blocks
@@ -247,7 +352,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         ptx::fence_mbar_init();
     }
     if (warp == 1) {
-        ptx::tmem_alloc(ptx::smem_addr(&tmem_base_slot), C::TMEM_COLS);
+        ptx::tmem_alloc(ptx::smem_addr(&tmem_base_slot), TMEM_COLS);
         ptx::tmem_relinquish();
     }
     if (threadIdx.x < BT) token_absmax[threadIdx.x] = 0u;
@@ -257,21 +362,26 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const uint32_t tmem_base = tmem_base_slot;
     const unsigned long long t_setup = p.stamps ? globaltimer_ns() : 0ull;
 
-    // per-thread output column (= weight row) and its constants; behind the quantizer they belong to the weights, not to
-    // the preceding kernel, so they are fetched now and their latency hides behind the main loop
+    // per-thread output columns (= weight rows, one per part) and their constants; behind the quantizer they belong to the
+    // weights, not to the preceding kernel, so they are fetched now and their latency hides behind the main loop
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     const int grp = warp >> 2; // which slice of the token columns it handles
     const int col_begin = grp * C::GROUP_COLS, col_end = col_begin + C::GROUP_COLS;
     // A tile holds tile_rows <= 128 weight rows; the MMA still spans 128 TMEM lanes, the upper ones compute on
     // whatever the rest of the shared-memory slot holds and are never read back.
-    const int n = n_tile * p.tile_rows + q * 32 + lane;
-    const bool n_ok = n < p.N && q * 32 + lane < p.tile_rows;
-    float sn = 0.0f;
-    half bias_h = __ushort_as_half((unsigned short)0x8000u); // x + (-0.0) == x for every x: no branch for "no bias"
+    const int nl = pack ? (q & 1) * 32 + lane : q * 32 + lane; // weight row inside the part
+    const bool nl_ok = nl < p.tile_rows;
+    const int n = tile_row0 + nl;
+    float sn[2] = {0.0f, 0.0f};
+    half bias_h[2] = {__ushort_as_half((unsigned short)0x8000u), __ushort_as_half((unsigned short)0x8000u)}; // x + (-0.0) == x for every x: no branch for "no bias"
     auto load_column_constants = [&] {
-        if (p.mode != EPI_RAW_I32 && n_ok) {
-            sn = __half2float(p.scale_n[n]);
-            if (p.bias != nullptr) bias_h = p.bias[n];
+        if (p.mode == EPI_RAW_I32 || !nl_ok) return;
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            const int na = n + (a != 0 ? p.part_stride : 0);
+            if ((a != 0 && !two_parts) || (SWIGLU ? n : na) >= p.N) break;
+            sn[a] = __half2float(p.scale_n[na]);
+            if (p.bias != nullptr) bias_h[a] = p.bias[na];
         }
     };
     if (p.early_weights) load_column_constants();
@@ -286,18 +396,27 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         const int prew = nkb < SW ? nkb : SW;
         if (!p.early_weights) {
             const int ahead = nkb < 2 * SW ? nkb : 2 * SW;
-            for (int i = 0; i < ahead; ++i) ptx::tma_prefetch_l2_2d(&tmap_w, PPLB200_KB(i) * BK, n_tile * p.tile_rows);
+            for (int i = 0; i < ahead; ++i) {
+                ptx::tma_prefetch_l2_2d(&tmap_w, PPLB200_KB(i) * BK, tile_row0);
+                if (two_parts) ptx::tma_prefetch_l2_2d(&tmap_w, PPLB200_KB(i) * BK, tile_row0 + p.part_stride);
+            }
             pdl_wait_prior_grid();
         }
+        // the second part lies on the lanes from 64 up (one accumulator), or densely behind the first (two accumulators)
+        const uint32_t part_off = (pack ? 64u : (uint32_t)p.tile_rows) * BK;
         for (int i = 0; i < prew; ++i) {
-            ptx::mbar_arrive_expect_tx(fw0 + i * 8u, w_stride);
-            ptx::tma_load_2d(ring + i * w_stride, &tmap_w, fw0 + i * 8u, PPLB200_KB(i) * BK, n_tile * p.tile_rows);
+            const uint32_t dst = ring + i * w_stride;
+            ptx::mbar_arrive_expect_tx(fw0 + i * 8u, (uint32_t)p.w_box_bytes);
+            ptx::tma_load_2d(dst, &tmap_w, fw0 + i * 8u, PPLB200_KB(i) * BK, tile_row0);
+            if (two_parts) ptx::tma_load_2d(dst + part_off, &tmap_w, fw0 + i * 8u, PPLB200_KB(i) * BK, tile_row0 + p.part_stride);
         }
         uint32_t sw = prew == SW ? 0u : (uint32_t)prew, pw = prew == SW ? 1u : 0u;
         for (int i = prew; i < nkb; ++i) {
             if (!ptx::mbar_wait(ew0 + sw * 8u, pw ^ 1u, p.status, ST_DEC_PRODUCER)) { ok = false; break; }
-            ptx::mbar_arrive_expect_tx(fw0 + sw * 8u, w_stride);
-            ptx::tma_load_2d(ring + sw * w_stride, &tmap_w, fw0 + sw * 8u, PPLB200_KB(i) * BK, n_tile * p.tile_rows);
+            const uint32_t dst = ring + sw * w_stride;
+            ptx::mbar_arrive_expect_tx(fw0 + sw * 8u, (uint32_t)p.w_box_bytes);
+            ptx::tma_load_2d(dst, &tmap_w, fw0 + sw * 8u, PPLB200_KB(i) * BK, tile_row0);
+            if (two_parts) ptx::tma_load_2d(dst + part_off, &tmap_w, fw0 + sw * 8u, PPLB200_KB(i) * BK, tile_row0 + p.part_stride);
             if (++sw == (uint32_t)SW) { sw = 0; pw ^= 1u; }
         }
     } else if (warp == 3 && lane == 0) {
@@ -321,7 +440,8 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         const uint32_t w_lo0 = ptx::desc_lo_sw128(ring), x_lo0 = ptx::desc_lo_sw128(x_ring);
         const uint32_t fw0 = ptx::smem_addr(&full_w[0]), ew0 = ptx::smem_addr(&empty_w[0]);
         const uint32_t fx0 = ptx::smem_addr(&full_x[0]), ex0 = ptx::smem_addr(&empty_x[0]);
-        const uint32_t tmem_d = tmem_base + (uint32_t)me * BT;
+        const uint32_t tmem_d = tmem_base + (uint32_t)(me * NPART) * BT;
+        const uint32_t part_lo = ((uint32_t)p.tile_rows * BK) >> 4;
         uint32_t sw = (uint32_t)me, pw = 0, sx = (uint32_t)me, px = 0; // both rings have at least two stages
         bool ready_w = false, ready_x = false;
         for (int i = me; i < nkb; i += C::NACC) {
@@ -338,6 +458,11 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
 #pragma unroll
             for (uint32_t k = 0; k < BK / UMMA_K; ++k)
                 ptx::mma_i8(tmem_d, ptx::desc_from_lo(w_lo + 2u * k), ptx::desc_from_lo(x_lo + 2u * k), idesc, k != 0 ? 1u : accumulate);
+            if (DUAL) {
+#pragma unroll
+                for (uint32_t k = 0; k < BK / UMMA_K; ++k)
+                    ptx::mma_i8(tmem_d + BT, ptx::desc_from_lo(w_lo + part_lo + 2u * k), ptx::desc_from_lo(x_lo + 2u * k), idesc, k != 0 ? 1u : accumulate);
+            }
             ptx::mma_commit(ew0 + sw * 8u);
             ptx::mma_commit(ex0 + sx * 8u);
             sw = nsw; pw = npw; sx = nsx; px = npx;
@@ -363,23 +488,27 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const unsigned long long t_main = p.stamps ? globaltimer_ns() : 0ull;
 
     const uint32_t taddr_row = tmem_base + ((uint32_t)(q * 32) << 16);
-    const uint32_t recv_pieces_per_owner = (C::PIECES + S - 1) / S;
     // piece index of (column chunk c, quarter q) is 4 c + q; owner = piece % S, slot = piece / S.
     // Both are tracked incrementally (no divisions in the loops): a step of one chunk adds 4.
-    const uint32_t step_div = 4u / S, step_rem = 4u % S;
+    // With x and gate rows on different lanes (pack) a CTA owns all four quarters of a chunk: owner = c % S, and the
+    // pieces of a chunk are neighbours, slot = 4 (c / S) + q.
+    const uint32_t recv_pieces_per_owner = pack ? 4u * ((BT / PIECE_COLS + S - 1) / S) : (C::PIECES + S - 1) / S;
+    const uint32_t step_div = pack ? 4u * (1u / S) : 4u / S, step_rem = pack ? 1u % S : 4u % S, slot_carry = pack ? 4u : 1u;
+    const uint32_t first_chunk = (uint32_t)(col_begin / PIECE_COLS);
+    const uint32_t own0 = pack ? first_chunk % S : (first_chunk * 4u + (uint32_t)q) % S;
+    const uint32_t slot0 = pack ? first_chunk / S * 4u + (uint32_t)q : (first_chunk * 4u + (uint32_t)q) / S;
     const bool have_acc = nkb > 0 && acc_ready;
 
     if (S > 1) {
         cluster_sync_all(); // every CTA of the cluster is done reading its ring: it may now receive
         // ---- send the pieces owned by other CTAs
-        const uint32_t first_piece = (uint32_t)(col_begin / PIECE_COLS) * 4u + (uint32_t)q;
-        uint32_t own = first_piece % S, slot = first_piece / S;
+        uint32_t own = own0, slot = slot0;
 #pragma unroll 1
         for (int c0 = col_begin; c0 < col_end; c0 += C::LD_COLS) {
             if (c0 >= p.M) break; // columns past the last token hold zeros nobody reads
             uint32_t acc[C::LD_COLS];
             if (have_acc) {
-                tmem_ld_sum<C::LD_COLS, C::NACC, BT>(taddr_row + c0, acc, nkb < C::NACC ? nkb : C::NACC);
+                tmem_ld_sum<C::LD_COLS, C::NACC, NPART * BT>(taddr_row + c0, acc, nkb < C::NACC ? nkb : C::NACC);
             } else {
 #pragma unroll
                 for (int j = 0; j < C::LD_COLS; ++j) acc[j] = 0u;
@@ -394,7 +523,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                     st_cluster_v4(remote + 16, acc[s8 * 8 + 4], acc[s8 * 8 + 5], acc[s8 * 8 + 6], acc[s8 * 8 + 7]);
                 }
                 own += step_rem; slot += step_div;
-                if (own >= S) { own -= S; slot += 1; }
+                if (own >= S) { own -= S; slot += slot_carry; }
             }
         }
         cluster_sync_all(); // all partial pieces have landed
@@ -412,11 +541,17 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     // clipped at the matrix bounds -- instead of a 2-byte (or 4-byte) store with its own address arithmetic per
     // element (lane = weight row, registers = tokens is the wrong way round for the row-major output).
     const bool staged = S == 1 && !p.raw_affine;
-    const uint32_t nl = (uint32_t)(q * 32 + lane);         // weight row inside the tile
-    const bool nl_ok = nl < (uint32_t)p.tile_rows;
-    {
-        const uint32_t first_piece = (uint32_t)(col_begin / PIECE_COLS) * 4u + (uint32_t)q;
-        uint32_t own = first_piece % S, slot = first_piece / S;
+    const uint32_t tile_cols = (uint32_t)(p.tile_rows * NPART);
+    if constexpr (SWIGLU) {
+        swiglu_epilogue<BT, DUAL>(p, taddr_row, ring, S, rank, own0, slot0, step_div, step_rem, slot_carry, recv_pieces_per_owner, have_acc,
+                                  nkb, col_begin, col_end, nl, n, q, lane, sn, token_scale, token_absmax);
+    } else {
+#pragma unroll
+    for (int part = 0; part < NPART; ++part) { // S == 1 with two parts
+        const uint32_t nlp = (uint32_t)(part * p.tile_rows + nl); // weight row inside the tile
+        const int np = n + part * p.part_stride;
+        const bool n_ok = nl_ok && np < p.N;
+        uint32_t own = own0, slot = slot0;
 #pragma unroll 1
         for (int c0 = col_begin; c0 < col_end; c0 += C::LD_COLS) {
             if (c0 >= M) break;
@@ -426,7 +561,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
             for (int j = 0; j < C::LD_COLS; ++j) absbits[j] = 0u;
 
             if (have_acc) {
-                tmem_ld_sum<C::LD_COLS, C::NACC, BT>(taddr_row + c0, acc, nkb < C::NACC ? nkb : C::NACC);
+                tmem_ld_sum<C::LD_COLS, C::NACC, NPART * BT>(taddr_row + part * BT + c0, acc, nkb < C::NACC ? nkb : C::NACC);
             } else {
 #pragma unroll
                 for (int j = 0; j < C::LD_COLS; ++j) acc[j] = 0u;
@@ -448,11 +583,11 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                         if (nl_ok) {
 #pragma unroll
                             for (int j = 0; j < 8; ++j)
-                                asm volatile("st.shared.u32 [%0], %1;" ::"r"(ring + ((uint32_t)(m0 + j) * (uint32_t)p.tile_rows + nl) * 4u), "r"(v[j]) : "memory");
+                                asm volatile("st.shared.u32 [%0], %1;" ::"r"(ring + ((uint32_t)(m0 + j) * tile_cols + nlp) * 4u), "r"(v[j]) : "memory");
                         }
                     } else if (mode == EPI_RAW_I32) {
-                        int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)m0 * p.ldc + n;
-                        const uint32_t add = (p.raw_affine && p.raw_bias != nullptr && n_ok) ? (uint32_t)p.raw_bias[n] : 0u;
+                        int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)m0 * p.ldc + np;
+                        const uint32_t add = (p.raw_affine && p.raw_bias != nullptr && n_ok) ? (uint32_t)p.raw_bias[np] : 0u;
 #pragma unroll
                         for (int j = 0; j < 8; ++j)
                             if (n_ok && m0 + j < M) {
@@ -471,19 +606,19 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                         half h[8];
 #pragma unroll
                         for (int j = 0; j < 8; ++j) {
-                            float t = __fmul_rn((float)(int32_t)v[j], sn);
+                            float t = __fmul_rn((float)(int32_t)v[j], sn[part]);
                             t = __fmul_rn(t, down_n);
                             t = __fmul_rn(t, ts[j]);
-                            h[j] = __hadd(__float2half_rn(t), bias_h);
+                            h[j] = __hadd(__float2half_rn(t), bias_h[part]);
                         }
                         if (staged) {
                             if (nl_ok) {
 #pragma unroll
                                 for (int j = 0; j < 8; ++j)
-                                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(ring + ((uint32_t)(m0 + j) * (uint32_t)p.tile_rows + nl) * 2u), "h"(__half_as_ushort(h[j])) : "memory");
+                                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(ring + ((uint32_t)(m0 + j) * tile_cols + nlp) * 2u), "h"(__half_as_ushort(h[j])) : "memory");
                             }
                         } else {
-                            half* dst = reinterpret_cast<half*>(p.out) + (int64_t)m0 * p.ldc + n;
+                            half* dst = reinterpret_cast<half*>(p.out) + (int64_t)m0 * p.ldc + np;
 #pragma unroll
                             for (int j = 0; j < 8; ++j)
                                 if (n_ok && m0 + j < M) dst[(int64_t)j * p.ldc] = h[j];
@@ -498,7 +633,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                     }
                 }
                 own += step_rem; slot += step_div;
-                if (own >= S) { own -= S; slot += 1; }
+                if (own >= S) { own -= S; slot += slot_carry; }
             }
             if (mode == EPI_DEQUANT_F16_REQUANT_I8) {
                 // per-token max |y| over this warp's 32 output columns; lane t ends up with token c0 + t
@@ -508,12 +643,24 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         }
     }
 
+    }
 #undef PPLB200_KB
-    if (staged) ptx::fence_proxy_async_smem(); // the tile written above is read by the TMA unit
+    if (staged || SWIGLU) ptx::fence_proxy_async_smem(); // the tile written above is read by the TMA unit
     ptx::tc_fence_before();
     __syncthreads();
-    if (staged && threadIdx.x == 0) {
-        ptx::tma_store_2d(&tmap_y, ring, n_tile * p.tile_rows, 0);
+    if constexpr (SWIGLU) { // eight tokens per store, those this CTA owns
+        if (threadIdx.x < BT / PIECE_COLS && threadIdx.x * PIECE_COLS < M && (!pack || threadIdx.x % S == rank)) {
+            ptx::tma_store_2d(&tmap_y, ring + C::SWIGLU_OUT + threadIdx.x * (uint32_t)(PIECE_COLS * 2 * p.tile_rows), tile_row0,
+                              (int)threadIdx.x * PIECE_COLS);
+            ptx::bulk_commit_group();
+            ptx::bulk_wait_group_read<0>();
+        }
+        // this CTA's share of the row maxima, [token][CTA]: a CTA writes every token (zero for those it does not own),
+        // so nothing has to be cleared beforehand and nothing is added atomically
+        const uint32_t cta = (uint32_t)n_tile * S + rank, ctas = gridDim.y * S;
+        for (int m = threadIdx.x; m < BT && m < M; m += NUM_THREADS) p.row_absmax_bits[(uint32_t)m * ctas + cta] = token_absmax[m];
+    } else if (staged && threadIdx.x == 0) {
+        ptx::tma_store_2d(&tmap_y, ring, tile_row0, 0);
         ptx::bulk_commit_group();
         ptx::bulk_wait_group_read<0>(); // shared memory must outlive the store's reads; the kernel boundary publishes the writes
     }
@@ -523,7 +670,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     }
     if (warp == 1) {
         ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem_base, C::TMEM_COLS);
+        ptx::tmem_dealloc(tmem_base, TMEM_COLS);
     }
     if (p.stamps && threadIdx.x == 0) {
         const unsigned cta = blockIdx.y * gridDim.x + blockIdx.x;
@@ -585,8 +732,9 @@ std::mutex g_mutex;
 DecDeviceInfo g_dev[64];
 
 template <int BT> bool set_attr(int* max_clusters) {
-    if (cudaFuncSetAttribute(gemm_i8_decode_kernel<BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, DCfg<BT>::SMEM_BYTES) != cudaSuccess)
-        return false;
+    for (auto kernel : {gemm_i8_decode_kernel<BT, false, false>, gemm_i8_decode_kernel<BT, true, false>, gemm_i8_decode_kernel<BT, false, true>,
+                        gemm_i8_decode_kernel<BT, true, true>})
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DCfg<BT>::SMEM_BYTES) != cudaSuccess) return false;
     for (int s = 2; s <= 8; ++s) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)s, 64, 1);
@@ -598,7 +746,7 @@ template <int BT> bool set_attr(int* max_clusters) {
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, gemm_i8_decode_kernel<BT>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        if (cudaOccupancyMaxActiveClusters(&n, gemm_i8_decode_kernel<BT, false, false>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
         max_clusters[s] = n;
     }
     return true;
@@ -635,38 +783,54 @@ int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecDeviceInfo& d
     p.raw_alpha = a.raw_alpha; p.raw_beta = a.raw_beta; p.raw_bias = a.raw_bias;
     p.raw_affine = (a.raw_alpha != 1 || a.raw_beta != 0 || a.raw_bias != nullptr) ? 1 : 0;
 
+    const bool swiglu = a.mode == EPI_SWIGLU_F16;
+    if (swiglu) p.N = (int32_t)(a.N / 2); // the x half and the gate half of the weight rows share the output columns
+    p.beta = a.beta;
+    // Weight rows a tile can hold: one per TMEM lane, or, x and gate rows paired, half as many channels.
+    const int bw = swiglu ? BW / 2 : BW;
+    // Two accumulators per tile where tiles of bw rows no longer run as one wave: with 172 tiles on 148 SMs the second
+    // wave costs as much as the first.
+    const bool dual = (p.N + bw - 1) / bw > dev.sms;
+
     // K split: one CTA per SM is resident (the rings take the whole shared memory), so split K only as
     // far as all clusters still fit in one wave; every CTA keeps at least two K blocks
-    int S = dev.sms / (int)((a.N + BW - 1) / BW);
+    int S = dual ? 1 : dev.sms / (int)((p.N + bw - 1) / bw);
     if (S > 8) S = 8;
     if (S > p.num_k_blocks / 2) S = p.num_k_blocks / 2;
     if (S < 1) S = 1;
     // Tile height: the smallest multiple of 8 rows with which the tiles still run as one wave -- e.g. 12288 weight
     // rows: 140 tiles of 88 rows on 148 SMs instead of 96 tiles of 128 rows on 96.  With a K split the wave holds
     // as many clusters as the device can co-schedule (fewer than SMs / S: a cluster stays inside one GPC).
-    int tile_rows = BW;
+    const int parts_out = dual && !swiglu ? 2 : 1; // parts of a tile that are output columns of their own
+    int tile_rows = dual ? BW : bw;
     {
-        const int64_t cap = S == 1 ? dev.sms : dev.max_clusters[BT == 16 ? 0 : BT == 32 ? 1 : BT == 64 ? 2 : 3][S];
-        if (cap > 0 && (a.N + BW - 1) / BW <= cap) {
-            int64_t r = (a.N + cap - 1) / cap;
+        int64_t cap = S == 1 ? dev.sms : dev.max_clusters[BT == 16 ? 0 : BT == 32 ? 1 : BT == 64 ? 2 : 3][S];
+        cap *= parts_out;
+        if (cap > 0 && (p.N + tile_rows - 1) / tile_rows <= cap) {
+            int64_t r = (p.N + cap - 1) / cap;
             r = (r + 7) / 8 * 8;
             if (r < 8) r = 8;
-            if (r < BW) tile_rows = (int)r;
+            if (r < tile_rows) tile_rows = (int)r;
         }
     }
     p.tile_rows = tile_rows;
-    p.w_stages = DCfg<BT>::X_RING_OFFSET / (tile_rows * BK);
+    p.part_stride = swiglu ? p.N : tile_rows;
+    p.w_box_bytes = tile_rows * BK * (dual || swiglu ? 2 : 1);
+    p.w_slot_bytes = dual ? 2 * tile_rows * BK : (swiglu ? 64 + tile_rows : tile_rows) * BK;
+    p.w_stages = DCfg<BT>::X_RING_OFFSET / p.w_slot_bytes;
     if (p.w_stages > MAX_W_STAGES) p.w_stages = MAX_W_STAGES;
     p.w_stages -= p.w_stages % DCfg<BT>::NACC; // see X_STAGES
     p.stamps = stall_counters();
     p.early_weights = a.after_quantizer ? 1 : 0;
 
-    const int n_tiles = (int)((a.N + tile_rows - 1) / tile_rows);
+    const int n_tiles = (int)((p.N + tile_rows * parts_out - 1) / (tile_rows * parts_out));
+    if (a.row_absmax_parts) *a.row_absmax_parts = n_tiles * S;
     if (!make_map(&tw, a.B, a.N, a.K, a.ldb, tile_rows)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (W) encode failed");
     CUtensorMap ty;
     memset(&ty, 0, sizeof(ty));
-    if (S == 1 && !p.raw_affine &&
-        !make_out_map(&ty, a.out, a.M, a.N, a.ldc, a.mode == EPI_RAW_I32 ? 4 : 2, tile_rows, BT))
+    if (swiglu ? !make_out_map(&ty, a.out, a.M, p.N, a.ldc, 2, tile_rows, PIECE_COLS)
+               : S == 1 && !p.raw_affine &&
+                     !make_out_map(&ty, a.out, a.M, a.N, a.ldc, a.mode == EPI_RAW_I32 ? 4 : 2, tile_rows * parts_out, BT))
         return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (Y) encode failed");
 
     cudaLaunchConfig_t cfg = {};
@@ -688,7 +852,9 @@ int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecDeviceInfo& d
     }
     cfg.attrs = attrs;
     cfg.numAttrs = na;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_i8_decode_kernel<BT>, tw, tx, ty, p);
+    const auto kernel = dual ? (swiglu ? gemm_i8_decode_kernel<BT, true, true> : gemm_i8_decode_kernel<BT, true, false>)
+                             : (swiglu ? gemm_i8_decode_kernel<BT, false, true> : gemm_i8_decode_kernel<BT, false, false>);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tw, tx, ty, p);
     if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "decode GEMM launch failed: %s", cudaGetErrorString(e));
     return RC_SUCCESS;
 }

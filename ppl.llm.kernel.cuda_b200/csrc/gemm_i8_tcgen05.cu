@@ -1069,6 +1069,7 @@ int32_t launch_gemm(cudaStream_t stream, const GemmArgs& a) {
     if (a.M > INT32_MAX - BM || a.N > INT32_MAX - 256 || a.K > INT32_MAX - BK)
         return fail(RC_UNSUPPORTED, "GEMM extent beyond 2^31");
 
+    if (a.mode == EPI_SWIGLU_F16 && a.M <= 128) return launch_gemm_decode(stream, a, dev->status, a.pdl);
     if (a.mode == EPI_SWIGLU_F16 || a.mode == EPI_PUSH_I32 || a.mode == EPI_GATHER_F16)
         return launch_pair(stream, a, *dev); // the caller checked the shape
 

@@ -59,7 +59,9 @@ struct QuantRow {
     float scale;   // max(amax / 127, 1e-7), what the reference divides by
     float inv_hi;  // (1 / scale) nudged up and down by 2^-21: v * inv_lo <= v / scale <= v * inv_hi for v >= 0
     float inv_lo;
-    bool exact;    // row holds a NaN or its maximum is infinite: every element takes the IEEE division
+    // Every element takes the IEEE division: the row holds a NaN, or an infinity -- the maximum may be that of fp32 values
+    // which became infinite when they were rounded to fp16 (65520 and above).
+    bool exact;
 };
 __device__ __forceinline__ QuantRow make_quant_row(float amax, bool saw_nan) {
     QuantRow q;
@@ -67,7 +69,7 @@ __device__ __forceinline__ QuantRow make_quant_row(float amax, bool saw_nan) {
     const float inv = __frcp_rn(q.scale);
     q.inv_hi = __fmul_rn(inv, 1.0f + 0x1p-21f);
     q.inv_lo = __fmul_rn(inv, 1.0f - 0x1p-21f);
-    q.exact = saw_nan || !(amax < __int_as_float(0x7f800000));
+    q.exact = saw_nan || !(amax < 65520.0f);
     return q;
 }
 

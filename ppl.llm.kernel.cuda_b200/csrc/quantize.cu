@@ -21,7 +21,7 @@ template <int UNITS>
 __global__ void __launch_bounds__(QTPB, UNITS <= 2 ? 5 : 1)
 quantize_rows_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, float up_scale, int32_t layout,
                      int8_t* __restrict__ q, half* __restrict__ scale_out, const uint32_t* __restrict__ given_absmax_bits,
-                     uint32_t* __restrict__ zero_absmax_bits) {
+                     uint32_t* __restrict__ zero_absmax_bits, int32_t given_parts) {
     __shared__ float red[QTPB / 32];
     const int64_t row = blockIdx.x;
     const int units = (int)(dim >> 4);
@@ -53,7 +53,15 @@ quantize_rows_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, fl
         amax = block_max_any(amax, saw_nan, red, blockDim.x >> 5, any_nan);
         qr = make_quant_row(amax, any_nan);
     } else {
-        qr = make_quant_row(__uint_as_float(given_absmax_bits[row]), false);
+        float amax;
+        if (given_parts == 1) {
+            amax = __uint_as_float(given_absmax_bits[row]);
+        } else { // partial maxima of the CTAs that produced the row: no NaN among them
+            amax = 0.0f;
+            for (int i = threadIdx.x; i < given_parts; i += blockDim.x) amax = fmaxf(amax, __uint_as_float(given_absmax_bits[row * given_parts + i]));
+            amax = block_max(amax, red, blockDim.x >> 5);
+        }
+        qr = make_quant_row(amax, false);
     }
     const float scale = qr.scale;
 
@@ -78,7 +86,7 @@ quantize_rows_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, fl
 __global__ void __launch_bounds__(QTPB)
 quantize_rows_twopass_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, float up_scale, int32_t layout,
                              int8_t* __restrict__ q, half* __restrict__ scale_out,
-                             const uint32_t* __restrict__ given_absmax_bits, uint32_t* __restrict__ zero_absmax_bits) {
+                             const uint32_t* __restrict__ given_absmax_bits, uint32_t* __restrict__ zero_absmax_bits, int32_t given_parts) {
     __shared__ float red[QTPB / 32];
     pdl_launch_dependents();
     pdl_wait_prior_grid();
@@ -96,7 +104,9 @@ quantize_rows_twopass_kernel(const half* __restrict__ in, int64_t batch, int64_t
         }
         amax = block_max(fmaxf(__low2float(m2), __high2float(m2)), red, blockDim.x >> 5);
     } else {
-        amax = __uint_as_float(given_absmax_bits[row]);
+        amax = 0.0f;
+        for (int i = threadIdx.x; i < given_parts; i += blockDim.x) amax = fmaxf(amax, __uint_as_float(given_absmax_bits[row * given_parts + i]));
+        amax = block_max(amax, red, blockDim.x >> 5);
     }
     const QuantRow qr = make_quant_row(amax, false);
     const float scale = qr.scale;
@@ -213,7 +223,7 @@ int grid_for(int64_t work_items, int tpb) {
 
 int32_t launch_quantize(cudaStream_t stream, const half* in, int64_t batch, int64_t dim, float up_scale,
                         int32_t layout, int8_t* q, half* scale, const uint32_t* given_absmax_bits,
-                        uint32_t* zero_absmax_bits, bool pdl) {
+                        uint32_t* zero_absmax_bits, bool pdl, int32_t given_parts) {
     if (batch == 0 || dim == 0) return RC_SUCCESS;
     const int64_t units = dim >> 4;
     cudaError_t e;
@@ -223,7 +233,7 @@ int32_t launch_quantize(cudaStream_t stream, const half* in, int64_t batch, int6
         int threads = (int)(units < QTPB ? (units + 31) / 32 * 32 : QTPB);
         const dim3 grid((unsigned)batch, (unsigned)((units + threads - 1) / threads), 1);
         e = launch_ex(quantize_rows_kernel<1>, grid, dim3(threads), stream, pdl, in, batch, dim, up_scale, layout, q, scale,
-                      given_absmax_bits, zero_absmax_bits);
+                      given_absmax_bits, zero_absmax_bits, given_parts);
     } else if (units <= QTPB * 8) {
         // threads: enough to give every thread the same small number of units
         int per = (int)((units + QTPB - 1) / QTPB);
@@ -236,14 +246,14 @@ int32_t launch_quantize(cudaStream_t stream, const half* in, int64_t batch, int6
         if (threads > QTPB) threads = QTPB;
         const dim3 grid((unsigned)batch, 1, 1), block(threads);
         switch (bucket) {
-        case 1: e = launch_ex(quantize_rows_kernel<1>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits); break;
-        case 2: e = launch_ex(quantize_rows_kernel<2>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits); break;
-        case 4: e = launch_ex(quantize_rows_kernel<4>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits); break;
-        default: e = launch_ex(quantize_rows_kernel<8>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits); break;
+        case 1: e = launch_ex(quantize_rows_kernel<1>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
+        case 2: e = launch_ex(quantize_rows_kernel<2>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
+        case 4: e = launch_ex(quantize_rows_kernel<4>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
+        default: e = launch_ex(quantize_rows_kernel<8>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
         }
     } else {
         e = launch_ex(quantize_rows_twopass_kernel, dim3((unsigned)batch), dim3(QTPB), stream, pdl, in, batch, dim, up_scale, layout, q, scale,
-                      given_absmax_bits, zero_absmax_bits);
+                      given_absmax_bits, zero_absmax_bits, given_parts);
     }
     if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "quantize launch failed: %s", cudaGetErrorString(e));
     return RC_SUCCESS;

@@ -171,3 +171,29 @@ def test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K):
     assert cuda.equal(act.view(cuda.int16), ws2.view(cuda.int16))
     assert cuda.equal(s.view(cuda.int16), s2.view(cuda.int16)) and cuda.equal(q, q2)
     assert float(act.float().abs().max()) > 0.01  # the scales put the values in SiLU's interesting range
+
+
+# One accumulator for x and gate rows with K split over 1 .. 8 CTAs (up to 64 channels per tile; 1280: seven, 16: eight),
+# two accumulators from 9473 channels up, K shorter than a K block, a last tile of 16 channels, every token width
+@pytest.mark.parametrize("M,D,K", [(1, 16, 16), (5, 16, 4096), (16, 1280, 1808), (17, 3584, 1024), (8, 11008, 512), (33, 9488, 272),
+                                   (64, 4672, 1040), (96, 3584, 2048), (128, 1280, 4096), (128, 9472, 384), (128, 19056, 144), (120, 640, 2064)])
+def test_small_batch_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K):
+    """The small-batch kernel's SwiGLU epilogue == raw-int32 linear followed by the stand-alone SwiGLU kernel, bit for bit."""
+    test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K)
+
+
+def test_small_batch_gate_up_swiglu_overflow(cuda):
+    """Activated values beyond the fp16 range (infinities in the row, a finite fp32 row maximum)."""
+    import pplb200
+    M, D, K = 4, 64, 256
+    g = cuda.Generator(device="cuda").manual_seed(3)
+    xq = cuda.randint(-127, 128, (M, K), generator=g, device="cuda", dtype=cuda.int8)
+    w = cuda.randint(-127, 128, (2 * D, K), generator=g, device="cuda", dtype=cuda.int8)
+    sm = cuda.full((M,), 4096 / 127, device="cuda").half()
+    sn = cuda.full((2 * D,), 8192 * 0.35, device="cuda").half()
+    acc = pplb200.column_parallel_linear(xq, w, None, None, None, K, 2 * D, gather_output=False)
+    two_step = pplb200.minmax_requantize_swiglu_fp16(acc, sm, sn)
+    fused = pplb200.gate_up_swiglu_requant(xq, w, sm, sn)
+    assert bool(cuda.isinf(two_step[0]).any()) and bool(cuda.isfinite(two_step[0]).any())
+    assert cuda.equal(fused[0].view(cuda.int16), two_step[0].view(cuda.int16))
+    assert cuda.equal(fused[1], two_step[1]) and cuda.equal(fused[2].view(cuda.int16), two_step[2].view(cuda.int16))

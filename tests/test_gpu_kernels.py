@@ -426,3 +426,10 @@ def test_back_to_back_launches_see_fresh_operands(cuda, M, N, K):
         (q, s), (p, t) = pplb200.minmax_quantize_fp16(x), pplb200.minmax_quantize_fp16(w)
         want = pplb200.minmax_dequantize_fp16((q.double() @ p.double().T).to(cuda.int32), s, t)  # int32 sums are exact in fp64
         assert cuda.equal(y.view(cuda.int16), want.view(cuda.int16))
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 19072, 144), (16, 22016, 256), (37, 18960, 400), (128, 28672, 272), (128, 37904, 128)])
+def test_decode_gemm_two_row_parts(cuda, oracle, M, N, K):
+    """More weight rows than one tile of 128 per SM: two accumulators per CTA (37904: a second wave of one ragged tile)."""
+    test_decode_gemm_all_modes(cuda, oracle, M, N, K)
+    test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
