@@ -155,12 +155,55 @@ int32_t launch_act(cudaStream_t stream, const ActParams& p) {
     return RC_SUCCESS;
 }
 
-// dequantize (+bias) and scatter the columns into three row-major outputs; 4 columns per thread
+// Dequantize (+bias) and scatter the columns into three outputs.  Row-major input with every extent a multiple of 8: eight
+// columns per thread, the same columns of R rows, so that the column constants are read once and 32 R bytes are
+// requested before anything is used.  1999 x 12288 (98 MB read, 49 written, part of both in L2): 21 us, as long as HBM takes for all of it.
+template <int R>
 __global__ void __launch_bounds__(256)
-dequantize_split3_kernel(const int32_t* __restrict__ acc, const half* __restrict__ bias, const half* __restrict__ scale_m,
-                         const half* __restrict__ scale_n, int64_t batch, int64_t dim, int64_t d0, int64_t d1, int64_t d2,
-                         float down_m, float down_n, int32_t layout, half* __restrict__ o0, half* __restrict__ o1,
-                         half* __restrict__ o2) {
+dequantize_split3_rows8_kernel(const int32_t* acc, const half* bias, const half* scale_m, const half* scale_n, int64_t batch, int64_t dim,
+                               int64_t d0, int64_t d1, int64_t d2, float down_m, float down_n, half* o0, half* o1, half* o2) {
+    pdl_launch_dependents();
+    pdl_wait_prior_grid();
+    const int64_t n = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) << 3;
+    if (n >= dim) return;
+    half* dst; int64_t ld; // a group of columns goes where its first column belongs, as the reference routes groups of four (split.cu:73-79)
+    if (n < d0) { dst = o0 + n; ld = d0; }
+    else if (n < d0 + d1) { dst = o1 + (n - d0); ld = d1; }
+    else if (n < d0 + d1 + d2) { dst = o2 + (n - d0 - d1); ld = d2; }
+    else return;
+    const uint4 snv = ld_global_16(scale_n + n);
+    uint4 bv = make_uint4(0x80008000u, 0x80008000u, 0x80008000u, 0x80008000u); // x + (-0.0) == x for every x
+    if (bias != nullptr) bv = ld_global_16(bias + n);
+    const half* sn = reinterpret_cast<const half*>(&snv);
+    const half* b = reinterpret_cast<const half*>(&bv);
+    for (int64_t m0 = (int64_t)blockIdx.y * R; m0 < batch; m0 += (int64_t)gridDim.y * R) {
+        uint4 a[R][2];
+        half sm[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int64_t m = m0 + r < batch ? m0 + r : batch - 1;
+            a[r][0] = ld_global_16(acc + m * dim + n);
+            a[r][1] = ld_global_16(acc + m * dim + n + 4);
+            sm[r] = ld_global_half(scale_m + m);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (m0 + r >= batch) break;
+            const float bs = __fmul_rn(__half2float(sm[r]), down_m);
+            const int32_t* v = reinterpret_cast<const int32_t*>(&a[r][0]);
+            uint4 ov;
+            half* o = reinterpret_cast<half*>(&ov);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] = __hadd(__float2half_rn(dq(v[j], sn[j], down_n, bs)), b[j]);
+            *reinterpret_cast<uint4*>(dst + (m0 + r) * ld) = ov;
+        }
+    }
+}
+
+// Any layout, extents that are multiples of 4: four columns per thread, per-element gather.
+__global__ void __launch_bounds__(256)
+dequantize_split3_kernel(const int32_t* acc, const half* bias, const half* scale_m, const half* scale_n, int64_t batch, int64_t dim,
+                         int64_t d0, int64_t d1, int64_t d2, float down_m, float down_n, int32_t layout, half* o0, half* o1, half* o2) {
     const int64_t chunks = dim >> 2, total = batch * chunks;
     pdl_launch_dependents();
     pdl_wait_prior_grid();
@@ -238,6 +281,19 @@ int32_t dequantize_split3(cudaStream_t stream, const void* acc, const void* bias
     if (d0 % 4 || d1 % 4 || d2 % 4) return fail(RC_INVALID_VALUE, "split sizes must be multiples of 4");
     if (batch == 0 || dim == 0) return RC_SUCCESS;
     if (!acc || !sm || !sn || (d0 && !o0) || (d1 && !o1) || (d2 && !o2)) return fail(RC_INVALID_VALUE, "null pointer");
+    if (layout == LAYOUT_ROW_MAJOR && dim % 8 == 0 && d0 % 8 == 0 && d1 % 8 == 0 && d2 % 8 == 0 && aligned16(acc) && aligned16(sn) &&
+        (!bias || aligned16(bias)) && aligned16(o0) && aligned16(o1) && aligned16(o2)) {
+        // four rows per thread once that still leaves a few CTAs for every SM
+        const unsigned gx = (unsigned)((dim / 8 + 255) / 256);
+        const bool four = batch * gx >= 4 * 4 * 148;
+        int64_t gy = four ? (batch + 3) / 4 : batch;
+        if (gy > 65535) gy = 65535;
+        const cudaError_t e = launch_ex(four ? dequantize_split3_rows8_kernel<4> : dequantize_split3_rows8_kernel<1>, dim3(gx, (unsigned)gy),
+                                        dim3(256), stream, /*pdl=*/true, (const int32_t*)acc, (const half*)bias, (const half*)sm, (const half*)sn,
+                                        batch, dim, d0, d1, d2, down_m, down_n, (half*)o0, (half*)o1, (half*)o2);
+        if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "dequantize_split3 launch failed: %s", cudaGetErrorString(e));
+        return RC_SUCCESS;
+    }
     int64_t blocks = (batch * (dim >> 2) + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
     const cudaError_t e = launch_ex(dequantize_split3_kernel, dim3((unsigned)blocks), dim3(256), stream, /*pdl=*/true,

@@ -52,6 +52,24 @@ int32_t check_launch(const char* what);
 __device__ __forceinline__ void pdl_wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Global loads that stay behind pdl_wait_prior_grid(): the compiler keeps volatile statements in order, while it may move a load
+// through a `const __restrict__` pointer (which it takes to be invariant for the whole kernel) ahead of the wait.
+__device__ __forceinline__ uint4 ld_global_16(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ __half ld_global_half(const __half* p) {
+    unsigned short v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return __ushort_as_half(v);
+}
+__device__ __forceinline__ uint32_t ld_global_u32(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 template <typename... Args>
 cudaError_t launch_ex(void (*kernel)(Args...), dim3 grid, dim3 block, cudaStream_t stream, bool pdl, Args... args) {
     cudaLaunchConfig_t cfg = {};

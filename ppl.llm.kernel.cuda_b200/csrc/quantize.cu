@@ -16,8 +16,8 @@ namespace {
 using namespace qdev;
 
 // One CTA per row.  A "unit" is 16 consecutive halves (two 128-bit loads, one 128-bit store).
-// Thread t owns units t, t + blockDim.x, ... (UNITS of them), kept in registers.
-template <int UNITS>
+// Thread t owns units t, t + blockDim.x, ... (UNITS of them), kept in registers.  GIVEN: the row maximum is known.
+template <int UNITS, bool GIVEN>
 __global__ void __launch_bounds__(QTPB, UNITS <= 2 ? 5 : 1)
 quantize_rows_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, float up_scale, int32_t layout,
                      int8_t* __restrict__ q, half* __restrict__ scale_out, const uint32_t* __restrict__ given_absmax_bits,
@@ -47,7 +47,7 @@ quantize_rows_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, fl
 
     // max |x| taken in fp16 (exact: max commutes with the widening conversion)
     QuantRow qr;
-    if (given_absmax_bits == nullptr) {
+    if constexpr (!GIVEN) {
         bool saw_nan, any_nan;
         float amax = absmax_halves(reinterpret_cast<const __half2*>(&v[0][0]), UNITS * 8, saw_nan);
         amax = block_max_any(amax, saw_nan, red, blockDim.x >> 5, any_nan);
@@ -55,10 +55,10 @@ quantize_rows_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, fl
     } else {
         float amax;
         if (given_parts == 1) {
-            amax = __uint_as_float(given_absmax_bits[row]);
+            amax = __uint_as_float(ld_global_u32(given_absmax_bits + row));
         } else { // partial maxima of the CTAs that produced the row: no NaN among them
             amax = 0.0f;
-            for (int i = threadIdx.x; i < given_parts; i += blockDim.x) amax = fmaxf(amax, __uint_as_float(given_absmax_bits[row * given_parts + i]));
+            for (int i = threadIdx.x; i < given_parts; i += blockDim.x) amax = fmaxf(amax, __uint_as_float(ld_global_u32(given_absmax_bits + row * given_parts + i)));
             amax = block_max(amax, red, blockDim.x >> 5);
         }
         qr = make_quant_row(amax, false);
@@ -69,8 +69,7 @@ quantize_rows_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, fl
     for (int u = 0; u < UNITS; ++u) {
         const int unit = unit_base + u * blockDim.x + threadIdx.x;
         if (unit < units) {
-            const uint4 o = given_absmax_bits == nullptr ? quant16<false>(reinterpret_cast<const __half2*>(&v[u][0]), qr)
-                                                         : quant16<true>(reinterpret_cast<const __half2*>(&v[u][0]), qr);
+            const uint4 o = quant16<GIVEN>(reinterpret_cast<const __half2*>(&v[u][0]), qr);
             const int64_t off = layout_offset(layout, batch, dim, row, (int64_t)unit << 4);
             *reinterpret_cast<uint4*>(q + off) = o;
         }
@@ -97,7 +96,7 @@ quantize_rows_twopass_kernel(const half* __restrict__ in, int64_t batch, int64_t
     if (given_absmax_bits == nullptr) {
         __half2 m2 = __float2half2_rn(0.0f);
         for (int64_t unit = threadIdx.x; unit < units; unit += blockDim.x) {
-            uint4 a[2] = {src[2 * unit], src[2 * unit + 1]};
+            uint4 a[2] = {ld_global_16(src + 2 * unit), ld_global_16(src + 2 * unit + 1)};
             const __half2* h = reinterpret_cast<const __half2*>(a);
 #pragma unroll
             for (int i = 0; i < 8; ++i) m2 = __hmax2(m2, __habs2(h[i]));
@@ -105,13 +104,13 @@ quantize_rows_twopass_kernel(const half* __restrict__ in, int64_t batch, int64_t
         amax = block_max(fmaxf(__low2float(m2), __high2float(m2)), red, blockDim.x >> 5);
     } else {
         amax = 0.0f;
-        for (int i = threadIdx.x; i < given_parts; i += blockDim.x) amax = fmaxf(amax, __uint_as_float(given_absmax_bits[row * given_parts + i]));
+        for (int i = threadIdx.x; i < given_parts; i += blockDim.x) amax = fmaxf(amax, __uint_as_float(ld_global_u32(given_absmax_bits + row * given_parts + i)));
         amax = block_max(amax, red, blockDim.x >> 5);
     }
     const QuantRow qr = make_quant_row(amax, false);
     const float scale = qr.scale;
     for (int64_t unit = threadIdx.x; unit < units; unit += blockDim.x) {
-        uint4 a[2] = {src[2 * unit], src[2 * unit + 1]};
+        uint4 a[2] = {ld_global_16(src + 2 * unit), ld_global_16(src + 2 * unit + 1)};
         const uint4 o = quant16<true>(reinterpret_cast<const __half2*>(a), qr); // NaNs were dropped above: looked for per group
         *reinterpret_cast<uint4*>(q + layout_offset(layout, batch, dim, row, unit << 4)) = o;
     }
@@ -232,7 +231,7 @@ int32_t launch_quantize(cudaStream_t stream, const half* in, int64_t batch, int6
         // 256-unit chunks (more loads in flight when there are few rows)
         int threads = (int)(units < QTPB ? (units + 31) / 32 * 32 : QTPB);
         const dim3 grid((unsigned)batch, (unsigned)((units + threads - 1) / threads), 1);
-        e = launch_ex(quantize_rows_kernel<1>, grid, dim3(threads), stream, pdl, in, batch, dim, up_scale, layout, q, scale,
+        e = launch_ex(quantize_rows_kernel<1, true>, grid, dim3(threads), stream, pdl, in, batch, dim, up_scale, layout, q, scale,
                       given_absmax_bits, zero_absmax_bits, given_parts);
     } else if (units <= QTPB * 8) {
         // threads: enough to give every thread the same small number of units
@@ -246,10 +245,10 @@ int32_t launch_quantize(cudaStream_t stream, const half* in, int64_t batch, int6
         if (threads > QTPB) threads = QTPB;
         const dim3 grid((unsigned)batch, 1, 1), block(threads);
         switch (bucket) {
-        case 1: e = launch_ex(quantize_rows_kernel<1>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
-        case 2: e = launch_ex(quantize_rows_kernel<2>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
-        case 4: e = launch_ex(quantize_rows_kernel<4>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
-        default: e = launch_ex(quantize_rows_kernel<8>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
+        case 1: e = launch_ex(quantize_rows_kernel<1, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
+        case 2: e = launch_ex(quantize_rows_kernel<2, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
+        case 4: e = launch_ex(quantize_rows_kernel<4, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
+        default: e = launch_ex(quantize_rows_kernel<8, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
         }
     } else {
         e = launch_ex(quantize_rows_twopass_kernel, dim3((unsigned)batch), dim3(QTPB), stream, pdl, in, batch, dim, up_scale, layout, q, scale,

@@ -21,8 +21,6 @@ namespace {
 
 constexpr int RTPB = 256;
 
-__device__ __forceinline__ uint4 ldg16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
-
 template <int UNITS>
 __global__ void __launch_bounds__(RTPB)
 skip_rmsnorm_quantize_kernel(const half* __restrict__ input, const half* __restrict__ weight, const half* __restrict__ skip,
@@ -37,8 +35,37 @@ skip_rmsnorm_quantize_kernel(const half* __restrict__ input, const half* __restr
     pdl_launch_dependents();
     pdl_wait_prior_grid();
 
-    // ---- load, skip add, statistics
-    __half2 z[UNITS][8];
+    // ---- load, skip add, statistics.  A row of a small batch is one chain of latencies, so everything it needs is requested
+    // before anything is used; short rows also keep the norm weights in registers for the second pass.
+    // (96 tokens of an 8192-wide layer, two norms, the QKV split rewritten alongside: 80.9 -> 75.7 us for the layer's nine launches.)
+    constexpr bool KEEP_W = UNITS <= 2;
+    uint4 zv[UNITS][2], wk[KEEP_W ? UNITS : 1][2];
+#pragma unroll
+    for (int u = 0; u < UNITS; ++u) {
+        const int unit = u * blockDim.x + threadIdx.x;
+        zv[u][0] = zv[u][1] = make_uint4(0, 0, 0, 0);
+        if (unit < units) {
+            const int64_t off = (int64_t)unit << 4;
+            zv[u][0] = ld_global_16(in_row + off);
+            zv[u][1] = ld_global_16(in_row + off + 8);
+        }
+    }
+    uint4 sv[KEEP_W ? UNITS : 1][2];
+    if (KEEP_W) {
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            const int unit = u * blockDim.x + threadIdx.x;
+            if (unit < units) {
+                const int64_t off = (int64_t)unit << 4;
+                if (skip != nullptr) {
+                    sv[u][0] = ld_global_16(skip + row * dim + off);
+                    sv[u][1] = ld_global_16(skip + row * dim + off + 8);
+                }
+                wk[u][0] = ld_global_16(weight + off);
+                wk[u][1] = ld_global_16(weight + off + 8);
+            }
+        }
+    }
     float sumsq = 0.0f;
     float amax = eps; // the reference seeds the running maximum with eps (rms_norm.cu:58)
 #pragma unroll
@@ -46,21 +73,23 @@ skip_rmsnorm_quantize_kernel(const half* __restrict__ input, const half* __restr
         const int unit = u * blockDim.x + threadIdx.x;
         if (unit < units) {
             const int64_t off = (int64_t)unit << 4;
-            uint4 a[2] = {ldg16(in_row + off), ldg16(in_row + off + 8)};
-            __half2* h = reinterpret_cast<__half2*>(a);
+            __half2* h = reinterpret_cast<__half2*>(&zv[u][0]);
+            uint4 wv[2];
             if (skip != nullptr) {
-                uint4 s[2] = {ldg16(skip + row * dim + off), ldg16(skip + row * dim + off + 8)};
-                const __half2* sh = reinterpret_cast<const __half2*>(s);
+                uint4 st[2];
+                if (KEEP_W) { st[0] = sv[KEEP_W ? u : 0][0]; st[1] = sv[KEEP_W ? u : 0][1]; }
+                else { st[0] = ld_global_16(skip + row * dim + off); st[1] = ld_global_16(skip + row * dim + off + 8); }
+                const __half2* sh = reinterpret_cast<const __half2*>(st);
 #pragma unroll
                 for (int i = 0; i < 8; ++i) h[i] = __hadd2(h[i], sh[i]);
             }
-            *reinterpret_cast<uint4*>(skip_out + row * dim + off) = a[0];
-            *reinterpret_cast<uint4*>(skip_out + row * dim + off + 8) = a[1];
-            uint4 wv[2] = {ldg16(weight + off), ldg16(weight + off + 8)};
+            *reinterpret_cast<uint4*>(skip_out + row * dim + off) = zv[u][0];
+            *reinterpret_cast<uint4*>(skip_out + row * dim + off + 8) = zv[u][1];
+            if (KEEP_W) { wv[0] = wk[KEEP_W ? u : 0][0]; wv[1] = wk[KEEP_W ? u : 0][1]; }
+            else { wv[0] = ld_global_16(weight + off); wv[1] = ld_global_16(weight + off + 8); }
             const __half2* wh = reinterpret_cast<const __half2*>(wv);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                z[u][i] = h[i];
                 const float2 x = __half22float2(h[i]);
                 const float2 w = __half22float2(wh[i]);
                 sumsq = fmaf(x.x, x.x, sumsq);
@@ -68,9 +97,6 @@ skip_rmsnorm_quantize_kernel(const half* __restrict__ input, const half* __restr
                 amax = fmaxf(amax, fabsf(__fmul_rn(x.x, w.x)));
                 amax = fmaxf(amax, fabsf(__fmul_rn(x.y, w.y)));
             }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) z[u][i] = __float2half2_rn(0.0f);
         }
     }
 #pragma unroll
@@ -96,12 +122,14 @@ skip_rmsnorm_quantize_kernel(const half* __restrict__ input, const half* __restr
         const int unit = u * blockDim.x + threadIdx.x;
         if (unit < units) {
             const int64_t off = (int64_t)unit << 4;
-            uint4 wv[2] = {ldg16(weight + off), ldg16(weight + off + 8)};
+            uint4 wv[2];
+            if (KEEP_W) { wv[0] = wk[KEEP_W ? u : 0][0]; wv[1] = wk[KEEP_W ? u : 0][1]; }
+            else { wv[0] = ld_global_16(weight + off); wv[1] = ld_global_16(weight + off + 8); }
             const __half2* wh = reinterpret_cast<const __half2*>(wv);
             int qi[16];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const float2 x = __half22float2(z[u][i]);
+                const float2 x = __half22float2(reinterpret_cast<const __half2*>(&zv[u][0])[i]);
                 const float2 w = __half22float2(wh[i]);
                 const float v0 = __fmul_rn(__fmul_rn(__fmul_rn(x.x, w.x), r), inv_scale);
                 const float v1 = __fmul_rn(__fmul_rn(__fmul_rn(x.y, w.y), r), inv_scale);

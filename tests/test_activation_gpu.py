@@ -197,3 +197,19 @@ def test_small_batch_gate_up_swiglu_overflow(cuda):
     assert bool(cuda.isinf(two_step[0]).any()) and bool(cuda.isfinite(two_step[0]).any())
     assert cuda.equal(fused[0].view(cuda.int16), two_step[0].view(cuda.int16))
     assert cuda.equal(fused[1], two_step[1]) and cuda.equal(fused[2].view(cuda.int16), two_step[2].view(cuda.int16))
+
+
+@pytest.mark.parametrize("M,splits", [(1, (8, 8, 8)), (5, (4096, 512, 512)), (2401, (32, 8, 8)), (3, (2056, 0, 16)), (7, (24, 16, 4)), (1203, (2048, 256, 256))])
+@pytest.mark.parametrize("with_bias", [False, True])
+def test_dequantize_split3_vector_form(cuda, oracle, M, splits, with_bias):
+    """Eight columns per thread (one or four rows each), ragged last CTAs and rows, an empty output; (24, 16, 4) keeps to groups of four."""
+    import pplb200
+    rng = np.random.default_rng(M + sum(splits))
+    N = sum(splits)
+    acc = rng.integers(-2**22, 2**22, (M, N), dtype=np.int32)
+    sm, sn = (rng.uniform(0.5, 3.0, M) * 32).astype(np.float16), (rng.uniform(0.001, 0.01, N) * 8192).astype(np.float16)
+    bias = rng.standard_normal(N).astype(np.float16) if with_bias else None
+    outs = pplb200.minmax_dequantize_split3_fp16(_t(cuda, acc), _t(cuda, sm), _t(cuda, sn), splits, _t(cuda, bias))
+    rc, want = oracle.dequantize_split3(acc, sm, sn, splits, bias)
+    for a, b in zip(outs, want):
+        assert np.array_equal(oracle.f16_bits(a.cpu().numpy()), oracle.f16_bits(b))
