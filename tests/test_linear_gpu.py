@@ -162,3 +162,10 @@ def test_linear_on_host_buffers_matches_device_path(cuda, oracle, M, K, N, chunk
     ref = oracle.linear(x.numpy()[:8], w, sn, bias)
     assert np.array_equal(oracle.f16_bits(y_host[:8].numpy()), oracle.f16_bits(ref["y"]))
     assert pplb200.gemm_status() == 0
+
+
+@pytest.mark.parametrize("M,K,N,chunk,requant", [(40, 512, 272, 0, False), (1024, 512, 528, 0, True), (1500, 256, 264, 1024, False),
+                                                 (2047, 2048, 1024, 1024, True), (1023, 4096, 1032, 0, False)])
+def test_linear_on_host_buffers_below_two_chunks(cuda, oracle, M, K, N, chunk, requant):
+    """Short first and last chunks inside the two staging buffers, which together hold the whole batch."""
+    test_linear_on_host_buffers_matches_device_path(cuda, oracle, M, K, N, chunk, requant)
