@@ -210,6 +210,8 @@ namespace {
 // The fused form needs the CTA-pair kernel: enough 256-row x 128-channel tiles for every pair, and
 // the x / gate halves of the weight matrix aligned to the 128-row tiles.
 bool swiglu_fusable(int64_t M, int64_t D) { return M > 128 && D % 128 == 0 && ((M + 255) / 256) * (D / 128) >= 74; }
+// Fused on single CTAs: batches for which the plain GEMM does not use CTA pairs either.
+bool swiglu_single(int64_t M, int64_t D) { return M <= 128 || ((M + 255) / 256) * ((2 * D + 255) / 256) < 74; }
 }
 
 int64_t pplb200_i8i8_gate_up_swiglu_workspace_bytes(int64_t M, int64_t act_dim, int64_t K) {
@@ -236,8 +238,9 @@ int32_t pplb200_i8i8_gate_up_swiglu_requant(pplb200_stream_t stream_, const void
     if ((reinterpret_cast<uintptr_t>(ws) & (WS_ALIGN - 1)) != 0) return fail(RC_INVALID_VALUE, "workspace must be 256-byte aligned");
     uint32_t* maxima = (uint32_t*)ws;
 
-    if (M > 128 && !swiglu_fusable(M, D)) {
-        // too few tiles for the CTA pairs, too many tokens for the small-batch kernel: raw int32 GEMM, then the stand-alone SwiGLU + re-quantize kernel
+    const bool pairs = swiglu_fusable(M, D);
+    if (!pairs && !swiglu_single(M, D)) {
+        // many tokens, but halves that do not fall on the CTA pairs' 128-row tiles: raw int32 GEMM, then the stand-alone SwiGLU + re-quantize kernel
         void* acc = (char*)ws + round_up(M * 4 + 4, WS_ALIGN);
         int32_t rc = gemm_entry(stream, input, lda, weight, K, M, 2 * D, K, EPI_RAW_I32, nullptr, nullptr, nullptr, 0.f, 0.f, 0.f,
                                 nullptr, 0, acc, 2 * D, nullptr, nullptr, false);
@@ -246,12 +249,12 @@ int32_t pplb200_i8i8_gate_up_swiglu_requant(pplb200_stream_t stream_, const void
                           activated, out_q, out_q_scale);
     }
 
-    // The small-batch kernel writes its CTAs' partial maxima, at most 2 D per row: the [M, 2 D] int32 that the workspace
+    // The single-CTA kernel writes its CTAs' partial maxima, at most 2 D per row: the [M, 2 D] int32 that the workspace
     // holds for such a batch.
     int32_t parts = 1;
-    if (M > 128 && cudaMemsetAsync(maxima, 0, (size_t)M * 4, stream) != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "memset failed");
+    if (pairs && cudaMemsetAsync(maxima, 0, (size_t)M * 4, stream) != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "memset failed");
     GemmArgs g;
-    g.row_absmax_parts = &parts;
+    g.row_absmax_parts = pairs ? nullptr : &parts;
     g.A = (const int8_t*)input; g.lda = lda; g.B = (const int8_t*)weight; g.ldb = K;
     g.M = M; g.N = 2 * D; g.K = K; g.mode = EPI_SWIGLU_F16;
     g.scale_m = (const half*)scale_M; g.scale_n = (const half*)scale_N; g.bias = nullptr;

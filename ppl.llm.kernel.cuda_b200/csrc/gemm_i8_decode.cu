@@ -40,6 +40,7 @@ constexpr unsigned ST_DEC_PRODUCER = 16u, ST_DEC_MMA = 32u, ST_DEC_EPI = 64u;
 struct DecodeParams {
     int32_t M, N;           // tokens, output columns (= weight rows; EPI_SWIGLU_F16: half of them)
     int32_t tile_rows;      // weight rows per tile (a multiple of 8, <= 128; two-part tiles: per part), chosen so that the tiles fill the SMs
+    int32_t tile_tokens;    // tokens per tile (a multiple of 16, <= BT): blockIdx.z counts the token tiles
     int32_t part_stride;    // two-part tiles: the second part starts this many weight rows after the first
     int32_t w_box_bytes;    // bytes of weights that one K block brings in
     int32_t w_slot_bytes;   // bytes between the slots of the weight ring
@@ -70,9 +71,11 @@ template <int BT> struct DCfg {
     static constexpr int X_BYTES = BT * BK;
     // Ring depths are multiples of the number of MMA issuers, so that every use of a slot belongs to the same issuer:
     // a thread then never polls a barrier more than one phase ahead (a parity wait cannot tell phase u from u + 2).
-    static constexpr int X_STAGES = BT >= 64 ? 6 : 8;
+    // A two-part tile's weight stages are up to 32 KB: four of them need the room of two activation stages (448 x 14336 x 9216
+    // with two weight stages: 107 us).
+    template <bool DUAL> static constexpr int x_stages() { return BT == 128 && DUAL ? 4 : BT >= 64 ? 6 : 8; }
     static constexpr int RING_BYTES = SMEM_BUDGET - 1024;
-    static constexpr int X_RING_OFFSET = RING_BYTES - X_STAGES * X_BYTES; // the weight ring grows from 0 up to here
+    template <bool DUAL> static constexpr int x_ring_offset() { return RING_BYTES - x_stages<DUAL>() * X_BYTES; } // the weight ring grows from 0 up to here
     static constexpr int SMEM_BYTES = SMEM_BUDGET;
     // Two MMA-issuing threads, each with its own accumulator tile.  With at most 128 token columns an MMA is issued
     // in 53 - 64 cycles, but the thread that issues it also waits on two barriers, polls the next two and commits
@@ -95,7 +98,8 @@ template <int BT> struct DCfg {
     static_assert(SWIGLU_OUT + BT * 128 * 2 <= RING_BYTES, "swiglu epilogue buffers fit the rings");
     static_assert(LD_COLS == 8 || LD_COLS == 16 || LD_COLS == 32, "tcgen05.ld shape");
     static_assert(BT == 16 || BT == 32 || BT == 64 || BT == 128, "token tile");
-    static_assert(X_RING_OFFSET % 1024 == 0 && X_RING_OFFSET >= 6 * BW * BK, "room for at least six full weight tiles");
+    static_assert(RING_BYTES % 1024 == 0 && RING_BYTES - 6 * X_BYTES >= 6 * BW * BK && RING_BYTES - 4 * X_BYTES >= 8 * BW * BK,
+                  "room for at least six full weight tiles, or four of two parts");
     // the rings double as the receive buffer of the reduce-scatter once the main loop is over
     static_assert(PIECES * PIECE_BYTES <= RING_BYTES, "receive buffer fits the rings");
 };
@@ -213,7 +217,7 @@ template <int BT, bool DUAL>
 __device__ __forceinline__ void swiglu_epilogue(const DecodeParams& p, uint32_t taddr_row, uint32_t ring, uint32_t S, uint32_t rank,
                                                 uint32_t own0, uint32_t slot0, uint32_t step_div, uint32_t step_rem, uint32_t slot_carry,
                                                 uint32_t recv_pieces, bool have_acc, int nkb, int col_begin, int col_end, int nl, int n,
-                                                int q, int lane, const float (&sn)[2], const float* token_scale, uint32_t* token_absmax) {
+                                                int q, int lane, const float (&sn)[2], const float* token_scale, uint32_t* token_absmax, int M) {
     using C = DCfg<BT>;
     constexpr int NPART = DUAL ? 2 : 1;
     const int valid = nkb < C::NACC ? nkb : C::NACC;
@@ -239,7 +243,7 @@ __device__ __forceinline__ void swiglu_epilogue(const DecodeParams& p, uint32_t 
         uint32_t own = own0, slot = slot0;
 #pragma unroll 1
         for (int c0 = col_begin; c0 < col_end; c0 += PIECE_COLS) {
-            if (c0 >= p.M) break;
+            if (c0 >= M) break;
             if (own == rank && ((c0 / PIECE_COLS) & 1) != side) {
                 uint32_t v[8];
                 load8(c0, slot, v);
@@ -254,7 +258,7 @@ __device__ __forceinline__ void swiglu_epilogue(const DecodeParams& p, uint32_t 
     uint32_t own = own0, slot = slot0;
 #pragma unroll 1
     for (int c0 = col_begin; c0 < col_end; c0 += PIECE_COLS) {
-        if (c0 >= p.M) break;
+        if (c0 >= M) break;
         if (DUAL || (own == rank && ((c0 / PIECE_COLS) & 1) == side)) {
             uint32_t v[8], w[8], absbits[8];
             load8(c0, slot, v);
@@ -278,7 +282,7 @@ __device__ __forceinline__ void swiglu_epilogue(const DecodeParams& p, uint32_t 
                                  "h"(__half_as_ushort(__float2half_rn(r))) : "memory");
             }
             const uint32_t tok_max = warp_token_max<8>(absbits, lane);
-            if (lane < 8 && c0 + lane < p.M && tok_max != 0u) atomicMax(&token_absmax[c0 + lane], tok_max);
+            if (lane < 8 && c0 + lane < M && tok_max != 0u) atomicMax(&token_absmax[c0 + lane], tok_max);
         }
         own += step_rem; slot += step_div;
         if (own >= S) { own -= S; slot += slot_carry; }
@@ -302,10 +306,11 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     using C = DCfg<BT>;
     constexpr int NUM_THREADS = C::NUM_THREADS;
     constexpr int NPART = DUAL ? 2 : 1;
+    constexpr int X_STAGES = C::template x_stages<DUAL>();
     constexpr int TMEM_COLS = C::template tmem_cols<DUAL>();
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_w[MAX_W_STAGES], empty_w[MAX_W_STAGES];
-    __shared__ __align__(8) uint64_t full_x[C::X_STAGES], empty_x[C::X_STAGES];
+    __shared__ __align__(8) uint64_t full_x[X_STAGES], empty_x[X_STAGES];
     __shared__ __align__(8) uint64_t acc_full_bar;
     __shared__ uint32_t tmem_base_slot;
     __shared__ __align__(16) float token_scale[BT];
@@ -321,8 +326,11 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const int SW = p.w_stages;
     const uint32_t w_stride = (uint32_t)p.w_slot_bytes;
     constexpr bool pack = SWIGLU && !DUAL, two_parts = SWIGLU || DUAL;
+    const int token0 = (int)blockIdx.z * p.tile_tokens;
+    const int M = p.M - token0 < p.tile_tokens ? p.M - token0 : p.tile_tokens; // tokens of this tile
+    const uint32_t x_box_bytes = (uint32_t)p.tile_tokens * BK;
     const int tile_row0 = n_tile * p.tile_rows * (DUAL && !SWIGLU ? 2 : 1); // first weight row (= output column)
-    const uint32_t x_ring = ring + C::X_RING_OFFSET;
+    const uint32_t x_ring = ring + C::template x_ring_offset<DUAL>();
 
     // this CTA's K blocks
     const int nkb_total = p.num_k_blocks;
@@ -345,7 +353,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
             ptx::mbar_init(ptx::smem_addr(&full_w[lane]), 1);
             ptx::mbar_init(ptx::smem_addr(&empty_w[lane]), 1);
         }
-        if (lane < C::X_STAGES) {
+        if (lane < X_STAGES) {
             ptx::mbar_init(ptx::smem_addr(&full_x[lane]), 1);
             ptx::mbar_init(ptx::smem_addr(&empty_x[lane]), 1);
         }
@@ -426,16 +434,16 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         pdl_wait_prior_grid(); // quantized activations are written by the preceding kernel
         uint32_t sx = 0, px = 0;
         for (int i = 0; i < nkb; ++i) {
-            if (i >= C::X_STAGES && !ptx::mbar_wait(ex0 + sx * 8u, px ^ 1u, p.status, ST_DEC_PRODUCER)) { ok = false; break; }
-            ptx::mbar_arrive_expect_tx(fx0 + sx * 8u, C::X_BYTES);
-            ptx::tma_load_2d(x_ring + sx * C::X_BYTES, &tmap_x, fx0 + sx * 8u, PPLB200_KB(i) * BK, 0);
-            if (++sx == (uint32_t)C::X_STAGES) { sx = 0; px ^= 1u; }
+            if (i >= X_STAGES && !ptx::mbar_wait(ex0 + sx * 8u, px ^ 1u, p.status, ST_DEC_PRODUCER)) { ok = false; break; }
+            ptx::mbar_arrive_expect_tx(fx0 + sx * 8u, x_box_bytes);
+            ptx::tma_load_2d(x_ring + sx * C::X_BYTES, &tmap_x, fx0 + sx * 8u, PPLB200_KB(i) * BK, token0);
+            if (++sx == (uint32_t)X_STAGES) { sx = 0; px ^= 1u; }
         }
     } else if ((warp == 1 || warp == 2) && lane == 0) {
         // ---- MMA issuers: two threads, K blocks me, me + 2, ... each, accumulator tile `me`.  Their own instruction
         // streams are kept short (descriptors are a 32-bit add away from the previous ones; the barriers of the next
         // K block are polled before this block's MMAs are issued).
-        constexpr uint32_t idesc = ptx::make_i8_idesc(BW, BT);
+        const uint32_t idesc = ptx::make_i8_idesc(BW, p.tile_tokens);
         const int me = warp - 1;
         const uint32_t w_lo0 = ptx::desc_lo_sw128(ring), x_lo0 = ptx::desc_lo_sw128(x_ring);
         const uint32_t fw0 = ptx::smem_addr(&full_w[0]), ew0 = ptx::smem_addr(&empty_w[0]);
@@ -450,7 +458,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
             ptx::tc_fence_after();
             uint32_t nsw = sw + C::NACC, npw = pw, nsx = sx + C::NACC, npx = px;
             if (nsw >= (uint32_t)SW) { nsw -= (uint32_t)SW; npw ^= 1u; }
-            if (nsx >= (uint32_t)C::X_STAGES) { nsx -= (uint32_t)C::X_STAGES; npx ^= 1u; }
+            if (nsx >= (uint32_t)X_STAGES) { nsx -= (uint32_t)X_STAGES; npx ^= 1u; }
             ready_w = ptx::mbar_try_wait(fw0 + nsw * 8u, npw);
             ready_x = ptx::mbar_try_wait(fx0 + nsx * 8u, npx);
             const uint32_t w_lo = w_lo0 + sw * (w_stride >> 4), x_lo = x_lo0 + sx * (uint32_t)(C::X_BYTES >> 4);
@@ -478,7 +486,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
 
     if (p.mode != EPI_RAW_I32) {
         for (int m = threadIdx.x; m < BT; m += NUM_THREADS)
-            token_scale[m] = m < p.M ? __fmul_rn(__half2float(p.scale_m[m]), p.down_m) : 0.0f;
+            token_scale[m] = m < M ? __fmul_rn(__half2float(p.scale_m[token0 + m]), p.down_m) : 0.0f;
     }
 
     // ---- all four warps: wait for this CTA's partial accumulator
@@ -505,7 +513,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         uint32_t own = own0, slot = slot0;
 #pragma unroll 1
         for (int c0 = col_begin; c0 < col_end; c0 += C::LD_COLS) {
-            if (c0 >= p.M) break; // columns past the last token hold zeros nobody reads
+            if (c0 >= M) break; // columns past the last token hold zeros nobody reads
             uint32_t acc[C::LD_COLS];
             if (have_acc) {
                 tmem_ld_sum<C::LD_COLS, C::NACC, NPART * BT>(taddr_row + c0, acc, nkb < C::NACC ? nkb : C::NACC);
@@ -534,7 +542,6 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
 
     // ---- epilogue over the pieces this CTA owns
     const int mode = p.mode;
-    const int M = p.M;
     const float down_n = p.down_n;
     // Without a K split the CTA owns its whole [tokens x tile_rows] output tile: the values are transposed through
     // shared memory (the rings are dead by now) into a dense [token][weight row] tile and leave as ONE TMA store,
@@ -544,7 +551,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const uint32_t tile_cols = (uint32_t)(p.tile_rows * NPART);
     if constexpr (SWIGLU) {
         swiglu_epilogue<BT, DUAL>(p, taddr_row, ring, S, rank, own0, slot0, step_div, step_rem, slot_carry, recv_pieces_per_owner, have_acc,
-                                  nkb, col_begin, col_end, nl, n, q, lane, sn, token_scale, token_absmax);
+                                  nkb, col_begin, col_end, nl, n, q, lane, sn, token_scale, token_absmax, M);
     } else {
 #pragma unroll
     for (int part = 0; part < NPART; ++part) { // S == 1 with two parts
@@ -586,7 +593,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                                 asm volatile("st.shared.u32 [%0], %1;" ::"r"(ring + ((uint32_t)(m0 + j) * tile_cols + nlp) * 4u), "r"(v[j]) : "memory");
                         }
                     } else if (mode == EPI_RAW_I32) {
-                        int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)m0 * p.ldc + np;
+                        int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)(token0 + m0) * p.ldc + np;
                         const uint32_t add = (p.raw_affine && p.raw_bias != nullptr && n_ok) ? (uint32_t)p.raw_bias[np] : 0u;
 #pragma unroll
                         for (int j = 0; j < 8; ++j)
@@ -618,7 +625,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                                     asm volatile("st.shared.u16 [%0], %1;" ::"r"(ring + ((uint32_t)(m0 + j) * tile_cols + nlp) * 2u), "h"(__half_as_ushort(h[j])) : "memory");
                             }
                         } else {
-                            half* dst = reinterpret_cast<half*>(p.out) + (int64_t)m0 * p.ldc + np;
+                            half* dst = reinterpret_cast<half*>(p.out) + (int64_t)(token0 + m0) * p.ldc + np;
 #pragma unroll
                             for (int j = 0; j < 8; ++j)
                                 if (n_ok && m0 + j < M) dst[(int64_t)j * p.ldc] = h[j];
@@ -651,29 +658,29 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     if constexpr (SWIGLU) { // eight tokens per store, those this CTA owns
         if (threadIdx.x < BT / PIECE_COLS && threadIdx.x * PIECE_COLS < M && (!pack || threadIdx.x % S == rank)) {
             ptx::tma_store_2d(&tmap_y, ring + C::SWIGLU_OUT + threadIdx.x * (uint32_t)(PIECE_COLS * 2 * p.tile_rows), tile_row0,
-                              (int)threadIdx.x * PIECE_COLS);
+                              token0 + (int)threadIdx.x * PIECE_COLS);
             ptx::bulk_commit_group();
             ptx::bulk_wait_group_read<0>();
         }
         // this CTA's share of the row maxima, [token][CTA]: a CTA writes every token (zero for those it does not own),
         // so nothing has to be cleared beforehand and nothing is added atomically
         const uint32_t cta = (uint32_t)n_tile * S + rank, ctas = gridDim.y * S;
-        for (int m = threadIdx.x; m < BT && m < M; m += NUM_THREADS) p.row_absmax_bits[(uint32_t)m * ctas + cta] = token_absmax[m];
+        for (int m = threadIdx.x; m < BT && m < M; m += NUM_THREADS) p.row_absmax_bits[(int64_t)(token0 + m) * ctas + cta] = token_absmax[m];
     } else if (staged && threadIdx.x == 0) {
-        ptx::tma_store_2d(&tmap_y, ring, tile_row0, 0);
+        ptx::tma_store_2d(&tmap_y, ring, tile_row0, token0);
         ptx::bulk_commit_group();
         ptx::bulk_wait_group_read<0>(); // shared memory must outlive the store's reads; the kernel boundary publishes the writes
     }
     if (p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
-        for (int m = threadIdx.x; m < BT && m < p.M; m += NUM_THREADS)
-            if (token_absmax[m] != 0u) atomicMax(p.row_absmax_bits + m, token_absmax[m]);
+        for (int m = threadIdx.x; m < BT && m < M; m += NUM_THREADS)
+            if (token_absmax[m] != 0u) atomicMax(p.row_absmax_bits + token0 + m, token_absmax[m]);
     }
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc(tmem_base, TMEM_COLS);
     }
     if (p.stamps && threadIdx.x == 0) {
-        const unsigned cta = blockIdx.y * gridDim.x + blockIdx.x;
+        const unsigned cta = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
         unsigned long long* st = p.stamps + (size_t)(cta < 296u ? cta : 295u) * 8;
         st[0] = t_start; st[1] = t_setup; st[2] = t_main; st[3] = t_exchange; st[4] = globaltimer_ns();
     }
@@ -767,10 +774,83 @@ const DecDeviceInfo* dec_device_info() {
     return &d;
 }
 
+// How a launch is cut: `tokens` x `rows` tiles (two-part tiles: rows per part), K split over S CTAs.
+struct DecodePlan {
+    int tokens, token_tiles, rows, row_tiles, S;
+    bool dual;
+};
+
+// Rows per tile for `cap` tiles that can run at once: the smallest multiple of 8 with which `columns` output columns
+// still are one wave -- e.g. 12288 weight rows: 140 tiles of 88 rows on 148 SMs instead of 96 tiles of 128 rows on 96.
+int rows_for(int64_t columns, int64_t cap, int max_rows) {
+    if (cap <= 0 || (columns + max_rows - 1) / max_rows > cap) return max_rows;
+    const int64_t r = ((columns + cap - 1) / cap + 7) / 8 * 8;
+    return r < 8 ? 8 : r < max_rows ? (int)r : max_rows;
+}
+
+// Up to 128 tokens: one token tile.
+DecodePlan plan_small(const DecDeviceInfo& dev, int variant, int64_t M, int64_t columns, int num_k_blocks, bool swiglu) {
+    DecodePlan d;
+    d.tokens = (int)((M + 15) / 16 * 16);
+    d.token_tiles = 1;
+    // Weight rows a tile can hold: one per TMEM lane, or, x and gate rows paired, half as many channels.
+    const int bw = swiglu ? BW / 2 : BW;
+    // Two accumulators per tile where tiles of bw rows no longer run as one wave: with 172 tiles on 148 SMs the second
+    // wave costs as much as the first.
+    d.dual = (columns + bw - 1) / bw > dev.sms;
+    // K split: one CTA per SM is resident (the rings take the whole shared memory), so split K only as far as all clusters
+    // still fit in one wave (fewer than SMs / S of them: a cluster stays inside one GPC); every CTA keeps at least two
+    // K blocks
+    int S = d.dual ? 1 : dev.sms / (int)((columns + bw - 1) / bw);
+    if (S > 8) S = 8;
+    if (S > num_k_blocks / 2) S = num_k_blocks / 2;
+    if (S < 1) S = 1;
+    d.S = S;
+    const int parts_out = d.dual && !swiglu ? 2 : 1; // parts of a tile that are output columns of their own
+    d.rows = rows_for(columns, (S == 1 ? dev.sms : dev.max_clusters[variant][S]) * (int64_t)parts_out, d.dual ? BW : bw);
+    d.row_tiles = (int)((columns + d.rows * parts_out - 1) / (d.rows * parts_out));
+    return d;
+}
+
+// More than 128 tokens, too few for the CTA pairs' 256 x 256 tiles: the cheapest cut by a model of one CTA's time in SM
+// cycles.  A K block costs the larger of its operands' way from L2 (60 bytes per cycle and SM), its four MMAs per part
+// (half a cycle per token, 53 at least) and the issuing threads' bookkeeping (390); a launch 3000, an
+// exchange of K partials 12000 (clusters also start and end together).
+DecodePlan plan_medium(const DecDeviceInfo& dev, int64_t M, int64_t columns, int num_k_blocks, bool swiglu) {
+    DecodePlan best = {};
+    double best_cost = 1e30;
+    for (int64_t t = (M + 127) / 128; t <= (M + 127) / 128 + 3; ++t) {
+        const int tokens = (int)(((M + t - 1) / t + 15) / 16 * 16);
+        if (tokens <= 64) break; // such tiles belong to another variant of the kernel
+        const int64_t token_tiles = (M + tokens - 1) / tokens;
+        for (int dual = 0; dual < 2; ++dual) {
+            const int max_rows = swiglu && !dual ? BW / 2 : BW;
+            const int parts_out = dual && !swiglu ? 2 : 1, parts = dual || swiglu ? 2 : 1;
+            for (int S = 1; S <= (dual ? 1 : 8) && (S == 1 || S <= num_k_blocks / 2); ++S) {
+                const int64_t slots = S == 1 ? dev.sms : dev.max_clusters[3][S];
+                if (slots <= 0) continue;
+                const int rows = rows_for(columns, slots / token_tiles * parts_out, max_rows);
+                const int64_t row_tiles = (columns + rows * parts_out - 1) / (rows * parts_out);
+                const int64_t waves = (row_tiles * token_tiles + slots - 1) / slots;
+                double kb = (rows * parts + tokens) * (double)BK / 60.0;
+                const double mma = (dual ? 8 : 4) * (tokens < 106 ? 53.0 : tokens / 2.0);
+                if (kb < mma) kb = mma;
+                if (kb < 390.0) kb = 390.0;
+                const double cost = (double)waves * ((num_k_blocks + S - 1) / S * kb + 3000.0 + (S > 1 ? 12000.0 : 0.0));
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best = {tokens, (int)token_tiles, rows, (int)row_tiles, S, dual != 0};
+                }
+            }
+        }
+    }
+    return best;
+}
+
 template <int BT>
-int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecDeviceInfo& dev, unsigned int* status, bool pdl) {
+int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecodePlan& plan, unsigned int* status, bool pdl) {
     CUtensorMap tw, tx;
-    if (!make_map(&tx, a.A, a.M, a.K, a.lda, BT)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (X) encode failed");
+    if (!make_map(&tx, a.A, a.M, a.K, a.lda, plan.tokens)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (X) encode failed");
     DecodeParams p;
     p.M = (int32_t)a.M; p.N = (int32_t)a.N;
     p.num_k_blocks = (int32_t)((a.K + BK - 1) / BK);
@@ -786,55 +866,31 @@ int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecDeviceInfo& d
     const bool swiglu = a.mode == EPI_SWIGLU_F16;
     if (swiglu) p.N = (int32_t)(a.N / 2); // the x half and the gate half of the weight rows share the output columns
     p.beta = a.beta;
-    // Weight rows a tile can hold: one per TMEM lane, or, x and gate rows paired, half as many channels.
-    const int bw = swiglu ? BW / 2 : BW;
-    // Two accumulators per tile where tiles of bw rows no longer run as one wave: with 172 tiles on 148 SMs the second
-    // wave costs as much as the first.
-    const bool dual = (p.N + bw - 1) / bw > dev.sms;
-
-    // K split: one CTA per SM is resident (the rings take the whole shared memory), so split K only as
-    // far as all clusters still fit in one wave; every CTA keeps at least two K blocks
-    int S = dual ? 1 : dev.sms / (int)((p.N + bw - 1) / bw);
-    if (S > 8) S = 8;
-    if (S > p.num_k_blocks / 2) S = p.num_k_blocks / 2;
-    if (S < 1) S = 1;
-    // Tile height: the smallest multiple of 8 rows with which the tiles still run as one wave -- e.g. 12288 weight
-    // rows: 140 tiles of 88 rows on 148 SMs instead of 96 tiles of 128 rows on 96.  With a K split the wave holds
-    // as many clusters as the device can co-schedule (fewer than SMs / S: a cluster stays inside one GPC).
-    const int parts_out = dual && !swiglu ? 2 : 1; // parts of a tile that are output columns of their own
-    int tile_rows = dual ? BW : bw;
-    {
-        int64_t cap = S == 1 ? dev.sms : dev.max_clusters[BT == 16 ? 0 : BT == 32 ? 1 : BT == 64 ? 2 : 3][S];
-        cap *= parts_out;
-        if (cap > 0 && (p.N + tile_rows - 1) / tile_rows <= cap) {
-            int64_t r = (p.N + cap - 1) / cap;
-            r = (r + 7) / 8 * 8;
-            if (r < 8) r = 8;
-            if (r < tile_rows) tile_rows = (int)r;
-        }
-    }
+    const int S = plan.S, tile_rows = plan.rows;
+    const bool dual = plan.dual;
+    const int parts_out = dual && !swiglu ? 2 : 1;
+    p.tile_tokens = plan.tokens;
     p.tile_rows = tile_rows;
     p.part_stride = swiglu ? p.N : tile_rows;
     p.w_box_bytes = tile_rows * BK * (dual || swiglu ? 2 : 1);
     p.w_slot_bytes = dual ? 2 * tile_rows * BK : (swiglu ? 64 + tile_rows : tile_rows) * BK;
-    p.w_stages = DCfg<BT>::X_RING_OFFSET / p.w_slot_bytes;
+    p.w_stages = (dual ? DCfg<BT>::template x_ring_offset<true>() : DCfg<BT>::template x_ring_offset<false>()) / p.w_slot_bytes;
     if (p.w_stages > MAX_W_STAGES) p.w_stages = MAX_W_STAGES;
     p.w_stages -= p.w_stages % DCfg<BT>::NACC; // see X_STAGES
     p.stamps = stall_counters();
     p.early_weights = a.after_quantizer ? 1 : 0;
 
-    const int n_tiles = (int)((p.N + tile_rows * parts_out - 1) / (tile_rows * parts_out));
-    if (a.row_absmax_parts) *a.row_absmax_parts = n_tiles * S;
+    if (a.row_absmax_parts) *a.row_absmax_parts = plan.row_tiles * S;
     if (!make_map(&tw, a.B, a.N, a.K, a.ldb, tile_rows)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (W) encode failed");
     CUtensorMap ty;
     memset(&ty, 0, sizeof(ty));
     if (swiglu ? !make_out_map(&ty, a.out, a.M, p.N, a.ldc, 2, tile_rows, PIECE_COLS)
                : S == 1 && !p.raw_affine &&
-                     !make_out_map(&ty, a.out, a.M, a.N, a.ldc, a.mode == EPI_RAW_I32 ? 4 : 2, tile_rows * parts_out, BT))
+                     !make_out_map(&ty, a.out, a.M, a.N, a.ldc, a.mode == EPI_RAW_I32 ? 4 : 2, tile_rows * parts_out, plan.tokens))
         return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (Y) encode failed");
 
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)S, (unsigned)n_tiles, 1);
+    cfg.gridDim = dim3((unsigned)S, (unsigned)plan.row_tiles, (unsigned)plan.token_tiles);
     cfg.blockDim = dim3(DCfg<BT>::NUM_THREADS, 1, 1);
     cfg.dynamicSmemBytes = DCfg<BT>::SMEM_BYTES;
     cfg.stream = stream;
@@ -864,10 +920,18 @@ int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecDeviceInfo& d
 int32_t launch_gemm_decode(cudaStream_t stream, const GemmArgs& a, unsigned int* status, bool pdl) {
     const DecDeviceInfo* dev = dec_device_info();
     if (!dev) return fail(RC_DEVICE_RUNTIME_ERROR, "device set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
-    if (a.M <= 16) return launch_bt<16>(stream, a, *dev, status, pdl);
-    if (a.M <= 32) return launch_bt<32>(stream, a, *dev, status, pdl);
-    if (a.M <= 64) return launch_bt<64>(stream, a, *dev, status, pdl);
-    return launch_bt<128>(stream, a, *dev, status, pdl);
+    const bool swiglu = a.mode == EPI_SWIGLU_F16;
+    const int64_t columns = swiglu ? a.N / 2 : a.N;
+    const int num_k_blocks = (int)((a.K + BK - 1) / BK);
+    if (a.M > 128) return launch_bt<128>(stream, a, plan_medium(*dev, a.M, columns, num_k_blocks, swiglu), status, pdl);
+    const int variant = a.M <= 16 ? 0 : a.M <= 32 ? 1 : a.M <= 64 ? 2 : 3;
+    const DecodePlan plan = plan_small(*dev, variant, a.M, columns, num_k_blocks, swiglu);
+    switch (variant) {
+    case 0: return launch_bt<16>(stream, a, plan, status, pdl);
+    case 1: return launch_bt<32>(stream, a, plan, status, pdl);
+    case 2: return launch_bt<64>(stream, a, plan, status, pdl);
+    default: return launch_bt<128>(stream, a, plan, status, pdl);
+    }
 }
 
 } // namespace pplb200

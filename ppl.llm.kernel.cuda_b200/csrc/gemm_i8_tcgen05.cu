@@ -6,12 +6,12 @@
 // C[M,N] = A[M,K] * B[N,K]^T, both operands K-major (row-major [rows, K]), exactly the
 // transa = false / transb = true convention of the reference's linear ops.
 //
-// Kernel shape: persistent, one CTA per SM, 6 warps:
+// Kernel shape: persistent, one CTA pair per two SMs, 6 warps per CTA:
 //   warp 0      TMA producer     (one elected lane)
-//   warp 1      MMA issuer       (one elected lane); also owns TMEM alloc / dealloc
-//   warps 2..5  epilogue         (tcgen05.ld -> scale -> fp16 -> global), one TMEM lane quarter each
-// Shared-memory ring of STAGES x {A tile 128 x 128 B, B tile BN x 128 B}; two TMEM accumulator
-// buffers of BN columns each so the epilogue of tile i overlaps the main loop of tile i + 1.
+//   warp 1      MMA issuer       (one elected lane of the leader CTA); also owns TMEM alloc / dealloc
+//   warps 2..   epilogue         (tcgen05.ld -> scale -> fp16 -> global), one TMEM lane quarter each
+// Shared-memory ring of stages; two TMEM accumulator buffers of 256 columns each so the epilogue of tile i
+// overlaps the main loop of tile i + 1.  Problems with fewer tiles than pairs go to gemm_i8_decode.cu.
 // No TMA multicast is used anywhere.
 #include "common.cuh"
 #include "ptx.cuh"
@@ -23,15 +23,9 @@ namespace pplb200 {
 
 namespace {
 
-constexpr int BM = 128;       // tile rows (TMEM lanes)
+constexpr int BM = 128;       // tile rows per CTA (TMEM lanes)
 constexpr int BK = 128;       // bytes (= int8 elements) of K per stage: one 128-byte swizzle row
 constexpr int UMMA_K = 32;    // K per tcgen05.mma kind::i8
-// warp 0: TMA producer, warp 1: MMA issuer, warps 2..: epilogue.  Four epilogue warps (one per TMEM
-// lane quarter) drain a 128 x 256 accumulator faster than its successor is produced; on the
-// power-capped part eight warps measured slower (more issue activity, lower clocks).
-constexpr int EPI_WARPS = 4;
-constexpr int NUM_THREADS = 64 + 32 * EPI_WARPS;
-
 // status bits recorded when a bounded wait gives up
 constexpr unsigned ST_PRODUCER_TIMEOUT = 1u, ST_MMA_FULL_TIMEOUT = 2u, ST_MMA_ACC_TIMEOUT = 4u, ST_EPI_TIMEOUT = 8u;
 
@@ -68,20 +62,6 @@ struct KernelParams {
     // EPI_GATHER_F16 (CTA-pair kernel only): see GemmArgs
     int32_t gather_ranks;
     int64_t gather_col0;
-};
-
-template <int BN> struct Cfg {
-    static constexpr int A_BYTES = BM * BK;
-    static constexpr int B_BYTES = BN * BK;
-    static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-    // the epilogue's staging buffers (EPI_STAGE_BYTES of static shared memory) come on top of the ring
-    static constexpr int STAGES = (BN >= 256) ? 4 : (BN >= 128) ? 6 : 8;
-    static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024; // + slack to align the ring to 1024 B
-    static constexpr int TMEM_COLS = (2 * BN <= 32) ? 32 : (2 * BN <= 64) ? 64 : (2 * BN <= 128) ? 128 : (2 * BN <= 256) ? 256 : 512;
-    static_assert(BN % 64 == 0 && BN >= 64 && BN <= 256, "UMMA N for M = 128; the epilogue stores 64-column slabs");
-    // More than half of the SM's shared memory: at most one CTA per SM, so two CTAs can never
-    // compete for (and block on) the same SM's tensor memory.
-    static_assert(SMEM_BYTES > 116 * 1024 && SMEM_BYTES <= 227 * 1024, "smem budget");
 };
 
 // Dequantize + optional bias for 8 consecutive columns; returns packed halves.
@@ -246,141 +226,6 @@ __device__ __forceinline__ void drain_tile(const KernelParams& p, const CUtensor
     if (want_absmax && row_ok) {
         const __half m = __hmax(__low2half(absmax2), __high2half(absmax2));
         atomicMax(p.row_absmax_bits + row, __float_as_uint(__half2float(m)));
-    }
-}
-
-template <int BN>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_i8_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                       const __grid_constant__ CUtensorMap tmap_out, const KernelParams p) {
-    using C = Cfg<BN>;
-    extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(1024) uint8_t epi_stage[EPI_STAGE_BYTES];
-    __shared__ __align__(8) uint64_t full_bar[C::STAGES];
-    __shared__ __align__(8) uint64_t empty_bar[C::STAGES];
-    __shared__ __align__(8) uint64_t acc_full_bar[2];
-    __shared__ __align__(8) uint64_t acc_empty_bar[2];
-    __shared__ uint32_t tmem_base_slot;
-
-    const int warp = threadIdx.x >> 5;
-    const int lane = threadIdx.x & 31;
-    const uint32_t ring = (ptx::smem_addr(smem_raw) + 1023u) & ~1023u;
-
-    if (warp == 0 && lane == 0) {
-        ptx::prefetch_tensormap(&tmap_a);
-        ptx::prefetch_tensormap(&tmap_b);
-        for (int s = 0; s < C::STAGES; ++s) {
-            ptx::mbar_init(ptx::smem_addr(&full_bar[s]), 1);
-            ptx::mbar_init(ptx::smem_addr(&empty_bar[s]), 1);
-        }
-        for (int b = 0; b < 2; ++b) {
-            ptx::mbar_init(ptx::smem_addr(&acc_full_bar[b]), 1);
-            ptx::mbar_init(ptx::smem_addr(&acc_empty_bar[b]), EPI_WARPS);
-        }
-        ptx::fence_mbar_init();
-    }
-    if (warp == 1) {
-        ptx::tmem_alloc(ptx::smem_addr(&tmem_base_slot), C::TMEM_COLS);
-        ptx::tmem_relinquish();
-    }
-    ptx::tc_fence_before();
-    __syncthreads();
-    ptx::tc_fence_after();
-    const uint32_t tmem_base = tmem_base_slot;
-    pdl_launch_dependents(); // every CTA is resident: a dependent kernel may set itself up under this one
-    pdl_wait_prior_grid();   // as a programmatic dependent: everything above ran under the tail of the preceding kernel
-
-    const int num_tiles = p.num_m_tiles * p.num_n_tiles;
-    const int nkb = p.num_k_blocks;
-
-    if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            uint32_t stage = 0, phase = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-                const int m_tile = tile % p.num_m_tiles;
-                const int n_tile = tile / p.num_m_tiles;
-                for (int kb = 0; kb < nkb; ++kb) {
-                    if (!ptx::mbar_wait(ptx::smem_addr(&empty_bar[stage]), phase ^ 1u, p.status, ST_PRODUCER_TIMEOUT)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t full = ptx::smem_addr(&full_bar[stage]);
-                    const uint32_t sa = ring + stage * C::STAGE_BYTES;
-                    ptx::mbar_arrive_expect_tx(full, C::STAGE_BYTES);
-                    ptx::tma_load_2d(sa, &tmap_a, full, kb * BK, m_tile * BM);
-                    ptx::tma_load_2d(sa + C::A_BYTES, &tmap_b, full, kb * BK, n_tile * BN);
-                    if (++stage == C::STAGES) { stage = 0; phase ^= 1u; }
-                }
-            }
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer
-        // One thread feeds the tensor cores, so its own instruction stream must stay well under the 128 cycles
-        // an MMA takes: descriptors are a 32-bit add away from the previous ones, and the barrier of the NEXT
-        // stage is polled before the current stage's MMAs are issued, so its latency hides behind them.
-        if (lane == 0) {
-            constexpr uint32_t idesc = ptx::make_i8_idesc(BM, BN);
-            const uint32_t a_lo0 = ptx::desc_lo_sw128(ring), full0 = ptx::smem_addr(&full_bar[0]), empty0 = ptx::smem_addr(&empty_bar[0]);
-            uint32_t stage = 0, phase = 0;
-            bool ok = true;
-            int it = 0;
-            bool ready = false;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++it) {
-                const uint32_t buf = it & 1, acc_phase = (it >> 1) & 1;
-                if (!ptx::mbar_wait(ptx::smem_addr(&acc_empty_bar[buf]), acc_phase ^ 1u, p.status, ST_MMA_ACC_TIMEOUT)) break;
-                ptx::tc_fence_after();
-                const uint32_t tmem_d = tmem_base + buf * BN;
-                for (int kb = 0; kb < nkb; ++kb) {
-                    if (!ready && !ptx::mbar_wait(full0 + stage * 8u, phase, p.status, ST_MMA_FULL_TIMEOUT)) {
-                        ok = false;
-                        break;
-                    }
-                    ptx::tc_fence_after();
-                    uint32_t nstage = stage + 1, nphase = phase;
-                    if (nstage == C::STAGES) { nstage = 0; nphase ^= 1u; }
-                    ready = ptx::mbar_try_wait(full0 + nstage * 8u, nphase); // used in the next iteration
-                    const uint32_t a_lo = a_lo0 + stage * (uint32_t)(C::STAGE_BYTES >> 4), b_lo = a_lo + (uint32_t)(C::A_BYTES >> 4);
-                    ptx::mma_i8(tmem_d, ptx::desc_from_lo(a_lo), ptx::desc_from_lo(b_lo), idesc, kb != 0 ? 1u : 0u);
-#pragma unroll
-                    for (uint32_t k = 1; k < BK / UMMA_K; ++k) // +32 bytes of K = +2 in descriptor address units
-                        ptx::mma_i8(tmem_d, ptx::desc_from_lo(a_lo + 2u * k), ptx::desc_from_lo(b_lo + 2u * k), idesc, 1u);
-                    ptx::mma_commit(empty0 + stage * 8u); // frees the smem slot when these MMAs retire
-                    stage = nstage; phase = nphase;
-                }
-                if (ok) ptx::mma_commit(ptx::smem_addr(&acc_full_bar[buf]));
-            }
-        }
-    } else {
-        // ------------------------------------------------------------------ epilogue
-        const int quarter = warp & 3; // TMEM lanes [32 * quarter, 32 * quarter + 32) belong to this warp
-        const uint32_t stage = ptx::smem_addr(epi_stage) + (uint32_t)(warp - 2) * 8192u;
-        uint32_t sel = 0;
-        if (lane == 0) ptx::prefetch_tensormap(&tmap_out);
-        int it = 0;
-        for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++it) {
-            const int m_tile = tile % p.num_m_tiles;
-            const int n_tile = tile / p.num_m_tiles;
-            const uint32_t buf = it & 1, acc_phase = (it >> 1) & 1;
-            if (!ptx::mbar_wait(ptx::smem_addr(&acc_full_bar[buf]), acc_phase, p.status, ST_EPI_TIMEOUT)) break;
-            ptx::tc_fence_after();
-            const uint32_t taddr_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * BN;
-            drain_tile<BN>(p, &tmap_out, taddr_row, m_tile * BM + quarter * 32, n_tile * BN, lane, stage, sel);
-
-            // accumulator buffer drained: hand it back to the MMA warp
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(ptx::smem_addr(&acc_empty_bar[buf]));
-        }
-        if (lane == 0) ptx::bulk_wait_group<0>(); // the staging buffers must outlive the stores that read them
-    }
-
-    ptx::tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        ptx::tc_fence_after();
-        ptx::tmem_dealloc(tmem_base, C::TMEM_COLS);
     }
 }
 
@@ -922,11 +767,6 @@ DeviceInfo g_dev[64];
 
 // One-time set-up for the current device: SM count, the device address of the status word,
 // and the opt-in shared-memory sizes of the kernel instantiations.
-template <int BN> bool set_smem_attr() {
-    return cudaFuncSetAttribute(gemm_i8_tcgen05_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                Cfg<BN>::SMEM_BYTES) == cudaSuccess;
-}
-
 const DeviceInfo* device_info() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
@@ -938,7 +778,6 @@ const DeviceInfo* device_info() {
         if (cudaGetSymbolAddress(&addr, g_gemm_status) != cudaSuccess) return nullptr;
         d.status = static_cast<unsigned int*>(addr);
         if (cudaStreamCreateWithFlags(&d.status_stream, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
-        if (!set_smem_attr<256>() || !set_smem_attr<128>() || !set_smem_attr<64>()) return nullptr;
         if (cudaFuncSetAttribute(gemm_i8_tcgen05_pair_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  PairCfg::SMEM_BYTES) != cudaSuccess) return nullptr;
         if (cudaFuncSetAttribute(gemm_i8_tcgen05_pair_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -946,34 +785,6 @@ const DeviceInfo* device_info() {
         d.ready = true;
     }
     return &d;
-}
-
-template <int BN>
-int32_t launch_bn(cudaStream_t stream, const GemmArgs& a, const DeviceInfo& dev) {
-    CUtensorMap ta, tb, tc;
-    if (!make_operand_map(&ta, a.A, a.M, a.K, a.lda, BM)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (A) encode failed");
-    if (!make_operand_map(&tb, a.B, a.N, a.K, a.ldb, BN)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (B) encode failed");
-    if (!make_output_map(&tc, a.out, a.M, a.N, a.ldc, a.mode == EPI_RAW_I32 ? 4 : 2))
-        return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (C) encode failed");
-    KernelParams p{};
-    fill_common(p, a, dev.status);
-    p.num_m_tiles = (int32_t)((a.M + BM - 1) / BM);
-    p.num_n_tiles = (int32_t)((a.N + BN - 1) / BN);
-    const int64_t tiles = (int64_t)p.num_m_tiles * p.num_n_tiles;
-    const int grid = (int)(tiles < dev.sms ? tiles : dev.sms);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid, 1, 1);
-    cfg.blockDim = dim3(NUM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = Cfg<BN>::SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = a.pdl ? 1 : 0;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_i8_tcgen05_kernel<BN>, ta, tb, tc, p);
-    if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "GEMM launch failed: %s", cudaGetErrorString(e));
-    return RC_SUCCESS;
 }
 
 // 256 x 256 tiles on CTA pairs (clusters of two), persistent: one pair per two SMs.
@@ -1069,7 +880,7 @@ int32_t launch_gemm(cudaStream_t stream, const GemmArgs& a) {
     if (a.M > INT32_MAX - BM || a.N > INT32_MAX - 256 || a.K > INT32_MAX - BK)
         return fail(RC_UNSUPPORTED, "GEMM extent beyond 2^31");
 
-    if (a.mode == EPI_SWIGLU_F16 && a.M <= 128) return launch_gemm_decode(stream, a, dev->status, a.pdl);
+    if (a.mode == EPI_SWIGLU_F16 && a.row_absmax_parts != nullptr) return launch_gemm_decode(stream, a, dev->status, a.pdl);
     if (a.mode == EPI_SWIGLU_F16 || a.mode == EPI_PUSH_I32 || a.mode == EPI_GATHER_F16)
         return launch_pair(stream, a, *dev); // the caller checked the shape
 
@@ -1080,11 +891,9 @@ int32_t launch_gemm(cudaStream_t stream, const GemmArgs& a) {
     if (((a.M + 255) / 256) * ((a.N + 255) / 256) >= dev->sms / 2)
         return launch_pair(stream, a, *dev);
 
-    // Tile width: the widest tile that still gives every SM work.
-    const int64_t m_tiles = (a.M + BM - 1) / BM;
-    if (m_tiles * ((a.N + 255) / 256) >= dev->sms) return launch_bn<256>(stream, a, *dev);
-    if (m_tiles * ((a.N + 127) / 128) >= dev->sms) return launch_bn<128>(stream, a, *dev);
-    return launch_bn<64>(stream, a, *dev);
+    // In between: one wave of smaller tiles on single CTAs.  (M333 K4096 N4096, linear: 16.4 us; the same on persistent
+    // 128 x 64 tiles, 192 of them in two waves, 26.4.)
+    return launch_gemm_decode(stream, a, dev->status, a.pdl);
 }
 
 void set_tail_split(int mode) { g_slice_leftover_tiles = mode; }

@@ -213,3 +213,9 @@ def test_dequantize_split3_vector_form(cuda, oracle, M, splits, with_bias):
     rc, want = oracle.dequantize_split3(acc, sm, sn, splits, bias)
     for a, b in zip(outs, want):
         assert np.array_equal(oracle.f16_bits(a.cpu().numpy()), oracle.f16_bits(b))
+
+
+@pytest.mark.parametrize("M,D,K", [(129, 16, 272), (333, 1376, 512), (200, 9344, 144), (1000, 2048, 272), (700, 208, 2064)])
+def test_medium_batch_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K):
+    """The same over several token tiles."""
+    test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K)

@@ -433,3 +433,12 @@ def test_decode_gemm_two_row_parts(cuda, oracle, M, N, K):
     """More weight rows than one tile of 128 per SM: two accumulators per CTA (37904: a second wave of one ragged tile)."""
     test_decode_gemm_all_modes(cuda, oracle, M, N, K)
     test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
+
+
+# Batches between the small-batch and the CTA-pair kernels: several token tiles, the last one ragged; K split over clusters
+# (few rows), one or two row parts, token tiles of 80 .. 128
+@pytest.mark.parametrize("M,N,K", [(129, 16, 16), (333, 4096, 512), (130, 1040, 4096), (255, 1024, 272), (1000, 4096, 272), (192, 18928, 144),
+                                   (385, 9216, 400), (700, 528, 2064), (4700, 256, 400)])
+def test_medium_batch_gemm_all_modes(cuda, oracle, M, N, K):
+    test_decode_gemm_all_modes(cuda, oracle, M, N, K)
+    test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
