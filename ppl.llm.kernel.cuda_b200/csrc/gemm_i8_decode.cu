@@ -686,6 +686,241 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     }
 }
 
+// ---- K folded onto the TMEM lanes ------------------------------------------------------------------
+// When there are fewer than 148 x 64 weight rows, a tile of 128 rows per CTA leaves SMs idle, and splitting K over a
+// cluster costs a distributed-shared-memory exchange (two cluster barriers around the stores).  Here a tile
+// has 128 / F rows and K is cut into F parts instead: part f's weight rows lie on lanes f * 128 / F .. , its
+// activations are MMA columns f * tokens .. , one MMA multiplies all F parts with all F, and the F diagonal blocks hold
+// the partial sums -- the other blocks are computed in the same cycles (up to 64 columns cost the same 53) and never
+// read.  The sums meet in this CTA's own shared memory.  Each CTA reads every activation, so the form pays
+// while they are fewer than the weights (plan_fold).
+template <int BT, int F> struct FCfg {
+    static constexpr int ROWS = BW / F;                 // weight rows per tile
+    static constexpr int W_BYTES = BW * BK;             // one stage: F parts
+    static constexpr int X_BYTES = F * BT * BK;
+    static constexpr int W_STAGES = X_BYTES >= 32 * 1024 ? 4 : X_BYTES <= 4 * 1024 ? 10 : 8; // multiples of the two issuers
+    static constexpr int X_STAGES = X_BYTES >= 16 * 1024 ? 4 : 8;
+    static constexpr int X_RING_OFFSET = W_STAGES * W_BYTES;
+    static constexpr int SMEM_BYTES = X_RING_OFFSET + X_STAGES * X_BYTES + 1024;
+    static constexpr int TMEM_COLS = 2 * F * BT;
+    static constexpr int GROUPS = DCfg<BT>::GROUPS;
+    static constexpr int NUM_THREADS = 128 * GROUPS;
+    static constexpr int GROUP_COLS = BT / GROUPS;
+    static_assert(F * BT <= 256 && SMEM_BYTES <= SMEM_BUDGET && SMEM_BYTES > 114 * 1024, "one CTA per SM");
+    static_assert(GROUP_COLS % 8 == 0 && F * BT * ROWS * 4 <= X_RING_OFFSET, "epilogue");
+};
+
+template <int BT, int F>
+__global__ void __launch_bounds__(FCfg<BT, F>::NUM_THREADS, 1)
+gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const DecodeParams p) {
+    using C = FCfg<BT, F>;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ __align__(8) uint64_t full_w[C::W_STAGES], empty_w[C::W_STAGES];
+    __shared__ __align__(8) uint64_t full_x[C::X_STAGES], empty_x[C::X_STAGES];
+    __shared__ __align__(8) uint64_t acc_full_bar;
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ float token_scale[BT];
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const uint32_t ring = (ptx::smem_addr(smem_raw) + 1023u) & ~1023u;
+    const uint32_t x_ring = ring + C::X_RING_OFFSET;
+    const int row0 = (int)blockIdx.x * p.tile_rows;
+    const unsigned long long t_start = p.stamps ? globaltimer_ns() : 0ull;
+
+    // stage i brings K block f * per_part + i of every part f (past the end of K: zeros); every CTA starts at another i,
+    // so that they do not all ask for the same activation lines at once
+    const int per_part = (p.num_k_blocks + F - 1) / F;
+    const int rot = (int)(blockIdx.x % (unsigned)per_part);
+    auto k_of = [&](int i, int f) { const int j = i + rot >= per_part ? i + rot - per_part : i + rot; return (f * per_part + j) * BK; };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            ptx::prefetch_tensormap(&tmap_w);
+            ptx::prefetch_tensormap(&tmap_x);
+            ptx::mbar_init(ptx::smem_addr(&acc_full_bar), 2);
+        }
+        if (lane < C::W_STAGES) {
+            ptx::mbar_init(ptx::smem_addr(&full_w[lane]), 1);
+            ptx::mbar_init(ptx::smem_addr(&empty_w[lane]), 1);
+        }
+        if (lane < C::X_STAGES) {
+            ptx::mbar_init(ptx::smem_addr(&full_x[lane]), 1);
+            ptx::mbar_init(ptx::smem_addr(&empty_x[lane]), 1);
+        }
+        ptx::fence_mbar_init();
+    }
+    if (warp == 1) {
+        ptx::tmem_alloc(ptx::smem_addr(&tmem_base_slot), C::TMEM_COLS);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem_base = tmem_base_slot;
+    const unsigned long long t_setup = p.stamps ? globaltimer_ns() : 0ull;
+
+    // output column of this thread in the final pass: lane = weight row, warps share rows (ROWS / 32 warps side by side) and tokens
+    constexpr int ROW_WARPS = C::ROWS / 32;
+    const int nl = (warp % ROW_WARPS) * 32 + lane;
+    const int n = row0 + nl;
+    const bool n_ok = nl < p.tile_rows && n < p.N;
+    float sn = 0.0f;
+    half bias_h = __ushort_as_half((unsigned short)0x8000u); // x + (-0.0) == x for every x: no branch for "no bias"
+    auto load_column_constants = [&] {
+        if (p.mode != EPI_RAW_I32 && n_ok) {
+            sn = __half2float(p.scale_n[n]);
+            if (p.bias != nullptr) bias_h = p.bias[n];
+        }
+    };
+    if (p.early_weights) load_column_constants();
+
+    bool ok = true;
+    if (warp == 0 && lane == 0) {
+        // ---- TMA producer of the weight ring (early_weights: as in gemm_i8_decode_kernel)
+        const uint32_t fw0 = ptx::smem_addr(&full_w[0]), ew0 = ptx::smem_addr(&empty_w[0]);
+        if (!p.early_weights) {
+            const int ahead = per_part < 2 * C::W_STAGES ? per_part : 2 * C::W_STAGES;
+            for (int i = 0; i < ahead; ++i)
+#pragma unroll
+                for (int f = 0; f < F; ++f) ptx::tma_prefetch_l2_2d(&tmap_w, k_of(i, f), row0);
+            pdl_wait_prior_grid();
+        }
+        uint32_t sw = 0, pw = 0;
+        for (int i = 0; i < per_part; ++i) {
+            if (i >= C::W_STAGES && !ptx::mbar_wait(ew0 + sw * 8u, pw ^ 1u, p.status, ST_DEC_PRODUCER)) { ok = false; break; }
+            ptx::mbar_arrive_expect_tx(fw0 + sw * 8u, (uint32_t)p.w_box_bytes);
+#pragma unroll
+            for (int f = 0; f < F; ++f)
+                ptx::tma_load_2d(ring + sw * C::W_BYTES + f * C::ROWS * BK, &tmap_w, fw0 + sw * 8u, k_of(i, f), row0);
+            if (++sw == (uint32_t)C::W_STAGES) { sw = 0; pw ^= 1u; }
+        }
+    } else if (warp == 3 && lane == 0) {
+        // ---- TMA producer of the activation ring
+        const uint32_t fx0 = ptx::smem_addr(&full_x[0]), ex0 = ptx::smem_addr(&empty_x[0]);
+        const uint32_t box = (uint32_t)p.tile_tokens * BK;
+        pdl_wait_prior_grid(); // quantized activations are written by the preceding kernel
+        uint32_t sx = 0, px = 0;
+        for (int i = 0; i < per_part; ++i) {
+            if (i >= C::X_STAGES && !ptx::mbar_wait(ex0 + sx * 8u, px ^ 1u, p.status, ST_DEC_PRODUCER)) { ok = false; break; }
+            ptx::mbar_arrive_expect_tx(fx0 + sx * 8u, F * box);
+#pragma unroll
+            for (int f = 0; f < F; ++f) ptx::tma_load_2d(x_ring + sx * C::X_BYTES + f * box, &tmap_x, fx0 + sx * 8u, k_of(i, f), 0);
+            if (++sx == (uint32_t)C::X_STAGES) { sx = 0; px ^= 1u; }
+        }
+    } else if ((warp == 1 || warp == 2) && lane == 0) {
+        // ---- MMA issuers: two threads, alternate stages, an accumulator tile each (see DCfg)
+        const uint32_t idesc = ptx::make_i8_idesc(BW, F * p.tile_tokens);
+        const int me = warp - 1;
+        const uint32_t w_lo0 = ptx::desc_lo_sw128(ring), x_lo0 = ptx::desc_lo_sw128(x_ring);
+        const uint32_t fw0 = ptx::smem_addr(&full_w[0]), ew0 = ptx::smem_addr(&empty_w[0]);
+        const uint32_t fx0 = ptx::smem_addr(&full_x[0]), ex0 = ptx::smem_addr(&empty_x[0]);
+        const uint32_t tmem_d = tmem_base + (uint32_t)me * (F * BT);
+        uint32_t sw = (uint32_t)me, pw = 0, sx = (uint32_t)me, px = 0;
+        bool ready_w = false, ready_x = false;
+        for (int i = me; i < per_part; i += 2) {
+            if (!ready_w && !ptx::mbar_wait(fw0 + sw * 8u, pw, p.status, ST_DEC_MMA)) { ok = false; break; }
+            if (!ready_x && !ptx::mbar_wait(fx0 + sx * 8u, px, p.status, ST_DEC_MMA)) { ok = false; break; }
+            ptx::tc_fence_after();
+            uint32_t nsw = sw + 2u, npw = pw, nsx = sx + 2u, npx = px;
+            if (nsw >= (uint32_t)C::W_STAGES) { nsw -= (uint32_t)C::W_STAGES; npw ^= 1u; }
+            if (nsx >= (uint32_t)C::X_STAGES) { nsx -= (uint32_t)C::X_STAGES; npx ^= 1u; }
+            ready_w = ptx::mbar_try_wait(fw0 + nsw * 8u, npw);
+            ready_x = ptx::mbar_try_wait(fx0 + nsx * 8u, npx);
+            const uint32_t w_lo = w_lo0 + sw * (uint32_t)(C::W_BYTES >> 4), x_lo = x_lo0 + sx * (uint32_t)(C::X_BYTES >> 4);
+            const uint32_t accumulate = i != me ? 1u : 0u;
+#pragma unroll
+            for (uint32_t k = 0; k < BK / UMMA_K; ++k)
+                ptx::mma_i8(tmem_d, ptx::desc_from_lo(w_lo + 2u * k), ptx::desc_from_lo(x_lo + 2u * k), idesc, k != 0 ? 1u : accumulate);
+            ptx::mma_commit(ew0 + sw * 8u);
+            ptx::mma_commit(ex0 + sx * 8u);
+            sw = nsw; pw = npw; sx = nsx; px = npx;
+        }
+        if (me < per_part) { if (ok) ptx::mma_commit(ptx::smem_addr(&acc_full_bar)); }
+        else ptx::mbar_arrive(ptx::smem_addr(&acc_full_bar));
+    }
+    (void)ok;
+    __syncwarp();
+    pdl_wait_prior_grid(); // every thread: scale_m / row_absmax come from the preceding kernel too
+    if (!p.early_weights) load_column_constants();
+    if (p.mode != EPI_RAW_I32) {
+        for (int m = threadIdx.x; m < BT; m += C::NUM_THREADS)
+            token_scale[m] = m < p.M ? __fmul_rn(__half2float(p.scale_m[m]), p.down_m) : 0.0f;
+    }
+
+    const bool acc_ready = ptx::mbar_wait(ptx::smem_addr(&acc_full_bar), 0, p.status, ST_DEC_EPI);
+    ptx::tc_fence_after();
+    pdl_launch_dependents();
+    const unsigned long long t_main = p.stamps ? globaltimer_ns() : 0ull;
+
+    // ---- the diagonal blocks, [part][token][row], into the dead weight ring
+    {
+        const int q = warp & 3, grp = warp >> 2;         // TMEM lane quarter, slice of the tokens
+        const int f = q / ROW_WARPS, row = (q % ROW_WARPS) * 32 + lane;
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(f * p.tile_tokens);
+        const uint32_t dst = ring + (uint32_t)(f * BT * C::ROWS + row) * 4u;
+#pragma unroll 1
+        for (int c0 = grp * C::GROUP_COLS; c0 < (grp + 1) * C::GROUP_COLS; c0 += 8) {
+            if (c0 >= p.M) break;
+            uint32_t v[8];
+            if (acc_ready) {
+                tmem_ld_sum<8, 2, F * BT>(taddr + c0, v, per_part < 2 ? per_part : 2);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = 0u;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (uint32_t)((c0 + j) * C::ROWS) * 4u), "r"(v[j]) : "memory");
+        }
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    const unsigned long long t_exchange = p.stamps ? globaltimer_ns() : 0ull;
+
+    // ---- sums and epilogue: a warp handles 32 rows of one token at a time
+    const uint32_t src = ring + (uint32_t)nl * 4u;
+#pragma unroll 4
+    for (int m = warp / ROW_WARPS; m < p.M; m += (C::NUM_THREADS / 32) / ROW_WARPS) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+            uint32_t t;
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(t) : "r"(src + (uint32_t)((f * BT + m) * C::ROWS) * 4u) : "memory");
+            v += t;
+        }
+        if (p.mode == EPI_RAW_I32) {
+            if (n_ok) {
+                int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)m * p.ldc + n;
+                if (p.raw_affine) {
+                    v = (uint32_t)p.raw_alpha * v + (p.raw_bias != nullptr ? (uint32_t)p.raw_bias[n] : 0u);
+                    if (p.raw_beta != 0) v += (uint32_t)p.raw_beta * (uint32_t)*dst;
+                }
+                *dst = (int32_t)v;
+            }
+            continue;
+        }
+        float t = __fmul_rn((float)(int32_t)v, sn);
+        t = __fmul_rn(t, p.down_n);
+        t = __fmul_rn(t, token_scale[m]);
+        const half h = __hadd(__float2half_rn(t), bias_h);
+        if (n_ok) reinterpret_cast<half*>(p.out)[(int64_t)m * p.ldc + n] = h;
+        if (p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
+            const float a = n_ok ? fabsf(__half2float(h)) : 0.0f;
+            const uint32_t bits = __reduce_max_sync(0xffffffffu, a == a ? __float_as_uint(a) : 0u); // NaNs are dropped, as fmax does
+            if (lane == 0 && bits != 0u) atomicMax(p.row_absmax_bits + m, bits);
+        }
+    }
+    if (warp == 1) {
+        __syncwarp();
+        ptx::tc_fence_after();
+        ptx::tmem_dealloc(tmem_base, C::TMEM_COLS);
+    }
+    if (p.stamps && threadIdx.x == 0) {
+        unsigned long long* st = p.stamps + (size_t)(blockIdx.x < 296u ? blockIdx.x : 295u) * 8;
+        st[0] = t_start; st[1] = t_setup; st[2] = t_main; st[3] = t_exchange; st[4] = globaltimer_ns();
+    }
+}
+
 // ---- host side ---------------------------------------------------------------------------------
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -759,6 +994,10 @@ template <int BT> bool set_attr(int* max_clusters) {
     return true;
 }
 
+template <int BT, int F> bool set_fold_attr() {
+    return cudaFuncSetAttribute(gemm_i8_fold_kernel<BT, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, FCfg<BT, F>::SMEM_BYTES) == cudaSuccess;
+}
+
 const DecDeviceInfo* dec_device_info() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
@@ -768,6 +1007,9 @@ const DecDeviceInfo* dec_device_info() {
         if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return nullptr;
         if (!set_attr<16>(d.max_clusters[0]) || !set_attr<32>(d.max_clusters[1]) || !set_attr<64>(d.max_clusters[2]) ||
             !set_attr<128>(d.max_clusters[3]))
+            return nullptr;
+        if (!set_fold_attr<16, 2>() || !set_fold_attr<16, 4>() || !set_fold_attr<32, 2>() || !set_fold_attr<32, 4>() ||
+            !set_fold_attr<64, 2>() || !set_fold_attr<64, 4>() || !set_fold_attr<128, 2>())
             return nullptr;
         d.ready = true;
     }
@@ -847,11 +1089,8 @@ DecodePlan plan_medium(const DecDeviceInfo& dev, int64_t M, int64_t columns, int
     return best;
 }
 
-template <int BT>
-int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecodePlan& plan, unsigned int* status, bool pdl) {
-    CUtensorMap tw, tx;
-    if (!make_map(&tx, a.A, a.M, a.K, a.lda, plan.tokens)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (X) encode failed");
-    DecodeParams p;
+DecodeParams make_params(const GemmArgs& a, unsigned int* status) {
+    DecodeParams p = {};
     p.M = (int32_t)a.M; p.N = (int32_t)a.N;
     p.num_k_blocks = (int32_t)((a.K + BK - 1) / BK);
     p.mode = a.mode;
@@ -862,10 +1101,61 @@ int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecodePlan& plan
     p.status = status;
     p.raw_alpha = a.raw_alpha; p.raw_beta = a.raw_beta; p.raw_bias = a.raw_bias;
     p.raw_affine = (a.raw_alpha != 1 || a.raw_beta != 0 || a.raw_bias != nullptr) ? 1 : 0;
+    p.beta = a.beta;
+    p.early_weights = a.after_quantizer ? 1 : 0;
+    p.stamps = stall_counters();
+    return p;
+}
 
+// Parts K is folded into (see gemm_i8_fold_kernel), 0 = not folded.  Both forms are modelled in SM cycles per CTA: a stage costs
+// the larger of its operands' way from L2 (60 bytes per cycle) and the issuing threads' bookkeeping (390), all weights come
+// from HBM at 3400, and sharing K inside a cluster adds 2500 and 80 per token up to 6500 (exchange and scattered stores;
+// measured 1.7 us at 16 tokens, 3.1 at 37, 3.6 at 96).  Folded, a CTA reads all of K for every token; `split` is the alternative.
+int plan_fold(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t K, const DecodePlan& split) {
+    if (split.S == 1 || split.dual) return 0; // every SM has a tile of its own already
+    const int F = columns <= dev.sms * (BW / 4) && split.tokens <= 64 ? 4 : 2;
+    if (columns > dev.sms * (BW / F)) return 0;
+    const int64_t kb = (K + BK - 1) / BK;
+    auto loop = [&](int64_t stages, double bytes) { return (double)stages * (bytes / 60.0 > 390.0 ? bytes / 60.0 : 390.0); };
+    const double hbm = (double)columns * K / 3400.0;
+    const double folded = loop((kb + F - 1) / F, (double)F * (rows_for(columns, dev.sms, BW / F) + M) * BK);
+    const double shared = loop((kb + split.S - 1) / split.S, (double)(split.rows + M) * BK);
+    const double exchange = 2500.0 + 80.0 * M < 6500.0 ? 2500.0 + 80.0 * M : 6500.0;
+    return (folded > hbm ? folded : hbm) < (shared > hbm ? shared : hbm) + exchange ? F : 0;
+}
+
+template <int BT, int F>
+int32_t launch_fold(cudaStream_t stream, const GemmArgs& a, const DecDeviceInfo& dev, unsigned int* status, bool pdl) {
+    using C = FCfg<BT, F>;
+    CUtensorMap tw, tx;
+    DecodeParams p = make_params(a, status);
+    p.tile_tokens = (int32_t)((a.M + 15) / 16 * 16);
+    p.tile_rows = rows_for(a.N, dev.sms, C::ROWS);
+    p.w_box_bytes = F * p.tile_rows * BK;
+    if (!make_map(&tx, a.A, a.M, a.K, a.lda, p.tile_tokens)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (X) encode failed");
+    if (!make_map(&tw, a.B, a.N, a.K, a.ldb, p.tile_rows)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (W) encode failed");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((a.N + p.tile_rows - 1) / p.tile_rows), 1, 1);
+    cfg.blockDim = dim3(C::NUM_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = C::SMEM_BYTES;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_i8_fold_kernel<BT, F>, tw, tx, p);
+    if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "folded GEMM launch failed: %s", cudaGetErrorString(e));
+    return RC_SUCCESS;
+}
+
+template <int BT>
+int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecodePlan& plan, unsigned int* status, bool pdl) {
+    CUtensorMap tw, tx;
+    if (!make_map(&tx, a.A, a.M, a.K, a.lda, plan.tokens)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (X) encode failed");
+    DecodeParams p = make_params(a, status);
     const bool swiglu = a.mode == EPI_SWIGLU_F16;
     if (swiglu) p.N = (int32_t)(a.N / 2); // the x half and the gate half of the weight rows share the output columns
-    p.beta = a.beta;
     const int S = plan.S, tile_rows = plan.rows;
     const bool dual = plan.dual;
     const int parts_out = dual && !swiglu ? 2 : 1;
@@ -877,8 +1167,6 @@ int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecodePlan& plan
     p.w_stages = (dual ? DCfg<BT>::template x_ring_offset<true>() : DCfg<BT>::template x_ring_offset<false>()) / p.w_slot_bytes;
     if (p.w_stages > MAX_W_STAGES) p.w_stages = MAX_W_STAGES;
     p.w_stages -= p.w_stages % DCfg<BT>::NACC; // see X_STAGES
-    p.stamps = stall_counters();
-    p.early_weights = a.after_quantizer ? 1 : 0;
 
     if (a.row_absmax_parts) *a.row_absmax_parts = plan.row_tiles * S;
     if (!make_map(&tw, a.B, a.N, a.K, a.ldb, tile_rows)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (W) encode failed");
@@ -926,6 +1214,15 @@ int32_t launch_gemm_decode(cudaStream_t stream, const GemmArgs& a, unsigned int*
     if (a.M > 128) return launch_bt<128>(stream, a, plan_medium(*dev, a.M, columns, num_k_blocks, swiglu), status, pdl);
     const int variant = a.M <= 16 ? 0 : a.M <= 32 ? 1 : a.M <= 64 ? 2 : 3;
     const DecodePlan plan = plan_small(*dev, variant, a.M, columns, num_k_blocks, swiglu);
+    const int fold = swiglu ? 0 : plan_fold(*dev, a.M, columns, a.K, plan);
+    if (fold == 4) {
+        return variant == 0 ? launch_fold<16, 4>(stream, a, *dev, status, pdl)
+             : variant == 1 ? launch_fold<32, 4>(stream, a, *dev, status, pdl) : launch_fold<64, 4>(stream, a, *dev, status, pdl);
+    }
+    if (fold == 2) {
+        return variant == 0 ? launch_fold<16, 2>(stream, a, *dev, status, pdl) : variant == 1 ? launch_fold<32, 2>(stream, a, *dev, status, pdl)
+             : variant == 2 ? launch_fold<64, 2>(stream, a, *dev, status, pdl) : launch_fold<128, 2>(stream, a, *dev, status, pdl);
+    }
     switch (variant) {
     case 0: return launch_bt<16>(stream, a, plan, status, pdl);
     case 1: return launch_bt<32>(stream, a, plan, status, pdl);

@@ -442,3 +442,14 @@ def test_decode_gemm_two_row_parts(cuda, oracle, M, N, K):
 def test_medium_batch_gemm_all_modes(cuda, oracle, M, N, K):
     test_decode_gemm_all_modes(cuda, oracle, M, N, K)
     test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
+
+
+# K folded onto the TMEM lanes in four and two parts: one to 64 (128) tokens, K of a fraction of a block and of one block per
+# part, ragged last tiles, more stages than the rings hold
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (16, 896, 16), (17, 4736, 144), (37, 4096, 11008), (64, 1040, 1024), (33, 4744, 528),
+                                   (48, 9472, 384), (96, 8192, 1024), (128, 5120, 272), (65, 7168, 2064)])
+def test_folded_gemm_all_modes(cuda, oracle, M, N, K):
+    if N % 16 == 0:
+        test_decode_gemm_all_modes(cuda, oracle, M, N, K)
+    test_gemm_i32_alpha_beta_bias(cuda, M, N, K, 1, 0, False)
+    test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
