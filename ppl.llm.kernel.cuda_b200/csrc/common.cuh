@@ -112,10 +112,11 @@ __host__ __device__ inline int64_t layout_offset(int32_t layout, int64_t rows, i
 
 // given_absmax_bits != null: rows are quantized with that precomputed max |x| (float bits) instead of
 // scanning the row, the maximum of given_parts values per row.  zero_absmax_bits != null: the kernel also clears that per-row array (for the
-// GEMM that follows).  pdl: launch as a programmatic dependent of the preceding kernel in the stream.
+// GEMM that follows).  pdl: launch as a programmatic dependent of the preceding kernel in the stream.  late_trigger: let the
+// dependent start only when everything before this kernel has completed.
 int32_t launch_quantize(cudaStream_t stream, const half* in, int64_t batch, int64_t dim, float up_scale,
                         int32_t layout, int8_t* q, half* scale, const uint32_t* given_absmax_bits,
-                        uint32_t* zero_absmax_bits = nullptr, bool pdl = false, int32_t given_parts = 1);
+                        uint32_t* zero_absmax_bits = nullptr, bool pdl = false, int32_t given_parts = 1, bool late_trigger = false);
 
 int32_t launch_dequantize(cudaStream_t stream, const int32_t* acc, const half* bias, const half* scale_m,
                           const half* scale_n, int64_t batch, int64_t dim, float down_m, float down_n,
@@ -153,8 +154,9 @@ struct GemmArgs {
     void* out; int64_t ldc;
     uint32_t* row_absmax_bits; // mode 2: per-row max |y| as float bits, zeroed by the launcher
     bool pdl = false;          // launch as a programmatic dependent of the preceding kernel
-    // The preceding kernel is the quantizer that the same call of the fused linear has just enqueued: it does not write
-    // the weights, and above 128 tokens it is an ordinary launch, so nothing before it still uses the scratch.
+    // The preceding kernel is the quantizer that the same call of the fused linear has just enqueued, with a late trigger
+    // (gemm_preloads_weights): whatever wrote the weights or used the K-slice scratch before that call has completed when
+    // this kernel starts.
     bool after_quantizer = false;
     float beta = 1.0f;         // EPI_SWIGLU_F16
     // EPI_SWIGLU_F16, M <= 128: the row maxima are written as *row_absmax_parts partial maxima per row, [M][parts] (at
@@ -185,6 +187,11 @@ constexpr int64_t kSkTileBytes = 256 * 256 * 4;
 constexpr int64_t kSkStateBytes = 2048;
 constexpr int64_t kSkWsBytes = kSkStateBytes + kSkMaxTiles * kSkTileBytes;
 static_assert(kSkMaxTiles * 8 * 4 <= kSkStateBytes, "arrival counters");
+// The quantizer of the fused linear lets the GEMM start at once -- the GEMM then waits before it loads weights, and brings them
+// into L2 until then -- or, where this is true, once everything before the call has completed, so that the GEMM fills its
+// weight ring while the quantizer runs.  That pays where the way from L2 into the SMs is what the GEMM is bound by: more than
+// 128 tokens (333 x 4096 x 4096: 15.8 against 18.4 us), and K shared by a cluster (48 x 11008 x 1024: 14.0 against 15.4 us).
+bool gemm_preloads_weights(int64_t M, int64_t N, int64_t K);
 int32_t launch_gemm_decode(cudaStream_t stream, const GemmArgs& a, unsigned int* status, bool pdl);
 int32_t launch_gemm(cudaStream_t stream, const GemmArgs& a);
 int32_t gemm_status(int32_t reset);

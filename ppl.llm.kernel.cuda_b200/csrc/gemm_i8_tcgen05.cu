@@ -675,8 +675,8 @@ gemm_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
     }
 }
 
-// Clears the K-slice scratch.  In the fused linear it is launched as a programmatic dependent of the quantizer, which is
-// an ordinary launch: nothing that came before still uses the scratch, so it is cleared under the quantizer's last wave
+// Clears the K-slice scratch.  In the fused linear it is launched as a programmatic dependent of the quantizer, which has
+// waited for everything before it: nothing still uses the scratch, so it is cleared under the quantizer's last wave
 // (idle) -- but the kernel only EXITS after the quantizer has completed (the wait below), because the GEMM, its own
 // programmatic dependent, takes the completion of this grid as its licence to read the quantizer's output.  Behind any
 // other kernel, which may itself have started before an earlier user of the scratch ended, it waits first.

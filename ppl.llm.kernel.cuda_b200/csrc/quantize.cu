@@ -21,7 +21,7 @@ template <int UNITS, bool GIVEN>
 __global__ void __launch_bounds__(QTPB, UNITS <= 2 ? 5 : 1)
 quantize_rows_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, float up_scale, int32_t layout,
                      int8_t* __restrict__ q, half* __restrict__ scale_out, const uint32_t* __restrict__ given_absmax_bits,
-                     uint32_t* __restrict__ zero_absmax_bits, int32_t given_parts) {
+                     uint32_t* __restrict__ zero_absmax_bits, int32_t given_parts, bool late_trigger) {
     __shared__ float red[QTPB / 32];
     const int64_t row = blockIdx.x;
     const int units = (int)(dim >> 4);
@@ -29,8 +29,11 @@ quantize_rows_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, fl
     // With a precomputed row maximum the row may be split over blockIdx.y; otherwise gridDim.y == 1.
     const int unit_base = blockIdx.y * blockDim.x * UNITS;
 
-    pdl_launch_dependents(); // a dependent kernel may start its own preamble now
-    pdl_wait_prior_grid();   // no-op unless launched as a programmatic dependent
+    // A dependent kernel may start its own preamble now; late_trigger: once everything before this grid has completed, so that
+    // it may also use what none of this call's own launches writes
+    if (!late_trigger) pdl_launch_dependents();
+    pdl_wait_prior_grid(); // no-op unless launched as a programmatic dependent
+    if (late_trigger) pdl_launch_dependents();
 
     uint4 v[UNITS][2];
 #pragma unroll
@@ -85,10 +88,11 @@ quantize_rows_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, fl
 __global__ void __launch_bounds__(QTPB)
 quantize_rows_twopass_kernel(const half* __restrict__ in, int64_t batch, int64_t dim, float up_scale, int32_t layout,
                              int8_t* __restrict__ q, half* __restrict__ scale_out,
-                             const uint32_t* __restrict__ given_absmax_bits, uint32_t* __restrict__ zero_absmax_bits, int32_t given_parts) {
+                             const uint32_t* __restrict__ given_absmax_bits, uint32_t* __restrict__ zero_absmax_bits, int32_t given_parts, bool late_trigger) {
     __shared__ float red[QTPB / 32];
-    pdl_launch_dependents();
+    if (!late_trigger) pdl_launch_dependents();
     pdl_wait_prior_grid();
+    if (late_trigger) pdl_launch_dependents();
     const int64_t row = blockIdx.x;
     const int64_t units = dim >> 4;
     const uint4* src = reinterpret_cast<const uint4*>(in + row * dim);
@@ -222,7 +226,7 @@ int grid_for(int64_t work_items, int tpb) {
 
 int32_t launch_quantize(cudaStream_t stream, const half* in, int64_t batch, int64_t dim, float up_scale,
                         int32_t layout, int8_t* q, half* scale, const uint32_t* given_absmax_bits,
-                        uint32_t* zero_absmax_bits, bool pdl, int32_t given_parts) {
+                        uint32_t* zero_absmax_bits, bool pdl, int32_t given_parts, bool late_trigger) {
     if (batch == 0 || dim == 0) return RC_SUCCESS;
     const int64_t units = dim >> 4;
     cudaError_t e;
@@ -232,7 +236,7 @@ int32_t launch_quantize(cudaStream_t stream, const half* in, int64_t batch, int6
         int threads = (int)(units < QTPB ? (units + 31) / 32 * 32 : QTPB);
         const dim3 grid((unsigned)batch, (unsigned)((units + threads - 1) / threads), 1);
         e = launch_ex(quantize_rows_kernel<1, true>, grid, dim3(threads), stream, pdl, in, batch, dim, up_scale, layout, q, scale,
-                      given_absmax_bits, zero_absmax_bits, given_parts);
+                      given_absmax_bits, zero_absmax_bits, given_parts, late_trigger);
     } else if (units <= QTPB * 8) {
         // threads: enough to give every thread the same small number of units
         int per = (int)((units + QTPB - 1) / QTPB);
@@ -245,14 +249,14 @@ int32_t launch_quantize(cudaStream_t stream, const half* in, int64_t batch, int6
         if (threads > QTPB) threads = QTPB;
         const dim3 grid((unsigned)batch, 1, 1), block(threads);
         switch (bucket) {
-        case 1: e = launch_ex(quantize_rows_kernel<1, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
-        case 2: e = launch_ex(quantize_rows_kernel<2, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
-        case 4: e = launch_ex(quantize_rows_kernel<4, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
-        default: e = launch_ex(quantize_rows_kernel<8, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts); break;
+        case 1: e = launch_ex(quantize_rows_kernel<1, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts, late_trigger); break;
+        case 2: e = launch_ex(quantize_rows_kernel<2, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts, late_trigger); break;
+        case 4: e = launch_ex(quantize_rows_kernel<4, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts, late_trigger); break;
+        default: e = launch_ex(quantize_rows_kernel<8, false>, grid, block, stream, pdl, in, batch, dim, up_scale, layout, q, scale, given_absmax_bits, zero_absmax_bits, given_parts, late_trigger); break;
         }
     } else {
         e = launch_ex(quantize_rows_twopass_kernel, dim3((unsigned)batch), dim3(QTPB), stream, pdl, in, batch, dim, up_scale, layout, q, scale,
-                      given_absmax_bits, zero_absmax_bits, given_parts);
+                      given_absmax_bits, zero_absmax_bits, given_parts, late_trigger);
     }
     if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "quantize launch failed: %s", cudaGetErrorString(e));
     return RC_SUCCESS;

@@ -169,3 +169,70 @@ def test_linear_on_host_buffers_matches_device_path(cuda, oracle, M, K, N, chunk
 def test_linear_on_host_buffers_below_two_chunks(cuda, oracle, M, K, N, chunk, requant):
     """Short first and last chunks inside the two staging buffers, which together hold the whole batch."""
     test_linear_on_host_buffers_matches_device_path(cuda, oracle, M, K, N, chunk, requant)
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 2048, 2048), (16, 1024, 12288), (37, 4096, 1024), (128, 1024, 4096), (300, 1024, 2048), (2400, 512, 2048)])
+def test_linear_sees_weights_written_right_before(cuda, M, K, N):
+    """The fused linear's launches overlap their predecessors: weights that the quantizer writes right before the call, round
+    after round into the same buffer, are the ones that are used."""
+    import pplb200
+    g = cuda.Generator(device="cuda").manual_seed(M + N + K)
+    x = cuda.randn((M, K), generator=g, device="cuda").half()
+    ws = [cuda.randn((N, K), generator=g, device="cuda").half() for _ in range(8)]
+    wq, sn = cuda.zeros((N, K), dtype=cuda.int8, device="cuda"), cuda.zeros((N,), dtype=cuda.float16, device="cuda")
+    lin = pplb200.W8A8Linear(wq, sn, None, max_tokens=M)
+    got = []
+    for w in ws:
+        pplb200.minmax_quantize_fp16(w, up_scale=pplb200.HIDDEN_UP_SCALE, out=wq, scale=sn)
+        got.append(lin(x).clone())
+    cuda.cuda.synchronize()
+    assert pplb200.gemm_status() == 0
+    q, s = pplb200.minmax_quantize_fp16(x)
+    for w, y in zip(ws, got):
+        p, t = pplb200.minmax_quantize_fp16(w, up_scale=pplb200.HIDDEN_UP_SCALE)
+        want = pplb200.minmax_dequantize_fp16((q.double() @ p.double().T).to(cuda.int32), s, t)  # int32 sums are exact in fp64
+        assert cuda.equal(y.view(cuda.int16), want.view(cuda.int16))
+
+
+@pytest.mark.parametrize("M,K,N", [(16, 1024, 2048), (300, 512, 1024)])
+def test_capture_with_joined_streams(cuda, M, K, N):
+    """A captured graph in which a call depends on kernels of two streams (one of them this library's, the other not) and on a
+    copy: replayed with new inputs, the result is that of the eager call."""
+    import pplb200
+    g = cuda.Generator(device="cuda").manual_seed(5)
+    wq = cuda.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=cuda.int8)
+    sn = (cuda.rand((N,), generator=g, device="cuda") * 8).half()
+    lin, lin2 = (pplb200.W8A8Linear(wq, sn, None, max_tokens=M) for _ in range(2))
+    a, b, c = (cuda.zeros((M, K), dtype=cuda.float16, device="cuda") for _ in range(3))
+    side = cuda.cuda.Stream()
+
+    def step():
+        cur = cuda.cuda.current_stream()
+        side.wait_stream(cur)
+        with cuda.cuda.stream(side):
+            b.copy_(a * 2)              # a kernel and a copy on the other stream
+            q, s = pplb200.minmax_quantize_fp16(b)
+        y = lin(a)                      # this library's kernels on this one
+        cur.wait_stream(side)
+        z = pplb200.row_parallel_linear(q, wq, s, sn, None, K, N)  # depends on both
+        c.copy_(b)
+        return y, z, lin2(c)            # behind a copy
+
+    warm = cuda.cuda.Stream()
+    warm.wait_stream(cuda.cuda.current_stream())
+    with cuda.cuda.stream(warm):
+        step()
+    cuda.cuda.current_stream().wait_stream(warm)
+    graph = cuda.cuda.CUDAGraph()
+    with cuda.cuda.graph(graph):
+        out = step()
+    for i in range(3):
+        a.copy_(cuda.randn((M, K), generator=g, device="cuda").half())
+        graph.replay()
+        got = [t.clone() for t in out]
+        cuda.cuda.synchronize()
+        want = [lin(a).clone(), lin((a * 2).contiguous()).clone()]
+        assert cuda.equal(got[0].view(cuda.int16), want[0].view(cuda.int16))
+        assert cuda.equal(got[1].view(cuda.int16), want[1].view(cuda.int16))
+        assert cuda.equal(got[2].view(cuda.int16), want[1].view(cuda.int16))
+    assert pplb200.gemm_status() == 0
