@@ -343,8 +343,8 @@ gemm_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
     const uint32_t tmem_base = tmem_base_slot;
     // Launched as a programmatic dependent (fused linear), everything above ran under the tail of the preceding
     // kernel; its results (quantized activations, row scales, cleared scratch) are needed from here on.  Every
-    // thread waits: all of them read such data.  A no-op in an ordinary launch.
-    pdl_launch_dependents(); // every CTA is resident: a dependent kernel may set itself up under this one
+    // thread waits: all of them read such data.  A no-op in an ordinary launch.  Dependents are not released before this
+    // grid ends: with the next kernel's CTAs already waiting on the SMs 3000 x 8192 x 4096 took 105 us instead of 100.
     pdl_wait_prior_grid();
 
     const int num_pairs = (int)(gridDim.x >> 1);
