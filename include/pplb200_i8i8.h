@@ -119,8 +119,9 @@ int32_t pplb200_i8i8_minmax_requantize_swiglu_fp16(pplb200_stream_t stream, cons
  * input int8 [M, K] (row stride lda); weight int8 [2 * act_dim, K] = [x rows | gate rows];
  * scale_N fp16 [2 * act_dim]; activated fp16 [M, act_dim] (the reference's `workspace`);
  * out_q int8 [M, act_dim]; out_q_scale fp16 [M].  ws: pplb200_i8i8_gate_up_swiglu_workspace_bytes().
- * Shapes that cannot use the fused kernel (M <= 128, act_dim % 128 != 0, too few tiles) run the two
- * steps separately inside this call (the workspace size accounts for the int32 buffer).
+ * Two kernels do this, one for large batches (act_dim % 128 == 0) and one for few tiles; large batches with another
+ * act_dim run the two steps separately inside this call.  The workspace size accounts for the int32 buffer, or for the
+ * partial row maxima that take its place.
  */
 int64_t pplb200_i8i8_gate_up_swiglu_workspace_bytes(int64_t M, int64_t act_dim, int64_t K);
 int32_t pplb200_i8i8_gate_up_swiglu_requant(pplb200_stream_t stream, const void* input, int64_t lda, const void* weight,
@@ -227,7 +228,7 @@ int32_t pplb200_i8i8_linear_fp16_args(pplb200_stream_t stream, const pplb200_lin
  * three streams at once (the two copy streams and their events are created per device at the first call, which
  * therefore should come before any stream capture), so a large batch costs little more than its slower copy
  * direction; with chunks of 1024 tokens or more the first chunk goes in as chunk_rows / 8, / 8, / 4 and / 2 tokens, so
- * that the copy out, usually the longest of the three, starts early.  Chunking is exact: the per-token quantizer and
+ * that the copy out, usually the longest of the three, starts early; a batch below two chunks is cut finer than chunk_rows.  Chunking is exact: the per-token quantizer and
  * the epilogue work row by row.  `ws` is DEVICE memory of
  * pplb200_i8i8_linear_host_workspace_bytes (two sets of staging buffers); weights, scales and bias are device
  * pointers as in pplb200_i8i8_linear_fp16.  Work enqueued on `stream` after the call runs after the last copy out.
