@@ -1133,7 +1133,7 @@ DecodeParams make_params(const GemmArgs& a, unsigned int* status) {
 }
 
 // Parts K is folded into (see gemm_i8_fold_kernel), 0 = not folded.  Both forms are modelled in SM cycles per CTA: a stage costs
-// the larger of its operands' way from L2 (60 bytes per cycle) and the issuing threads' bookkeeping (390), all weights come
+// the larger of its operands' way from L2 (60 bytes per cycle) and the issuing threads' bookkeeping (390; 450 with F boxes each), all weights come
 // from HBM at 3400, and sharing K inside a cluster adds 2500 and 80 per token up to 6500 (exchange and scattered stores;
 // measured 1.7 us at 16 tokens, 3.1 at 37, 3.6 at 96).  Folded, a CTA reads all of K for every token; `split` is the alternative.
 int plan_fold(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t K, const DecodePlan& split) {
@@ -1141,10 +1141,10 @@ int plan_fold(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t K, c
     const int F = columns <= dev.sms * (BW / 4) && split.tokens <= 64 ? 4 : 2;
     if (columns > dev.sms * (BW / F)) return 0;
     const int64_t kb = (K + BK - 1) / BK;
-    auto loop = [&](int64_t stages, double bytes) { return (double)stages * (bytes / 60.0 > 390.0 ? bytes / 60.0 : 390.0); };
+    auto loop = [&](int64_t stages, double bytes, double issue) { return (double)stages * (bytes / 60.0 > issue ? bytes / 60.0 : issue); };
     const double hbm = (double)columns * K / 3400.0;
-    const double folded = loop((kb + F - 1) / F, (double)F * (rows_for(columns, dev.sms, BW / F) + M) * BK);
-    const double shared = loop((kb + split.S - 1) / split.S, (double)(split.rows + M) * BK);
+    const double folded = loop((kb + F - 1) / F, (double)F * (rows_for(columns, dev.sms, BW / F) + M) * BK, 450.0);
+    const double shared = loop((kb + split.S - 1) / split.S, (double)(split.rows + M) * BK, 390.0);
     const double exchange = 2500.0 + 80.0 * M < 6500.0 ? 2500.0 + 80.0 * M : 6500.0;
     return (folded > hbm ? folded : hbm) < (shared > hbm ? shared : hbm) + exchange ? F : 0;
 }
