@@ -148,6 +148,11 @@ template <int BN>
 __device__ __forceinline__ void drain_tile(const KernelParams& p, const CUtensorMap* tmap_out, uint32_t taddr_row,
                                            int row0, int n_base, int lane, uint32_t stage, uint32_t& sel,
                                            const int32_t* sums = nullptr) {
+    // Warps whose rows all lie past the last token leave at once.  Filling the staging buffers without handing them to the TMA
+    // unit is not an option: the waits below count committed stores (at most one of them may still be reading its buffer), so
+    // a slab that commits nothing lets the next but one be written into a buffer that the previous tile's last store still
+    // reads -- a wrong product in the last 32 columns of such a tile where the next tile is ready at once (behind a K slice, or with a short K).
+    if (row0 >= p.M) return;
     const int row = row0 + lane;
     const bool row_ok = row < p.M;
     const uint32_t my_row = (uint32_t)lane * 128u, sw = (uint32_t)(lane & 7);
@@ -182,7 +187,7 @@ __device__ __forceinline__ void drain_tile(const KernelParams& p, const CUtensor
                 ptx::st_shared_v4(buf + my_row + (((uint32_t)j ^ sw) << 4), make_uint4(acc[4 * j], acc[4 * j + 1], acc[4 * j + 2], acc[4 * j + 3]));
             ptx::fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0 && row0 < p.M) {
+            if (lane == 0) {
                 ptx::tma_store_2d(tmap_out, buf, n0, row0);
                 ptx::bulk_commit_group();
             }
@@ -217,7 +222,7 @@ __device__ __forceinline__ void drain_tile(const KernelParams& p, const CUtensor
         }
         ptx::fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0 && row0 < p.M) {
+        if (lane == 0) {
             ptx::tma_store_2d(tmap_out, buf, n0, row0);
             ptx::bulk_commit_group();
         }

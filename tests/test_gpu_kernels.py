@@ -336,6 +336,75 @@ def test_gemm_random_shapes(cuda):
         assert torch.equal(c, _exact_gemm(torch, a, b)), (M, N, K)
 
 
+def _differing_tiles(torch, got, want):
+    """{(256-row tile, 256-column tile): (elements that differ, largest difference)}"""
+    r, c = (got != want).nonzero(as_tuple=True)
+    tiles = {}
+    for i, j in sorted(set(zip((r // 256).tolist(), (c // 256).tolist()))):
+        d = (got[256 * i:256 * i + 256, 256 * j:256 * j + 256].double() - want[256 * i:256 * i + 256, 256 * j:256 * j + 256].double()).abs()
+        tiles[(i, j)] = (int((d != 0).sum()), float(d.max()))
+    return tiles
+
+
+# A tile whose rows end before a warp's 32 follows one that is stored in full: right behind a K slice (the first two: 6 leftover
+# tiles in 8 slices), with a short K (the epilogue is behind the main loop all the time), odd and even numbers of 32- and 64-column slabs
+@pytest.mark.parametrize("M,N,K", [(1625, 5584, 4720), (2340, 2016, 4096), (1625, 5584, 16), (2100, 4096, 128), (1311, 10312, 256), (4865, 2072, 144)])
+@pytest.mark.parametrize("dequant", [False, True])
+def test_gemm_rows_past_the_last_token(cuda, M, N, K, dequant):
+    import pplb200
+    g = cuda.Generator(device="cuda").manual_seed(M + N + K)
+    a = cuda.randint(-127, 128, (M, K), dtype=cuda.int8, device="cuda", generator=g)
+    b = cuda.randint(-127, 128, (N, K), dtype=cuda.int8, device="cuda", generator=g)
+    want = _exact_gemm(cuda, a, b)
+    kw = {}
+    if dequant:
+        sm = (cuda.rand((M,), generator=g, device="cuda") + 0.5).half()
+        sn = (cuda.rand((N,), generator=g, device="cuda") + 0.5).half()
+        want = pplb200.minmax_dequantize_fp16(want, sm, sn)
+        kw = dict(mode=pplb200.EPI_DEQUANT_F16, scale_m=sm, scale_n=sn)
+    outs = [cuda.empty_like(want) for _ in range(4)]
+    wrong = cuda.zeros((), dtype=cuda.int64, device="cuda")
+    for _ in range(25):
+        for c in outs:
+            c.fill_(-1)
+        for c in outs:
+            pplb200.gemm_i8i8(a, b, out=c, **kw)
+        for c in outs:
+            wrong += (c != want).sum()
+    assert int(wrong) == 0, _differing_tiles(cuda, outs[-1], want)
+    assert pplb200.gemm_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(1625, 5584, 4720), (2560, 2048, 4096)])
+@pytest.mark.parametrize("writer", ["copy", "quantizer"])
+def test_sliced_gemm_sees_fresh_operands(cuda, M, N, K, writer):
+    """Leftover tiles in K slices whose scratch is cleared between the launches that write both operands and the GEMM."""
+    import pplb200
+    g = cuda.Generator(device="cuda").manual_seed(M + N + K)
+    fa = [cuda.randn((M, K), generator=g, device="cuda").half() for _ in range(3)]
+    fb = [cuda.randn((N, K), generator=g, device="cuda").half() for _ in range(3)]
+    qa, qb = [pplb200.minmax_quantize_fp16(t)[0] for t in fa], [pplb200.minmax_quantize_fp16(t)[0] for t in fb]
+    want = [_exact_gemm(cuda, x, y) for x, y in zip(qa, qb)]
+    a, b = cuda.empty_like(qa[0]), cuda.empty_like(qb[0])
+    sa, sb = cuda.empty((M,), dtype=cuda.float16, device="cuda"), cuda.empty((N,), dtype=cuda.float16, device="cuda")
+    ws = cuda.empty((pplb200.gemm_workspace_bytes(M, N, K, pplb200.EPI_RAW_I32),), dtype=cuda.uint8, device="cuda")
+    c = cuda.empty_like(want[0])
+    wrong, first = cuda.zeros((200,), dtype=cuda.int64, device="cuda"), None
+    for i in range(200):
+        j = i % 3
+        if writer == "copy":
+            a.copy_(qa[j])
+            b.copy_(qb[j])
+        else:
+            pplb200.minmax_quantize_fp16(fa[j], out=a, scale=sa)
+            pplb200.minmax_quantize_fp16(fb[j], out=b, scale=sb)
+        pplb200.gemm_i8i8(a, b, out=c, ws=ws)
+        wrong[i] = (c != want[j]).sum()
+    bad = wrong.nonzero().flatten().tolist()
+    assert not bad, (bad, wrong[bad].tolist(), _differing_tiles(cuda, c, want[199 % 3]))
+    assert pplb200.gemm_status() == 0
+
+
 def test_gemm_error_codes(cuda):
     import pplb200
     a = cuda.zeros((8, 40), dtype=cuda.int8, device="cuda")
