@@ -425,7 +425,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         const uint32_t fw0 = ptx::smem_addr(&full_w[0]), ew0 = ptx::smem_addr(&empty_w[0]);
         const int prew = nkb < SW ? nkb : SW;
         if (!p.early_weights) {
-            pdl_wait_prior_grid();
+            pdl_wait_before_tma();
             *static_cast<volatile int*>(&loads_started) = 1;
         }
         // the second part lies on the lanes from 64 up (one accumulator), or densely behind the first (two accumulators)
@@ -455,7 +455,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         // ---- TMA producer of the activation ring (a thread of its own: each barrier operation costs on the order of
         // a hundred cycles, and one thread serving both rings was as slow as the MMA issue it feeds)
         const uint32_t fx0 = ptx::smem_addr(&full_x[0]), ex0 = ptx::smem_addr(&empty_x[0]);
-        pdl_wait_prior_grid(); // quantized activations are written by the preceding kernel
+        pdl_wait_before_tma(); // quantized activations are written by the preceding kernel
         uint32_t sx = 0, px = 0;
         for (int i = 0; i < nkb; ++i) {
             if (i >= X_STAGES && !ptx::mbar_wait(ex0 + sx * 8u, px ^ 1u, p.status, ST_DEC_PRODUCER)) { ok = false; break; }
@@ -804,7 +804,7 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     if (warp == 0 && lane == 0) {
         // ---- TMA producer of the weight ring
         const uint32_t fw0 = ptx::smem_addr(&full_w[0]), ew0 = ptx::smem_addr(&empty_w[0]);
-        pdl_wait_prior_grid();
+        pdl_wait_before_tma();
         *static_cast<volatile int*>(&loads_started) = 1;
         uint32_t sw = 0, pw = 0;
         for (int i = 0; i < per_part; ++i) {
@@ -824,7 +824,7 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         // ---- TMA producer of the activation ring
         const uint32_t fx0 = ptx::smem_addr(&full_x[0]), ex0 = ptx::smem_addr(&empty_x[0]);
         const uint32_t box = (uint32_t)p.tile_tokens * BK;
-        pdl_wait_prior_grid(); // quantized activations are written by the preceding kernel
+        pdl_wait_before_tma(); // quantized activations are written by the preceding kernel
         uint32_t sx = 0, px = 0;
         for (int i = 0; i < per_part; ++i) {
             if (i >= C::X_STAGES && !ptx::mbar_wait(ex0 + sx * 8u, px ^ 1u, p.status, ST_DEC_PRODUCER)) { ok = false; break; }

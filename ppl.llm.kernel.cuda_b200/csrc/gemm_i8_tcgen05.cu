@@ -350,7 +350,7 @@ gemm_i8_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
     // kernel; its results (quantized activations, row scales, cleared scratch) are needed from here on.  Every
     // thread waits: all of them read such data.  A no-op in an ordinary launch.  Dependents are not released before this
     // grid ends: with the next kernel's CTAs already waiting on the SMs 3000 x 8192 x 4096 took 105 us instead of 100.
-    pdl_wait_prior_grid();
+    pdl_wait_before_tma();
 
     const int num_pairs = (int)(gridDim.x >> 1);
     const int pair_id = (int)(blockIdx.x >> 1);
