@@ -452,7 +452,7 @@ int32_t pplb200_i8i8_linear_fp16_host(pplb200_stream_t stream_, const void* x_ho
     const bool flat = M < 2 * c;
     const int64_t row_bytes = 2 * (K > N ? K : N);
     int64_t fine = (N * K / 5000 + 10000) * 55 / row_bytes; // ns x bytes per ns / bytes per row
-    fine = round_up(fine, 128);
+    fine = fine < 128 ? 128 : round_up(fine, 128);          // 0 where a row alone takes longer than the launches (K 16, N 524288)
     int64_t chunk = 0, rows = 0;
     int last = 0;
     for (int64_t m0 = 0; m0 < M; m0 += rows, ++chunk) {

@@ -171,6 +171,12 @@ def test_linear_on_host_buffers_below_two_chunks(cuda, oracle, M, K, N, chunk, r
     test_linear_on_host_buffers_matches_device_path(cuda, oracle, M, K, N, chunk, requant)
 
 
+# A row takes longer on the wire than the launches of its linear: chunks stay at 128 rows (two and a part; one)
+@pytest.mark.parametrize("M,K,N", [(300, 16, 524288), (40, 600000, 16)])
+def test_linear_on_host_buffers_very_wide_rows(cuda, oracle, M, K, N):
+    test_linear_on_host_buffers_matches_device_path(cuda, oracle, M, K, N, 0, False)
+
+
 @pytest.mark.parametrize("M,K,N", [(1, 2048, 2048), (16, 1024, 12288), (37, 4096, 1024), (128, 1024, 4096), (300, 1024, 2048), (2400, 512, 2048)])
 def test_linear_sees_weights_written_right_before(cuda, M, K, N):
     """The fused linear's launches overlap their predecessors: weights that the quantizer writes right before the call, round
