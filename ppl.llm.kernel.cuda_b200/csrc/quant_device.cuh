@@ -10,9 +10,11 @@ namespace qdev {
 
 constexpr int QTPB = 256;
 
+// Read once, kept out of L1.  Not through the non-coherent path: that is for data which nobody writes while the grid runs, and a
+// grid that starts as a programmatic dependent runs while its predecessor still writes the rows.
 __device__ __forceinline__ uint4 ldg_stream(const uint4* p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
         : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }

@@ -497,6 +497,29 @@ def test_back_to_back_launches_see_fresh_operands(cuda, M, N, K):
         assert cuda.equal(y.view(cuda.int16), want.view(cuda.int16))
 
 
+@pytest.mark.parametrize("M,N,K", [(5, 512, 256), (40, 4096, 512), (96, 8192, 128), (700, 2048, 144), (2400, 2048, 128)])
+def test_quantizer_sees_rows_written_right_before(cuda, M, N, K):
+    """The stand-alone quantizer's input is rewritten by the GEMM before it, round after round on the same buffers."""
+    import pplb200
+    g = cuda.Generator(device="cuda").manual_seed(M + N + K)
+    a = [cuda.randint(-127, 128, (M, K), generator=g, device="cuda", dtype=cuda.int8) for _ in range(3)]
+    b = cuda.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=cuda.int8)
+    kw = dict(mode=pplb200.EPI_DEQUANT_F16, scale_m=cuda.ones((M,), device="cuda").half(), scale_n=cuda.ones((N,), device="cuda").half())
+    want = []
+    for x in a:
+        y = pplb200.gemm_i8i8(x, b, **kw)
+        cuda.cuda.synchronize()
+        want.append(pplb200.minmax_quantize_fp16(y))
+    y = cuda.empty((M, N), dtype=cuda.float16, device="cuda")
+    q, s = cuda.empty_like(want[0][0]), cuda.empty_like(want[0][1])
+    wrong = cuda.zeros((), dtype=cuda.int64, device="cuda")
+    for i in range(150):
+        pplb200.gemm_i8i8(a[i % 3], b, out=y, **kw)
+        pplb200.minmax_quantize_fp16(y, out=q, scale=s)
+        wrong += (q != want[i % 3][0]).sum() + (s.view(cuda.int16) != want[i % 3][1].view(cuda.int16)).sum()
+    assert int(wrong) == 0 and pplb200.gemm_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 19072, 144), (16, 22016, 256), (37, 18960, 400), (128, 28672, 272), (128, 37904, 128)])
 def test_decode_gemm_two_row_parts(cuda, oracle, M, N, K):
     """More weight rows than one tile of 128 per SM: two accumulators per CTA (37904: a second wave of one ragged tile)."""
