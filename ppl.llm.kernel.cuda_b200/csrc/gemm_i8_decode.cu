@@ -392,8 +392,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const uint32_t tmem_base = tmem_base_slot;
     const unsigned long long t_setup = p.stamps ? globaltimer_ns() : 0ull;
 
-    // per-thread output columns (= weight rows, one per part) and their constants; behind the quantizer they belong to the
-    // weights, not to the preceding kernel, so they are fetched now and their latency hides behind the main loop
+    // per-thread output columns (= weight rows, one per part) and their constants
     const int q = warp & 3;  // TMEM lane quarter this warp may read
     const int grp = warp >> 2; // which slice of the token columns it handles
     const int col_begin = grp * C::GROUP_COLS, col_end = col_begin + C::GROUP_COLS;
@@ -404,17 +403,6 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const int n = tile_row0 + nl;
     float sn[2] = {0.0f, 0.0f};
     half bias_h[2] = {__ushort_as_half((unsigned short)0x8000u), __ushort_as_half((unsigned short)0x8000u)}; // x + (-0.0) == x for every x: no branch for "no bias"
-    auto load_column_constants = [&] {
-        if (p.mode == EPI_RAW_I32 || !nl_ok) return;
-#pragma unroll
-        for (int a = 0; a < 2; ++a) {
-            const int na = n + (a != 0 ? p.part_stride : 0);
-            if ((a != 0 && !two_parts) || (SWIGLU ? n : na) >= p.N) break;
-            sn[a] = __half2float(p.scale_n[na]);
-            if (p.bias != nullptr) bias_h[a] = p.bias[na];
-        }
-    };
-    if (p.early_weights) load_column_constants();
 
     bool ok = true;
     if (warp == 0 && lane == 0) {
@@ -506,7 +494,17 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     (void)ok;
     __syncwarp();
     pdl_wait_prior_grid(); // every thread: scale_m / row_absmax come from the preceding kernel too
-    if (!p.early_weights) load_column_constants();
+    // The column constants are fetched behind the wait even where the weights are not: these are ordinary loads, and an L1 line
+    // of an earlier launch is out of date until the wait has returned.  Their latency hides behind the main loop.
+    if (p.mode != EPI_RAW_I32 && nl_ok) {
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            const int na = n + (a != 0 ? p.part_stride : 0);
+            if ((a != 0 && !two_parts) || (SWIGLU ? n : na) >= p.N) break;
+            sn[a] = __half2float(p.scale_n[na]);
+            if (p.bias != nullptr) bias_h[a] = p.bias[na];
+        }
+    }
 
     if (p.mode != EPI_RAW_I32) {
         for (int m = threadIdx.x; m < BT; m += NUM_THREADS)

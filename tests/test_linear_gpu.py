@@ -200,6 +200,28 @@ def test_linear_sees_weights_written_right_before(cuda, M, K, N):
         assert cuda.equal(y.view(cuda.int16), want.view(cuda.int16))
 
 
+# The first two: K shared by a cluster, weights requested ahead of the dependency wait; then token tiles, CTA pairs, K folded
+@pytest.mark.parametrize("M,K,N", [(14, 8192, 1056), (68, 15792, 2080), (300, 1024, 2048), (2400, 512, 2048), (24, 2048, 1040)])
+def test_linear_sees_scales_and_bias_written_right_before(cuda, M, K, N):
+    import pplb200
+    g = cuda.Generator(device="cuda").manual_seed(M + N + K)
+    x = cuda.randn((M, K), generator=g, device="cuda").half()
+    wq = cuda.randint(-127, 128, (N, K), generator=g, device="cuda", dtype=cuda.int8)
+    sns = [(cuda.rand((N,), generator=g, device="cuda") * 8).half() for _ in range(3)]
+    biases = [cuda.randn((N,), generator=g, device="cuda").half() for _ in range(3)]
+    sn, bias = cuda.empty_like(sns[0]), cuda.empty_like(biases[0])
+    lin = pplb200.W8A8Linear(wq, sn, bias, max_tokens=M)
+    q, s = pplb200.minmax_quantize_fp16(x)
+    acc = (q.double() @ wq.double().T).to(cuda.int32)
+    want = [pplb200.minmax_dequantize_fp16(acc, s, t, bias=b) for t, b in zip(sns, biases)]
+    wrong = cuda.zeros((), dtype=cuda.int64, device="cuda")
+    for i in range(60):
+        sn.copy_(sns[i % 3])
+        bias.copy_(biases[i % 3])
+        wrong += (lin(x).view(cuda.int16) != want[i % 3].view(cuda.int16)).sum()
+    assert int(wrong) == 0 and pplb200.gemm_status() == 0
+
+
 @pytest.mark.parametrize("M,K,N", [(16, 1024, 2048), (300, 512, 1024)])
 def test_capture_with_joined_streams(cuda, M, K, N):
     """A captured graph in which a call depends on kernels of two streams (one of them this library's, the other not) and on a
