@@ -71,11 +71,11 @@ int32_t check_gemm_args(const void* A, int64_t lda, const void* B, int64_t ldb, 
 } // namespace
 
 // chained: the caller has just enqueued the activation quantizer on `stream`, which also cleared the
-// row-maximum scratch; the GEMM and the re-quantizer are then launched as programmatic dependents.
+// row-maximum scratch.  preloads: with a late trigger, because gemm_preloads_weights says so.
 int32_t gemm_entry(cudaStream_t stream, const void* A, int64_t lda, const void* B, int64_t ldb, int64_t M, int64_t N,
                    int64_t K, int32_t mode, const void* scale_M, const void* scale_N, const void* bias, float down_M,
                    float down_N, float requant_up, void* ws, int64_t ws_bytes, void* out, int64_t ldc, void* out_q,
-                   void* out_q_scale, bool chained) {
+                   void* out_q_scale, bool chained, bool preloads = false) {
     int32_t rc = check_gemm_args(A, lda, B, ldb, M, N, K, mode, scale_M, scale_N, bias, out, ldc, out_q, out_q_scale);
     if (rc != RC_SUCCESS || M == 0 || N == 0) return rc;
     GemmArgs g;
@@ -97,7 +97,7 @@ int32_t gemm_entry(cudaStream_t stream, const void* A, int64_t lda, const void* 
         g.sk_ws_bytes = ws_bytes - need;
     }
     g.pdl = true;
-    g.after_quantizer = chained && gemm_preloads_weights(M, N, K);
+    g.after_quantizer = chained && preloads;
     rc = launch_gemm(stream, g);
     if (rc != RC_SUCCESS) return rc;
     if (mode == EPI_DEQUANT_F16_REQUANT_I8)
@@ -331,11 +331,12 @@ int32_t pplb200_i8i8_linear_fp16(pplb200_stream_t stream, const void* x, const v
     // touches no memory before its griddepcontrol.wait, so this only hides its launch latency.  Where the GEMM
     // loads weights before it waits for the quantizer, it may start only after that wait: the weights may have been written
     // right before this call.
+    const bool preloads = gemm_preloads_weights(M, N, K);
     int32_t rc = launch_quantize((cudaStream_t)stream, (const half*)x, M, K, up_scale, LAYOUT_ROW_MAJOR, (int8_t*)xq,
-                                 (half*)sm, nullptr, absmax, /*pdl=*/true, 1, /*late_trigger=*/gemm_preloads_weights(M, N, K));
+                                 (half*)sm, nullptr, absmax, /*pdl=*/true, 1, /*late_trigger=*/preloads);
     if (rc != RC_SUCCESS) return rc;
     return gemm_entry((cudaStream_t)stream, xq, K, W, K, M, N, K, epilogue_mode, sm, scale_N, optional_bias, down_scale_M,
-                      down_scale_N, requant_up_scale, gws, gemm_ws_bytes(M, epilogue_mode), y, N, y_q, y_q_scale, true);
+                      down_scale_N, requant_up_scale, gws, gemm_ws_bytes(M, epilogue_mode), y, N, y_q, y_q_scale, true, preloads);
 }
 
 int32_t pplb200_i8i8_linear_fp16_args(pplb200_stream_t stream, const pplb200_linear_args* a) {

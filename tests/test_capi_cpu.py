@@ -73,6 +73,27 @@ def test_workspace_sizes():
     assert pplb200.lib.pplb200_i8i8_row_parallel_p2p_bytes(2048, 8192, 0) == -1
 
 
+@pytest.mark.parametrize("requant", [False, True])
+def test_linear_results_are_tensors_of_their_own(monkeypatch, requant):
+    """W8A8Linear hands out its buffers' memory, not the buffer objects: reshaping a result in place leaves the next call alone."""
+    import torch
+    import pplb200
+    calls = []
+    monkeypatch.setattr(pplb200, "_stream", lambda: 0)
+    monkeypatch.setattr(pplb200, "_linear_fp16_args", lambda stream, block: calls.append(block) or 0)
+    lin = pplb200.W8A8Linear(torch.zeros((32, 16), dtype=torch.int8), torch.ones((32,), dtype=torch.float16), max_tokens=4, requant=requant)
+    for x in (torch.zeros((4, 16), dtype=torch.float16), torch.zeros((4, 16, 1), dtype=torch.float16), torch.zeros((3, 16), dtype=torch.float16)):
+        M = x.shape[0]
+        for _ in range(2):
+            out = lin(x)
+            out = out if requant else (out,)
+            assert [tuple(t.shape) for t in out] == [(M, 32), (M, 32), (M,)][:len(out)]
+            assert [t.data_ptr() for t in out] == [t.data_ptr() for t in (lin.y, lin.yq, lin.ys)[:len(out)]]
+            for t in out:
+                t.unsqueeze_(0)
+    assert len(calls) == 6
+
+
 def test_reference_compatible_headers_compile(tmp_path):
     """A translation unit written against the reference's operator API (same namespaces, names and
     argument lists as its own call sites) compiles unchanged against include/."""
