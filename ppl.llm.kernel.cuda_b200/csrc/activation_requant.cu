@@ -158,7 +158,9 @@ int32_t launch_act(cudaStream_t stream, const ActParams& p) {
 // Dequantize (+bias) and scatter the columns into three outputs.  Row-major input with every extent a multiple of 8: eight
 // columns per thread, the same columns of R rows, so that the column constants are read once and 32 R bytes are
 // requested before anything is used.  1999 x 12288 (98 MB read, 49 written, part of both in L2): 21 us, as long as HBM takes for all of it.
-template <int R>
+// PACK: rows of at most 1024 columns share a CTA (blockDim.y).  8192 x 48: 4.4 -> 2.4 us, 100000 x 48: 28.5 -> 5.7; a form of its own, since a row
+// number that differs between the threads costs the wide one (1999 x 12288: 22.4 -> 27.6 us).
+template <int R, bool PACK>
 __global__ void __launch_bounds__(256)
 dequantize_split3_rows8_kernel(const int32_t* acc, const half* bias, const half* scale_m, const half* scale_n, int64_t batch, int64_t dim,
                                int64_t d0, int64_t d1, int64_t d2, float down_m, float down_n, half* o0, half* o1, half* o2) {
@@ -176,7 +178,9 @@ dequantize_split3_rows8_kernel(const int32_t* acc, const half* bias, const half*
     if (bias != nullptr) bv = ld_global_16(bias + n);
     const half* sn = reinterpret_cast<const half*>(&snv);
     const half* b = reinterpret_cast<const half*>(&bv);
-    for (int64_t m0 = (int64_t)blockIdx.y * R; m0 < batch; m0 += (int64_t)gridDim.y * R) {
+    const int64_t m_first = PACK ? ((int64_t)blockIdx.y * blockDim.y + threadIdx.y) * R : (int64_t)blockIdx.y * R;
+    const int64_t m_step = PACK ? (int64_t)gridDim.y * blockDim.y * R : (int64_t)gridDim.y * R;
+    for (int64_t m0 = m_first; m0 < batch; m0 += m_step) {
         uint4 a[R][2];
         half sm[R];
 #pragma unroll
@@ -283,14 +287,17 @@ int32_t dequantize_split3(cudaStream_t stream, const void* acc, const void* bias
     if (!acc || !sm || !sn || (d0 && !o0) || (d1 && !o1) || (d2 && !o2)) return fail(RC_INVALID_VALUE, "null pointer");
     if (layout == LAYOUT_ROW_MAJOR && dim % 8 == 0 && d0 % 8 == 0 && d1 % 8 == 0 && d2 % 8 == 0 && aligned16(acc) && aligned16(sn) &&
         (!bias || aligned16(bias)) && aligned16(o0) && aligned16(o1) && aligned16(o2)) {
-        // four rows per thread once that still leaves a few CTAs for every SM
-        const unsigned gx = (unsigned)((dim / 8 + 255) / 256);
-        const bool four = batch * gx >= 4 * 4 * 148;
-        int64_t gy = four ? (batch + 3) / 4 : batch;
+        // the groups of eight columns dealt evenly over CTAs, narrow rows side by side in one; four rows per thread once that
+        // still leaves a few CTAs for every SM
+        const int64_t groups = dim / 8;
+        const unsigned gx = (unsigned)((groups + 255) / 256), tx = (unsigned)((groups + gx - 1) / gx), ty = 256 / tx;
+        const bool four = batch * gx / ty >= 4 * 4 * 148;
+        int64_t gy = (batch + (four ? 4 * ty : ty) - 1) / (four ? 4 * ty : ty);
         if (gy > 65535) gy = 65535;
-        const cudaError_t e = launch_ex(four ? dequantize_split3_rows8_kernel<4> : dequantize_split3_rows8_kernel<1>, dim3(gx, (unsigned)gy),
-                                        dim3(256), stream, /*pdl=*/true, (const int32_t*)acc, (const half*)bias, (const half*)sm, (const half*)sn,
-                                        batch, dim, d0, d1, d2, down_m, down_n, (half*)o0, (half*)o1, (half*)o2);
+        const auto kernel = ty > 1 ? (four ? dequantize_split3_rows8_kernel<4, true> : dequantize_split3_rows8_kernel<1, true>)
+                                   : (four ? dequantize_split3_rows8_kernel<4, false> : dequantize_split3_rows8_kernel<1, false>);
+        const cudaError_t e = launch_ex(kernel, dim3(gx, (unsigned)gy), dim3(tx, ty), stream, /*pdl=*/true, (const int32_t*)acc,
+                                        (const half*)bias, (const half*)sm, (const half*)sn, batch, dim, d0, d1, d2, down_m, down_n, (half*)o0, (half*)o1, (half*)o2);
         if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "dequantize_split3 launch failed: %s", cudaGetErrorString(e));
         return RC_SUCCESS;
     }

@@ -199,10 +199,12 @@ def test_small_batch_gate_up_swiglu_overflow(cuda):
     assert cuda.equal(fused[1], two_step[1]) and cuda.equal(fused[2].view(cuda.int16), two_step[2].view(cuda.int16))
 
 
-@pytest.mark.parametrize("M,splits", [(1, (8, 8, 8)), (5, (4096, 512, 512)), (2401, (32, 8, 8)), (3, (2056, 0, 16)), (7, (24, 16, 4)), (1203, (2048, 256, 256))])
+@pytest.mark.parametrize("M,splits", [(1, (8, 8, 8)), (5, (4096, 512, 512)), (2401, (32, 8, 8)), (3, (2056, 0, 16)), (7, (24, 16, 4)), (1203, (2048, 256, 256)),
+                                      (1, (8, 0, 0)), (70001, (8, 8, 8)), (9999, (32, 8, 8)), (37, (680, 8, 8)), (2400, (1024, 512, 504)), (6, (2040, 8, 16))])
 @pytest.mark.parametrize("with_bias", [False, True])
 def test_dequantize_split3_vector_form(cuda, oracle, M, splits, with_bias):
-    """Eight columns per thread (one or four rows each), ragged last CTAs and rows, an empty output; (24, 16, 4) keeps to groups of four."""
+    """Eight columns per thread (one or four rows each), ragged last CTAs and rows, narrow rows side by side, an empty output; (24, 16, 4)
+    keeps to groups of four."""
     import pplb200
     rng = np.random.default_rng(M + sum(splits))
     N = sum(splits)
