@@ -742,7 +742,6 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     __shared__ __align__(8) uint64_t acc_full_bar;
     __shared__ uint32_t tmem_base_slot;
     __shared__ float token_scale[BT];
-    __shared__ uint32_t token_absmax[BT];
     __shared__ int loads_started;
 
     const int warp = threadIdx.x >> 5;
@@ -779,7 +778,6 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         ptx::tmem_alloc(ptx::smem_addr(&tmem_base_slot), C::TMEM_COLS);
         ptx::tmem_relinquish();
     }
-    if (threadIdx.x < BT) token_absmax[threadIdx.x] = 0u;
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
@@ -932,15 +930,25 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
         if (p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
             const float a = n_ok ? fabsf(__half2float(h)) : 0.0f;
             const uint32_t bits = __reduce_max_sync(0xffffffffu, a == a ? __float_as_uint(a) : 0u); // NaNs are dropped, as fmax does
-            if (lane == 0 && bits != 0u) atomicMax(&token_absmax[m], bits);
+            if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(x_ring + (uint32_t)((warp % ROW_WARPS) * BT + m) * 4u), "r"(bits) : "memory");
         }
     }
     if (p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
         // Neighbouring tokens leave in one instruction per CTA.  One global atomic per token and warp as the rows are finished,
-        // all CTAs on the same few lines of L2, took as long as the rest of the kernel (59 tokens, N 8928, K 2944: the call 20.9 -> 12.5 us; one token: 8.4 -> 8.5).
+        // all CTAs on the same few lines of L2, took as long as the rest of the kernel (59 x 8928 x 2944: the call 20.9 -> 11.8 us).
+        // They meet in the dead activation ring, not in memory of their own: 1 KB more, and under the 196 KB carve-out that the driver picks for
+        // this kernel no quantizer CTA starts beside it any more (70 x 8192 x 4096 without re-quantizing: 12.9 -> 13.8 us).
         __syncthreads();
-        for (int m = threadIdx.x; m < BT && m < p.M; m += C::NUM_THREADS)
-            if (token_absmax[m] != 0u) atomicMax(p.row_absmax_bits + m, token_absmax[m]);
+        for (int m = threadIdx.x; m < BT && m < p.M; m += C::NUM_THREADS) {
+            uint32_t bits = 0u;
+#pragma unroll
+            for (int w = 0; w < ROW_WARPS; ++w) {
+                uint32_t t;
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(t) : "r"(x_ring + (uint32_t)(w * BT + m) * 4u) : "memory");
+                bits = t > bits ? t : bits;
+            }
+            if (bits != 0u) atomicMax(p.row_absmax_bits + m, bits);
+        }
     }
     if (warp == 1) {
         __syncwarp();
