@@ -196,7 +196,7 @@ static_assert(kSkMaxTiles * 8 * 4 <= kSkStateBytes, "arrival counters");
 // The quantizer of the fused linear lets the GEMM start at once -- the GEMM then waits before it loads weights, and brings them
 // into L2 until then -- or, where this is true, once everything before the call has completed, so that the GEMM fills its
 // weight ring while the quantizer runs.  That pays where the way from L2 into the SMs is what the GEMM is bound by: more than
-// 128 tokens (333 x 4096 x 4096: 15.8 against 18.4 us), and K shared by a cluster (48 x 11008 x 1024: 14.0 against 15.4 us).
+// 128 tokens (333 x 4096 x 4096: 15.8 against 18.4 us); for fewer see the rule itself.
 bool gemm_preloads_weights(int64_t M, int64_t N, int64_t K);
 int32_t launch_gemm_decode(cudaStream_t stream, const GemmArgs& a, unsigned int* status, bool pdl);
 int32_t launch_gemm(cudaStream_t stream, const GemmArgs& a);

@@ -715,7 +715,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
 // activations are MMA columns f * tokens .. , one MMA multiplies all F parts with all F, and the F diagonal blocks hold
 // the partial sums -- the other blocks are computed in the same cycles (up to 64 columns cost the same 53) and never
 // read.  The sums meet in this CTA's own shared memory.  Each CTA reads every activation, so the form pays
-// while they are fewer than the weights (plan_fold).
+// while they are fewer than the weights (plan_small).
 template <int BT, int F> struct FCfg {
     static constexpr int ROWS = BW / F;                 // weight rows per tile
     static constexpr int W_BYTES = BW * BK;             // one stage: F parts
@@ -802,8 +802,10 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     if (warp == 0 && lane == 0) {
         // ---- TMA producer of the weight ring
         const uint32_t fw0 = ptx::smem_addr(&full_w[0]), ew0 = ptx::smem_addr(&empty_w[0]);
-        pdl_wait_before_tma();
-        *static_cast<volatile int*>(&loads_started) = 1;
+        if (!p.early_weights) { // as in gemm_i8_decode_kernel
+            pdl_wait_before_tma();
+            *static_cast<volatile int*>(&loads_started) = 1;
+        }
         uint32_t sw = 0, pw = 0;
         for (int i = 0; i < per_part; ++i) {
             if (i >= C::W_STAGES && !ptx::mbar_wait(ew0 + sw * 8u, pw ^ 1u, p.status, ST_DEC_PRODUCER)) { ok = false; break; }
@@ -814,10 +816,11 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
             if (++sw == (uint32_t)C::W_STAGES) { sw = 0; pw ^= 1u; }
         }
     } else if (warp == 4 && lane == 0) {
-        prefetch_weights(per_part, &loads_started, [&](int i) {
+        if (!p.early_weights)
+            prefetch_weights(per_part, &loads_started, [&](int i) {
 #pragma unroll
-            for (int f = 0; f < F; ++f) ptx::tma_prefetch_l2_2d(&tmap_w, k_of(i, f), row0);
-        });
+                for (int f = 0; f < F; ++f) ptx::tma_prefetch_l2_2d(&tmap_w, k_of(i, f), row0);
+            });
     } else if (warp == 3 && lane == 0) {
         // ---- TMA producer of the activation ring
         const uint32_t fx0 = ptx::smem_addr(&full_x[0]), ex0 = ptx::smem_addr(&empty_x[0]);
@@ -1060,6 +1063,7 @@ const DecDeviceInfo* dec_device_info() {
 struct DecodePlan {
     int tokens, token_tiles, rows, row_tiles, S;
     bool dual;
+    int fold; // parts K is folded into (gemm_i8_fold_kernel), 0 = row tiles
 };
 
 // Rows per tile for `cap` tiles that can run at once: the smallest multiple of 8 with which `columns` output columns
@@ -1070,28 +1074,64 @@ int rows_for(int64_t columns, int64_t cap, int max_rows) {
     return r < 8 ? 8 : r < max_rows ? (int)r : max_rows;
 }
 
-// Up to 128 tokens: one token tile.
-DecodePlan plan_small(const DecDeviceInfo& dev, int variant, int64_t M, int64_t columns, int num_k_blocks, bool swiglu) {
-    DecodePlan d;
-    d.tokens = (int)((M + 15) / 16 * 16);
-    d.token_tiles = 1;
+int variant_of(int64_t M) { return M <= 16 ? 0 : M <= 32 ? 1 : M <= 64 ? 2 : 3; }
+
+// Up to 128 tokens: one token tile.  Where tiles of full height leave SMs idle, K is shared: by the S CTAs of a cluster, or
+// folded onto the lanes of one CTA (gemm_i8_fold_kernel).  All forms that run as one wave are modelled in SM cycles per CTA: a
+// stage costs the larger of its operands' way from L2 (60 bytes per cycle) and the issuing threads' bookkeeping (415; 425 and 500
+// with two and four boxes per operand), all weights arrive at 4500 bytes per cycle (between HBM's 3400 and the rate of what is
+// still in L2), and sharing K inside a cluster adds 3800 and 45 per token (exchange, scattered stores).  Fitted to 420 shapes of
+// 1024 .. 9472 columns, every form timed; on 520 others on average 1.3 % behind the fastest form, with SwiGLU (160 shapes) 3.1 %.  (16 x 2560 x 17424: 12.8 us
+// with clusters of six, 21.1 of seven, which need a second wave, 15.6 folded in four.)
+DecodePlan plan_small(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t K, bool swiglu) {
+    DecodePlan best = {};
+    best.tokens = (int)((M + 15) / 16 * 16);
+    best.token_tiles = 1;
+    const int64_t kb = (K + BK - 1) / BK;
     // Weight rows a tile can hold: one per TMEM lane, or, x and gate rows paired, half as many channels.
     const int bw = swiglu ? BW / 2 : BW;
+    const int64_t full_tiles = (columns + bw - 1) / bw;
     // Two accumulators per tile where tiles of bw rows no longer run as one wave: with 172 tiles on 148 SMs the second
     // wave costs as much as the first.
-    d.dual = (columns + bw - 1) / bw > dev.sms;
-    // K split: one CTA per SM is resident (the rings take the whole shared memory), so split K only as far as all clusters
-    // still fit in one wave (fewer than SMs / S of them: a cluster stays inside one GPC); every CTA keeps at least two
-    // K blocks
-    int S = d.dual ? 1 : dev.sms / (int)((columns + bw - 1) / bw);
-    if (S > 8) S = 8;
-    if (S > num_k_blocks / 2) S = num_k_blocks / 2;
-    if (S < 1) S = 1;
-    d.S = S;
-    const int parts_out = d.dual && !swiglu ? 2 : 1; // parts of a tile that are output columns of their own
-    d.rows = rows_for(columns, (S == 1 ? dev.sms : dev.max_clusters[variant][S]) * (int64_t)parts_out, d.dual ? BW : bw);
-    d.row_tiles = (int)((columns + d.rows * parts_out - 1) / (d.rows * parts_out));
-    return d;
+    best.dual = full_tiles > dev.sms;
+    if (best.dual) {
+        const int parts_out = swiglu ? 1 : 2; // parts of a tile that are output columns of their own
+        best.S = 1;
+        best.rows = rows_for(columns, dev.sms * (int64_t)parts_out, BW);
+        best.row_tiles = (int)((columns + best.rows * parts_out - 1) / (best.rows * parts_out));
+        return best;
+    }
+    const double from_hbm = (double)columns * (swiglu ? 2 : 1) * K / 4500.0;
+    auto main_loop = [&](int64_t stages, double bytes, double issue) {
+        const double c = (double)stages * (bytes / 60.0 > issue ? bytes / 60.0 : issue);
+        return c > from_hbm ? c : from_hbm;
+    };
+    double best_cost = 1e30;
+    const double exchange = 3800.0 + (45.0 * M < 6000.0 ? 45.0 * M : 6000.0);
+    for (int S = 1; S <= 8 && (S == 1 || S <= kb / 2); ++S) { // every CTA keeps at least two K blocks
+        // Fewer than SMs / S clusters: each stays inside one GPC.  From three CTAs up two fewer again: filled to the last cluster, some find
+        // no GPC with S free SMs while the kernel before is ending, and run as a second wave (117 x 4320 x 23376: 58.9 us, now 40.7).
+        const int64_t slots = S == 1 ? dev.sms : dev.max_clusters[variant_of(M)][S] - (S > 2 ? 2 : 0);
+        if (full_tiles > slots) continue;
+        const int rows = rows_for(columns, slots, bw);
+        const double cost = main_loop((kb + S - 1) / S, (double)(rows * (swiglu ? 2 : 1) + best.tokens) * BK, 415.0) + (S > 1 ? exchange : 0.0);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best.S = S;
+            best.rows = rows;
+            best.row_tiles = (int)((columns + rows - 1) / rows);
+        }
+    }
+    for (int F = 2; F <= 4 && !swiglu; F += 2) {
+        if (columns > dev.sms * (BW / F) || F * best.tokens > 256 || kb < 4) continue; // below four K blocks there is nothing to share
+        const int rows = rows_for(columns, dev.sms, BW / F);
+        const double cost = main_loop((kb + F - 1) / F, (double)F * (rows + best.tokens) * BK, F == 4 ? 500.0 : 425.0);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best.fold = F;
+        }
+    }
+    return best;
 }
 
 // More than 128 tokens, too few for the CTA pairs' 256 x 256 tiles: the cheapest cut by a model of one CTA's time in SM
@@ -1121,7 +1161,7 @@ DecodePlan plan_medium(const DecDeviceInfo& dev, int64_t M, int64_t columns, int
                 const double cost = (double)waves * ((num_k_blocks + S - 1) / S * kb + 3000.0 + (S > 1 ? 12000.0 : 0.0));
                 if (cost < best_cost) {
                     best_cost = cost;
-                    best = {tokens, (int)token_tiles, rows, (int)row_tiles, S, dual != 0};
+                    best = {tokens, (int)token_tiles, rows, (int)row_tiles, S, dual != 0, 0};
                 }
             }
         }
@@ -1145,23 +1185,6 @@ DecodeParams make_params(const GemmArgs& a, unsigned int* status) {
     p.early_weights = a.after_quantizer ? 1 : 0;
     p.stamps = stall_counters();
     return p;
-}
-
-// Parts K is folded into (see gemm_i8_fold_kernel), 0 = not folded.  Both forms are modelled in SM cycles per CTA: a stage costs
-// the larger of its operands' way from L2 (60 bytes per cycle) and the issuing threads' bookkeeping (390; 450 with F boxes each), all weights come
-// from HBM at 3400, and sharing K inside a cluster adds 2500 and 80 per token up to 6500 (exchange and scattered stores;
-// measured 1.7 us at 16 tokens, 3.1 at 37, 3.6 at 96).  Folded, a CTA reads all of K for every token; `split` is the alternative.
-int plan_fold(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t K, const DecodePlan& split) {
-    if (split.S == 1 || split.dual) return 0; // every SM has a tile of its own already
-    const int F = columns <= dev.sms * (BW / 4) && split.tokens <= 64 ? 4 : 2;
-    if (columns > dev.sms * (BW / F)) return 0;
-    const int64_t kb = (K + BK - 1) / BK;
-    auto loop = [&](int64_t stages, double bytes, double issue) { return (double)stages * (bytes / 60.0 > issue ? bytes / 60.0 : issue); };
-    const double hbm = (double)columns * K / 3400.0;
-    const double folded = loop((kb + F - 1) / F, (double)F * (rows_for(columns, dev.sms, BW / F) + M) * BK, 450.0);
-    const double shared = loop((kb + split.S - 1) / split.S, (double)(split.rows + M) * BK, 390.0);
-    const double exchange = 2500.0 + 80.0 * M < 6500.0 ? 2500.0 + 80.0 * M : 6500.0;
-    return (folded > hbm ? folded : hbm) < (shared > hbm ? shared : hbm) + exchange ? F : 0;
 }
 
 template <int BT, int F>
@@ -1249,9 +1272,15 @@ bool gemm_preloads_weights(int64_t M, int64_t N, int64_t K) {
     if (M > 128) return true;
     const DecDeviceInfo* dev = dec_device_info();
     if (!dev) return false;
-    const int kb = (int)((K + BK - 1) / BK);
-    const DecodePlan plan = plan_small(*dev, M <= 16 ? 0 : M <= 32 ? 1 : M <= 64 ? 2 : 3, M, N, kb, false);
-    return plan.S > 1 && plan_fold(*dev, M, N, K, plan) == 0;
+    const DecodePlan plan = plan_small(*dev, M, N, K, false);
+    // Starting late exposes part of the GEMM's launch, unless the quantizer itself takes long; starting early, the weight ring fills
+    // only once the quantizer has ended.  Early -> late, us, tokens x N x K, weights from L2 (warm) or HBM (cold):
+    // one wide MMA (fold * M columns) or a short K: 83 x 7168 x 4096 cold 13.2 -> 14.4, 2 x 5120 x 1024 cold 5.3 -> 5.5; else 1 x 8192 x 4096 warm 8.8 -> 8.4, 16 x 9216 x 4784 cold 13.3 -> 12.6
+    if (plan.fold) return plan.fold * M <= 128 && K >= 2048;
+    // 16 x 5120 x 14336 warm 15.0 -> 14.3, 48 x 1024 x 11008 cold 12.5 -> 12.1
+    if (plan.S > 1) return true;
+    // 24 x 12288 x 5120 cold 15.7 -> 16.4, 24 x 22016 x 5120 cold (two row parts) 23.2 -> 24.1; 128 x 12288 x 8192 cold 30.0 -> 29.3, 96 x 12288 x 8192 warm 27.3 -> 26.1
+    return !plan.dual && M * K >= 320 * 1024;
 }
 
 int32_t launch_gemm_decode(cudaStream_t stream, const GemmArgs& a, unsigned int* status, bool pdl) {
@@ -1259,16 +1288,14 @@ int32_t launch_gemm_decode(cudaStream_t stream, const GemmArgs& a, unsigned int*
     if (!dev) return fail(RC_DEVICE_RUNTIME_ERROR, "device set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
     const bool swiglu = a.mode == EPI_SWIGLU_F16;
     const int64_t columns = swiglu ? a.N / 2 : a.N;
-    const int num_k_blocks = (int)((a.K + BK - 1) / BK);
-    if (a.M > 128) return launch_bt<128>(stream, a, plan_medium(*dev, a.M, columns, num_k_blocks, swiglu), status, pdl);
-    const int variant = a.M <= 16 ? 0 : a.M <= 32 ? 1 : a.M <= 64 ? 2 : 3;
-    const DecodePlan plan = plan_small(*dev, variant, a.M, columns, num_k_blocks, swiglu);
-    const int fold = swiglu ? 0 : plan_fold(*dev, a.M, columns, a.K, plan);
-    if (fold == 4) {
+    if (a.M > 128) return launch_bt<128>(stream, a, plan_medium(*dev, a.M, columns, (int)((a.K + BK - 1) / BK), swiglu), status, pdl);
+    const int variant = variant_of(a.M);
+    const DecodePlan plan = plan_small(*dev, a.M, columns, a.K, swiglu);
+    if (plan.fold == 4) {
         return variant == 0 ? launch_fold<16, 4>(stream, a, *dev, status, pdl)
              : variant == 1 ? launch_fold<32, 4>(stream, a, *dev, status, pdl) : launch_fold<64, 4>(stream, a, *dev, status, pdl);
     }
-    if (fold == 2) {
+    if (plan.fold == 2) {
         return variant == 0 ? launch_fold<16, 2>(stream, a, *dev, status, pdl) : variant == 1 ? launch_fold<32, 2>(stream, a, *dev, status, pdl)
              : variant == 2 ? launch_fold<64, 2>(stream, a, *dev, status, pdl) : launch_fold<128, 2>(stream, a, *dev, status, pdl);
     }
