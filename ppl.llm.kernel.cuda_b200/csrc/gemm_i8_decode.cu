@@ -412,7 +412,9 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         // later write still reaches them.
         const uint32_t fw0 = ptx::smem_addr(&full_w[0]), ew0 = ptx::smem_addr(&empty_w[0]);
         const int prew = nkb < SW ? nkb : SW;
-        if (!p.early_weights) {
+        if (p.early_weights) {
+            order_before_tma();
+        } else {
             pdl_wait_before_tma();
             *static_cast<volatile int*>(&loads_started) = 1;
         }
@@ -802,7 +804,9 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     if (warp == 0 && lane == 0) {
         // ---- TMA producer of the weight ring
         const uint32_t fw0 = ptx::smem_addr(&full_w[0]), ew0 = ptx::smem_addr(&empty_w[0]);
-        if (!p.early_weights) { // as in gemm_i8_decode_kernel
+        if (p.early_weights) { // as in gemm_i8_decode_kernel
+            order_before_tma();
+        } else {
             pdl_wait_before_tma();
             *static_cast<volatile int*>(&loads_started) = 1;
         }
