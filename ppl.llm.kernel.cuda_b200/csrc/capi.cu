@@ -209,9 +209,9 @@ int32_t pplb200_i8i8_minmax_requantize_swiglu_fp16(pplb200_stream_t stream, cons
 namespace {
 // The fused form needs the CTA-pair kernel: enough 256-row x 128-channel tiles for every pair, and
 // the x / gate halves of the weight matrix aligned to the 128-row tiles.
-bool swiglu_fusable(int64_t M, int64_t D) { return M > 128 && D % 128 == 0 && ((M + 255) / 256) * (D / 128) >= 74; }
+bool swiglu_fusable(int64_t M, int64_t D) { return M > 128 && D % 128 == 0 && ((M + 255) / 256) * (D / 128) >= kCtaPairs; }
 // Fused on single CTAs: batches for which the plain GEMM does not use CTA pairs either.
-bool swiglu_single(int64_t M, int64_t D) { return M <= 128 || ((M + 255) / 256) * ((2 * D + 255) / 256) < 74; }
+bool swiglu_single(int64_t M, int64_t D) { return M <= 128 || ((M + 255) / 256) * ((2 * D + 255) / 256) < kCtaPairs; }
 }
 
 int64_t pplb200_i8i8_gate_up_swiglu_workspace_bytes(int64_t M, int64_t act_dim, int64_t K) {

@@ -194,6 +194,9 @@ constexpr int64_t kSkTileBytes = 256 * 256 * 4;
 constexpr int64_t kSkStateBytes = 2048;
 constexpr int64_t kSkWsBytes = kSkStateBytes + kSkMaxTiles * kSkTileBytes;
 static_assert(kSkMaxTiles * 8 * 4 <= kSkStateBytes, "arrival counters");
+// CTA pairs of a B200 (148 SMs): products with fewer 256 x 256 tiles go to the small-batch kernels.  Workspace sizes depend on it, which
+// are asked for without a device, so it is not read from the device.
+constexpr int64_t kCtaPairs = 74;
 // The quantizer of the fused linear lets the GEMM start at once -- the GEMM then waits before it loads weights, and brings them
 // into L2 until then -- or, where this is true, once everything before the call has completed, so that the GEMM fills its
 // weight ring while the quantizer runs.  That pays where the way from L2 into the SMs is what the GEMM is bound by: more than

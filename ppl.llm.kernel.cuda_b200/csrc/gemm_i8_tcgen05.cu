@@ -893,7 +893,7 @@ int32_t launch_gemm(cudaStream_t stream, const GemmArgs& a) {
     if (a.M <= 128) return launch_gemm_decode(stream, a, dev->status, a.pdl);
 
     // Large problems: 256 x 256 tiles on CTA pairs, as long as every pair gets at least one tile.
-    if (((a.M + 255) / 256) * ((a.N + 255) / 256) >= dev->sms / 2)
+    if (((a.M + 255) / 256) * ((a.N + 255) / 256) >= kCtaPairs)
         return launch_pair(stream, a, *dev);
 
     // In between: one wave of smaller tiles on single CTAs.  (M333 K4096 N4096, linear: 16.4 us; the same on persistent
