@@ -419,6 +419,15 @@ void pplb200_debug_gemm_stall_counters(void* counters);
 void pplb200_debug_gemm_tail_split(int32_t enabled);
 
 /*
+ * Diagnostics: how the small-batch GEMM (up to 128 tokens, and larger batches with too few 256 x 256 tiles for the CTA pairs)
+ * cuts a product of N output columns on the current device.  plan: [0] tokens per tile, [1] token tiles, [2] weight rows per
+ * tile and part, [3] row tiles, [4] CTAs of a cluster that share K, [5] row parts of a tile, [6] parts that K is folded into
+ * (0: not folded; else [2] .. [5] do not apply), [7] whether the fused linear requests weights ahead of the dependency wait.
+ * swiglu != 0: the GEMM of gate_up_swiglu_requant, N = act_dim.
+ */
+int32_t pplb200_debug_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t swiglu, int32_t* plan);
+
+/*
  * Storage-order change of a [rows, cols] matrix of int8 (elem_bytes 1) or int32 (elem_bytes 4) elements between
  * any two of ROW_MAJOR, COL32, COL32_2R_4R4 and COL4_4R2_8C (index maps of
  * include/ppl/kernel/llm/cuda/common/matrix_layout.h:34-142; no counterpart function in the reference, whose

@@ -500,6 +500,10 @@ int32_t pplb200_i8i8_linear_fp16_host(pplb200_stream_t stream_, const void* x_ho
 
 int32_t pplb200_i8i8_gemm_status(int32_t reset) { return gemm_status(reset); }
 void pplb200_debug_gemm_stall_counters(void* counters) { set_stall_counters(counters); }
+int32_t pplb200_debug_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t swiglu, int32_t* plan) {
+    if (!plan || M <= 0 || N <= 0 || K <= 0) return fail(RC_INVALID_VALUE, "bad extents or null plan");
+    return gemm_decode_plan(M, N, K, swiglu != 0, plan);
+}
 void pplb200_debug_gemm_tail_split(int32_t enabled) { set_tail_split(enabled < 0 ? 0 : enabled > 2 ? 2 : enabled); }
 
 // Host helper for tests: the library's (row, col) -> offset map for a layout.

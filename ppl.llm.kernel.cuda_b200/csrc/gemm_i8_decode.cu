@@ -1287,6 +1287,16 @@ bool gemm_preloads_weights(int64_t M, int64_t N, int64_t K) {
     return !plan.dual && M * K >= 320 * 1024;
 }
 
+int32_t gemm_decode_plan(int64_t M, int64_t columns, int64_t K, bool swiglu, int32_t* out) {
+    const DecDeviceInfo* dev = dec_device_info();
+    if (!dev) return fail(RC_DEVICE_RUNTIME_ERROR, "device set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
+    const DecodePlan d = M > 128 ? plan_medium(*dev, M, columns, (int)((K + BK - 1) / BK), swiglu) : plan_small(*dev, M, columns, K, swiglu);
+    out[0] = d.tokens; out[1] = d.token_tiles; out[2] = d.rows; out[3] = d.row_tiles;
+    out[4] = d.S; out[5] = d.dual ? 2 : 1; out[6] = d.fold;
+    out[7] = !swiglu && gemm_preloads_weights(M, columns, K) ? 1 : 0;
+    return RC_SUCCESS;
+}
+
 int32_t launch_gemm_decode(cudaStream_t stream, const GemmArgs& a, unsigned int* status, bool pdl) {
     const DecDeviceInfo* dev = dec_device_info();
     if (!dev) return fail(RC_DEVICE_RUNTIME_ERROR, "device set-up failed: %s", cudaGetErrorString(cudaGetLastError()));

@@ -173,7 +173,7 @@ def test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K):
     assert float(act.float().abs().max()) > 0.01  # the scales put the values in SiLU's interesting range
 
 
-# One accumulator for x and gate rows with K split over 1 .. 8 CTAs (up to 64 channels per tile; 1280: seven, 16: eight),
+# One accumulator for x and gate rows with K split over 1 .. 8 CTAs (up to 64 channels per tile; 1280: five and six, 16: eight),
 # two accumulators from 9473 channels up, K shorter than a K block, a last tile of 16 channels, every token width
 @pytest.mark.parametrize("M,D,K", [(1, 16, 16), (5, 16, 4096), (16, 1280, 1808), (17, 3584, 1024), (8, 11008, 512), (33, 9488, 272),
                                    (64, 4672, 1040), (96, 3584, 2048), (128, 1280, 4096), (128, 9472, 384), (128, 19056, 144), (120, 640, 2064)])
@@ -220,4 +220,13 @@ def test_dequantize_split3_vector_form(cuda, oracle, M, splits, with_bias):
 @pytest.mark.parametrize("M,D,K", [(129, 16, 272), (333, 1376, 512), (200, 9344, 144), (1000, 2048, 272), (700, 208, 2064)])
 def test_medium_batch_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K):
     """The same over several token tiles."""
+    test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K)
+
+
+@pytest.mark.parametrize("M,D,K", [(40, 2800, 5120), (128, 448, 8192), (144, 1552, 8496), (131, 864, 7136), (226, 192, 5232), (195, 128, 5600)])
+def test_gate_up_swiglu_k_shared_by_a_cluster(cuda, oracle, M, D, K):
+    """One and several token tiles whose K is shared by two to eight CTAs."""
+    import pplb200
+    plan = pplb200.gemm_plan(M, D, K, swiglu=True)
+    assert plan["split"] > 1 and (M <= 128 or plan["token_tiles"] > 1), plan
     test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K)

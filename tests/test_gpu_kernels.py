@@ -175,8 +175,8 @@ DECODE_SHAPES = [(128, 6272, 2048), (100, 12288, 4096), (64, 8192, 1024), (72, 3
 
 @pytest.mark.parametrize("M,N,K", DECODE_SHAPES + [(16, 4096, 4096), (128, 19072, 1024), (8, 1024, 256), (1, 2048, 8192)])
 def test_decode_gemm_all_modes(cuda, oracle, M, N, K):
-    """Small-batch kernel across its variants: one or two weight-row tiles per CTA, K split over clusters of
-    different sizes, an odd number of weight-row tiles, token counts that are not multiples of 8."""
+    """Small-batch kernels: whole K per CTA with one or two row parts, K folded onto the lanes, an odd number of weight-row
+    tiles, token counts that are not multiples of 8."""
     import pplb200
     rng = np.random.default_rng(M + N + K)
     x = rng.standard_normal((M, K)).astype(np.float16)
@@ -318,8 +318,8 @@ def test_gemm_tile_groups_ragged(cuda, M, N, K):
 
 
 def test_gemm_random_shapes(cuda):
-    """Seeded sweep over shapes of the large-batch kernels (CTA pairs and single CTAs, every tile width, sliced and whole
-    leftover tiles): raw int32 result against the exact product."""
+    """Seeded sweep over shapes of more than 128 tokens (CTA pairs, one shape with sliced leftover tiles; token tiles on
+    single CTAs): raw int32 result against the exact product."""
     import pplb200
     torch = cuda
     rng = np.random.default_rng(20240611)
@@ -527,8 +527,8 @@ def test_decode_gemm_two_row_parts(cuda, oracle, M, N, K):
     test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
 
 
-# Batches between the small-batch and the CTA-pair kernels: several token tiles, the last one ragged; K split over clusters
-# (few rows), one or two row parts, token tiles of 80 .. 128
+# Batches between the small-batch and the CTA-pair kernels: several token tiles, the last one ragged; one or two row parts,
+# token tiles of 80 .. 128
 @pytest.mark.parametrize("M,N,K", [(129, 16, 16), (333, 4096, 512), (130, 1040, 4096), (255, 1024, 272), (1000, 4096, 272), (192, 18928, 144),
                                    (385, 9216, 400), (700, 528, 2064), (4700, 256, 400)])
 def test_medium_batch_gemm_all_modes(cuda, oracle, M, N, K):
@@ -536,12 +536,47 @@ def test_medium_batch_gemm_all_modes(cuda, oracle, M, N, K):
     test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
 
 
-# K folded onto the TMEM lanes in four and two parts: one to 64 (128) tokens, K of a fraction of a block and of one block per
-# part, ragged last tiles, more stages than the rings hold
+# K folded onto the TMEM lanes in four and two parts: one to 64 (128) tokens, ragged last tiles, more stages than the rings
+# hold; and neighbours with fewer than four K blocks, which are not folded
 @pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (16, 896, 16), (17, 4736, 144), (37, 4096, 11008), (64, 1040, 1024), (33, 4744, 528),
                                    (48, 9472, 384), (96, 8192, 1024), (128, 5120, 272), (65, 7168, 2064)])
 def test_folded_gemm_all_modes(cuda, oracle, M, N, K):
     if N % 16 == 0:
         test_decode_gemm_all_modes(cuda, oracle, M, N, K)
     test_gemm_i32_alpha_beta_bias(cuda, M, N, K, 1, 0, False)
+    test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
+
+
+# Every instantiation of the folded kernel: one K block per part (the second issuer has none), a last part that lies partly or
+# wholly past the end of K, weights requested ahead of the wait in the fused linear
+@pytest.mark.parametrize("M,N,K,fold,early", [(1, 896, 400, 4, 0), (20, 1040, 512, 4, 0), (24, 2048, 528, 4, 0), (64, 1040, 1024, 4, 0), (16, 8192, 1024, 2, 0),
+                                              (32, 8192, 1024, 2, 0), (96, 8192, 1024, 2, 0), (128, 4096, 4096, 2, 0), (16, 4736, 2064, 4, 1),
+                                              (30, 4736, 2048, 4, 1), (40, 9472, 2304, 2, 1)])
+def test_folded_gemm_forms(cuda, oracle, M, N, K, fold, early):
+    import pplb200
+    plan = pplb200.gemm_plan(M, N, K)
+    assert plan["fold"] == fold and plan["early_weights"] == early, plan
+    test_decode_gemm_all_modes(cuda, oracle, M, N, K)
+    test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
+
+
+# K shared by the CTAs of a cluster (two to eight of them): partial sums through distributed shared memory, every CTA storing the
+# pieces that it owns, at every token width
+@pytest.mark.parametrize("M,N,K", [(1, 2704, 10864), (5, 256, 6784), (31, 256, 8976), (31, 4800, 8720), (60, 1712, 8208), (60, 2592, 7744),
+                                   (100, 256, 5712), (128, 272, 5200), (128, 3168, 5968), (128, 5536, 9008)])
+def test_decode_gemm_k_shared_by_a_cluster(cuda, oracle, M, N, K):
+    import pplb200
+    plan = pplb200.gemm_plan(M, N, K)
+    assert plan["split"] > 1 and plan["fold"] == 0 and plan["early_weights"] == 1, plan
+    test_decode_gemm_all_modes(cuda, oracle, M, N, K)
+    test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
+
+
+# The same with several token tiles, the last one ragged
+@pytest.mark.parametrize("M,N,K", [(160, 160, 4560), (197, 128, 5248), (145, 1824, 5504), (274, 1504, 6400), (398, 1488, 8368)])
+def test_medium_batch_gemm_k_shared_by_a_cluster(cuda, oracle, M, N, K):
+    import pplb200
+    plan = pplb200.gemm_plan(M, N, K)
+    assert plan["split"] > 1 and plan["token_tiles"] > 1, plan
+    test_decode_gemm_all_modes(cuda, oracle, M, N, K)
     test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)

@@ -177,7 +177,11 @@ def test_linear_on_host_buffers_very_wide_rows(cuda, oracle, M, K, N):
     test_linear_on_host_buffers_matches_device_path(cuda, oracle, M, K, N, 0, False)
 
 
-@pytest.mark.parametrize("M,K,N", [(1, 2048, 2048), (16, 1024, 12288), (37, 4096, 1024), (128, 1024, 4096), (300, 1024, 2048), (2400, 512, 2048)])
+# weights requested ahead of the dependency wait: K folded, K shared by a cluster, whole K per CTA
+EARLY_WEIGHTS = [(16, 4096, 2048), (5, 6784, 256), (128, 5200, 272), (128, 2576, 12288)]
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 2048, 2048), (16, 1024, 12288), (37, 4096, 1024), (128, 1024, 4096), (300, 1024, 2048), (2400, 512, 2048)] + EARLY_WEIGHTS)
 def test_linear_sees_weights_written_right_before(cuda, M, K, N):
     """The fused linear's launches overlap their predecessors: weights that the quantizer writes right before the call, round
     after round into the same buffer, are the ones that are used."""
@@ -186,6 +190,7 @@ def test_linear_sees_weights_written_right_before(cuda, M, K, N):
     x = cuda.randn((M, K), generator=g, device="cuda").half()
     ws = [cuda.randn((N, K), generator=g, device="cuda").half() for _ in range(8)]
     wq, sn = cuda.zeros((N, K), dtype=cuda.int8, device="cuda"), cuda.zeros((N,), dtype=cuda.float16, device="cuda")
+    assert (M, K, N) not in EARLY_WEIGHTS or pplb200.gemm_plan(M, N, K)["early_weights"] == 1
     lin = pplb200.W8A8Linear(wq, sn, None, max_tokens=M)
     got = []
     for w in ws:
