@@ -21,8 +21,9 @@ namespace {
 
 constexpr int RTPB = 256;
 
-template <int UNITS>
-__global__ void __launch_bounds__(RTPB)
+// FEW: few rows, each a chain of latencies; otherwise many rows per SM hide each other's, if their registers leave room for them.
+template <int UNITS, bool FEW>
+__global__ void __launch_bounds__(RTPB, !FEW && UNITS <= 4 ? 4 : 1)
 skip_rmsnorm_quantize_kernel(const half* __restrict__ input, const half* __restrict__ weight, const half* __restrict__ skip,
                              float eps, int64_t batch, int64_t dim, float up_scale, int32_t layout,
                              half* __restrict__ skip_out, half* __restrict__ scale_out, int8_t* __restrict__ q) {
@@ -32,14 +33,15 @@ skip_rmsnorm_quantize_kernel(const half* __restrict__ input, const half* __restr
     const int units = (int)(dim >> 4);
     const half* in_row = input + row * dim;
 
-    pdl_launch_dependents();
-    pdl_wait_prior_grid();
+    // Ordinary launches of thousands of one-unit rows spare themselves both instructions (7627 x 512: 9.0 -> 6.1 us).
+    if (UNITS > 1 || batch <= 8) pdl_wait_prior_grid();
 
-    // ---- load, skip add, statistics.  A row of a small batch is one chain of latencies, so everything it needs is requested
-    // before anything is used; short rows also keep the norm weights in registers for the second pass.
-    // (96 tokens of an 8192-wide layer, two norms, the QKV split rewritten alongside: 80.9 -> 75.7 us for the layer's nine launches.)
-    constexpr bool KEEP_W = UNITS <= 2;
-    uint4 zv[UNITS][2], wk[KEEP_W ? UNITS : 1][2];
+    // ---- load, skip add, statistics.  Volatile loads do not move ahead of stores.  With few rows, what four units per thread need is
+    // therefore requested before any of it is used or stored (a whole row up to 16384 wide, whose norm weights then also stay in registers
+    // for the second pass); otherwise rows up to that width are stored in the second pass.
+    constexpr int G = !FEW ? 1 : UNITS < 4 ? UNITS : 4;
+    constexpr bool KEEP_W = UNITS == G, STORE_LATE = !FEW && UNITS <= 4;
+    uint4 zv[UNITS][2], wk[G][2];
 #pragma unroll
     for (int u = 0; u < UNITS; ++u) {
         const int unit = u * blockDim.x + threadIdx.x;
@@ -50,55 +52,53 @@ skip_rmsnorm_quantize_kernel(const half* __restrict__ input, const half* __restr
             zv[u][1] = ld_global_16(in_row + off + 8);
         }
     }
-    uint4 sv[KEEP_W ? UNITS : 1][2];
-    if (KEEP_W) {
-#pragma unroll
-        for (int u = 0; u < UNITS; ++u) {
-            const int unit = u * blockDim.x + threadIdx.x;
-            if (unit < units) {
-                const int64_t off = (int64_t)unit << 4;
-                if (skip != nullptr) {
-                    sv[u][0] = ld_global_16(skip + row * dim + off);
-                    sv[u][1] = ld_global_16(skip + row * dim + off + 8);
-                }
-                wk[u][0] = ld_global_16(weight + off);
-                wk[u][1] = ld_global_16(weight + off + 8);
-            }
-        }
-    }
     float sumsq = 0.0f;
     float amax = eps; // the reference seeds the running maximum with eps (rms_norm.cu:58)
 #pragma unroll
-    for (int u = 0; u < UNITS; ++u) {
-        const int unit = u * blockDim.x + threadIdx.x;
-        if (unit < units) {
-            const int64_t off = (int64_t)unit << 4;
-            __half2* h = reinterpret_cast<__half2*>(&zv[u][0]);
-            uint4 wv[2];
-            if (skip != nullptr) {
-                uint4 st[2];
-                if (KEEP_W) { st[0] = sv[KEEP_W ? u : 0][0]; st[1] = sv[KEEP_W ? u : 0][1]; }
-                else { st[0] = ld_global_16(skip + row * dim + off); st[1] = ld_global_16(skip + row * dim + off + 8); }
-                const __half2* sh = reinterpret_cast<const __half2*>(st);
+    for (int u0 = 0; u0 < UNITS; u0 += G) {
+        uint4 sv[G][2];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) h[i] = __hadd2(h[i], sh[i]);
+        for (int g = 0; g < G; ++g) {
+            const int unit = (u0 + g) * blockDim.x + threadIdx.x;
+            if (unit < units) {
+                const int64_t off = (int64_t)unit << 4;
+                if (skip != nullptr) {
+                    sv[g][0] = ld_global_16(skip + row * dim + off);
+                    sv[g][1] = ld_global_16(skip + row * dim + off + 8);
+                }
+                wk[g][0] = ld_global_16(weight + off);
+                wk[g][1] = ld_global_16(weight + off + 8);
             }
-            *reinterpret_cast<uint4*>(skip_out + row * dim + off) = zv[u][0];
-            *reinterpret_cast<uint4*>(skip_out + row * dim + off + 8) = zv[u][1];
-            if (KEEP_W) { wv[0] = wk[KEEP_W ? u : 0][0]; wv[1] = wk[KEEP_W ? u : 0][1]; }
-            else { wv[0] = ld_global_16(weight + off); wv[1] = ld_global_16(weight + off + 8); }
-            const __half2* wh = reinterpret_cast<const __half2*>(wv);
+        }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float2 x = __half22float2(h[i]);
-                const float2 w = __half22float2(wh[i]);
-                sumsq = fmaf(x.x, x.x, sumsq);
-                sumsq = fmaf(x.y, x.y, sumsq);
-                amax = fmaxf(amax, fabsf(__fmul_rn(x.x, w.x)));
-                amax = fmaxf(amax, fabsf(__fmul_rn(x.y, w.y)));
+        for (int g = 0; g < G; ++g) {
+            const int unit = (u0 + g) * blockDim.x + threadIdx.x;
+            if (unit < units) {
+                const int64_t off = (int64_t)unit << 4;
+                __half2* h = reinterpret_cast<__half2*>(&zv[u0 + g][0]);
+                if (skip != nullptr) {
+                    const __half2* sh = reinterpret_cast<const __half2*>(&sv[g][0]);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) h[i] = __hadd2(h[i], sh[i]);
+                }
+                if (!STORE_LATE) {
+                    *reinterpret_cast<uint4*>(skip_out + row * dim + off) = zv[u0 + g][0];
+                    *reinterpret_cast<uint4*>(skip_out + row * dim + off + 8) = zv[u0 + g][1];
+                }
+                const __half2* wh = reinterpret_cast<const __half2*>(&wk[g][0]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const float2 x = __half22float2(h[i]);
+                    const float2 w = __half22float2(wh[i]);
+                    sumsq = fmaf(x.x, x.x, sumsq);
+                    sumsq = fmaf(x.y, x.y, sumsq);
+                    amax = fmaxf(amax, fabsf(__fmul_rn(x.x, w.x)));
+                    amax = fmaxf(amax, fabsf(__fmul_rn(x.y, w.y)));
+                }
             }
         }
     }
+    if (UNITS > 1 || batch <= 1024) pdl_launch_dependents();
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) {
         sumsq += __shfl_xor_sync(0xffffffffu, sumsq, m);
@@ -120,12 +120,23 @@ skip_rmsnorm_quantize_kernel(const half* __restrict__ input, const half* __restr
 #pragma unroll
     for (int u = 0; u < UNITS; ++u) {
         const int unit = u * blockDim.x + threadIdx.x;
+        if (!KEEP_W && u % G == 0) {
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const int64_t off = (int64_t)((u + g) * blockDim.x + threadIdx.x) << 4;
+                if (off < dim) {
+                    wk[g][0] = ld_global_16(weight + off);
+                    wk[g][1] = ld_global_16(weight + off + 8);
+                }
+            }
+        }
         if (unit < units) {
             const int64_t off = (int64_t)unit << 4;
-            uint4 wv[2];
-            if (KEEP_W) { wv[0] = wk[KEEP_W ? u : 0][0]; wv[1] = wk[KEEP_W ? u : 0][1]; }
-            else { wv[0] = ld_global_16(weight + off); wv[1] = ld_global_16(weight + off + 8); }
-            const __half2* wh = reinterpret_cast<const __half2*>(wv);
+            if (STORE_LATE) {
+                *reinterpret_cast<uint4*>(skip_out + row * dim + off) = zv[u][0];
+                *reinterpret_cast<uint4*>(skip_out + row * dim + off + 8) = zv[u][1];
+            }
+            const __half2* wh = reinterpret_cast<const __half2*>(&wk[u % G][0]);
             int qi[16];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -163,11 +174,18 @@ int32_t launch_skip_rmsnorm_quantize(cudaStream_t stream, const half* input, con
     if (threads > RTPB) threads = RTPB;
     const dim3 grid((unsigned)batch), block(threads);
     cudaError_t e;
+    // Few rows: up to two per SM (205 x 14336: 9.4 -> 6.4 us, 1052 x 11008 in the other form 17.4 -> 15.3).  A programmatic dependent only up
+    // to 8 rows (behind a GEMM, 8 x 4096: 6.7 -> 6.4 us): CTAs of more rows that start early pile up on the SMs that the GEMM before leaves
+    // free (64 x 8192, us as a dependent / as an ordinary launch: 10.7 / 9.1; 128 x 4096: 14.1 / 12.1; 1024 x 4096: 26.4 / 25.9).
+    const bool few = batch <= 2 * 148, pdl = batch <= 8;
+    auto go = [&](auto kernel) {
+        e = launch_ex(kernel, grid, block, stream, pdl, input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q);
+    };
     switch (bucket) {
-    case 1: e = launch_ex(skip_rmsnorm_quantize_kernel<1>, grid, block, stream, /*pdl=*/true, input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
-    case 2: e = launch_ex(skip_rmsnorm_quantize_kernel<2>, grid, block, stream, /*pdl=*/true, input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
-    case 4: e = launch_ex(skip_rmsnorm_quantize_kernel<4>, grid, block, stream, /*pdl=*/true, input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
-    default: e = launch_ex(skip_rmsnorm_quantize_kernel<8>, grid, block, stream, /*pdl=*/true, input, weight, skip, eps, batch, dim, up_scale, layout, skip_out, scale_out, q); break;
+    case 1: go(skip_rmsnorm_quantize_kernel<1, true>); break;
+    case 2: go(skip_rmsnorm_quantize_kernel<2, true>); break;
+    case 4: few ? go(skip_rmsnorm_quantize_kernel<4, true>) : go(skip_rmsnorm_quantize_kernel<4, false>); break;
+    default: few ? go(skip_rmsnorm_quantize_kernel<8, true>) : go(skip_rmsnorm_quantize_kernel<8, false>); break;
     }
     if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "skip_rmsnorm_quantize launch failed: %s", cudaGetErrorString(e));
     return RC_SUCCESS;
