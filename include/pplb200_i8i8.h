@@ -119,8 +119,8 @@ int32_t pplb200_i8i8_minmax_requantize_swiglu_fp16(pplb200_stream_t stream, cons
  * input int8 [M, K] (row stride lda); weight int8 [2 * act_dim, K] = [x rows | gate rows];
  * scale_N fp16 [2 * act_dim]; activated fp16 [M, act_dim] (the reference's `workspace`);
  * out_q int8 [M, act_dim]; out_q_scale fp16 [M].  ws: pplb200_i8i8_gate_up_swiglu_workspace_bytes().
- * Two kernels do this, one for large batches (act_dim % 128 == 0) and one for few tiles; large batches with another
- * act_dim run the two steps separately inside this call.  The workspace size accounts for the int32 buffer, or for the
+ * Two kernels do this, one for large batches (act_dim % 128 == 0) and one for few tiles; act_dim below 2368 and large batches
+ * with another act_dim run the two steps separately inside this call.  The workspace size accounts for the int32 buffer, or for the
  * partial row maxima that take its place.
  */
 int64_t pplb200_i8i8_gate_up_swiglu_workspace_bytes(int64_t M, int64_t act_dim, int64_t K);

@@ -210,8 +210,11 @@ namespace {
 // The fused form needs the CTA-pair kernel: enough 256-row x 128-channel tiles for every pair, and
 // the x / gate halves of the weight matrix aligned to the 128-row tiles.
 bool swiglu_fusable(int64_t M, int64_t D) { return M > 128 && D % 128 == 0 && ((M + 255) / 256) * (D / 128) >= kCtaPairs; }
-// Fused on single CTAs: batches for which the plain GEMM does not use CTA pairs either.
-bool swiglu_single(int64_t M, int64_t D) { return M <= 128 || ((M + 255) / 256) * ((2 * D + 255) / 256) < kCtaPairs; }
+// Fused on single CTAs: batches for which the plain GEMM does not use CTA pairs either, from 16 channels per SM up.  With fewer the raw GEMM
+// (narrow enough to fold K) and the stand-alone kernel are faster: us fused / in two steps, tokens x channels x K: 38 x 304 x 2048
+// 12.2 / 8.2, 89 x 576 x 4096 15.9 / 12.0, 47 x 2000 x 5120 12.3 / 10.3; up to 4736 channels the two are close, beyond
+// fusing wins (83 x 8608 x 2048 15.1 / 21.2).
+bool swiglu_single(int64_t M, int64_t D) { return D >= 16 * 2 * kCtaPairs && (M <= 128 || ((M + 255) / 256) * ((2 * D + 255) / 256) < kCtaPairs); }
 }
 
 int64_t pplb200_i8i8_gate_up_swiglu_workspace_bytes(int64_t M, int64_t act_dim, int64_t K) {
@@ -240,7 +243,7 @@ int32_t pplb200_i8i8_gate_up_swiglu_requant(pplb200_stream_t stream_, const void
 
     const bool pairs = swiglu_fusable(M, D);
     if (!pairs && !swiglu_single(M, D)) {
-        // many tokens, but halves that do not fall on the CTA pairs' 128-row tiles: raw int32 GEMM, then the stand-alone SwiGLU + re-quantize kernel
+        // few channels, or many tokens and halves that do not fall on the CTA pairs' 128-row tiles: raw int32 GEMM, then the stand-alone kernel
         void* acc = (char*)ws + round_up(M * 4 + 4, WS_ALIGN);
         int32_t rc = gemm_entry(stream, input, lda, weight, K, M, 2 * D, K, EPI_RAW_I32, nullptr, nullptr, nullptr, 0.f, 0.f, 0.f,
                                 nullptr, 0, acc, 2 * D, nullptr, nullptr, false);
