@@ -20,321 +20,15 @@
 // gemm_i8_fold_kernel below is a second form for few weight rows that needs no cluster.
 // Math and operand conventions as in gemm_i8_tcgen05.cu; reference:
 // src/ppl/kernel/llm/cuda/cublas/gemm.cu:171-363, src/ppl/kernel/llm/cuda/pmx/i8i8/quantize.cu:126-169.
-#include "common.cuh"
-#include "ptx.cuh"
+#include "gemm_i8_decode.cuh"
 
-#include <mutex>
 #include <string.h>
 
 namespace pplb200 {
 
+using namespace dec;
+
 namespace {
-
-constexpr int BW = 128;      // weight rows per tile (TMEM lanes)
-constexpr int BK = 128;      // bytes of K per stage
-constexpr int UMMA_K = 32;
-constexpr int PIECE_COLS = 8; // reduce-scatter granule: 32 lanes x 8 columns x 4 B = 1 KiB
-constexpr int PIECE_BYTES = 32 * PIECE_COLS * 4;
-constexpr int SMEM_BUDGET = 210 * 1024; // one CTA per SM: the whole shared memory is one TMA ring
-
-constexpr unsigned ST_DEC_PRODUCER = 16u, ST_DEC_MMA = 32u, ST_DEC_EPI = 64u;
-
-struct DecodeParams {
-    int32_t M, N;           // tokens, output columns (= weight rows; EPI_SWIGLU_F16: half of them)
-    int32_t tile_rows;      // weight rows per tile (a multiple of 8, <= 128; two-part tiles: per part), chosen so that the tiles fill the SMs
-    int32_t tile_tokens;    // tokens per tile (a multiple of 16, <= BT): blockIdx.z counts the token tiles
-    int32_t part_stride;    // two-part tiles: the second part starts this many weight rows after the first
-    int32_t w_box_bytes;    // bytes of weights that one K block brings in
-    int32_t w_slot_bytes;   // bytes between the slots of the weight ring
-    float beta;             // EPI_SWIGLU_F16
-    int32_t num_k_blocks;
-    int32_t mode;
-    void* out; int64_t ldc; // [M, ldc] int32 or fp16
-    const half* scale_m; const half* scale_n; const half* bias;
-    float down_m, down_n;
-    uint32_t* row_absmax_bits;
-    unsigned int* status;
-    // EPI_RAW_I32 with raw_affine != 0: out = raw_alpha * acc + raw_beta * out + raw_bias[n] (wrapping int32)
-    int32_t raw_affine, raw_alpha, raw_beta;
-    const int32_t* raw_bias;
-    int32_t early_weights;       // nothing that is still running writes the weights: load them before the dependency wait
-    int32_t w_stages;            // stages of the weight ring (tile_rows * 128 bytes each)
-    unsigned long long* stamps;  // optional diagnostics: 8 x uint64 per CTA, global-timer stamps of its phases
-};
-
-// Shared memory is two independent TMA rings: weight tiles come from HBM (about two microseconds away under
-// load), activation tiles from L2 (re-read by every CTA, about one microsecond away), so the weight ring gets
-// as many stages as fit and the activation ring only what its shorter latency needs.  With one ring of
-// {weights, activations} stages the activation bytes occupied half of the memory that could hold weights in
-// flight, and the weight stream ran latency-bound at two thirds of the HBM rate.
-constexpr int MAX_W_STAGES = 16;
-
-template <int BT> struct DCfg {
-    static constexpr int X_BYTES = BT * BK;
-    // Ring depths are multiples of the number of MMA issuers, so that every use of a slot belongs to the same issuer:
-    // a thread then never polls a barrier more than one phase ahead (a parity wait cannot tell phase u from u + 2).
-    // A two-part tile's weight stages are up to 32 KB: four of them need the room of two activation stages (448 x 14336 x 9216
-    // with two weight stages: 107 us).
-    template <bool DUAL> static constexpr int x_stages() { return BT == 128 && DUAL ? 4 : BT >= 64 ? 6 : 8; }
-    static constexpr int RING_BYTES = SMEM_BUDGET - 1024;
-    template <bool DUAL> static constexpr int x_ring_offset() { return RING_BYTES - x_stages<DUAL>() * X_BYTES; } // the weight ring grows from 0 up to here
-    static constexpr int SMEM_BYTES = SMEM_BUDGET;
-    // Two MMA-issuing threads, each with its own accumulator tile.  With at most 128 token columns an MMA is issued
-    // in 53 - 64 cycles, but the thread that issues it also waits on two barriers, polls the next two and commits
-    // to two per K block: about 780 cycles per K block in all, whatever the token count and wherever the operands
-    // come from (measured), which capped the weight stream at two thirds of the HBM rate.  Two threads taking
-    // alternate K blocks halve that; the epilogue adds the two partial tiles while it reads them.
-    static constexpr int NACC = 2;
-    template <bool DUAL> static constexpr int tmem_cols() { return NACC * BT * (DUAL ? 2 : 1) < 32 ? 32 : NACC * BT * (DUAL ? 2 : 1); }
-    static_assert(NACC * BT * 2 <= 512 && (BT & (BT - 1)) == 0, "tensor-memory allocation size");
-    // A lone warp per scheduler runs the epilogue at a fraction of an instruction per clock, so
-    // the accumulator columns are spread over GROUPS sets of four warps (one warp per TMEM lane
-    // quarter in each set).
-    static constexpr int GROUPS = BT >= 32 ? 4 : 2;
-    static constexpr int NUM_THREADS = 128 * GROUPS;
-    static constexpr int GROUP_COLS = BT / GROUPS;
-    static constexpr int LD_COLS = GROUP_COLS < 32 ? GROUP_COLS : 32; // columns per tcgen05.ld
-    static constexpr int PIECES = 4 * (BT / PIECE_COLS);
-    // EPI_SWIGLU_F16: once the main loop is over, [received partials | partner accumulators | output tile] share the rings
-    static constexpr int SWIGLU_PARTNER = 72 * 1024, SWIGLU_OUT = 104 * 1024; // at most 72 KB are received (split in 7)
-    static_assert(SWIGLU_OUT + BT * 128 * 2 <= RING_BYTES, "swiglu epilogue buffers fit the rings");
-    static_assert(LD_COLS == 8 || LD_COLS == 16 || LD_COLS == 32, "tcgen05.ld shape");
-    static_assert(BT == 16 || BT == 32 || BT == 64 || BT == 128, "token tile");
-    static_assert(RING_BYTES % 1024 == 0 && RING_BYTES - 6 * X_BYTES >= 6 * BW * BK && RING_BYTES - 4 * X_BYTES >= 8 * BW * BK,
-                  "room for at least six full weight tiles, or four of two parts");
-    // the rings double as the receive buffer of the reduce-scatter once the main loop is over
-    static_assert(PIECES * PIECE_BYTES <= RING_BYTES, "receive buffer fits the rings");
-};
-
-__device__ __forceinline__ unsigned long long globaltimer_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ uint32_t cluster_nctarank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_smem_addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
-    return r;
-}
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-    return v;
-}
-
-// Per-token maximum over the 32 lanes of a warp for NV tokens held as a[0..NV) in every lane
-// (halving butterfly: NV - 1 shuffles instead of NV full warp reductions).  Returns, in every lane,
-// the maximum for token (lane % NV).
-template <int NV>
-__device__ __forceinline__ uint32_t warp_token_max(uint32_t (&a)[NV], int lane) {
-#pragma unroll
-    for (int off = NV / 2; off >= 1; off >>= 1) {
-        const bool upper = (lane & off) != 0;
-#pragma unroll
-        for (int i = 0; i < off; ++i) {
-            const uint32_t send = upper ? a[i] : a[i + off];
-            const uint32_t keep = upper ? a[i + off] : a[i];
-            const uint32_t got = __shfl_xor_sync(0xffffffffu, send, off);
-            a[i] = keep > got ? keep : got;
-        }
-    }
-    uint32_t r = a[0];
-#pragma unroll
-    for (int off = NV; off < 32; off <<= 1) {
-        const uint32_t got = __shfl_xor_sync(0xffffffffu, r, off);
-        r = r > got ? r : got;
-    }
-    return r;
-}
-
-// Largest |y| per token of a finished fp16 tile [tokens][cols] in shared memory (cols a multiple of 8), one global atomic per token.
-// Neighbouring lanes share a token and read 16 bytes each, so a tile takes a few loads per thread and up to five shuffles.  Taken from
-// the accumulator registers instead, where a token's columns lie in 32 lanes, the maxima cost 31 shuffles per 32 tokens and
-// shared-memory atomics (128 x 12288 x 4096: the GEMM's epilogue 4.4 us, now 2.9).  NaNs are dropped, as fmax does.  Called by every
-// thread of the CTA.
-template <int THREADS>
-__device__ __forceinline__ void staged_row_maxima(uint32_t tile, int tokens, int cols, uint32_t* row_absmax_bits) {
-    int lanes = 1; // per token
-    while (lanes < 32 && lanes * 2 * tokens <= THREADS) lanes *= 2;
-    const int t = (int)threadIdx.x / lanes;
-    __half2 m2 = __float2half2_rn(0.0f);
-    if (t < tokens) {
-        for (int c = ((int)threadIdx.x & (lanes - 1)) * 8; c < cols; c += lanes * 8) {
-            const uint4 v = ld_shared_v4(tile + (uint32_t)(t * cols + c) * 2u);
-            const __half2* h = reinterpret_cast<const __half2*>(&v);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) m2 = __hmax2(m2, __habs2(h[j]));
-        }
-    }
-    uint32_t bits = __float_as_uint(fmaxf(__low2float(m2), __high2float(m2)));
-    for (int off = lanes >> 1; off >= 1; off >>= 1) {
-        const uint32_t other = __shfl_xor_sync(0xffffffffu, bits, off);
-        bits = other > bits ? other : bits;
-    }
-    if (((int)threadIdx.x & (lanes - 1)) == 0 && t < tokens && bits != 0u) atomicMax(row_absmax_bits + t, bits);
-}
-
-template <int N> struct TmemLd;
-template <> struct TmemLd<32> {
-    __device__ static __forceinline__ void run(uint32_t taddr, uint32_t (&r)[32]) { ptx::tmem_ld_32x32(taddr, r); }
-};
-template <> struct TmemLd<8> {
-    __device__ static __forceinline__ void run(uint32_t taddr, uint32_t (&r)[8]) {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-            : "r"(taddr)
-            : "memory");
-    }
-};
-template <> struct TmemLd<16> {
-    __device__ static __forceinline__ void run(uint32_t taddr, uint32_t (&r)[16]) {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(taddr)
-            : "memory");
-    }
-};
-
-// Reads N columns of each of the first `valid` accumulator tiles (STRIDE columns apart) and returns their sum.
-template <int N, int NACC, int STRIDE>
-__device__ __forceinline__ void tmem_ld_sum(uint32_t taddr, uint32_t (&acc)[N], int valid) {
-    TmemLd<N>::run(taddr, acc);
-    ptx::tmem_ld_wait();
-#pragma unroll
-    for (int a = 1; a < NACC; ++a) { // one partial tile at a time: two register arrays live, not NACC
-        if (a >= valid) break; // warp-uniform: that issuer had no K block
-        uint32_t part[N];
-        TmemLd<N>::run(taddr + a * STRIDE, part);
-        ptx::tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < N; ++j) acc[j] += part[j];
-    }
-}
-
-// Brings this CTA's weight stages into L2 while the kernel still waits for its predecessors: two at once, then one per 400
-// cycles (11 KB x 140 CTAs: about the HBM rate) until the loads proper start.  Unpaced, tens of megabytes of requests queue up
-// in front of the few that the small kernel still running waits for (a quantizer, a norm).  One thread of an idle warp.
-// Back to back in a graph, us without / all at once / paced: layer of 8 tokens 56.1 / 53.5 / 53.5, layer shard of 96 tokens
-// 68.9 / 65.9 / 65.2, linear 37 x 11008 x 4096 17.6 / 17.0 / 16.5, 96 x 4096 x 8192 15.6 / 14.7 / 14.3.
-template <typename Fetch>
-__device__ __forceinline__ void prefetch_weights(int stages, int* loads_started, Fetch fetch) {
-    long long due = clock64();
-    for (int i = 0; i < stages; ++i) {
-        if (i >= 2) {
-            due += 400;
-            while (clock64() < due && *static_cast<volatile int*>(loads_started) == 0) {}
-        }
-        if (*static_cast<volatile int*>(loads_started) != 0) break;
-        fetch(i);
-    }
-}
-
-// One activated value of the fused gate + up projection, operation by operation as the stand-alone kernel of
-// activation_requant.cu computes it.
-__device__ __forceinline__ float swiglu_value(uint32_t xi, uint32_t gi, float sx, float sg, float down_n, float ts, float beta) {
-    const float x = __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)xi, sx), down_n), ts);
-    const float g = __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)gi, sg), down_n), ts);
-    return __fmul_rn(__fdiv_rn(x, __fadd_rn(1.0f, __expf(__fmul_rn(-x, beta)))), g);
-}
-
-// SwiGLU over the accumulators this CTA owns: activated fp16 values into the output tile [token][channel] at
-// ring + SWIGLU_OUT, row maxima (of the fp32 values) into token_absmax.  Called by every thread of the CTA.
-template <int BT, bool DUAL>
-__device__ __forceinline__ void swiglu_epilogue(const DecodeParams& p, uint32_t taddr_row, uint32_t ring, uint32_t S, uint32_t rank,
-                                                uint32_t own0, uint32_t slot0, uint32_t step_div, uint32_t step_rem, uint32_t slot_carry,
-                                                uint32_t recv_pieces, bool have_acc, int nkb, int col_begin, int col_end, int nl, int n,
-                                                int q, int lane, const float (&sn)[2], const float* token_scale, uint32_t* token_absmax, int M) {
-    using C = DCfg<BT>;
-    constexpr int NPART = DUAL ? 2 : 1;
-    const int valid = nkb < C::NACC ? nkb : C::NACC;
-    const bool ok = nl < p.tile_rows && n < p.N;
-    auto load8 = [&](int col, uint32_t slot, uint32_t (&v)[8]) { // eight tokens of this lane's row, K slices summed
-        if (have_acc) {
-            tmem_ld_sum<8, C::NACC, NPART * BT>(taddr_row + col, v, valid);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = 0u;
-        }
-        for (uint32_t r = 0; r + 1 < S; ++r) {
-            const uint32_t addr = ring + (r * recv_pieces + slot) * PIECE_BYTES + lane * 32;
-            const uint4 a = ld_shared_v4(addr), b = ld_shared_v4(addr + 16);
-            v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-            v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
-        }
-    };
-    const uint32_t partner = ring + C::SWIGLU_PARTNER + (uint32_t)nl * 4u; // [token][64 rows] int32
-    const int side = q >> 1;                                              // lanes of the x rows (0) or of the gate rows (1)
-    if (!DUAL) {
-        // each half of the lanes computes every other chunk and hands the accumulators of the rest to the other half
-        uint32_t own = own0, slot = slot0;
-#pragma unroll 1
-        for (int c0 = col_begin; c0 < col_end; c0 += PIECE_COLS) {
-            if (c0 >= M) break;
-            if (own == rank && ((c0 / PIECE_COLS) & 1) != side) {
-                uint32_t v[8];
-                load8(c0, slot, v);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(partner + (uint32_t)(c0 + j) * 256u), "r"(v[j]) : "memory");
-            }
-            own += step_rem; slot += step_div;
-            if (own >= S) { own -= S; slot += slot_carry; }
-        }
-        __syncthreads();
-    }
-    uint32_t own = own0, slot = slot0;
-#pragma unroll 1
-    for (int c0 = col_begin; c0 < col_end; c0 += PIECE_COLS) {
-        if (c0 >= M) break;
-        if (DUAL || (own == rank && ((c0 / PIECE_COLS) & 1) == side)) {
-            uint32_t v[8], w[8], absbits[8];
-            load8(c0, slot, v);
-            if (DUAL) {
-                load8(BT + c0, slot, w);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[j]) : "r"(partner + (uint32_t)(c0 + j) * 256u) : "memory");
-            }
-            const float4 ts0 = *reinterpret_cast<const float4*>(&token_scale[c0]);
-            const float4 ts1 = *reinterpret_cast<const float4*>(&token_scale[c0 + 4]);
-            const float ts[8] = {ts0.x, ts0.y, ts0.z, ts0.w, ts1.x, ts1.y, ts1.z, ts1.w};
-#pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const bool swap = !DUAL && side != 0; // this lane holds the gate, its partner the x value
-                const float r = swiglu_value(swap ? w[j] : v[j], swap ? v[j] : w[j], sn[0], sn[1], p.down_n, ts[j], p.beta);
-                const float a = ok ? fabsf(r) : 0.0f;
-                absbits[j] = a == a ? __float_as_uint(a) : 0u; // NaNs are dropped, as fmax does
-                if (nl < p.tile_rows)
-                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(ring + C::SWIGLU_OUT + ((uint32_t)(c0 + j) * (uint32_t)p.tile_rows + (uint32_t)nl) * 2u),
-                                 "h"(__half_as_ushort(__float2half_rn(r))) : "memory");
-            }
-            const uint32_t tok_max = warp_token_max<8>(absbits, lane);
-            if (lane < 8 && c0 + lane < M && tok_max != 0u) atomicMax(&token_absmax[c0 + lane], tok_max);
-        }
-        own += step_rem; slot += step_div;
-        if (own >= S) { own -= S; slot += slot_carry; }
-    }
-}
 
 // grid = (S, weight-row tiles); cluster = (S, 1, 1): the S CTAs of a cluster share one weight-row
 // tile and each takes a contiguous range of K blocks.
@@ -917,80 +611,8 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     pdl_launch_dependents();
     const unsigned long long t_main = p.stamps ? globaltimer_ns() : 0ull;
 
-    // ---- the diagonal blocks, [part][token][row], into the dead weight ring
-    {
-        const int q = warp & 3, grp = warp >> 2;         // TMEM lane quarter, slice of the tokens
-        const int f = q / ROW_WARPS, row = (q % ROW_WARPS) * 32 + lane;
-        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(f * p.tile_tokens);
-        const uint32_t dst = ring + (uint32_t)(f * BT * C::ROWS + row) * 4u;
-#pragma unroll 1
-        for (int c0 = grp * C::GROUP_COLS; c0 < (grp + 1) * C::GROUP_COLS; c0 += 8) {
-            if (c0 >= p.M) break;
-            uint32_t v[8];
-            if (acc_ready) {
-                tmem_ld_sum<8, 2, F * BT>(taddr + c0, v, per_part < 2 ? per_part : 2);
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = 0u;
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (uint32_t)((c0 + j) * C::ROWS) * 4u), "r"(v[j]) : "memory");
-        }
-    }
-    ptx::tc_fence_before();
-    __syncthreads();
-    const unsigned long long t_exchange = p.stamps ? globaltimer_ns() : 0ull;
-
-    // ---- sums and epilogue: a warp handles 32 rows of one token at a time
-    const uint32_t src = ring + (uint32_t)nl * 4u;
-#pragma unroll 4
-    for (int m = warp / ROW_WARPS; m < p.M; m += (C::NUM_THREADS / 32) / ROW_WARPS) {
-        uint32_t v = 0;
-#pragma unroll
-        for (int f = 0; f < F; ++f) {
-            uint32_t t;
-            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(t) : "r"(src + (uint32_t)((f * BT + m) * C::ROWS) * 4u) : "memory");
-            v += t;
-        }
-        if (p.mode == EPI_RAW_I32) {
-            if (n_ok) {
-                int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)m * p.ldc + n;
-                if (p.raw_affine) {
-                    v = (uint32_t)p.raw_alpha * v + (p.raw_bias != nullptr ? (uint32_t)p.raw_bias[n] : 0u);
-                    if (p.raw_beta != 0) v += (uint32_t)p.raw_beta * (uint32_t)*dst;
-                }
-                *dst = (int32_t)v;
-            }
-            continue;
-        }
-        float t = __fmul_rn((float)(int32_t)v, sn);
-        t = __fmul_rn(t, p.down_n);
-        t = __fmul_rn(t, token_scale[m]);
-        const half h = __hadd(__float2half_rn(t), bias_h);
-        if (n_ok) reinterpret_cast<half*>(p.out)[(int64_t)m * p.ldc + n] = h;
-        if (p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
-            const float a = n_ok ? fabsf(__half2float(h)) : 0.0f;
-            const uint32_t bits = __reduce_max_sync(0xffffffffu, a == a ? __float_as_uint(a) : 0u); // NaNs are dropped, as fmax does
-            if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(x_ring + (uint32_t)((warp % ROW_WARPS) * BT + m) * 4u), "r"(bits) : "memory");
-        }
-    }
-    if (p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
-        // Neighbouring tokens leave in one instruction per CTA.  One global atomic per token and warp as the rows are finished,
-        // all CTAs on the same few lines of L2, took as long as the rest of the kernel (59 x 8928 x 2944: the call 20.9 -> 11.8 us).
-        // They meet in the dead activation ring, not in memory of their own: 1 KB more, and under the 196 KB carve-out that the driver picks for
-        // this kernel no quantizer CTA starts beside it any more (70 x 8192 x 4096 without re-quantizing: 12.9 -> 13.8 us).
-        __syncthreads();
-        for (int m = threadIdx.x; m < BT && m < p.M; m += C::NUM_THREADS) {
-            uint32_t bits = 0u;
-#pragma unroll
-            for (int w = 0; w < ROW_WARPS; ++w) {
-                uint32_t t;
-                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(t) : "r"(x_ring + (uint32_t)(w * BT + m) * 4u) : "memory");
-                bits = t > bits ? t : bits;
-            }
-            if (bits != 0u) atomicMax(p.row_absmax_bits + m, bits);
-        }
-    }
+    const unsigned long long t_exchange = fold_epilogue<BT, F, F * BT, C::NUM_THREADS, false>(p, tmem_base, ring, x_ring, per_part < 2 ? per_part : 2, acc_ready,
+                                                                                       nl, n, n_ok, sn, bias_h, token_scale);
     if (warp == 1) {
         __syncwarp();
         ptx::tc_fence_after();
@@ -1003,48 +625,6 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
 }
 
 // ---- host side ---------------------------------------------------------------------------------
-
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qr) == cudaSuccess &&
-            qr == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(sym);
-    });
-    return fn;
-}
-
-// Output [M, N] (fp16 or int32, leading dimension ldc elements); box = {tile_rows weight rows, BT tokens}, dense.
-bool make_out_map(CUtensorMap* map, void* base, int64_t M, int64_t N, int64_t ldc, int elem_bytes, int box_cols, int box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
-    const cuuint64_t strides[1] = {(cuuint64_t)(ldc * elem_bytes)};
-    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
-    const cuuint32_t elem_strides[2] = {1, 1};
-    return fn(map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_INT32, 2, base, dims, strides, box,
-              elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld, int box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld};
-    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
-    const cuuint32_t elem_strides[2] = {1, 1};
-    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem_strides,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 
 struct DecDeviceInfo {
     bool ready = false;
@@ -1092,27 +672,38 @@ const DecDeviceInfo* dec_device_info() {
         if (!set_fold_attr<16, 2>() || !set_fold_attr<16, 4>() || !set_fold_attr<32, 2>() || !set_fold_attr<32, 4>() ||
             !set_fold_attr<64, 2>() || !set_fold_attr<64, 4>() || !set_fold_attr<128, 2>())
             return nullptr;
+        if (!token_pair_setup()) return nullptr;
         d.ready = true;
     }
     return &d;
 }
 
-// How a launch is cut: `tokens` x `rows` tiles (two-part tiles: rows per part), K split over S CTAs.
-struct DecodePlan {
-    int tokens, token_tiles, rows, row_tiles, S;
-    bool dual;
-    int fold; // parts K is folded into (gemm_i8_fold_kernel), 0 = row tiles
-};
-
-// Rows per tile for `cap` tiles that can run at once: the smallest multiple of 8 with which `columns` output columns
-// still are one wave -- e.g. 12288 weight rows: 140 tiles of 88 rows on 148 SMs instead of 96 tiles of 128 rows on 96.
-int rows_for(int64_t columns, int64_t cap, int max_rows) {
-    if (cap <= 0 || (columns + max_rows - 1) / max_rows > cap) return max_rows;
-    const int64_t r = ((columns + cap - 1) / cap + 7) / 8 * 8;
-    return r < 8 ? 8 : r < max_rows ? (int)r : max_rows;
-}
-
 int variant_of(int64_t M) { return M <= 16 ? 0 : M <= 32 ? 1 : M <= 64 ? 2 : 3; }
+
+// CTA pairs that share the activations (gemm_i8_token_pair_kernel) instead of the form in `best`.  They bring in half of the
+// activations per CTA and have one barrier per stage, but setting a pair up costs about 0.4 us more, and one MMA of a
+// pair at least 60 cycles for up to 120 columns, 2 per 4 columns beyond.  So they pay where there are stages enough to earn
+// the fixed part back.  Median time of quantizer + GEMM, best single-CTA form / pair, over 3035 random shapes of 17 .. 128 tokens:
+//   folded in four: 48 tokens 0.95 up to 7 stages, 1.00 up to 15, 1.07 from 16, 1.12 from 24; 32 tokens 1.01 at most
+//   folded in two:  80 tokens 1.05 from 8 stages, 1.12 from 24; 128 tokens 0.97 from 8, 1.02 from 16, 1.12 from 24; 64 tokens 1.00 at most
+//   whole K: 1.05 (up to 64 tokens) and 1.11 (beyond) up to 63 stages; then the weight stream bounds both, 0.93 .. 1.00
+// With these lines 801 of the shapes go to pairs; 8 of them lose more than 3 %.
+void plan_pair(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t kb, DecodePlan& best) {
+    if ((best.S > 1 && !best.fold) || best.dual) return;
+    const int ctas = dev.sms / 2 * 2;
+    const int t16 = (int)((M + 15) / 16 * 16), t32 = (int)((M + 31) / 32 * 32);
+    int F = 0;
+    if (best.fold == 4 && t16 >= 48 && (kb + 3) / 4 >= 16) F = 4;
+    else if (best.fold != 4 && t16 >= 80 && columns <= (int64_t)ctas * (BW / 2) && (kb + 1) / 2 >= t16 / 8) F = 2;
+    else if (!best.fold && columns <= (int64_t)ctas * BW && kb < 64) F = 1;
+    if (F == 0) return;
+    best.pair = true;
+    best.S = 1;
+    best.fold = F == 1 ? 0 : F;
+    best.tokens = F == 1 ? t32 : t16;
+    best.rows = rows_for(columns, ctas, BW / F);
+    best.row_tiles = (int)(((columns + best.rows - 1) / best.rows + 1) / 2 * 2);
+}
 
 // Up to 128 tokens: one token tile.  Where tiles of full height leave SMs idle, K is shared: by the S CTAs of a cluster, or
 // folded onto the lanes of one CTA (gemm_i8_fold_kernel).  All forms that run as one wave are modelled in SM cycles per CTA: a
@@ -1169,6 +760,7 @@ DecodePlan plan_small(const DecDeviceInfo& dev, int64_t M, int64_t columns, int6
             best.fold = F;
         }
     }
+    if (!swiglu) plan_pair(dev, M, columns, kb, best);
     return best;
 }
 
@@ -1199,9 +791,29 @@ DecodePlan plan_medium(const DecDeviceInfo& dev, int64_t M, int64_t columns, int
                 const double cost = (double)waves * ((num_k_blocks + S - 1) / S * kb + 3000.0 + (S > 1 ? 12000.0 : 0.0));
                 if (cost < best_cost) {
                     best_cost = cost;
-                    best = {tokens, (int)token_tiles, rows, (int)row_tiles, S, dual != 0, 0};
+                    best = {tokens, (int)token_tiles, rows, (int)row_tiles, S, dual != 0, 0, false};
                 }
             }
+        }
+    }
+    // CTA pairs that share the activations (gemm_i8_token_pair_kernel), up to 256 tokens per tile, against a whole K per CTA.  Their K
+    // block: 65 bytes per cycle, 380 cycles of bookkeeping, a fixed 1500 and 8 per token.  Fitted to 1881 shapes of 129 .. 1024 tokens:
+    // on average 8 % faster than without pairs and 0.4 % slower than the faster of the two; 5 % of distance keeps close calls where they were.
+    if (swiglu || best.S > 1) return best;
+    best_cost *= 0.95;
+    for (int64_t t = (M + 255) / 256; t <= (M + 63) / 64; ++t) {
+        const int tokens = (int)(((M + t - 1) / t + 31) / 32 * 32);
+        const int64_t token_tiles = (M + tokens - 1) / tokens, ctas = dev.sms / 2 / token_tiles * 2;
+        if (ctas == 0 || columns > ctas * BW) continue; // one wave
+        const int rows = rows_for(columns, ctas, BW);
+        double kb = (rows + tokens / 2) * (double)BK / 65.0;
+        const double mma = tokens < 120 ? 240.0 : tokens * 2.0;
+        if (kb < mma) kb = mma;
+        if (kb < 380.0) kb = 380.0;
+        const double cost = num_k_blocks * kb + 1500.0 + 8.0 * tokens;
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = {tokens, (int)token_tiles, rows, (int)(((columns + rows - 1) / rows + 1) / 2 * 2), 1, false, 0, true};
         }
     }
     return best;
@@ -1314,6 +926,9 @@ bool gemm_preloads_weights(int64_t M, int64_t N, int64_t K) {
     // Starting late exposes part of the GEMM's launch, unless the quantizer itself takes long; starting early, the weight ring fills
     // only once the quantizer has ended.  Early -> late, us, tokens x N x K, weights from L2 (warm) or HBM (cold):
     // one wide MMA (fold * M columns) or a short K: 83 x 7168 x 4096 cold 13.2 -> 14.4, 2 x 5120 x 1024 cold 5.3 -> 5.5; else 1 x 8192 x 4096 warm 8.8 -> 8.4, 16 x 9216 x 4784 cold 13.3 -> 12.6
+    // On pairs (2275 shapes, cold; median early / late): folded in four late, 1.02; folded in two early, 0.98 below K 6144 and 1.00 beyond; whole K early,
+    // 0.90 .. 0.96 below K 6144 -- but for the widest tiles, where graph replays are 2 % faster early and eager calls 1 % late.
+    if (plan.pair) return plan.fold == 4 || (plan.fold == 0 && M > 112 && M * K >= 320 * 1024);
     if (plan.fold) return plan.fold * M <= 128 && K >= 2048;
     // 16 x 5120 x 14336 warm 15.0 -> 14.3, 48 x 1024 x 11008 cold 12.5 -> 12.1
     if (plan.S > 1) return true;
@@ -1331,14 +946,21 @@ int32_t gemm_decode_plan(int64_t M, int64_t columns, int64_t K, bool swiglu, int
     return RC_SUCCESS;
 }
 
+int32_t gemm_decode_on_pairs(int64_t M, int64_t columns, int64_t K) {
+    const DecDeviceInfo* dev = dec_device_info();
+    if (!dev) return fail(RC_DEVICE_RUNTIME_ERROR, "device set-up failed: %s", cudaGetErrorString(cudaGetLastError())), -1;
+    return (M > 128 ? plan_medium(*dev, M, columns, (int)((K + BK - 1) / BK), false) : plan_small(*dev, M, columns, K, false)).pair ? 1 : 0;
+}
+
 int32_t launch_gemm_decode(cudaStream_t stream, const GemmArgs& a, unsigned int* status, bool pdl) {
     const DecDeviceInfo* dev = dec_device_info();
     if (!dev) return fail(RC_DEVICE_RUNTIME_ERROR, "device set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
     const bool swiglu = a.mode == EPI_SWIGLU_F16;
     const int64_t columns = swiglu ? a.N / 2 : a.N;
-    if (a.M > 128) return launch_bt<128>(stream, a, plan_medium(*dev, a.M, columns, (int)((a.K + BK - 1) / BK), swiglu), status, pdl);
+    const DecodePlan plan = a.M > 128 ? plan_medium(*dev, a.M, columns, (int)((a.K + BK - 1) / BK), swiglu) : plan_small(*dev, a.M, columns, a.K, swiglu);
+    if (plan.pair) return launch_token_pair(stream, a, plan, make_params(a, status), pdl);
+    if (a.M > 128) return launch_bt<128>(stream, a, plan, status, pdl);
     const int variant = variant_of(a.M);
-    const DecodePlan plan = plan_small(*dev, a.M, columns, a.K, swiglu);
     if (plan.fold == 4) {
         return variant == 0 ? launch_fold<16, 4>(stream, a, *dev, status, pdl)
              : variant == 1 ? launch_fold<32, 4>(stream, a, *dev, status, pdl) : launch_fold<64, 4>(stream, a, *dev, status, pdl);

@@ -1,0 +1,495 @@
+// Shared by the small-batch GEMM kernels (gemm_i8_decode.cu, gemm_i8_token_pair.cu): parameters, tensor-memory and cluster
+// helpers, the epilogue pieces, tensor maps and the cut of a launch.
+#pragma once
+
+#include "common.cuh"
+#include "ptx.cuh"
+
+#include <mutex>
+
+namespace pplb200 {
+
+namespace dec {
+
+constexpr int BW = 128;      // weight rows per tile (TMEM lanes)
+constexpr int BK = 128;      // bytes of K per stage
+constexpr int UMMA_K = 32;
+constexpr int PIECE_COLS = 8; // reduce-scatter granule: 32 lanes x 8 columns x 4 B = 1 KiB
+constexpr int PIECE_BYTES = 32 * PIECE_COLS * 4;
+constexpr int SMEM_BUDGET = 210 * 1024; // one CTA per SM: the whole shared memory is one TMA ring
+
+constexpr unsigned ST_DEC_PRODUCER = 16u, ST_DEC_MMA = 32u, ST_DEC_EPI = 64u;
+
+struct DecodeParams {
+    int32_t M, N;           // tokens, output columns (= weight rows; EPI_SWIGLU_F16: half of them)
+    int32_t tile_rows;      // weight rows per tile (a multiple of 8, <= 128; two-part tiles: per part), chosen so that the tiles fill the SMs
+    int32_t tile_tokens;    // tokens per tile (a multiple of 16, <= BT): blockIdx.z counts the token tiles
+    int32_t part_stride;    // two-part tiles: the second part starts this many weight rows after the first
+    int32_t w_box_bytes;    // bytes of weights that one K block brings in
+    int32_t fold_box;       // CTA pairs, folded K: one 3-D box brings all parts (make_fold_map), else a 2-D box per part
+    int32_t w_slot_bytes;   // bytes between the slots of the weight ring
+    float beta;             // EPI_SWIGLU_F16
+    int32_t num_k_blocks;
+    int32_t mode;
+    void* out; int64_t ldc; // [M, ldc] int32 or fp16
+    const half* scale_m; const half* scale_n; const half* bias;
+    float down_m, down_n;
+    uint32_t* row_absmax_bits;
+    unsigned int* status;
+    // EPI_RAW_I32 with raw_affine != 0: out = raw_alpha * acc + raw_beta * out + raw_bias[n] (wrapping int32)
+    int32_t raw_affine, raw_alpha, raw_beta;
+    const int32_t* raw_bias;
+    int32_t early_weights;       // nothing that is still running writes the weights: load them before the dependency wait
+    int32_t w_stages;            // stages of the weight ring (tile_rows * 128 bytes each)
+    unsigned long long* stamps;  // optional diagnostics: 8 x uint64 per CTA, global-timer stamps of its phases
+};
+
+// Shared memory is two independent TMA rings: weight tiles come from HBM (about two microseconds away under
+// load), activation tiles from L2 (re-read by every CTA, about one microsecond away), so the weight ring gets
+// as many stages as fit and the activation ring only what its shorter latency needs.  With one ring of
+// {weights, activations} stages the activation bytes occupied half of the memory that could hold weights in
+// flight, and the weight stream ran latency-bound at two thirds of the HBM rate.
+constexpr int MAX_W_STAGES = 16;
+
+template <int BT> struct DCfg {
+    static constexpr int X_BYTES = BT * BK;
+    // Ring depths are multiples of the number of MMA issuers, so that every use of a slot belongs to the same issuer:
+    // a thread then never polls a barrier more than one phase ahead (a parity wait cannot tell phase u from u + 2).
+    // A two-part tile's weight stages are up to 32 KB: four of them need the room of two activation stages (448 x 14336 x 9216
+    // with two weight stages: 107 us).
+    template <bool DUAL> static constexpr int x_stages() { return BT == 128 && DUAL ? 4 : BT >= 64 ? 6 : 8; }
+    static constexpr int RING_BYTES = SMEM_BUDGET - 1024;
+    template <bool DUAL> static constexpr int x_ring_offset() { return RING_BYTES - x_stages<DUAL>() * X_BYTES; } // the weight ring grows from 0 up to here
+    static constexpr int SMEM_BYTES = SMEM_BUDGET;
+    // Two MMA-issuing threads, each with its own accumulator tile.  With at most 128 token columns an MMA is issued
+    // in 53 - 64 cycles, but the thread that issues it also waits on two barriers, polls the next two and commits
+    // to two per K block: about 780 cycles per K block in all, whatever the token count and wherever the operands
+    // come from (measured), which capped the weight stream at two thirds of the HBM rate.  Two threads taking
+    // alternate K blocks halve that; the epilogue adds the two partial tiles while it reads them.
+    static constexpr int NACC = 2;
+    template <bool DUAL> static constexpr int tmem_cols() { return NACC * BT * (DUAL ? 2 : 1) < 32 ? 32 : NACC * BT * (DUAL ? 2 : 1); }
+    static_assert(NACC * BT * 2 <= 512 && (BT & (BT - 1)) == 0, "tensor-memory allocation size");
+    // A lone warp per scheduler runs the epilogue at a fraction of an instruction per clock, so
+    // the accumulator columns are spread over GROUPS sets of four warps (one warp per TMEM lane
+    // quarter in each set).
+    static constexpr int GROUPS = BT >= 32 ? 4 : 2;
+    static constexpr int NUM_THREADS = 128 * GROUPS;
+    static constexpr int GROUP_COLS = BT / GROUPS;
+    static constexpr int LD_COLS = GROUP_COLS < 32 ? GROUP_COLS : 32; // columns per tcgen05.ld
+    static constexpr int PIECES = 4 * (BT / PIECE_COLS);
+    // EPI_SWIGLU_F16: once the main loop is over, [received partials | partner accumulators | output tile] share the rings
+    static constexpr int SWIGLU_PARTNER = 72 * 1024, SWIGLU_OUT = 104 * 1024; // at most 72 KB are received (split in 7)
+    static_assert(SWIGLU_OUT + BT * 128 * 2 <= RING_BYTES, "swiglu epilogue buffers fit the rings");
+    static_assert(LD_COLS == 8 || LD_COLS == 16 || LD_COLS == 32, "tcgen05.ld shape");
+    static_assert(BT == 16 || BT == 32 || BT == 64 || BT == 128, "token tile");
+    static_assert(RING_BYTES % 1024 == 0 && RING_BYTES - 6 * X_BYTES >= 6 * BW * BK && RING_BYTES - 4 * X_BYTES >= 8 * BW * BK,
+                  "room for at least six full weight tiles, or four of two parts");
+    // the rings double as the receive buffer of the reduce-scatter once the main loop is over
+    static_assert(PIECES * PIECE_BYTES <= RING_BYTES, "receive buffer fits the rings");
+};
+
+__device__ __forceinline__ unsigned long long globaltimer_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_nctarank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_cta(uint32_t local_smem_addr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
+// Per-token maximum over the 32 lanes of a warp for NV tokens held as a[0..NV) in every lane
+// (halving butterfly: NV - 1 shuffles instead of NV full warp reductions).  Returns, in every lane,
+// the maximum for token (lane % NV).
+template <int NV>
+__device__ __forceinline__ uint32_t warp_token_max(uint32_t (&a)[NV], int lane) {
+#pragma unroll
+    for (int off = NV / 2; off >= 1; off >>= 1) {
+        const bool upper = (lane & off) != 0;
+#pragma unroll
+        for (int i = 0; i < off; ++i) {
+            const uint32_t send = upper ? a[i] : a[i + off];
+            const uint32_t keep = upper ? a[i + off] : a[i];
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, send, off);
+            a[i] = keep > got ? keep : got;
+        }
+    }
+    uint32_t r = a[0];
+#pragma unroll
+    for (int off = NV; off < 32; off <<= 1) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, r, off);
+        r = r > got ? r : got;
+    }
+    return r;
+}
+
+// Largest |y| per token of a finished fp16 tile [tokens][cols] in shared memory (cols a multiple of 8), one global atomic per token.
+// Neighbouring lanes share a token and read 16 bytes each, so a tile takes a few loads per thread and up to five shuffles.  Taken from
+// the accumulator registers instead, where a token's columns lie in 32 lanes, the maxima cost 31 shuffles per 32 tokens and
+// shared-memory atomics (128 x 12288 x 4096: the GEMM's epilogue 4.4 us, now 2.9).  NaNs are dropped, as fmax does.  Called by every
+// thread of the CTA.
+template <int THREADS>
+__device__ __forceinline__ void staged_row_maxima(uint32_t tile, int tokens, int cols, uint32_t* row_absmax_bits) {
+    int lanes = 1; // per token
+    while (lanes < 32 && lanes * 2 * tokens <= THREADS) lanes *= 2;
+    const int t = (int)threadIdx.x / lanes;
+    __half2 m2 = __float2half2_rn(0.0f);
+    if (t < tokens) {
+        for (int c = ((int)threadIdx.x & (lanes - 1)) * 8; c < cols; c += lanes * 8) {
+            const uint4 v = ld_shared_v4(tile + (uint32_t)(t * cols + c) * 2u);
+            const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) m2 = __hmax2(m2, __habs2(h[j]));
+        }
+    }
+    uint32_t bits = __float_as_uint(fmaxf(__low2float(m2), __high2float(m2)));
+    for (int off = lanes >> 1; off >= 1; off >>= 1) {
+        const uint32_t other = __shfl_xor_sync(0xffffffffu, bits, off);
+        bits = other > bits ? other : bits;
+    }
+    if (((int)threadIdx.x & (lanes - 1)) == 0 && t < tokens && bits != 0u) atomicMax(row_absmax_bits + t, bits);
+}
+
+template <int N> struct TmemLd;
+template <> struct TmemLd<32> {
+    __device__ static __forceinline__ void run(uint32_t taddr, uint32_t (&r)[32]) { ptx::tmem_ld_32x32(taddr, r); }
+};
+template <> struct TmemLd<8> {
+    __device__ static __forceinline__ void run(uint32_t taddr, uint32_t (&r)[8]) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+            : "r"(taddr)
+            : "memory");
+    }
+};
+template <> struct TmemLd<16> {
+    __device__ static __forceinline__ void run(uint32_t taddr, uint32_t (&r)[16]) {
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(taddr)
+            : "memory");
+    }
+};
+
+// Reads N columns of each of the first `valid` accumulator tiles (STRIDE columns apart) and returns their sum.
+template <int N, int NACC, int STRIDE>
+__device__ __forceinline__ void tmem_ld_sum(uint32_t taddr, uint32_t (&acc)[N], int valid) {
+    TmemLd<N>::run(taddr, acc);
+    ptx::tmem_ld_wait();
+#pragma unroll
+    for (int a = 1; a < NACC; ++a) { // one partial tile at a time: two register arrays live, not NACC
+        if (a >= valid) break; // warp-uniform: that issuer had no K block
+        uint32_t part[N];
+        TmemLd<N>::run(taddr + a * STRIDE, part);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < N; ++j) acc[j] += part[j];
+    }
+}
+
+// Brings this CTA's weight stages into L2 while the kernel still waits for its predecessors: two at once, then one per 400
+// cycles (11 KB x 140 CTAs: about the HBM rate) until the loads proper start.  Unpaced, tens of megabytes of requests queue up
+// in front of the few that the small kernel still running waits for (a quantizer, a norm).  One thread of an idle warp.
+// Back to back in a graph, us without / all at once / paced: layer of 8 tokens 56.1 / 53.5 / 53.5, layer shard of 96 tokens
+// 68.9 / 65.9 / 65.2, linear 37 x 11008 x 4096 17.6 / 17.0 / 16.5, 96 x 4096 x 8192 15.6 / 14.7 / 14.3.
+template <typename Fetch>
+__device__ __forceinline__ void prefetch_weights(int stages, int* loads_started, Fetch fetch) {
+    long long due = clock64();
+    for (int i = 0; i < stages; ++i) {
+        if (i >= 2) {
+            due += 400;
+            while (clock64() < due && *static_cast<volatile int*>(loads_started) == 0) {}
+        }
+        if (*static_cast<volatile int*>(loads_started) != 0) break;
+        fetch(i);
+    }
+}
+
+// One activated value of the fused gate + up projection, operation by operation as the stand-alone kernel of
+// activation_requant.cu computes it.
+__device__ __forceinline__ float swiglu_value(uint32_t xi, uint32_t gi, float sx, float sg, float down_n, float ts, float beta) {
+    const float x = __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)xi, sx), down_n), ts);
+    const float g = __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)gi, sg), down_n), ts);
+    return __fmul_rn(__fdiv_rn(x, __fadd_rn(1.0f, __expf(__fmul_rn(-x, beta)))), g);
+}
+
+// SwiGLU over the accumulators this CTA owns: activated fp16 values into the output tile [token][channel] at
+// ring + SWIGLU_OUT, row maxima (of the fp32 values) into token_absmax.  Called by every thread of the CTA.
+template <int BT, bool DUAL>
+__device__ __forceinline__ void swiglu_epilogue(const DecodeParams& p, uint32_t taddr_row, uint32_t ring, uint32_t S, uint32_t rank,
+                                                uint32_t own0, uint32_t slot0, uint32_t step_div, uint32_t step_rem, uint32_t slot_carry,
+                                                uint32_t recv_pieces, bool have_acc, int nkb, int col_begin, int col_end, int nl, int n,
+                                                int q, int lane, const float (&sn)[2], const float* token_scale, uint32_t* token_absmax, int M) {
+    using C = DCfg<BT>;
+    constexpr int NPART = DUAL ? 2 : 1;
+    const int valid = nkb < C::NACC ? nkb : C::NACC;
+    const bool ok = nl < p.tile_rows && n < p.N;
+    auto load8 = [&](int col, uint32_t slot, uint32_t (&v)[8]) { // eight tokens of this lane's row, K slices summed
+        if (have_acc) {
+            tmem_ld_sum<8, C::NACC, NPART * BT>(taddr_row + col, v, valid);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = 0u;
+        }
+        for (uint32_t r = 0; r + 1 < S; ++r) {
+            const uint32_t addr = ring + (r * recv_pieces + slot) * PIECE_BYTES + lane * 32;
+            const uint4 a = ld_shared_v4(addr), b = ld_shared_v4(addr + 16);
+            v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
+            v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+        }
+    };
+    const uint32_t partner = ring + C::SWIGLU_PARTNER + (uint32_t)nl * 4u; // [token][64 rows] int32
+    const int side = q >> 1;                                              // lanes of the x rows (0) or of the gate rows (1)
+    if (!DUAL) {
+        // each half of the lanes computes every other chunk and hands the accumulators of the rest to the other half
+        uint32_t own = own0, slot = slot0;
+#pragma unroll 1
+        for (int c0 = col_begin; c0 < col_end; c0 += PIECE_COLS) {
+            if (c0 >= M) break;
+            if (own == rank && ((c0 / PIECE_COLS) & 1) != side) {
+                uint32_t v[8];
+                load8(c0, slot, v);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(partner + (uint32_t)(c0 + j) * 256u), "r"(v[j]) : "memory");
+            }
+            own += step_rem; slot += step_div;
+            if (own >= S) { own -= S; slot += slot_carry; }
+        }
+        __syncthreads();
+    }
+    uint32_t own = own0, slot = slot0;
+#pragma unroll 1
+    for (int c0 = col_begin; c0 < col_end; c0 += PIECE_COLS) {
+        if (c0 >= M) break;
+        if (DUAL || (own == rank && ((c0 / PIECE_COLS) & 1) == side)) {
+            uint32_t v[8], w[8], absbits[8];
+            load8(c0, slot, v);
+            if (DUAL) {
+                load8(BT + c0, slot, w);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[j]) : "r"(partner + (uint32_t)(c0 + j) * 256u) : "memory");
+            }
+            const float4 ts0 = *reinterpret_cast<const float4*>(&token_scale[c0]);
+            const float4 ts1 = *reinterpret_cast<const float4*>(&token_scale[c0 + 4]);
+            const float ts[8] = {ts0.x, ts0.y, ts0.z, ts0.w, ts1.x, ts1.y, ts1.z, ts1.w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const bool swap = !DUAL && side != 0; // this lane holds the gate, its partner the x value
+                const float r = swiglu_value(swap ? w[j] : v[j], swap ? v[j] : w[j], sn[0], sn[1], p.down_n, ts[j], p.beta);
+                const float a = ok ? fabsf(r) : 0.0f;
+                absbits[j] = a == a ? __float_as_uint(a) : 0u; // NaNs are dropped, as fmax does
+                if (nl < p.tile_rows)
+                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(ring + C::SWIGLU_OUT + ((uint32_t)(c0 + j) * (uint32_t)p.tile_rows + (uint32_t)nl) * 2u),
+                                 "h"(__half_as_ushort(__float2half_rn(r))) : "memory");
+            }
+            const uint32_t tok_max = warp_token_max<8>(absbits, lane);
+            if (lane < 8 && c0 + lane < M && tok_max != 0u) atomicMax(&token_absmax[c0 + lane], tok_max);
+        }
+        own += step_rem; slot += step_div;
+        if (own >= S) { own -= S; slot += slot_carry; }
+    }
+}
+
+// Epilogue of the kernels that fold K onto the TMEM lanes in F parts: the F diagonal blocks of the accumulators (part f: lanes
+// f * (DENSE ? tile_rows : 128 / F) .., columns f * tile_tokens ..; two accumulator tiles ACC_STRIDE columns apart, `valid` of them used) meet in shared
+// memory at `blocks`, [part][token][row] with BT >= tokens, and leave summed; a warp handles 32 rows of one token at a time.
+// Row maxima for the re-quantizer are gathered at `maxima`.  nl / n: this thread's row in the tile and output column, sn / bias its
+// constants.  Called by every thread; returns the time stamp between the two halves.
+template <int BT, int F, int ACC_STRIDE, int THREADS, bool DENSE>
+__device__ __forceinline__ unsigned long long fold_epilogue(const DecodeParams& p, uint32_t tmem_base, uint32_t blocks, uint32_t maxima, int valid,
+                                                            bool acc_ready, int nl, int n, bool n_ok, float sn, half bias_h, const float* token_scale) {
+    constexpr int ROWS = BW / F, ROW_WARPS = ROWS / 32, GROUPS = THREADS / 128;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    {
+        const int q = warp & 3, grp = warp >> 2;         // TMEM lane quarter, slice of the tokens
+        // the parts that this quarter of the lanes holds rows of: one, or, densely packed, neighbouring ones
+        const int lanes = DENSE ? p.tile_rows : ROWS;
+        const int f0 = q * 32 / lanes, f1 = DENSE ? ((q * 32 + 31) / lanes < F - 1 ? (q * 32 + 31) / lanes : F - 1) : f0;
+#pragma unroll 1
+        for (int f = f0; f <= f1; ++f) {
+            const int row = q * 32 + lane - f * lanes;
+            const bool mine = row >= 0 && row < lanes;
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(f * p.tile_tokens);
+            const uint32_t dst = blocks + (uint32_t)(f * BT * ROWS + row) * 4u;
+#pragma unroll 1
+            for (int c0 = grp * 8; c0 < p.M; c0 += 8 * GROUPS) {
+                uint32_t v[8];
+                if (acc_ready) {
+                    tmem_ld_sum<8, 2, ACC_STRIDE>(taddr + c0, v, valid);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[j] = 0u;
+                }
+                if (mine) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (uint32_t)((c0 + j) * ROWS) * 4u), "r"(v[j]) : "memory");
+                }
+            }
+        }
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    const unsigned long long t_exchange = p.stamps ? globaltimer_ns() : 0ull;
+
+    // ---- sums and epilogue: a warp handles 32 rows of one token at a time
+    const uint32_t src = blocks + (uint32_t)nl * 4u;
+#pragma unroll 4
+    for (int m = warp / ROW_WARPS; m < p.M; m += (THREADS / 32) / ROW_WARPS) {
+        uint32_t v = 0;
+#pragma unroll
+        for (int f = 0; f < F; ++f) {
+            uint32_t t;
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(t) : "r"(src + (uint32_t)((f * BT + m) * ROWS) * 4u) : "memory");
+            v += t;
+        }
+        if (p.mode == EPI_RAW_I32) {
+            if (n_ok) {
+                int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)m * p.ldc + n;
+                if (p.raw_affine) {
+                    v = (uint32_t)p.raw_alpha * v + (p.raw_bias != nullptr ? (uint32_t)p.raw_bias[n] : 0u);
+                    if (p.raw_beta != 0) v += (uint32_t)p.raw_beta * (uint32_t)*dst;
+                }
+                *dst = (int32_t)v;
+            }
+            continue;
+        }
+        float t = __fmul_rn((float)(int32_t)v, sn);
+        t = __fmul_rn(t, p.down_n);
+        t = __fmul_rn(t, token_scale[m]);
+        const half h = __hadd(__float2half_rn(t), bias_h);
+        if (n_ok) reinterpret_cast<half*>(p.out)[(int64_t)m * p.ldc + n] = h;
+        if (p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
+            const float a = n_ok ? fabsf(__half2float(h)) : 0.0f;
+            const uint32_t bits = __reduce_max_sync(0xffffffffu, a == a ? __float_as_uint(a) : 0u); // NaNs are dropped, as fmax does
+            if (lane == 0) asm volatile("st.shared.u32 [%0], %1;" ::"r"(maxima + (uint32_t)((warp % ROW_WARPS) * BT + m) * 4u), "r"(bits) : "memory");
+        }
+    }
+    if (p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
+        // Neighbouring tokens leave in one instruction per CTA.  One global atomic per token and warp as the rows are finished,
+        // all CTAs on the same few lines of L2, took as long as the rest of the kernel (59 x 8928 x 2944: the call 20.9 -> 11.8 us).
+        // They meet in the dead activation ring, not in memory of their own: 1 KB more, and under the 196 KB carve-out that the driver picks for
+        // this kernel no quantizer CTA starts beside it any more (70 x 8192 x 4096 without re-quantizing: 12.9 -> 13.8 us).
+        __syncthreads();
+        for (int m = threadIdx.x; m < BT && m < p.M; m += THREADS) {
+            uint32_t bits = 0u;
+#pragma unroll
+            for (int w = 0; w < ROW_WARPS; ++w) {
+                uint32_t t;
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(t) : "r"(maxima + (uint32_t)(w * BT + m) * 4u) : "memory");
+                bits = t > bits ? t : bits;
+            }
+            if (bits != 0u) atomicMax(p.row_absmax_bits + m, bits);
+        }
+    }
+    return t_exchange;
+}
+
+// ---- host side ---------------------------------------------------------------------------------
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+inline EncodeTiledFn encode_fn() {
+    static EncodeTiledFn fn = nullptr;
+    static std::once_flag once;
+    std::call_once(once, [] {
+        void* sym = nullptr;
+        cudaDriverEntryPointQueryResult qr;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qr) == cudaSuccess &&
+            qr == cudaDriverEntryPointSuccess)
+            fn = reinterpret_cast<EncodeTiledFn>(sym);
+    });
+    return fn;
+}
+
+// Output [M, N] (fp16 or int32, leading dimension ldc elements); box = {tile_rows weight rows, BT tokens}, dense.
+inline bool make_out_map(CUtensorMap* map, void* base, int64_t M, int64_t N, int64_t ldc, int elem_bytes, int box_cols, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
+    const cuuint64_t strides[1] = {(cuuint64_t)(ldc * elem_bytes)};
+    const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows};
+    const cuuint32_t elem_strides[2] = {1, 1};
+    return fn(map, elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16 : CU_TENSOR_MAP_DATA_TYPE_INT32, 2, base, dims, strides, box,
+              elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+inline bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld, int box_rows) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)ld};
+    const cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
+    const cuuint32_t elem_strides[2] = {1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem_strides,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// A [rows, K] int8 matrix with K cut into F parts of K / F bytes, [part][row][byte of the part]: one box of {128 bytes, box_rows,
+// box_parts} brings the same K block of several parts.  What lies past the end of a part is zero.  K % (16 F) == 0.
+inline bool make_fold_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld, int F, int box_rows, int box_parts) {
+    EncodeTiledFn fn = encode_fn();
+    if (!fn) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)(K / F), (cuuint64_t)rows, (cuuint64_t)F};
+    const cuuint64_t strides[2] = {(cuuint64_t)ld, (cuuint64_t)(K / F)};
+    const cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, (cuuint32_t)box_parts};
+    const cuuint32_t elem_strides[3] = {1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, elem_strides,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// How a launch is cut: `tokens` x `rows` tiles (two-part tiles: rows per part), K split over S CTAs.
+struct DecodePlan {
+    int tokens, token_tiles, rows, row_tiles, S;
+    bool dual;
+    int fold; // parts K is folded into (gemm_i8_fold_kernel), 0 = row tiles
+    bool pair; // on CTA pairs that share the activations (gemm_i8_token_pair_kernel), folded or not
+};
+
+// Rows per tile for `cap` tiles that can run at once: the smallest multiple of 8 with which `columns` output columns
+// still are one wave -- e.g. 12288 weight rows: 140 tiles of 88 rows on 148 SMs instead of 96 tiles of 128 rows on 96.
+inline int rows_for(int64_t columns, int64_t cap, int max_rows) {
+    if (cap <= 0 || (columns + max_rows - 1) / max_rows > cap) return max_rows;
+    const int64_t r = ((columns + cap - 1) / cap + 7) / 8 * 8;
+    return r < 8 ? 8 : r < max_rows ? (int)r : max_rows;
+}
+
+} // namespace dec
+
+// gemm_i8_token_pair.cu
+bool token_pair_setup();
+int32_t launch_token_pair(cudaStream_t stream, const GemmArgs& a, const dec::DecodePlan& plan, dec::DecodeParams p, bool pdl);
+
+} // namespace pplb200

@@ -75,6 +75,11 @@ __device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* m, int32_t
                  ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y) : "memory");
 }
 
+__device__ __forceinline__ void tma_prefetch_l2_3d(const CUtensorMap* m, int32_t x, int32_t y, int32_t z) {
+    asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];"
+                 ::"l"(reinterpret_cast<uint64_t>(m)), "r"(x), "r"(y), "r"(z) : "memory");
+}
+
 // 2-D tiled store, shared -> global, tracked by the thread's bulk async-group.  The box is clipped at the
 // tensor's bounds; x * element size must be a multiple of 16 bytes and neither coordinate negative.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* m, uint32_t src, int32_t x, int32_t y) {
@@ -181,7 +186,14 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(x), "r"(y)
         : "memory");
 }
-// the same with an L2 eviction-priority hint for the lines the load touches
+// the same from a 3-D tensor: one instruction brings several 2-D boxes, one behind the other
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int32_t x, int32_t y, int32_t z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+// the 2-D load with an L2 eviction-priority hint for the lines the load touches
 __device__ __forceinline__ void tma_load_2d_pair_hint(uint32_t dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int32_t x, int32_t y,
                                                       uint64_t policy) {
     asm volatile(
