@@ -10,8 +10,8 @@
 //     fewer weight-row tiles than SMs, K is split over a thread-block cluster of S CTAs (one
 //     weight-row tile per cluster) so that all clusters still fit in one wave;
 //   * the S partial accumulators are combined inside the cluster through distributed shared
-//     memory (a reduce-scatter over 8-column pieces), never through global memory, and each CTA
-//     runs the dequant epilogue for the pieces it owns.  Integer addition makes the result
+//     memory (a reduce-scatter over groups of eight tokens, one bulk copy per pair of CTAs), never through global memory, and each CTA
+//     runs the dequant epilogue for the groups it owns.  Integer addition makes the result
 //     independent of the split.
 //   * sixteen epilogue warps: a lone warp per scheduler issues well under one instruction per clock,
 //     and the epilogue is not overlapped with anything in a one-tile-per-CTA kernel;
@@ -52,7 +52,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_w[MAX_W_STAGES], empty_w[MAX_W_STAGES];
     __shared__ __align__(8) uint64_t full_x[X_STAGES], empty_x[X_STAGES];
-    __shared__ __align__(8) uint64_t acc_full_bar;
+    __shared__ __align__(8) uint64_t acc_full_bar, recv_bar;
     __shared__ uint32_t tmem_base_slot;
     __shared__ __align__(16) float token_scale[BT];
     __shared__ uint32_t token_absmax[BT];
@@ -90,6 +90,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
             ptx::prefetch_tensormap(&tmap_w);
             ptx::prefetch_tensormap(&tmap_x);
             ptx::mbar_init(ptx::smem_addr(&acc_full_bar), C::NACC);
+            ptx::mbar_init(ptx::smem_addr(&recv_bar), 1);
             loads_started = 0;
         }
         if (lane < MAX_W_STAGES) {
@@ -113,13 +114,16 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const uint32_t tmem_base = tmem_base_slot;
     const unsigned long long t_setup = p.stamps ? globaltimer_ns() : 0ull;
 
-    // per-thread output columns (= weight rows, one per part) and their constants
-    const int q = warp & 3;  // TMEM lane quarter this warp may read
-    const int grp = warp >> 2; // which slice of the token columns it handles
-    const int col_begin = grp * C::GROUP_COLS, col_end = col_begin + C::GROUP_COLS;
+    const int q = warp & 3;    // TMEM lane quarter this warp may read
+    const int grp = warp >> 2; // which groups of eight token columns it handles
+    // Where K is shared or x and gate rows meet, the accumulators pass through shared memory and a warp finishes 32 rows of
+    // one token at a time; else it finishes what it reads from its lanes.
+    const bool exchanged = pack || S > 1;
+    const int row_warps = p.tile_rows > 64 ? 4 : p.tile_rows > 32 ? 2 : 1; // warps side by side in that last pass
+    // per-thread output column (= weight row, one per part) and its constants
     // A tile holds tile_rows <= 128 weight rows; the MMA still spans 128 TMEM lanes, the upper ones compute on
     // whatever the rest of the shared-memory slot holds and are never read back.
-    const int nl = pack ? (q & 1) * 32 + lane : q * 32 + lane; // weight row inside the part
+    const int nl = exchanged ? (warp & (row_warps - 1)) * 32 + lane : q * 32 + lane; // weight row inside the part
     const bool nl_ok = nl < p.tile_rows;
     const int n = tile_row0 + nl;
     float sn[2] = {0.0f, 0.0f};
@@ -241,192 +245,245 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const unsigned long long t_main = p.stamps ? globaltimer_ns() : 0ull;
 
     const uint32_t taddr_row = tmem_base + ((uint32_t)(q * 32) << 16);
-    // piece index of (column chunk c, quarter q) is 4 c + q; owner = piece % S, slot = piece / S.
-    // Both are tracked incrementally (no divisions in the loops): a step of one chunk adds 4.
-    // With x and gate rows on different lanes (pack) a CTA owns all four quarters of a chunk: owner = c % S, and the
-    // pieces of a chunk are neighbours, slot = 4 (c / S) + q.
-    const uint32_t recv_pieces_per_owner = pack ? 4u * ((BT / PIECE_COLS + S - 1) / S) : (C::PIECES + S - 1) / S;
-    const uint32_t step_div = pack ? 4u * (1u / S) : 4u / S, step_rem = pack ? 1u % S : 4u % S, slot_carry = pack ? 4u : 1u;
-    const uint32_t first_chunk = (uint32_t)(col_begin / PIECE_COLS);
-    const uint32_t own0 = pack ? first_chunk % S : (first_chunk * 4u + (uint32_t)q) % S;
-    const uint32_t slot0 = pack ? first_chunk / S * 4u + (uint32_t)q : (first_chunk * 4u + (uint32_t)q) / S;
     const bool have_acc = nkb > 0 && acc_ready;
-
-    if (S > 1) {
-        cluster_sync_all(); // every CTA of the cluster is done reading its ring: it may now receive
-        // ---- send the pieces owned by other CTAs
-        uint32_t own = own0, slot = slot0;
-#pragma unroll 1
-        for (int c0 = col_begin; c0 < col_end; c0 += C::LD_COLS) {
-            if (c0 >= M) break; // columns past the last token hold zeros nobody reads
-            uint32_t acc[C::LD_COLS];
-            if (have_acc) {
-                tmem_ld_sum<C::LD_COLS, C::NACC, NPART * BT>(taddr_row + c0, acc, nkb < C::NACC ? nkb : C::NACC);
-            } else {
-#pragma unroll
-                for (int j = 0; j < C::LD_COLS; ++j) acc[j] = 0u;
-            }
-#pragma unroll
-            for (int s8 = 0; s8 < C::LD_COLS / PIECE_COLS; ++s8) {
-                if (own != rank) {
-                    const uint32_t sender_slot = rank < own ? rank : rank - 1;
-                    const uint32_t local = ring + (sender_slot * recv_pieces_per_owner + slot) * PIECE_BYTES + lane * 32;
-                    const uint32_t remote = map_to_cta(local, own);
-                    st_cluster_v4(remote, acc[s8 * 8 + 0], acc[s8 * 8 + 1], acc[s8 * 8 + 2], acc[s8 * 8 + 3]);
-                    st_cluster_v4(remote + 16, acc[s8 * 8 + 4], acc[s8 * 8 + 5], acc[s8 * 8 + 6], acc[s8 * 8 + 7]);
-                }
-                own += step_rem; slot += step_div;
-                if (own >= S) { own -= S; slot += slot_carry; }
-            }
-        }
-        cluster_sync_all(); // all partial pieces have landed
-    } else {
+    const int valid = nkb < C::NACC ? nkb : C::NACC;
+    unsigned long long t_exchange = t_main;
+    if (!exchanged) {
+        // The CTA owns its whole [tokens x tile_rows] output tile: the values are transposed through shared memory (the rings
+        // are dead by now) into a dense [token][weight row] tile and leave as ONE TMA store, clipped at the matrix bounds.
+        const bool staged = !p.raw_affine;
+        const int tile_cols = p.tile_rows * NPART;
         __syncthreads(); // token_scale visible
-    }
-    const unsigned long long t_exchange = p.stamps ? globaltimer_ns() : 0ull;
-
-    // ---- epilogue over the pieces this CTA owns
-    const int mode = p.mode;
-    const float down_n = p.down_n;
-    // Without a K split the CTA owns its whole [tokens x tile_rows] output tile: the values are transposed through
-    // shared memory (the rings are dead by now) into a dense [token][weight row] tile and leave as ONE TMA store,
-    // clipped at the matrix bounds -- instead of a 2-byte (or 4-byte) store with its own address arithmetic per
-    // element (lane = weight row, registers = tokens is the wrong way round for the row-major output).
-    const bool staged = S == 1 && !p.raw_affine;
-    const bool scattered_maxima = mode == EPI_DEQUANT_F16_REQUANT_I8 && !staged; // a staged tile's row maxima are read back from it
-    const uint32_t tile_cols = (uint32_t)(p.tile_rows * NPART);
-    if constexpr (SWIGLU) {
-        swiglu_epilogue<BT, DUAL>(p, taddr_row, ring, S, rank, own0, slot0, step_div, step_rem, slot_carry, recv_pieces_per_owner, have_acc,
-                                  nkb, col_begin, col_end, nl, n, q, lane, sn, token_scale, token_absmax, M);
-    } else {
+        if constexpr (SWIGLU) { // two parts: x and gate of a channel lie on the same lane
+            uint32_t x[8], g[8], x1[8], g1[8];
 #pragma unroll
-    for (int part = 0; part < NPART; ++part) { // S == 1 with two parts
-        const uint32_t nlp = (uint32_t)(part * p.tile_rows + nl); // weight row inside the tile
-        const int np = n + part * p.part_stride;
-        const bool n_ok = nl_ok && np < p.N;
-        uint32_t own = own0, slot = slot0;
+            for (int j = 0; j < 8; ++j) { x1[j] = 0u; g1[j] = 0u; x[j] = 0u; g[j] = 0u; }
+            const bool n_ok = nl_ok && n < p.N;
 #pragma unroll 1
-        for (int c0 = col_begin; c0 < col_end; c0 += C::LD_COLS) {
-            if (c0 >= M) break;
-            uint32_t acc[C::LD_COLS];
-            uint32_t absbits[C::LD_COLS]; // |y| as float bits per token column (0 where not owned)
-#pragma unroll
-            for (int j = 0; j < C::LD_COLS; ++j) absbits[j] = 0u;
-
-            if (have_acc) {
-                tmem_ld_sum<C::LD_COLS, C::NACC, NPART * BT>(taddr_row + part * BT + c0, acc, nkb < C::NACC ? nkb : C::NACC);
-            } else {
-#pragma unroll
-                for (int j = 0; j < C::LD_COLS; ++j) acc[j] = 0u;
-            }
-#pragma unroll
-            for (int s8 = 0; s8 < C::LD_COLS / PIECE_COLS; ++s8) {
-                if (own == rank) {
-                    uint32_t v[8];
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] = acc[s8 * 8 + j];
-                    for (uint32_t r = 0; r + 1 < S; ++r) { // partials of the other S - 1 CTAs
-                        const uint32_t addr = ring + (r * recv_pieces_per_owner + slot) * PIECE_BYTES + lane * 32;
-                        const uint4 a = ld_shared_v4(addr), b = ld_shared_v4(addr + 16);
-                        v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-                        v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
+            for (int c0 = grp * 8; c0 < M; c0 += 8 * C::GROUPS) {
+                if (have_acc) {
+                    TmemLd<8>::run(taddr_row + c0, x);
+                    TmemLd<8>::run(taddr_row + BT + c0, g);
+                    if (valid > 1) {
+                        TmemLd<8>::run(taddr_row + NPART * BT + c0, x1);
+                        TmemLd<8>::run(taddr_row + NPART * BT + BT + c0, g1);
                     }
-                    const int m0 = c0 + s8 * 8;
-                    if (mode == EPI_RAW_I32 && staged) {
-                        if (nl_ok) {
+                    tmem_ld_wait8x2(x, g);
+                    tmem_ld_wait8x2(x1, g1);
+                }
+                uint32_t most = 0u;
 #pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                asm volatile("st.shared.u32 [%0], %1;" ::"r"(ring + ((uint32_t)(m0 + j) * tile_cols + nlp) * 4u), "r"(v[j]) : "memory");
-                        }
-                    } else if (mode == EPI_RAW_I32) {
-                        int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)(token0 + m0) * p.ldc + np;
-                        const uint32_t add = (p.raw_affine && p.raw_bias != nullptr && n_ok) ? (uint32_t)p.raw_bias[np] : 0u;
+                for (int h = 0; h < 8; h += 4) {
+                    uint32_t xs[4], gs[4];
+                    float r[4];
+                    const float4 tsv = *reinterpret_cast<const float4*>(&token_scale[c0 + h]);
+                    const float ts[4] = {tsv.x, tsv.y, tsv.z, tsv.w};
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            if (n_ok && m0 + j < M) {
-                                uint32_t r = v[j];
-                                if (p.raw_affine) {
-                                    r = (uint32_t)p.raw_alpha * r + add;
-                                    if (p.raw_beta != 0) r += (uint32_t)p.raw_beta * (uint32_t)dst[(int64_t)j * p.ldc];
-                                }
-                                dst[(int64_t)j * p.ldc] = (int32_t)r;
-                            }
-                    } else {
-                        // eight independent chains, no control flow between them
-                        const float4 ts0 = *reinterpret_cast<const float4*>(&token_scale[m0]);
-                        const float4 ts1 = *reinterpret_cast<const float4*>(&token_scale[m0 + 4]);
-                        const float ts[8] = {ts0.x, ts0.y, ts0.z, ts0.w, ts1.x, ts1.y, ts1.z, ts1.w};
-                        half h[8];
+                    for (int j = 0; j < 4; ++j) { xs[j] = x[h + j] + x1[h + j]; gs[j] = g[h + j] + g1[h + j]; }
+                    swiglu_values<4>(xs, gs, sn[0], sn[1], p.down_n, ts, p.beta, n_ok, r);
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            float t = __fmul_rn((float)(int32_t)v[j], sn[part]);
-                            t = __fmul_rn(t, down_n);
-                            t = __fmul_rn(t, ts[j]);
-                            h[j] = __hadd(__float2half_rn(t), bias_h[part]);
-                        }
-                        if (staged) {
-                            if (nl_ok) {
-#pragma unroll
-                                for (int j = 0; j < 8; ++j)
-                                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(ring + ((uint32_t)(m0 + j) * tile_cols + nlp) * 2u), "h"(__half_as_ushort(h[j])) : "memory");
-                            }
-                        } else {
-                            half* dst = reinterpret_cast<half*>(p.out) + (int64_t)(token0 + m0) * p.ldc + np;
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                if (n_ok && m0 + j < M) dst[(int64_t)j * p.ldc] = h[j];
-                        }
-                        if (scattered_maxima) {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                const float a = n_ok ? fabsf(__half2float(h[j])) : 0.0f;
-                                absbits[s8 * 8 + j] = a == a ? __float_as_uint(a) : 0u; // NaNs are dropped, as fmax does
-                            }
-                        }
+                    for (int j = 0; j < 4; ++j) {
+                        if (nl_ok)
+                            asm volatile("st.shared.u16 [%0], %1;" ::"r"(ring + (uint32_t)((c0 + h + j) * p.tile_rows + nl) * 2u), "h"(__half_as_ushort(__float2half_rn(r[j]))) : "memory");
+                        const float a = fabsf(r[j]);
+                        const uint32_t bits = __reduce_max_sync(0xffffffffu, n_ok && a == a ? __float_as_uint(a) : 0u); // NaNs are dropped, as fmax does
+                        if (lane == h + j) most = bits;
                     }
                 }
-                own += step_rem; slot += step_div;
-                if (own >= S) { own -= S; slot += slot_carry; }
+                if (lane < 8 && c0 + lane < M && most != 0u) atomicMax(&token_absmax[c0 + lane], most);
             }
-            if (scattered_maxima) {
-                // per-token max |y| over this warp's 32 output columns; lane t ends up with token c0 + t
-                const uint32_t tok_max = warp_token_max<C::LD_COLS>(absbits, lane);
-                if (lane < C::LD_COLS && c0 + lane < M && tok_max != 0u) atomicMax(&token_absmax[c0 + lane], tok_max);
+            ptx::fence_proxy_async_smem(); // the tile is read by the TMA unit
+            ptx::tc_fence_before();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                ptx::tma_store_2d(&tmap_y, ring, tile_row0, token0);
+                ptx::bulk_commit_group();
+            }
+            // this CTA's row maxima, [token][CTA]: nothing has to be cleared beforehand and nothing is added atomically
+            for (int m = threadIdx.x; m < M; m += NUM_THREADS) p.row_absmax_bits[(int64_t)(token0 + m) * gridDim.y + n_tile] = token_absmax[m];
+            if (threadIdx.x == 0) ptx::bulk_wait_group_read<0>(); // shared memory must outlive the store's reads
+        } else {
+        t_exchange = p.stamps ? globaltimer_ns() : 0ull;
+#pragma unroll
+        for (int part = 0; part < NPART; ++part)
+            tile_epilogue<NPART * BT, C::GROUPS>(p, taddr_row + part * BT, valid, have_acc, ring, tile_cols, part * p.tile_rows + nl, nl_ok,
+                                                 n + part * p.part_stride, sn[part], bias_h[part], token_scale, token0, M, grp);
+        if (staged) {
+            ptx::fence_proxy_async_smem(); // the tile is read by the TMA unit
+            ptx::tc_fence_before();
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                ptx::tma_store_2d(&tmap_y, ring, tile_row0, token0);
+                ptx::bulk_commit_group();
+            }
+            if (p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
+                __syncwarp();
+                staged_row_maxima<NUM_THREADS>(ring, M, tile_cols, p.row_absmax_bits + token0);
+            }
+            if (threadIdx.x == 0) ptx::bulk_wait_group_read<0>(); // shared memory must outlive the store's reads; the kernel boundary publishes the writes
+        }
+        }
+    } else {
+        // ---- Groups of eight tokens belong to the CTAs of the cluster in turn (group c to CTA c % S).  Each CTA writes its accumulators,
+        // [owner][its groups][token][row], into its own dead ring, and one bulk copy per owner takes a block over into a
+        // receive area there, counted by the owner's barrier; the owner sums S blocks.  Copies, because stores of the
+        // accumulators into the other CTAs' memory, 16 bytes per lane, moved about 10 bytes per cycle: 96 x 1280 x 8192 with K
+        // shared by eight 4.4 us until the partial sums had arrived and 2.3 for the epilogue, now 3.2 and 0.8.
+        const int pitch = p.tile_rows * (SWIGLU ? 2 : 1); // rows of a token: x rows, then gate rows
+        const int groups = (M + PIECE_COLS - 1) / PIECE_COLS, per_owner = (groups + (int)S - 1) / (int)S;
+        const uint32_t group_bytes = (uint32_t)(PIECE_COLS * pitch) * 4u, block_bytes = (uint32_t)per_owner * group_bytes;
+        const uint32_t recv = ring + S * block_bytes;
+        if (S > 1) {
+            __syncwarp();
+            cluster_arrive(); // this CTA's ring may be written from now on
+        }
+        {
+            uint32_t a[8], b[8];
+#pragma unroll
+            for (int part = 0; part < NPART; ++part) { // two parts: S is 1 and nothing is exchanged
+                const int lane_row = pack ? (q & 1) * 32 + lane : q * 32 + lane;
+                const int row = lane_row + (pack ? (q >> 1) : part) * p.tile_rows;
+                const uint32_t taddr = taddr_row + part * BT;
+                auto fetch = [&](int c) {
+                    TmemLd<8>::run(taddr + c * PIECE_COLS, a);
+                    if (valid > 1) TmemLd<8>::run(taddr + NPART * BT + c * PIECE_COLS, b);
+                };
+#pragma unroll
+                for (int j = 0; j < 8; ++j) { a[j] = 0u; b[j] = 0u; }
+                int c = grp;
+                if (c < groups && have_acc) fetch(c);
+#pragma unroll 1
+                for (; c < groups; c += C::GROUPS) {
+                    uint32_t v[8];
+                    tmem_ld_wait8x2(a, b);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[j] = a[j] + b[j];
+                    if (c + C::GROUPS < groups && have_acc) fetch(c + C::GROUPS);
+                    if (lane_row < p.tile_rows) {
+                        const uint32_t dst = ring + (S == 1 ? (uint32_t)c * group_bytes : (uint32_t)c % S * block_bytes + (uint32_t)c / S * group_bytes) + (uint32_t)row * 4u;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (uint32_t)(j * pitch) * 4u), "r"(v[j]) : "memory");
+                    }
+                }
             }
         }
-    }
+        const int mine = groups > (int)rank ? (groups - (int)rank + (int)S - 1) / (int)S : 0; // groups this CTA owns
+        if (S > 1) {
+            ptx::fence_proxy_async_smem(); // the blocks are read by the bulk copies
+            ptx::tc_fence_before();
+            __syncthreads();
+            cluster_wait(); // every CTA of the cluster is done reading its ring: it may receive
+            if (warp == 0) {
+                const uint32_t bar = ptx::smem_addr(&recv_bar);
+                if (lane == 0) ptx::mbar_arrive_expect_tx(bar, (S - 1) * (uint32_t)mine * group_bytes);
+                const uint32_t to = (uint32_t)lane; // one lane per owner
+                const uint32_t bytes = groups > lane ? (uint32_t)((groups - lane + (int)S - 1) / (int)S) * group_bytes : 0u;
+                if (to < S && to != rank && bytes != 0u)
+                    ptx::bulk_copy_to_cta(map_to_cta(recv + (rank < to ? rank : rank - 1) * block_bytes, to), ring + to * block_bytes, bytes, map_to_cta(bar, to));
+                __syncwarp();
+            }
+            ok = ptx::mbar_wait(ptx::smem_addr(&recv_bar), 0, p.status, ST_DEC_EPI);
+            __syncwarp();
+            cluster_arrive(); // received: the others' copies out of their rings to this CTA are done
+        } else {
+            ptx::tc_fence_before();
+            __syncthreads();
+        }
+        t_exchange = p.stamps ? globaltimer_ns() : 0ull;
 
+        // ---- sums and epilogue: a warp finishes 32 rows of four tokens at a time (one by one, the steps of a value would wait for each other)
+        constexpr int NV = 4;
+        const uint32_t own = ring + rank * block_bytes + (uint32_t)nl * 4u, got = recv + (uint32_t)nl * 4u;
+        const bool n_ok = nl_ok && n < p.N;
+        const int step = NV * (NUM_THREADS / 32) / row_warps;
+        auto sums = [&](uint32_t off, uint32_t (&v)[NV]) {
+#pragma unroll
+            for (int j = 0; j < NV; ++j) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v[j]) : "r"(own + off + (uint32_t)(j * pitch) * 4u) : "memory");
+#pragma unroll 1
+            for (uint32_t r = 0; r + 1 < S; ++r) {
+                uint32_t t[NV];
+#pragma unroll
+                for (int j = 0; j < NV; ++j) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(t[j]) : "r"(got + r * block_bytes + off + (uint32_t)(j * pitch) * 4u) : "memory");
+#pragma unroll
+                for (int j = 0; j < NV; ++j) v[j] += t[j];
+            }
+        };
+        const int owned = nl - lane < p.tile_rows ? mine * PIECE_COLS : 0; // 65 .. 96 rows: three row warps of four
+#pragma unroll 1
+        for (int i = NV * (warp / row_warps); i < owned; i += step) {
+            const int m0 = ((i / PIECE_COLS) * (int)S + (int)rank) * PIECE_COLS + (i & (PIECE_COLS - 1));
+            if (m0 >= M) break;
+            const uint32_t off = (uint32_t)(i * pitch) * 4u;
+            uint32_t v[NV];
+            float a[NV];
+            const float4 tsv = *reinterpret_cast<const float4*>(&token_scale[m0]);
+            const float ts[NV] = {tsv.x, tsv.y, tsv.z, tsv.w};
+            sums(off, v); // lanes past the last row read their neighbours' words
+            if constexpr (SWIGLU) {
+                uint32_t g[NV];
+                float r[NV];
+                sums(off + (uint32_t)p.tile_rows * 4u, g);
+                swiglu_values<NV>(v, g, sn[0], sn[1], p.down_n, ts, p.beta, n_ok, r);
+                half* dst = reinterpret_cast<half*>(p.out) + (int64_t)(token0 + m0) * p.ldc + n;
+#pragma unroll
+                for (int j = 0; j < NV; ++j) {
+                    if (n_ok && m0 + j < M) dst[(int64_t)j * p.ldc] = __float2half_rn(r[j]);
+                    a[j] = fabsf(r[j]);
+                }
+            } else if (p.mode == EPI_RAW_I32) {
+                int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)(token0 + m0) * p.ldc + n;
+#pragma unroll
+                for (int j = 0; j < NV; ++j)
+                    if (n_ok && m0 + j < M) {
+                        uint32_t r = v[j];
+                        if (p.raw_affine) {
+                            r = (uint32_t)p.raw_alpha * r + (p.raw_bias != nullptr ? (uint32_t)p.raw_bias[n] : 0u);
+                            if (p.raw_beta != 0) r += (uint32_t)p.raw_beta * (uint32_t)dst[(int64_t)j * p.ldc];
+                        }
+                        dst[(int64_t)j * p.ldc] = (int32_t)r;
+                    }
+                continue;
+            } else {
+                half* dst = reinterpret_cast<half*>(p.out) + (int64_t)(token0 + m0) * p.ldc + n;
+#pragma unroll
+                for (int j = 0; j < NV; ++j) {
+                    float t = __fmul_rn((float)(int32_t)v[j], sn[0]);
+                    t = __fmul_rn(t, p.down_n);
+                    t = __fmul_rn(t, ts[j]);
+                    const half h = __hadd(__float2half_rn(t), bias_h[0]);
+                    if (n_ok && m0 + j < M) dst[(int64_t)j * p.ldc] = h;
+                    a[j] = fabsf(__half2float(h));
+                }
+            }
+            if (SWIGLU || p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
+                uint32_t most = 0u;
+#pragma unroll
+                for (int j = 0; j < NV; ++j) {
+                    const uint32_t bits = __reduce_max_sync(0xffffffffu, n_ok && a[j] == a[j] ? __float_as_uint(a[j]) : 0u); // NaNs are dropped, as fmax does
+                    if (lane == j) most = bits;
+                }
+                if (lane < NV && most != 0u) atomicMax(&token_absmax[m0 + lane], most);
+            }
+        }
+        if (SWIGLU || p.mode == EPI_DEQUANT_F16_REQUANT_I8) {
+            __syncthreads();
+            // SwiGLU: this CTA's share of the row maxima, [token][CTA]: a CTA writes every token (zero for those it does not own),
+            // so nothing has to be cleared beforehand and nothing is added atomically
+            const uint32_t cta = (uint32_t)n_tile * S + rank, ctas = gridDim.y * S;
+            for (int m = threadIdx.x; m < BT && m < M; m += NUM_THREADS) {
+                if (SWIGLU) p.row_absmax_bits[(int64_t)(token0 + m) * ctas + cta] = token_absmax[m];
+                else if (token_absmax[m] != 0u) atomicMax(p.row_absmax_bits + token0 + m, token_absmax[m]);
+            }
+        }
+        if (S > 1) {
+            __syncwarp();
+            cluster_wait(); // nobody reads this CTA's ring any more
+        }
     }
 #undef PPLB200_KB
-    if (staged || SWIGLU) ptx::fence_proxy_async_smem(); // the tile written above is read by the TMA unit
+    (void)ok;
     ptx::tc_fence_before();
     __syncthreads();
-    if constexpr (SWIGLU) { // eight tokens per store, those this CTA owns
-        if (threadIdx.x < BT / PIECE_COLS && threadIdx.x * PIECE_COLS < M && (!pack || threadIdx.x % S == rank)) {
-            ptx::tma_store_2d(&tmap_y, ring + C::SWIGLU_OUT + threadIdx.x * (uint32_t)(PIECE_COLS * 2 * p.tile_rows), tile_row0,
-                              token0 + (int)threadIdx.x * PIECE_COLS);
-            ptx::bulk_commit_group();
-            ptx::bulk_wait_group_read<0>();
-        }
-        // this CTA's share of the row maxima, [token][CTA]: a CTA writes every token (zero for those it does not own),
-        // so nothing has to be cleared beforehand and nothing is added atomically
-        const uint32_t cta = (uint32_t)n_tile * S + rank, ctas = gridDim.y * S;
-        for (int m = threadIdx.x; m < BT && m < M; m += NUM_THREADS) p.row_absmax_bits[(int64_t)(token0 + m) * ctas + cta] = token_absmax[m];
-    } else if (staged) {
-        if (threadIdx.x == 0) {
-            ptx::tma_store_2d(&tmap_y, ring, tile_row0, token0);
-            ptx::bulk_commit_group();
-        }
-        if (mode == EPI_DEQUANT_F16_REQUANT_I8) {
-            __syncwarp();
-            staged_row_maxima<NUM_THREADS>(ring, M, (int)tile_cols, p.row_absmax_bits + token0);
-        }
-        if (threadIdx.x == 0) ptx::bulk_wait_group_read<0>(); // shared memory must outlive the store's reads; the kernel boundary publishes the writes
-    }
-    if (scattered_maxima) {
-        for (int m = threadIdx.x; m < BT && m < M; m += NUM_THREADS)
-            if (token_absmax[m] != 0u) atomicMax(p.row_absmax_bits + token0 + m, token_absmax[m]);
-    }
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc(tmem_base, TMEM_COLS);
@@ -885,9 +942,8 @@ int32_t launch_bt(cudaStream_t stream, const GemmArgs& a, const DecodePlan& plan
     if (!make_map(&tw, a.B, a.N, a.K, a.ldb, tile_rows)) return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (W) encode failed");
     CUtensorMap ty;
     memset(&ty, 0, sizeof(ty));
-    if (swiglu ? !make_out_map(&ty, a.out, a.M, p.N, a.ldc, 2, tile_rows, PIECE_COLS)
-               : S == 1 && !p.raw_affine &&
-                     !make_out_map(&ty, a.out, a.M, a.N, a.ldc, a.mode == EPI_RAW_I32 ? 4 : 2, tile_rows * parts_out, plan.tokens))
+    if ((swiglu ? dual : S == 1 && !p.raw_affine) &&
+        !make_out_map(&ty, a.out, a.M, p.N, a.ldc, a.mode == EPI_RAW_I32 ? 4 : 2, tile_rows * parts_out, plan.tokens))
         return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (Y) encode failed");
 
     cudaLaunchConfig_t cfg = {};

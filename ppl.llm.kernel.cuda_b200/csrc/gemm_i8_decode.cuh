@@ -14,8 +14,7 @@ namespace dec {
 constexpr int BW = 128;      // weight rows per tile (TMEM lanes)
 constexpr int BK = 128;      // bytes of K per stage
 constexpr int UMMA_K = 32;
-constexpr int PIECE_COLS = 8; // reduce-scatter granule: 32 lanes x 8 columns x 4 B = 1 KiB
-constexpr int PIECE_BYTES = 32 * PIECE_COLS * 4;
+constexpr int PIECE_COLS = 8; // tokens of a group in the exchange of K partials
 constexpr int SMEM_BUDGET = 210 * 1024; // one CTA per SM: the whole shared memory is one TMA ring
 
 constexpr unsigned ST_DEC_PRODUCER = 16u, ST_DEC_MMA = 32u, ST_DEC_EPI = 64u;
@@ -74,18 +73,12 @@ template <int BT> struct DCfg {
     // quarter in each set).
     static constexpr int GROUPS = BT >= 32 ? 4 : 2;
     static constexpr int NUM_THREADS = 128 * GROUPS;
-    static constexpr int GROUP_COLS = BT / GROUPS;
-    static constexpr int LD_COLS = GROUP_COLS < 32 ? GROUP_COLS : 32; // columns per tcgen05.ld
-    static constexpr int PIECES = 4 * (BT / PIECE_COLS);
-    // EPI_SWIGLU_F16: once the main loop is over, [received partials | partner accumulators | output tile] share the rings
-    static constexpr int SWIGLU_PARTNER = 72 * 1024, SWIGLU_OUT = 104 * 1024; // at most 72 KB are received (split in 7)
-    static_assert(SWIGLU_OUT + BT * 128 * 2 <= RING_BYTES, "swiglu epilogue buffers fit the rings");
-    static_assert(LD_COLS == 8 || LD_COLS == 16 || LD_COLS == 32, "tcgen05.ld shape");
     static_assert(BT == 16 || BT == 32 || BT == 64 || BT == 128, "token tile");
     static_assert(RING_BYTES % 1024 == 0 && RING_BYTES - 6 * X_BYTES >= 6 * BW * BK && RING_BYTES - 4 * X_BYTES >= 8 * BW * BK,
                   "room for at least six full weight tiles, or four of two parts");
-    // the rings double as the receive buffer of the reduce-scatter once the main loop is over
-    static_assert(PIECES * PIECE_BYTES <= RING_BYTES, "receive buffer fits the rings");
+    // once the main loop is over the rings hold the accumulators and what is received of them: at most 13 blocks of three groups (K
+    // shared by seven), or 256 rows (SwiGLU, two parts)
+    static_assert(13 * 3 * PIECE_COLS * BW * 4 <= RING_BYTES && BT * 2 * BW * 4 <= RING_BYTES, "exchange buffers fit the rings");
 };
 
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
@@ -104,46 +97,19 @@ __device__ __forceinline__ uint32_t cluster_nctarank() {
     asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
     return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
+// The two halves of a cluster barrier that publishes no data (a release costs some 1000 cycles): it tells the other CTAs only that
+// this one's tensor cores and bulk copies are done with its shared memory.  Every thread executes both.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t local_smem_addr, uint32_t rank) {
     uint32_t r;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_smem_addr), "r"(rank));
     return r;
 }
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
 __device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
-}
-
-// Per-token maximum over the 32 lanes of a warp for NV tokens held as a[0..NV) in every lane
-// (halving butterfly: NV - 1 shuffles instead of NV full warp reductions).  Returns, in every lane,
-// the maximum for token (lane % NV).
-template <int NV>
-__device__ __forceinline__ uint32_t warp_token_max(uint32_t (&a)[NV], int lane) {
-#pragma unroll
-    for (int off = NV / 2; off >= 1; off >>= 1) {
-        const bool upper = (lane & off) != 0;
-#pragma unroll
-        for (int i = 0; i < off; ++i) {
-            const uint32_t send = upper ? a[i] : a[i + off];
-            const uint32_t keep = upper ? a[i + off] : a[i];
-            const uint32_t got = __shfl_xor_sync(0xffffffffu, send, off);
-            a[i] = keep > got ? keep : got;
-        }
-    }
-    uint32_t r = a[0];
-#pragma unroll
-    for (int off = NV; off < 32; off <<= 1) {
-        const uint32_t got = __shfl_xor_sync(0xffffffffu, r, off);
-        r = r > got ? r : got;
-    }
-    return r;
 }
 
 // Largest |y| per token of a finished fp16 tile [tokens][cols] in shared memory (cols a multiple of 8), one global atomic per token.
@@ -174,9 +140,6 @@ __device__ __forceinline__ void staged_row_maxima(uint32_t tile, int tokens, int
 }
 
 template <int N> struct TmemLd;
-template <> struct TmemLd<32> {
-    __device__ static __forceinline__ void run(uint32_t taddr, uint32_t (&r)[32]) { ptx::tmem_ld_32x32(taddr, r); }
-};
 template <> struct TmemLd<8> {
     __device__ static __forceinline__ void run(uint32_t taddr, uint32_t (&r)[8]) {
         asm volatile(
@@ -186,18 +149,6 @@ template <> struct TmemLd<8> {
             : "memory");
     }
 };
-template <> struct TmemLd<16> {
-    __device__ static __forceinline__ void run(uint32_t taddr, uint32_t (&r)[16]) {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-            "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(taddr)
-            : "memory");
-    }
-};
-
 // Reads N columns of each of the first `valid` accumulator tiles (STRIDE columns apart) and returns their sum.
 template <int N, int NACC, int STRIDE>
 __device__ __forceinline__ void tmem_ld_sum(uint32_t taddr, uint32_t (&acc)[N], int valid) {
@@ -232,89 +183,103 @@ __device__ __forceinline__ void prefetch_weights(int stages, int* loads_started,
     }
 }
 
-// One activated value of the fused gate + up projection, operation by operation as the stand-alone kernel of
-// activation_requant.cu computes it.
-__device__ __forceinline__ float swiglu_value(uint32_t xi, uint32_t gi, float sx, float sg, float down_n, float ts, float beta) {
-    const float x = __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)xi, sx), down_n), ts);
-    const float g = __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)gi, sg), down_n), ts);
-    return __fmul_rn(__fdiv_rn(x, __fadd_rn(1.0f, __expf(__fmul_rn(-x, beta)))), g);
+// NV activated values of the fused gate + up projection: x / (1 + exp(-beta x)) * gate of the dequantized accumulators, bit for bit as the
+// stand-alone kernel of activation_requant.cu computes them.  The division there is the compiler's, whose special cases branch; with a
+// branch per value the NV chains run one after another (128 x 11008 x 4096: 11.7 us for the epilogue).  Here the quotient is Markstein's
+// ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): a reciprocal refined once, the quotient
+// corrected twice by its exact residual, which rounds correctly while nothing over- or underflows.  The denominator is at least 1; values
+// for which it is not well below 2^127, or whose x is tiny, infinite or no number, take the compiler's division, a warp at a time (live:
+// this lane's values are used).
+template <int NV>
+__device__ __forceinline__ void swiglu_values(const uint32_t (&xi)[NV], const uint32_t (&gi)[NV], float sx, float sg, float down_n, const float (&ts)[NV],
+                                              float beta, bool live, float (&r)[NV]) {
+    float x[NV], d[NV];
+    bool special = false;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        x[j] = __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)xi[j], sx), down_n), ts[j]);
+        d[j] = __fadd_rn(1.0f, __expf(__fmul_rn(-x[j], beta)));
+        // +0 / d comes out as +0 either way, -0 / d would not; the comparisons are false for NaNs
+        special |= !(d[j] < 0x1p100f && fabsf(x[j]) < 0x1p100f && (fabsf(x[j]) > 0x1p-20f || __float_as_uint(x[j]) == 0u));
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        float y;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d[j]));
+        y = __fmaf_rn(y, __fmaf_rn(-d[j], y, 1.0f), y);
+        float q = __fmul_rn(x[j], y);
+        q = __fmaf_rn(__fmaf_rn(-d[j], q, x[j]), y, q);
+        r[j] = __fmaf_rn(__fmaf_rn(-d[j], q, x[j]), y, q);
+    }
+    if (__any_sync(0xffffffffu, special && live)) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) r[j] = __fdiv_rn(x[j], d[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j) r[j] = __fmul_rn(r[j], __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)gi[j], sg), down_n), ts[j]));
 }
 
-// SwiGLU over the accumulators this CTA owns: activated fp16 values into the output tile [token][channel] at
-// ring + SWIGLU_OUT, row maxima (of the fp32 values) into token_absmax.  Called by every thread of the CTA.
-template <int BT, bool DUAL>
-__device__ __forceinline__ void swiglu_epilogue(const DecodeParams& p, uint32_t taddr_row, uint32_t ring, uint32_t S, uint32_t rank,
-                                                uint32_t own0, uint32_t slot0, uint32_t step_div, uint32_t step_rem, uint32_t slot_carry,
-                                                uint32_t recv_pieces, bool have_acc, int nkb, int col_begin, int col_end, int nl, int n,
-                                                int q, int lane, const float (&sn)[2], const float* token_scale, uint32_t* token_absmax, int M) {
-    using C = DCfg<BT>;
-    constexpr int NPART = DUAL ? 2 : 1;
-    const int valid = nkb < C::NACC ? nkb : C::NACC;
-    const bool ok = nl < p.tile_rows && n < p.N;
-    auto load8 = [&](int col, uint32_t slot, uint32_t (&v)[8]) { // eight tokens of this lane's row, K slices summed
-        if (have_acc) {
-            tmem_ld_sum<8, C::NACC, NPART * BT>(taddr_row + col, v, valid);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = 0u;
-        }
-        for (uint32_t r = 0; r + 1 < S; ++r) {
-            const uint32_t addr = ring + (r * recv_pieces + slot) * PIECE_BYTES + lane * 32;
-            const uint4 a = ld_shared_v4(addr), b = ld_shared_v4(addr + 16);
-            v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
-            v[4] += b.x; v[5] += b.y; v[6] += b.z; v[7] += b.w;
-        }
+// Waits for the tcgen05.ld's of this thread; the operands tie the registers' first use to the wait.
+__device__ __forceinline__ void tmem_ld_wait8x2(uint32_t (&a)[8], uint32_t (&b)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                   "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7])
+                 :: "memory");
+}
+
+// Finishes the accumulators at taddr (two tiles ACC_STRIDE columns apart, `valid` of them used) into the output tile
+// [token][cols] at `tile`, at column `col` (tile_ok: inside it); with an int32 affine step, into global memory, element by element.
+// The GROUPS warps of a lane quarter take every GROUPS-th group of eight tokens; the next group's accumulators are fetched under this one's arithmetic.
+template <int ACC_STRIDE, int GROUPS>
+__device__ __forceinline__ void tile_epilogue(const DecodeParams& p, uint32_t taddr, int valid, bool have_acc, uint32_t tile, int cols, int col, bool tile_ok,
+                                              int n, float sn, half bias_h, const float* token_scale, int token0, int M, int grp) {
+    const bool n_ok = tile_ok && n < p.N;
+    uint32_t a[8], b[8];
+    auto fetch = [&](int c) {
+        TmemLd<8>::run(taddr + c, a);
+        if (valid > 1) TmemLd<8>::run(taddr + ACC_STRIDE + c, b);
     };
-    const uint32_t partner = ring + C::SWIGLU_PARTNER + (uint32_t)nl * 4u; // [token][64 rows] int32
-    const int side = q >> 1;                                              // lanes of the x rows (0) or of the gate rows (1)
-    if (!DUAL) {
-        // each half of the lanes computes every other chunk and hands the accumulators of the rest to the other half
-        uint32_t own = own0, slot = slot0;
-#pragma unroll 1
-        for (int c0 = col_begin; c0 < col_end; c0 += PIECE_COLS) {
-            if (c0 >= M) break;
-            if (own == rank && ((c0 / PIECE_COLS) & 1) != side) {
-                uint32_t v[8];
-                load8(c0, slot, v);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(partner + (uint32_t)(c0 + j) * 256u), "r"(v[j]) : "memory");
-            }
-            own += step_rem; slot += step_div;
-            if (own >= S) { own -= S; slot += slot_carry; }
-        }
-        __syncthreads();
-    }
-    uint32_t own = own0, slot = slot0;
+    for (int j = 0; j < 8; ++j) { a[j] = 0u; b[j] = 0u; }
+    int c0 = grp * 8;
+    if (c0 < M && have_acc) fetch(c0);
 #pragma unroll 1
-    for (int c0 = col_begin; c0 < col_end; c0 += PIECE_COLS) {
-        if (c0 >= M) break;
-        if (DUAL || (own == rank && ((c0 / PIECE_COLS) & 1) == side)) {
-            uint32_t v[8], w[8], absbits[8];
-            load8(c0, slot, v);
-            if (DUAL) {
-                load8(BT + c0, slot, w);
-            } else {
+    for (; c0 < M; c0 += 8 * GROUPS) {
+        uint32_t v[8];
+        tmem_ld_wait8x2(a, b);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w[j]) : "r"(partner + (uint32_t)(c0 + j) * 256u) : "memory");
+        for (int j = 0; j < 8; ++j) v[j] = a[j] + b[j];
+        if (c0 + 8 * GROUPS < M && have_acc) fetch(c0 + 8 * GROUPS);
+        if (p.mode == EPI_RAW_I32 && !p.raw_affine) {
+            if (tile_ok) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    asm volatile("st.shared.u32 [%0], %1;" ::"r"(tile + (uint32_t)((c0 + j) * cols + col) * 4u), "r"(v[j]) : "memory");
             }
+        } else if (p.mode == EPI_RAW_I32) {
+            int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)(token0 + c0) * p.ldc + n;
+            const uint32_t add = (p.raw_bias != nullptr && n_ok) ? (uint32_t)p.raw_bias[n] : 0u;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (n_ok && c0 + j < M) {
+                    uint32_t r = (uint32_t)p.raw_alpha * v[j] + add;
+                    if (p.raw_beta != 0) r += (uint32_t)p.raw_beta * (uint32_t)dst[(int64_t)j * p.ldc];
+                    dst[(int64_t)j * p.ldc] = (int32_t)r;
+                }
+        } else {
             const float4 ts0 = *reinterpret_cast<const float4*>(&token_scale[c0]);
             const float4 ts1 = *reinterpret_cast<const float4*>(&token_scale[c0 + 4]);
             const float ts[8] = {ts0.x, ts0.y, ts0.z, ts0.w, ts1.x, ts1.y, ts1.z, ts1.w};
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-                const bool swap = !DUAL && side != 0; // this lane holds the gate, its partner the x value
-                const float r = swiglu_value(swap ? w[j] : v[j], swap ? v[j] : w[j], sn[0], sn[1], p.down_n, ts[j], p.beta);
-                const float a = ok ? fabsf(r) : 0.0f;
-                absbits[j] = a == a ? __float_as_uint(a) : 0u; // NaNs are dropped, as fmax does
-                if (nl < p.tile_rows)
-                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(ring + C::SWIGLU_OUT + ((uint32_t)(c0 + j) * (uint32_t)p.tile_rows + (uint32_t)nl) * 2u),
-                                 "h"(__half_as_ushort(__float2half_rn(r))) : "memory");
+                float t = __fmul_rn((float)(int32_t)v[j], sn);
+                t = __fmul_rn(t, p.down_n);
+                t = __fmul_rn(t, ts[j]);
+                const half h = __hadd(__float2half_rn(t), bias_h);
+                if (tile_ok)
+                    asm volatile("st.shared.u16 [%0], %1;" ::"r"(tile + (uint32_t)((c0 + j) * cols + col) * 2u), "h"(__half_as_ushort(h)) : "memory");
             }
-            const uint32_t tok_max = warp_token_max<8>(absbits, lane);
-            if (lane < 8 && c0 + lane < M && tok_max != 0u) atomicMax(&token_absmax[c0 + lane], tok_max);
         }
-        own += step_rem; slot += step_div;
-        if (own >= S) { own -= S; slot += slot_carry; }
     }
 }
 

@@ -28,14 +28,6 @@ struct TPCfg {
     static constexpr int ACC_STRIDE = 256;
 };
 
-// Waits for the tcgen05.ld's of this thread; the operands tie the registers' first use to the wait.
-__device__ __forceinline__ void tmem_ld_wait8x2(uint32_t (&a)[8], uint32_t (&b)[8]) {
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
-                   "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7])
-                 :: "memory");
-}
-
 // grid = (2, row pairs, token tiles), cluster = (2, 1, 1).  A stage is one slot of [weights | activations] in each CTA; the leader's
 // full barrier counts the bytes of both CTAs, one multicast commit (a signal, not a load) frees the slot in both.
 template <int F>
@@ -218,59 +210,10 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         t_exchange = fold_epilogue<256 / F, F, C::ACC_STRIDE, C::NUM_THREADS, true>(p, tmem_base, ring, ring + 256 * ROWS * 4, valid, acc_ready, nl, n, n_ok, sn,
                                                                               bias_h, token_scale);
     } else {
-        // The output tile goes through the dead ring, [token][weight row], and leaves as one TMA store (with an int32 affine step:
-        // element by element).  Four warps share a lane quarter and take every fourth group of eight tokens; the next group's
-        // accumulators are fetched under this one's arithmetic.
+        // the output tile goes through the dead ring, [token][weight row], and leaves as one TMA store
         const bool staged = !p.raw_affine;
-        const uint32_t cols = (uint32_t)p.tile_rows;
-        const uint32_t taddr_row = tmem_base + ((uint32_t)(q * 32) << 16);
-        uint32_t a[8], b[8];
-        auto fetch = [&](int c) {
-            TmemLd<8>::run(taddr_row + c, a);
-            if (valid > 1) TmemLd<8>::run(taddr_row + C::ACC_STRIDE + c, b);
-        };
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { a[j] = 0u; b[j] = 0u; }
-        int c0 = grp * 8;
-        if (c0 < M && acc_ready) fetch(c0);
-#pragma unroll 1
-        for (; c0 < M; c0 += 32) {
-            uint32_t v[8];
-            tmem_ld_wait8x2(a, b);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = a[j] + b[j];
-            if (c0 + 32 < M && acc_ready) fetch(c0 + 32);
-            if (p.mode == EPI_RAW_I32 && staged) {
-                if (nl < p.tile_rows) {
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        asm volatile("st.shared.u32 [%0], %1;" ::"r"(ring + ((uint32_t)(c0 + j) * cols + (uint32_t)nl) * 4u), "r"(v[j]) : "memory");
-                }
-            } else if (p.mode == EPI_RAW_I32) {
-                int32_t* dst = reinterpret_cast<int32_t*>(p.out) + (int64_t)(token0 + c0) * p.ldc + n;
-                const uint32_t add = (p.raw_bias != nullptr && n_ok) ? (uint32_t)p.raw_bias[n] : 0u;
-#pragma unroll
-                for (int j = 0; j < 8; ++j)
-                    if (n_ok && c0 + j < M) {
-                        uint32_t r = (uint32_t)p.raw_alpha * v[j] + add;
-                        if (p.raw_beta != 0) r += (uint32_t)p.raw_beta * (uint32_t)dst[(int64_t)j * p.ldc];
-                        dst[(int64_t)j * p.ldc] = (int32_t)r;
-                    }
-            } else {
-                const float4 ts0 = *reinterpret_cast<const float4*>(&token_scale[c0]);
-                const float4 ts1 = *reinterpret_cast<const float4*>(&token_scale[c0 + 4]);
-                const float ts[8] = {ts0.x, ts0.y, ts0.z, ts0.w, ts1.x, ts1.y, ts1.z, ts1.w};
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    float t = __fmul_rn((float)(int32_t)v[j], sn);
-                    t = __fmul_rn(t, p.down_n);
-                    t = __fmul_rn(t, ts[j]);
-                    const half h = __hadd(__float2half_rn(t), bias_h);
-                    if (nl < p.tile_rows)
-                        asm volatile("st.shared.u16 [%0], %1;" ::"r"(ring + ((uint32_t)(c0 + j) * cols + (uint32_t)nl) * 2u), "h"(__half_as_ushort(h)) : "memory");
-                }
-            }
-        }
+        tile_epilogue<C::ACC_STRIDE, C::NUM_THREADS / 128>(p, tmem_base + ((uint32_t)(q * 32) << 16), valid, acc_ready, ring, p.tile_rows, nl, nl < p.tile_rows, n,
+                                                           sn, bias_h, token_scale, token0, M, grp);
         if (staged) {
             ptx::fence_proxy_async_smem(); // the tile is read by the TMA unit
             __syncthreads();

@@ -231,3 +231,24 @@ def test_gate_up_swiglu_k_shared_by_a_cluster(cuda, oracle, M, D, K):
     plan = pplb200.gemm_plan(M, D, K, swiglu=True)
     assert plan["token_tiles" if M > 128 else "split"] > 1, plan
     test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K)
+
+
+# Both row parts on a lane, x and gate on different lanes, K shared by a cluster
+@pytest.mark.parametrize("M,D,K", [(40, 11008, 272), (64, 2800, 144), (33, 2688, 8192)])
+def test_fused_swiglu_of_values_of_every_magnitude(cuda, M, D, K):
+    """Row scales over the whole fp16 range: x from far below the smallest quotient that the fast division handles to far beyond exp's
+    overflow, zeros among them.  The division is exact in both kernels, so the results are the same bits."""
+    import pplb200
+    g = cuda.Generator(device="cuda").manual_seed(M + D + K)
+    xq = cuda.randint(-127, 128, (M, K), generator=g, device="cuda", dtype=cuda.int8)
+    xq[M // 2] = 0
+    w = cuda.randint(-127, 128, (2 * D, K), generator=g, device="cuda", dtype=cuda.int8)
+    sm = (2.0 ** cuda.linspace(-24, 15, M, device="cuda")).half()
+    sn = (2.0 ** (cuda.rand((2 * D,), generator=g, device="cuda") * 24 - 16)).half()
+    acc = pplb200.column_parallel_linear(xq, w, None, None, None, K, 2 * D, gather_output=False)
+    for beta in (1.0, -0.5):
+        two_step = pplb200.minmax_requantize_swiglu_fp16(acc, sm, sn, beta=beta)
+        fused = pplb200.gate_up_swiglu_requant(xq, w, sm, sn, beta=beta)
+        for a, b in zip(fused, two_step):
+            assert cuda.equal(a.view(cuda.int8), b.view(cuda.int8))
+    assert pplb200.gemm_status() == 0
