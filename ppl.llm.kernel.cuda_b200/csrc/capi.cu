@@ -447,12 +447,12 @@ int32_t pplb200_i8i8_linear_fp16_host(pplb200_stream_t stream_, const void* x_ho
     // c/4, c/2 rows (each step's copy-in + compute still fits under the previous step's copy-out), which starts the
     // copy-out after an eighth of the fill time.
     const bool ramp = c >= 1024 && M >= 2 * c;
-    // A batch below two chunks fits the two staging buffers as a whole: no part of them is used twice, and the chunks can
-    // be as short as pays.  `fine` rows take as long on the wire as their linear does (the weights at about 5 TB/s plus
-    // 10 us of launches, against 55 GB/s of PCIe); the first and the last chunk have that length, so that little of the
-    // copies in and out is exposed, those between twice that; less than two such chunks are not cut at all.
-    // (1024 x 4096 x 4096: 354 -> 309 us; 256 rows: 177 -> 100 us.  Two directions at once, short copies and their events cost more
-    // than their bytes: finer chunks gain nothing.)
+    // A batch below two chunks fits the two staging buffers as a whole: no part of them is used twice.  Its chunks are few: while
+    // results leave, the end of a copy in is seen some 15 us late, by the kernel that waits for it and by the next copy.  Up to
+    // 12 MB a quarter, a half and a quarter, beyond 15, 30 .. 35 and 20 % (us per call, with chunks of 128 and 256 rows / now:
+    // 1024 x 4096 x 4096 308 / 286, 1000 x 8192 x 1024 re-quantized 414 / 375, 1999 x 4096 x 5120 re-quantized 777 / 750; even shares
+    // 300 at the first).  A first and last chunk no shorter than `fine` rows, which take as long on the wire as their linear does
+    // (the weights at about 5 TB/s plus 10 us of launches, against 55 GB/s of PCIe); less than two such chunks are not cut at all.
     const bool flat = M < 2 * c;
     const int64_t row_bytes = 2 * (K > N ? K : N);
     int64_t fine = (N * K / 5000 + 10000) * 55 / row_bytes; // ns x bytes per ns / bytes per row
@@ -464,7 +464,15 @@ int32_t pplb200_i8i8_linear_fp16_host(pplb200_stream_t stream_, const void* x_ho
         const int64_t r0 = flat ? m0 - b * c : 0; // first row inside the staging buffer
         if (flat) {
             const int64_t left = M - m0;
-            rows = left < 2 * fine ? left : chunk == 0 ? fine : left < 3 * fine ? round_up(left - fine, 8) : 2 * fine;
+            const bool wide = M * row_bytes > (12 << 20);
+            const auto share = [&](int64_t percent) { const int64_t r = round_up(M * percent / 100, 8); return r > fine ? r : fine; };
+            const int64_t last_rows = share(wide ? 20 : 25);
+            if (left < 2 * fine) rows = left;
+            else if (chunk == 0) rows = share(wide ? 15 : 25);
+            else if (M > c && m0 < c) rows = c - m0; // the rest of the first staging buffer
+            else if (wide && M <= c && chunk == 1) rows = share(30);
+            else rows = left - last_rows >= fine ? left - last_rows : left;
+            if (rows > left) rows = left;
             if (rows > c - r0) rows = c - r0;
         } else {
             rows = !ramp || chunk >= 4 ? c : chunk < 2 ? c / 8 : chunk == 2 ? c / 4 : c / 2;
