@@ -740,19 +740,18 @@ int variant_of(int64_t M) { return M <= 16 ? 0 : M <= 32 ? 1 : M <= 64 ? 2 : 3; 
 // CTA pairs that share the activations (gemm_i8_token_pair_kernel) instead of the form in `best`.  They bring in half of the
 // activations per CTA and have one barrier per stage, but setting a pair up costs about 0.4 us more, and one MMA of a
 // pair at least 60 cycles for up to 120 columns, 2 per 4 columns beyond.  So they pay where there are stages enough to earn
-// the fixed part back.  Median time of quantizer + GEMM, best single-CTA form / pair, over 3035 random shapes of 17 .. 128 tokens:
-//   folded in four: 48 tokens 0.95 up to 7 stages, 1.00 up to 15, 1.07 from 16, 1.12 from 24; 32 tokens 1.01 at most
-//   folded in two:  80 tokens 1.05 from 8 stages, 1.12 from 24; 128 tokens 0.97 from 8, 1.02 from 16, 1.12 from 24; 64 tokens 1.00 at most
-//   whole K: 1.05 (up to 64 tokens) and 1.11 (beyond) up to 63 stages; then the weight stream bounds both, 0.93 .. 1.00
-// With these lines 801 of the shapes go to pairs; 8 of them lose more than 3 %.
+// the fixed part back.  Median time of quantizer + GEMM, single CTAs / pairs, over 4302 random shapes of 1 .. 128 tokens:
+//   folded in four: 32 tokens 0.91 up to 7 stages, 1.00 up to 15, 1.11 from 16; 48 tokens 0.93, 1.03, 1.11; 64 tokens 0.91, 0.99, 1.06
+//   folded in two:  80 tokens 0.99 up to 7 stages, 1.08 up to 15, 1.15 .. 1.25 from 16; 128 tokens 0.97, 1.01, 1.06 .. 1.19; 64 tokens 1.00 throughout
+//   whole K: 1.14 up to 15 stages, 1.12 up to 31, 1.04 .. 1.10 beyond
 void plan_pair(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t kb, DecodePlan& best) {
     if ((best.S > 1 && !best.fold) || best.dual) return;
     const int ctas = dev.sms / 2 * 2;
     const int t16 = (int)((M + 15) / 16 * 16), t32 = (int)((M + 31) / 32 * 32);
     int F = 0;
-    if (best.fold == 4 && t16 >= 48 && (kb + 3) / 4 >= 16) F = 4;
-    else if (best.fold != 4 && t16 >= 80 && columns <= (int64_t)ctas * (BW / 2) && (kb + 1) / 2 >= t16 / 8) F = 2;
-    else if (!best.fold && columns <= (int64_t)ctas * BW && kb < 64) F = 1;
+    if (best.fold == 4 && t16 >= 32 && (kb + 3) / 4 >= 12) F = 4;
+    else if (best.fold != 4 && t16 >= 80 && columns <= (int64_t)ctas * (BW / 2) && (kb + 1) / 2 * 10 >= t16) F = 2;
+    else if (!best.fold && columns <= (int64_t)ctas * BW) F = 1;
     if (F == 0) return;
     best.pair = true;
     best.S = 1;

@@ -585,8 +585,8 @@ def test_medium_batch_gemm_k_shared_by_a_cluster(cuda, oracle, M, N, K):
 # CTA pairs that share the activations: K folded in four and two (by one box per operand, or, where the parts of K are no multiple of
 # 16 bytes, by a box per part), whole K, token tiles; ragged tiles of tokens and rows, a last pair without second rows, one to many
 # stages, rows that share a quarter of the lanes with another part's
-@pytest.mark.parametrize("M,N,K,fold", [(37, 4096, 11008, 4), (48, 1032, 8208, 4), (64, 4728, 7744, 4), (33, 888, 8192, 4), (80, 9472, 2576, 2), (128, 1040, 4096, 2),
-                                        (100, 7000, 3360, 2), (17, 9480, 128, 0), (128, 18944, 256, 0), (20, 12288, 8064, 0), (33, 18936, 144, 0), (129, 2048, 528, 0),
+@pytest.mark.parametrize("M,N,K,fold", [(37, 4096, 11008, 4), (48, 1032, 8208, 4), (64, 4728, 7744, 4), (33, 888, 8192, 4), (80, 9472, 2576, 2), (128, 5000, 4112, 2), (20, 3000, 6160, 4),
+                                        (100, 7000, 3360, 2), (17, 9480, 128, 0), (128, 18944, 256, 0), (20, 12288, 8208, 0), (1, 9480, 1040, 0), (33, 18936, 144, 0), (129, 2048, 528, 0),
                                         (256, 4096, 1024, 0), (333, 4096, 4096, 0), (700, 528, 2064, 0), (130, 1048, 16, 0)])
 def test_gemm_on_pairs_that_share_the_activations(cuda, oracle, M, N, K, fold):
     import pplb200
