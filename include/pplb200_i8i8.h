@@ -428,7 +428,7 @@ void pplb200_debug_gemm_tail_split(int32_t enabled);
 int32_t pplb200_debug_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t swiglu, int32_t* plan);
 
 /* The same: 1 when it runs on CTA pairs that share the activations (folded or not), 0 on single CTAs, -1 on an error. */
-int32_t pplb200_debug_gemm_on_pairs(int64_t M, int64_t N, int64_t K);
+int32_t pplb200_debug_gemm_on_pairs(int64_t M, int64_t N, int64_t K, int32_t swiglu);
 
 /*
  * Storage-order change of a [rows, cols] matrix of int8 (elem_bytes 1) or int32 (elem_bytes 4) elements between

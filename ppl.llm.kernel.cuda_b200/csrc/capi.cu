@@ -515,9 +515,9 @@ int32_t pplb200_debug_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t swiglu,
     if (!plan || M <= 0 || N <= 0 || K <= 0) return fail(RC_INVALID_VALUE, "bad extents or null plan");
     return gemm_decode_plan(M, N, K, swiglu != 0, plan);
 }
-int32_t pplb200_debug_gemm_on_pairs(int64_t M, int64_t N, int64_t K) {
+int32_t pplb200_debug_gemm_on_pairs(int64_t M, int64_t N, int64_t K, int32_t swiglu) {
     if (M <= 0 || N <= 0 || K <= 0) return fail(RC_INVALID_VALUE, "bad extents"), -1;
-    return gemm_decode_on_pairs(M, N, K);
+    return gemm_decode_on_pairs(M, N, K, swiglu != 0);
 }
 void pplb200_debug_gemm_tail_split(int32_t enabled) { set_tail_split(enabled < 0 ? 0 : enabled > 2 ? 2 : enabled); }
 

@@ -204,7 +204,7 @@ constexpr int64_t kCtaPairs = 74;
 bool gemm_preloads_weights(int64_t M, int64_t N, int64_t K);
 int32_t launch_gemm_decode(cudaStream_t stream, const GemmArgs& a, unsigned int* status, bool pdl);
 int32_t gemm_decode_plan(int64_t M, int64_t columns, int64_t K, bool swiglu, int32_t* out);
-int32_t gemm_decode_on_pairs(int64_t M, int64_t columns, int64_t K); // 1 / 0, -1: no device
+int32_t gemm_decode_on_pairs(int64_t M, int64_t columns, int64_t K, bool swiglu); // 1 / 0, -1: no device
 int32_t launch_gemm(cudaStream_t stream, const GemmArgs& a);
 int32_t gemm_status(int32_t reset);
 void set_stall_counters(void* dev_ptr);

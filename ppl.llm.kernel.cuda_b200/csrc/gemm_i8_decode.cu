@@ -761,6 +761,18 @@ void plan_pair(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t kb,
     best.row_tiles = (int)(((columns + best.rows - 1) / best.rows + 1) / 2 * 2);
 }
 
+// The same for x and gate rows, K whole.  Against x and gate on the two halves of one CTA's lanes (2775 shapes of 8 .. 128 tokens): 1.13 up to
+// K 2048, 1.11 up to 4096, 1.05 .. 1.10 beyond; against K shared by two CTAs 1.08 up to 4096 and 0.96 beyond, by three 0.80 .. 0.96.
+void plan_pair_swiglu(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t kb, DecodePlan& best) {
+    const int ctas = dev.sms / 2 * 2;
+    if (best.dual || best.S > 2 || (best.S == 2 && kb > 32) || columns > (int64_t)ctas * (BW / 2)) return;
+    best.pair = true;
+    best.S = 1;
+    best.tokens = (int)((M + 31) / 32 * 32);
+    best.rows = rows_for(columns, ctas, BW / 2);
+    best.row_tiles = (int)(((columns + best.rows - 1) / best.rows + 1) / 2 * 2);
+}
+
 // Up to 128 tokens: one token tile.  Where tiles of full height leave SMs idle, K is shared: by the S CTAs of a cluster, or
 // folded onto the lanes of one CTA (gemm_i8_fold_kernel).  All forms that run as one wave are modelled in SM cycles per CTA: a
 // stage costs the larger of its operands' way from L2 (60 bytes per cycle) and the issuing threads' bookkeeping (415; 425 and 500
@@ -817,6 +829,7 @@ DecodePlan plan_small(const DecDeviceInfo& dev, int64_t M, int64_t columns, int6
         }
     }
     if (!swiglu) plan_pair(dev, M, columns, kb, best);
+    else plan_pair_swiglu(dev, M, columns, kb, best);
     return best;
 }
 
@@ -853,16 +866,18 @@ DecodePlan plan_medium(const DecDeviceInfo& dev, int64_t M, int64_t columns, int
         }
     }
     // CTA pairs that share the activations (gemm_i8_token_pair_kernel), up to 256 tokens per tile, against a whole K per CTA.  Their K
-    // block: 65 bytes per cycle, 380 cycles of bookkeeping, a fixed 1500 and 8 per token.  Fitted to 1881 shapes of 129 .. 1024 tokens:
+    // block: 65 bytes per cycle, 380 cycles of bookkeeping, a fixed 1500 and 8 per token.  Fitted to 1881 shapes (without SwiGLU; with it, on 2260 shapes, up
+    // to 13 % faster up to 256 tokens, level beyond) of 129 .. 1024 tokens:
     // on average 8 % faster than without pairs and 0.4 % slower than the faster of the two; 5 % of distance keeps close calls where they were.
-    if (swiglu || best.S > 1) return best;
+    if (best.S > 1) return best;
+    const int parts = swiglu ? 2 : 1, max_rows = BW / parts;
     best_cost *= 0.95;
     for (int64_t t = (M + 255) / 256; t <= (M + 63) / 64; ++t) {
         const int tokens = (int)(((M + t - 1) / t + 31) / 32 * 32);
         const int64_t token_tiles = (M + tokens - 1) / tokens, ctas = dev.sms / 2 / token_tiles * 2;
-        if (ctas == 0 || columns > ctas * BW) continue; // one wave
-        const int rows = rows_for(columns, ctas, BW);
-        double kb = (rows + tokens / 2) * (double)BK / 65.0;
+        if (ctas == 0 || columns > ctas * max_rows) continue; // one wave
+        const int rows = rows_for(columns, ctas, max_rows);
+        double kb = (rows * parts + tokens / 2) * (double)BK / 65.0;
         const double mma = tokens < 120 ? 240.0 : tokens * 2.0;
         if (kb < mma) kb = mma;
         if (kb < 380.0) kb = 380.0;
@@ -1001,10 +1016,10 @@ int32_t gemm_decode_plan(int64_t M, int64_t columns, int64_t K, bool swiglu, int
     return RC_SUCCESS;
 }
 
-int32_t gemm_decode_on_pairs(int64_t M, int64_t columns, int64_t K) {
+int32_t gemm_decode_on_pairs(int64_t M, int64_t columns, int64_t K, bool swiglu) {
     const DecDeviceInfo* dev = dec_device_info();
     if (!dev) return fail(RC_DEVICE_RUNTIME_ERROR, "device set-up failed: %s", cudaGetErrorString(cudaGetLastError())), -1;
-    return (M > 128 ? plan_medium(*dev, M, columns, (int)((K + BK - 1) / BK), false) : plan_small(*dev, M, columns, K, false)).pair ? 1 : 0;
+    return (M > 128 ? plan_medium(*dev, M, columns, (int)((K + BK - 1) / BK), swiglu) : plan_small(*dev, M, columns, K, swiglu)).pair ? 1 : 0;
 }
 
 int32_t launch_gemm_decode(cudaStream_t stream, const GemmArgs& a, unsigned int* status, bool pdl) {

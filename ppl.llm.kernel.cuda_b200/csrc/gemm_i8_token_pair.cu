@@ -9,6 +9,7 @@
 // F = 1: tokens [0, tile_tokens / 2) come from CTA 0, the rest from CTA 1; K is not shared.
 // F = 2, 4: K is folded onto the TMEM lanes as in gemm_i8_fold_kernel (part f of K: lanes f * tile_rows .., columns f * tokens ..);
 // CTA 0 brings the activations of the first F / 2 parts, CTA 1 those of the others.
+// SWIGLU (F = 1): a CTA's x rows on lanes 0 .., the gate rows of the same channels on the lanes behind them, both by one 3-D box.
 #include "gemm_i8_decode.cuh"
 
 #include <string.h>
@@ -30,7 +31,7 @@ struct TPCfg {
 
 // grid = (2, row pairs, token tiles), cluster = (2, 1, 1).  A stage is one slot of [weights | activations] in each CTA; the leader's
 // full barrier counts the bytes of both CTAs, one multicast commit (a signal, not a load) frees the slot in both.
-template <int F>
+template <int F, bool SWIGLU>
 __global__ void __launch_bounds__(TPCfg::NUM_THREADS, 1)
 gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                           const __grid_constant__ CUtensorMap tmap_y, const DecodeParams p) {
@@ -42,6 +43,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     __shared__ __align__(8) uint64_t acc_full_bar;
     __shared__ uint32_t tmem_base_slot;
     __shared__ __align__(16) float token_scale[256];
+    __shared__ uint32_t token_absmax[SWIGLU ? 256 : 1];
     __shared__ int loads_started;
 
     const int warp = threadIdx.x >> 5;
@@ -78,6 +80,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         ptx::tmem_alloc_pair(ptx::smem_addr(&tmem_base_slot), C::TMEM_COLS);
         ptx::tmem_relinquish_pair();
     }
+    if (SWIGLU && threadIdx.x < 256) token_absmax[threadIdx.x] = 0u;
     ptx::tc_fence_before();
     ptx::cluster_sync_all(); // the barriers of both CTAs are initialised before anyone signals them
     ptx::tc_fence_after();
@@ -93,7 +96,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         auto load_weights = [&](int i, uint32_t s) {
             if (rank == 0) ptx::mbar_arrive_expect_tx(full0 + s * 8u, 2u * ((uint32_t)p.w_box_bytes + x_bytes));
             const uint32_t dst = ring + s * slot;
-            if (F > 1 && p.fold_box) {
+            if (SWIGLU || (F > 1 && p.fold_box)) {
                 ptx::tma_load_3d_pair(dst, &tmap_w, full_leader0 + s * 8u, x_of(i), row0, 0);
             } else {
 #pragma unroll
@@ -139,7 +142,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     } else if (warp == 4 && lane == 0) {
         if (!p.early_weights)
             prefetch_weights(stages, &loads_started, [&](int i) {
-                if (F > 1 && p.fold_box) {
+                if (SWIGLU || (F > 1 && p.fold_box)) {
                     ptx::tma_prefetch_l2_3d(&tmap_w, x_of(i), row0, 0);
                 } else {
 #pragma unroll
@@ -183,14 +186,17 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
 
     // this thread's output column and its constants: lane = weight row
     const int q = warp & 3, grp = warp >> 2;
-    const int nl = F > 1 ? (warp % (ROWS / 32)) * 32 + lane : q * 32 + lane;
+    // (where parts of K or x and gate rows meet in shared memory, of the last pass: warps side by side over the rows)
+    const int row_warps = SWIGLU ? (p.tile_rows > 32 ? 2 : 1) : ROWS / 32;
+    const int nl = F > 1 || SWIGLU ? (warp % row_warps) * 32 + lane : q * 32 + lane;
     const int n = row0 + nl;
     const bool n_ok = nl < p.tile_rows && n < p.N;
-    float sn = 0.0f;
+    float sn = 0.0f, sg = 0.0f;
     half bias_h = __ushort_as_half((unsigned short)0x8000u); // x + (-0.0) == x for every x: no branch for "no bias"
     if (p.mode != EPI_RAW_I32) {
         if (n_ok) {
             sn = __half2float(p.scale_n[n]);
+            if (SWIGLU) sg = __half2float(p.scale_n[n + p.N]);
             if (p.bias != nullptr) bias_h = p.bias[n];
         }
         for (int m = threadIdx.x; m < 256; m += C::NUM_THREADS)
@@ -209,6 +215,64 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         // the blocks take F * (256 / F) * ROWS * 4 bytes of the dead ring, the maxima the next KB
         t_exchange = fold_epilogue<256 / F, F, C::ACC_STRIDE, C::NUM_THREADS, true>(p, tmem_base, ring, ring + 256 * ROWS * 4, valid, acc_ready, nl, n, n_ok, sn,
                                                                               bias_h, token_scale);
+    } else if constexpr (SWIGLU) {
+        // accumulators into the dead ring, [token][x rows, gate rows]; then a warp finishes 32 channels of four tokens at a time
+        const int pitch = 2 * p.tile_rows, lane_row = q * 32 + lane;
+        {
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
+            uint32_t a[8], b[8];
+            auto fetch = [&](int c) {
+                TmemLd<8>::run(taddr + c, a);
+                if (valid > 1) TmemLd<8>::run(taddr + C::ACC_STRIDE + c, b);
+            };
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { a[j] = 0u; b[j] = 0u; }
+            int c0 = grp * 8;
+            if (c0 < M && acc_ready) fetch(c0);
+#pragma unroll 1
+            for (; c0 < M; c0 += 32) {
+                uint32_t v[8];
+                tmem_ld_wait8x2(a, b);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) v[j] = a[j] + b[j];
+                if (c0 + 32 < M && acc_ready) fetch(c0 + 32);
+                if (lane_row < pitch) {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(ring + (uint32_t)((c0 + j) * pitch + lane_row) * 4u), "r"(v[j]) : "memory");
+                }
+            }
+        }
+        ptx::tc_fence_before();
+        __syncthreads();
+        t_exchange = p.stamps ? globaltimer_ns() : 0ull;
+        constexpr int NV = 4;
+#pragma unroll 1
+        for (int m0 = NV * (warp / row_warps); m0 < M; m0 += NV * (C::NUM_THREADS / 32) / row_warps) {
+            uint32_t x[NV], g[NV];
+            float r[NV];
+            const float4 tsv = *reinterpret_cast<const float4*>(&token_scale[m0]);
+            const float ts[NV] = {tsv.x, tsv.y, tsv.z, tsv.w};
+#pragma unroll
+            for (int j = 0; j < NV; ++j) { // lanes past the last row read their neighbours' words
+                const uint32_t addr = ring + (uint32_t)((m0 + j) * pitch + nl) * 4u;
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(x[j]) : "r"(addr) : "memory");
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(g[j]) : "r"(addr + (uint32_t)p.tile_rows * 4u) : "memory");
+            }
+            swiglu_values<NV>(x, g, sn, sg, p.down_n, ts, p.beta, n_ok, r);
+            half* dst = reinterpret_cast<half*>(p.out) + (int64_t)(token0 + m0) * p.ldc + n;
+            uint32_t most = 0u;
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                if (n_ok && m0 + j < M) dst[(int64_t)j * p.ldc] = __float2half_rn(r[j]);
+                const float a = fabsf(r[j]);
+                const uint32_t bits = __reduce_max_sync(0xffffffffu, n_ok && a == a ? __float_as_uint(a) : 0u); // NaNs are dropped, as fmax does
+                if (lane == j) most = bits;
+            }
+            if (lane < NV && most != 0u) atomicMax(&token_absmax[m0 + lane], most);
+        }
+        __syncthreads();
+        const uint32_t ctas = gridDim.y * 2u; // this CTA's row maxima, [token][CTA], as in gemm_i8_decode_kernel
+        for (int m = threadIdx.x; m < M; m += C::NUM_THREADS) p.row_absmax_bits[(int64_t)(token0 + m) * ctas + blockIdx.y * 2u + rank] = token_absmax[m];
     } else {
         // the output tile goes through the dead ring, [token][weight row], and leaves as one TMA store
         const bool staged = !p.raw_affine;
@@ -244,13 +308,13 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     }
 }
 
-template <int F> bool set_attr() {
-    return cudaFuncSetAttribute(gemm_i8_token_pair_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, TPCfg::SMEM_BYTES) == cudaSuccess;
+template <int F, bool SWIGLU> bool set_attr() {
+    return cudaFuncSetAttribute(gemm_i8_token_pair_kernel<F, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, TPCfg::SMEM_BYTES) == cudaSuccess;
 }
 
 } // namespace
 
-bool token_pair_setup() { return set_attr<1>() && set_attr<2>() && set_attr<4>(); }
+bool token_pair_setup() { return set_attr<1, false>() && set_attr<2, false>() && set_attr<4, false>() && set_attr<1, true>(); }
 
 int32_t launch_token_pair(cudaStream_t stream, const GemmArgs& a, const DecodePlan& plan, DecodeParams p, bool pdl) {
     using C = TPCfg;
@@ -258,7 +322,12 @@ int32_t launch_token_pair(cudaStream_t stream, const GemmArgs& a, const DecodePl
     const int F = plan.fold ? plan.fold : 1;
     p.tile_tokens = plan.tokens;
     p.tile_rows = plan.rows;
-    p.w_box_bytes = p.w_slot_bytes = F * plan.rows * BK;
+    const bool swiglu = a.mode == EPI_SWIGLU_F16;
+    if (swiglu) {
+        p.N = (int32_t)(a.N / 2); // x and gate halves of the weight rows share the output columns
+        *a.row_absmax_parts = plan.row_tiles;
+    }
+    p.w_box_bytes = p.w_slot_bytes = F * plan.rows * BK * (swiglu ? 2 : 1);
     p.fold_box = F > 1 && a.K % (16 * F) == 0;
     const int x_rows = F == 1 ? plan.tokens / 2 : plan.tokens;
     const int slot = p.w_slot_bytes + (F == 1 ? x_rows : F / 2 * x_rows) * BK;
@@ -269,10 +338,11 @@ int32_t launch_token_pair(cudaStream_t stream, const GemmArgs& a, const DecodePl
     p.w_stages = depth;
     if (!(p.fold_box ? make_fold_map(&tx, a.A, a.M, a.K, a.lda, F, x_rows, F / 2) : make_map(&tx, a.A, a.M, a.K, a.lda, x_rows)))
         return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (X) encode failed");
-    if (!(p.fold_box ? make_fold_map(&tw, a.B, a.N, a.K, a.ldb, F, plan.rows, F) : make_map(&tw, a.B, a.N, a.K, a.ldb, plan.rows)))
+    if (!(swiglu ? make_halves_map(&tw, a.B, p.N, a.K, a.ldb, plan.rows)
+                 : p.fold_box ? make_fold_map(&tw, a.B, a.N, a.K, a.ldb, F, plan.rows, F) : make_map(&tw, a.B, a.N, a.K, a.ldb, plan.rows)))
         return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (W) encode failed");
     memset(&ty, 0, sizeof(ty)); // only touched by staged tiles
-    if (F == 1 && !p.raw_affine && !make_out_map(&ty, a.out, a.M, a.N, a.ldc, a.mode == EPI_RAW_I32 ? 4 : 2, plan.rows, plan.tokens))
+    if (F == 1 && !swiglu && !p.raw_affine && !make_out_map(&ty, a.out, a.M, a.N, a.ldc, a.mode == EPI_RAW_I32 ? 4 : 2, plan.rows, plan.tokens))
         return fail(RC_DEVICE_RUNTIME_ERROR, "tensor map (Y) encode failed");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2, (unsigned)(plan.row_tiles / 2), (unsigned)plan.token_tiles);
@@ -288,7 +358,8 @@ int32_t launch_token_pair(cudaStream_t stream, const GemmArgs& a, const DecodePl
     attrs[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = pdl ? 2 : 1;
-    const auto kernel = F == 1 ? gemm_i8_token_pair_kernel<1> : F == 2 ? gemm_i8_token_pair_kernel<2> : gemm_i8_token_pair_kernel<4>;
+    const auto kernel = swiglu ? gemm_i8_token_pair_kernel<1, true> : F == 1 ? gemm_i8_token_pair_kernel<1, false>
+                      : F == 2 ? gemm_i8_token_pair_kernel<2, false> : gemm_i8_token_pair_kernel<4, false>;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, tw, tx, ty, p);
     if (e != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "pair GEMM (tokens) launch failed: %s", cudaGetErrorString(e));
     return RC_SUCCESS;

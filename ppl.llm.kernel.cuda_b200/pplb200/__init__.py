@@ -103,7 +103,7 @@ def _load():
     lib.pplb200_debug_gemm_tail_split.argtypes = [i32]
     lib.pplb200_debug_gemm_tail_split.restype = None
     lib.pplb200_debug_gemm_plan.argtypes = [i64, i64, i64, i32, vp]
-    lib.pplb200_debug_gemm_on_pairs.argtypes = [i64, i64, i64]
+    lib.pplb200_debug_gemm_on_pairs.argtypes = [i64, i64, i64, i32]
     lib.pplb200_probe_stream_read.argtypes = [vp, vp, i64, vp]
     lib.pplb200_nccl_get_unique_id.argtypes = [vp]
     lib.pplb200_nccl_comm_init.argtypes = [vp, i32, i32, ctypes.POINTER(vp)]
@@ -590,7 +590,7 @@ def gemm_plan(M, N, K, swiglu=False):
     plan = (ctypes.c_int32 * 8)()
     _check(lib.pplb200_debug_gemm_plan(M, N, K, int(swiglu), plan))
     return dict(zip(("tokens", "token_tiles", "rows", "row_tiles", "split", "parts", "fold", "early_weights"), plan),
-                pairs=not swiglu and lib.pplb200_debug_gemm_on_pairs(M, N, K) == 1)
+                pairs=lib.pplb200_debug_gemm_on_pairs(M, N, K, int(swiglu)) == 1)
 
 
 def gemm_stall_profile(fn):

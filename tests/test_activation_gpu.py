@@ -252,3 +252,12 @@ def test_fused_swiglu_of_values_of_every_magnitude(cuda, M, D, K):
         for a, b in zip(fused, two_step):
             assert cuda.equal(a.view(cuda.int8), b.view(cuda.int8))
     assert pplb200.gemm_status() == 0
+
+
+# CTA pairs, x and gate rows by one box: one to many stages, ragged tokens and channels, a last CTA without channels, token tiles of more than 128
+@pytest.mark.parametrize("M,D,K", [(1, 4752, 1040), (16, 9472, 144), (128, 9472, 272), (70, 4736, 4112), (33, 4800, 2064), (97, 5520, 16), (64, 3200, 4096), (200, 2384, 1040),
+                                   (250, 4608, 528)])
+def test_gate_up_swiglu_on_pairs(cuda, oracle, M, D, K):
+    import pplb200
+    assert pplb200.gemm_plan(M, D, K, swiglu=True)["pairs"]
+    test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K)
