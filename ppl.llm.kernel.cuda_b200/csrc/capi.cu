@@ -470,7 +470,7 @@ int32_t pplb200_i8i8_linear_fp16_host(pplb200_stream_t stream_, const void* x_ho
             if (left < 2 * fine) rows = left;
             else if (chunk == 0) rows = share(wide ? 15 : 25);
             else if (M > c && m0 < c) rows = c - m0; // the rest of the first staging buffer
-            else if (wide && M <= c && chunk == 1) rows = share(30);
+            else if (wide && M <= c && chunk == 1 && left - share(30) >= last_rows + fine) rows = share(30);
             else rows = left - last_rows >= fine ? left - last_rows : left;
             if (rows > left) rows = left;
             if (rows > c - r0) rows = c - r0;
