@@ -1002,8 +1002,8 @@ bool gemm_preloads_weights(int64_t M, int64_t N, int64_t K) {
     if (plan.fold) return plan.fold * M <= 128 && K >= 2048;
     // 16 x 5120 x 14336 warm 15.0 -> 14.3, 48 x 1024 x 11008 cold 12.5 -> 12.1
     if (plan.S > 1) return true;
-    // 24 x 12288 x 5120 cold 15.7 -> 16.4, 24 x 22016 x 5120 cold (two row parts) 23.2 -> 24.1; 128 x 12288 x 8192 cold 30.0 -> 29.3, 96 x 12288 x 8192 warm 27.3 -> 26.1
-    return !plan.dual && M * K >= 320 * 1024;
+    // two row parts: 24 x 22016 x 5120 cold 23.2 -> 24.1
+    return false;
 }
 
 int32_t gemm_decode_plan(int64_t M, int64_t columns, int64_t K, bool swiglu, int32_t* out) {
