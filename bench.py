@@ -706,6 +706,13 @@ def static_config(res, others):
     }
 
 
+def _small_batch_kernel(res):
+    """Name of the kernel that the library's small-batch GEMM takes for a configuration."""
+    import pplb200
+    plan = pplb200.gemm_plan(res["M"], res["Nw"], res["Kw"])
+    return "gemm_i8_token_pair_kernel" if plan["pairs"] else "gemm_i8_fold_kernel" if plan["fold"] else "gemm_i8_decode_kernel"
+
+
 def kernel_roofline(res, args, peaks, tensor_peak, impl):
     """roofline-shaped object for the dominant kernel of one configuration."""
     kt = res["ms_k"] / args.steps * 1e-3
@@ -714,7 +721,7 @@ def kernel_roofline(res, args, peaks, tensor_peak, impl):
     if res["bound"] == "hbm":
         ach = res["gemm_bytes"] / kt / 1e9
         return {"bound": "hbm", "achieved": ach, "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": ach / peaks["hbm_gbs"],
-                "traffic": traffic, "kernel": "gemm_i8_decode_kernel" if impl == "ours" else ref_kernel,
+                "traffic": traffic, "kernel": _small_batch_kernel(res) if impl == "ours" else ref_kernel,
                 "kernel_us": kt * 1e6, "algorithmic_bytes_per_launch": res["gemm_bytes"],
                 "peak_source": "%s STREAM-copy GB/s" % peaks["source"], "frac_of_8TBs_datasheet": ach / HBM_DATASHEET_GBS}
     ach = 2.0 * res["M"] * res["Nw"] * res["Kw"] / kt / 1e12
