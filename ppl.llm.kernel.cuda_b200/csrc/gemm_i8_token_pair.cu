@@ -88,6 +88,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     const unsigned long long t_setup = p.stamps ? globaltimer_ns() : 0ull;
 
     bool ok = true;
+    int issued = 0; // the producer thread: stages requested so far
     const uint32_t full0 = ptx::smem_addr(&full_bar[0]), empty0 = ptx::smem_addr(&empty_bar[0]);
     if (warp == 0 && lane == 0) {
         // ---- TMA producer of this CTA's half of every stage.  Weights ahead of the dependency wait only where nothing still
@@ -128,6 +129,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
             load_weights(i, (uint32_t)i);
             if (!p.early_weights) load_tokens(i, (uint32_t)i);
         }
+        issued = pre;
         if (p.early_weights) {
             pdl_wait_before_tma(); // quantized activations are written by the preceding kernel
             for (int i = 0; i < pre; ++i) load_tokens(i, (uint32_t)i);
@@ -137,6 +139,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
             if (!ptx::mbar_wait(empty0 + s * 8u, phase, p.status, ST_DEC_PRODUCER)) { ok = false; break; }
             load_weights(i, s);
             load_tokens(i, s);
+            issued = i + 1;
             if (++s == depth) { s = 0; phase ^= 1u; }
         }
     } else if (warp == 4 && lane == 0) {
@@ -204,6 +207,12 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     }
 
     const bool acc_ready = ptx::mbar_wait(ptx::smem_addr(&acc_full_bar), 0, p.status, ST_DEC_EPI);
+    // A wait has run out: no MMA waits for the boxes still under way, so the thread that counts them does (both CTAs' are counted in
+    // the leader, and the partner stays until this warp has arrived at the cluster barrier below).
+    if (!acc_ready && warp == 0 && lane == 0 && rank == 0)
+        for (int u = issued > (int)depth ? issued - (int)depth : 0; u < issued; ++u)
+            if (!ptx::mbar_wait(full0 + (uint32_t)(u % (int)depth) * 8u, (uint32_t)(u / (int)depth) & 1u, p.status, ST_DEC_PRODUCER)) break;
+    __syncwarp();
     ptx::tc_fence_after();
     pdl_launch_dependents();
     const unsigned long long t_main = p.stamps ? globaltimer_ns() : 0ull;
@@ -213,7 +222,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
 
     if constexpr (F > 1) {
         // the blocks take F * (256 / F) * ROWS * 4 bytes of the dead ring, the maxima the next KB
-        t_exchange = fold_epilogue<256 / F, F, C::ACC_STRIDE, C::NUM_THREADS, true>(p, tmem_base, ring, ring + 256 * ROWS * 4, valid, acc_ready, nl, n, n_ok, sn,
+        t_exchange = fold_epilogue<256 / F, F, C::ACC_STRIDE, C::NUM_THREADS, true, true>(p, tmem_base, ring, ring + 256 * ROWS * 4, valid, acc_ready, nl, n, n_ok, sn,
                                                                               bias_h, token_scale);
     } else if constexpr (SWIGLU) {
         // accumulators into the dead ring, [token][x rows, gate rows]; then a warp finishes 32 channels of four tokens at a time
@@ -244,6 +253,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         }
         ptx::tc_fence_before();
         __syncthreads();
+        cluster_arrive(); // see the end
         t_exchange = p.stamps ? globaltimer_ns() : 0ull;
         constexpr int NV = 4;
 #pragma unroll 1
@@ -278,6 +288,9 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         const bool staged = !p.raw_affine;
         tile_epilogue<C::ACC_STRIDE, C::NUM_THREADS / 128>(p, tmem_base + ((uint32_t)(q * 32) << 16), valid, acc_ready, ring, p.tile_rows, nl, nl < p.tile_rows, n,
                                                            sn, bias_h, token_scale, token0, M, grp);
+        ptx::tc_fence_before();
+        __syncwarp();
+        cluster_arrive(); // see the end
         if (staged) {
             ptx::fence_proxy_async_smem(); // the tile is read by the TMA unit
             __syncthreads();
@@ -293,10 +306,11 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         }
     }
 
-    // Either CTA may leave now: whatever its partner signals has been waited for -- the leader's full barriers before each MMA, the
-    // commits that free slots (none for the last uses) by the producers, the end of all MMAs by every thread.
-    ptx::tc_fence_before();
-    __syncthreads();
+    // Tensor memory was allocated by both CTAs together and is given back by both: each thread has arrived at the cluster barrier
+    // once its own tcgen05.ld's were complete, so nobody reads it any more when the wait returns, and neither CTA leaves while boxes
+    // of its partner are still counted on its barriers.  The arrival lies before the second half of the epilogue, which hides the wait.
+    __syncwarp();
+    cluster_wait();
     if (warp == 1) {
         ptx::tc_fence_after();
         ptx::tmem_dealloc_pair(tmem_base, C::TMEM_COLS);

@@ -596,3 +596,24 @@ def test_gemm_on_pairs_that_share_the_activations(cuda, oracle, M, N, K, fold):
         test_decode_gemm_all_modes(cuda, oracle, M, N, K)
     test_gemm_i32_alpha_beta_bias(cuda, M, N, K, 1, 0, False)
     test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
+
+
+# The second CTA of the last pair has no weight rows and is done first: whole K (one and several token tiles), K folded in two and four
+@pytest.mark.parametrize("M,N,K,fold", [(128, 12224, 1040, 0), (129, 2064, 528, 0), (128, 8192, 4096, 2), (64, 4064, 8192, 4)])
+def test_pair_gemm_with_an_idle_partner_between_others(cuda, M, N, K, fold):
+    """Both CTAs of a pair give their tensor memory back together: launches in turn with kernels that allocate it in other shapes."""
+    import pplb200
+    plan = pplb200.gemm_plan(M, N, K)
+    assert plan["pairs"] and plan["fold"] == fold and plan["rows"] * (plan["row_tiles"] - 1) >= N, plan
+    g = cuda.Generator(device="cuda").manual_seed(M + N + K)
+    ops = []
+    for m, n, k in ((M, N, K), (16, 1024, 512), (2400, 2048, 256)):
+        a, b = (cuda.randint(-127, 128, (r, k), generator=g, device="cuda", dtype=cuda.int8) for r in (m, n))
+        ops.append((a, b, cuda.empty((m, n), dtype=cuda.int32, device="cuda"), (a.double() @ b.double().T).to(cuda.int32)))  # exact in fp64
+    wrong = cuda.zeros((), dtype=cuda.int64, device="cuda")
+    for i in range(60):
+        for a, b, out, want in (ops[0], ops[1 + i % 2], ops[0]):
+            out.zero_() if i % 3 == 0 else None
+            pplb200.gemm_i8i8(a, b, out=out)
+            wrong += (out != want).sum()
+    assert int(wrong) == 0 and pplb200.gemm_status() == 0
