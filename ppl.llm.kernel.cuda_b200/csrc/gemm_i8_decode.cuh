@@ -187,9 +187,12 @@ __device__ __forceinline__ void prefetch_weights(int stages, int* loads_started,
 // stand-alone kernel of activation_requant.cu computes them.  The division there is the compiler's, whose special cases branch; with a
 // branch per value the NV chains run one after another (128 x 11008 x 4096: 11.7 us for the epilogue).  Here the quotient is Markstein's
 // ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): a reciprocal refined once, the quotient
-// corrected twice by its exact residual, which rounds correctly while nothing over- or underflows.  The denominator is at least 1; values
-// for which it is not well below 2^127, or whose x is tiny, infinite or no number, take the compiler's division, a warp at a time (live:
-// this lane's values are used).
+// corrected twice by its exact residual, which rounds correctly while nothing over- or underflows, wherever the reciprocal is the
+// correctly rounded one.  With an approximation anywhere within two ulps of it that holds for all but a few dozen mantissas of the denominator, and
+// over all numerators only three of them, 7ffffb, 7ffffd and 7fffff, give a wrong quotient (enumerated with fmaf on the host; B200's own
+// approximation refines to the correctly rounded reciprocal for all 2^23).  The denominator is at least 1; values whose denominator has
+// one of the last eight mantissas or is not well below 2^127, or whose x is tiny, infinite or no number, take the compiler's division, a warp
+// at a time (live: this lane's values are used).
 template <int NV>
 __device__ __forceinline__ void swiglu_values(const uint32_t (&xi)[NV], const uint32_t (&gi)[NV], float sx, float sg, float down_n, const float (&ts)[NV],
                                               float beta, bool live, float (&r)[NV]) {
@@ -200,6 +203,7 @@ __device__ __forceinline__ void swiglu_values(const uint32_t (&xi)[NV], const ui
         x[j] = __fmul_rn(__fmul_rn(__fmul_rn((float)(int32_t)xi[j], sx), down_n), ts[j]);
         d[j] = __fadd_rn(1.0f, __expf(__fmul_rn(-x[j], beta)));
         // +0 / d comes out as +0 either way, -0 / d would not; the comparisons are false for NaNs
+        special |= (__float_as_uint(d[j]) | 0xff800007u) == 0xffffffffu;
         special |= !(d[j] < 0x1p100f && fabsf(x[j]) < 0x1p100f && (fabsf(x[j]) > 0x1p-20f || __float_as_uint(x[j]) == 0u));
     }
 #pragma unroll

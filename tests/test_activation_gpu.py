@@ -261,3 +261,30 @@ def test_gate_up_swiglu_on_pairs(cuda, oracle, M, D, K):
     import pplb200
     assert pplb200.gemm_plan(M, D, K, swiglu=True)["pairs"]
     test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K)
+
+
+@pytest.mark.parametrize("M,D,K,form", [(40, 11008, 272, "two parts"), (64, 2800, 144, "pairs"), (33, 2688, 8192, "shared")])
+def test_fused_swiglu_quotient_by_all_ones(cuda, M, D, K, form):
+    """x a power of two over 1 + exp(-beta x) = 2 - 2^-23, whose mantissa bits are all ones: a quotient that a refined reciprocal and two
+    corrections round wrongly unless the approximate reciprocal is the nearest one.  The gate is 2^16 (1 + 2^-11), so that without its
+    last bit the quotient would turn a value just above the middle of two fp16 numbers into the middle itself."""
+    import pplb200
+    plan = pplb200.gemm_plan(M, D, K, swiglu=True)
+    assert {"two parts": plan["parts"] == 2, "pairs": plan["pairs"], "shared": plan["split"] > 1}[form], plan
+    xq = cuda.zeros((M, K), dtype=cuda.int8, device="cuda")
+    w = cuda.zeros((2 * D, K), dtype=cuda.int8, device="cuda")
+    xq[:, 0], xq[:, 1] = 1, 127
+    w[:D, 0] = 1                    # x rows: 1
+    w[D:, 0], w[D:, 1] = 17, 16     # gate rows: 17 + 127 * 16 = 2049
+    sm = cuda.full((M,), 2.0 ** 15, device="cuda").half()
+    sn = cuda.full((2 * D,), 2.0 ** 15, device="cuda").half()
+    sn[:D] = 2.0 ** -9              # x = 2^-9 2^15 2^-25 = 2^-19
+    acc = pplb200.column_parallel_linear(xq, w, None, None, None, K, 2 * D, gather_output=False)
+    hit = False
+    for t in (0.5, 0.625, 0.75, 0.875, 1.0, 1.125, 1.25, 1.375, 1.5):  # beta x about 2^-23: one of them gives 2 - 2^-23
+        two_step = pplb200.minmax_requantize_swiglu_fp16(acc, sm, sn, beta=t * 2.0 ** -4)
+        fused = pplb200.gate_up_swiglu_requant(xq, w, sm, sn, beta=t * 2.0 ** -4)
+        hit |= bool((two_step[0] == 2.0 ** -4 * (1 + 2.0 ** -10)).any())
+        for a, b in zip(fused, two_step):
+            assert cuda.equal(a.view(cuda.int8), b.view(cuda.int8)), t
+    assert hit and pplb200.gemm_status() == 0
