@@ -431,6 +431,12 @@ int32_t pplb200_debug_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t swiglu,
 int32_t pplb200_debug_gemm_on_pairs(int64_t M, int64_t N, int64_t K, int32_t swiglu);
 
 /*
+ * Diagnostics: the chunks of pplb200_i8i8_linear_fp16_host for a batch below two of chunk_rows (0: the default).  Writes the row at which each
+ * ends (at most five) and the first row that lies in the second staging buffer (M: none), returns how many there are; 0 for larger batches, -1 on an error.
+ */
+int32_t pplb200_debug_host_cut(int64_t M, int64_t N, int64_t K, int64_t chunk_rows, int64_t* ends, int64_t* split);
+
+/*
  * Storage-order change of a [rows, cols] matrix of int8 (elem_bytes 1) or int32 (elem_bytes 4) elements between
  * any two of ROW_MAJOR, COL32, COL32_2R_4R4 and COL4_4R2_8C (index maps of
  * include/ppl/kernel/llm/cuda/common/matrix_layout.h:34-142; no counterpart function in the reference, whose

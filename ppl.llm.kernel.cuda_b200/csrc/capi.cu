@@ -399,6 +399,55 @@ int64_t host_chunk_rows(int64_t M, int64_t chunk_rows) {
     if (chunk_rows <= 0) chunk_rows = 1024;
     return chunk_rows < M ? chunk_rows : M;
 }
+
+// How a batch is cut into chunks of rows, over two staging buffers of c rows.
+//
+// Two chunks and more: the copy-out of the results is the longest of the three pipelines (PCIe, fp16 [rows, N]), and it can
+// only start once the first chunk has been copied in and computed.  So the first full chunk is fed in as c/8, c/8,
+// c/4, c/2 rows (each step's copy-in + compute still fits under the previous step's copy-out), which starts the
+// copy-out after an eighth of the fill time.
+//
+// A batch below two chunks fits the two staging buffers as a whole: no part of them is used twice.  Its chunks are few: while
+// results leave, the end of a copy in is seen some 15 us late, by the kernel that waits for it and by the next copy.  Up to
+// 12 MB a quarter, a half and a quarter, beyond 15, 30, 35 and 20 % (us per call, with chunks of 128 and 256 rows / now:
+// 1024 x 4096 x 4096 308 / 286, 1000 x 8192 x 1024 re-quantized 414 / 375, 1999 x 4096 x 5120 re-quantized 777 / 750; even shares
+// 300 at the first).  A first and last chunk no shorter than `fine` rows, which take as long on the wire as their linear does
+// (the weights at about 5 TB/s plus 10 us of launches, against 55 GB/s of PCIe); less than two such chunks are not cut at all.
+// A chunk lies in one buffer.  Above c rows the second buffer begins behind the first two of four chunks, or before the last of three; where
+// that would leave more than c rows on one side, as near to it as fits.
+struct HostCut {
+    int64_t M, c, end[5], split; // end: rows up to the end of each chunk of a batch below two of c; split: first row of the second buffer
+    bool flat, ramp;
+
+    HostCut(int64_t M_, int64_t N, int64_t K, int64_t c_) : M(M_), c(c_), split(M_), flat(M_ < 2 * c_), ramp(c_ >= 1024 && M_ >= 2 * c_) {
+        if (!flat) return;
+        const int64_t row_bytes = 2 * (K > N ? K : N);
+        int64_t fine = (N * K / 5000 + 10000) * 55 / row_bytes; // ns x bytes per ns / bytes per row
+        fine = fine < 128 ? 128 : round_up(fine, 128);          // 0 where a row alone takes longer than the launches (K 16, N 524288)
+        const auto share = [&](int64_t percent) { const int64_t r = round_up(M * percent / 100, 8); return r > fine ? r : fine; };
+        const bool large = M * row_bytes > (12 << 20);
+        const int64_t first = share(large ? 15 : 25), second = first + share(30), before_last = M - share(large ? 20 : 25);
+        const bool four = large && before_last - second >= fine;
+        if (M > c) { // both sides of the split hold at most c rows
+            split = four ? second : M >= 2 * fine ? before_last : round_up(M / 2, 8);
+            if (split > c) split = c;
+            if (split < M - c) split = M - c;
+        }
+        int n = 0;
+        const auto cut = [&](int64_t at) { if (at > (n ? end[n - 1] : 0) && at < M) end[n++] = at; };
+        if (M >= 2 * fine && (M <= c || split - first >= fine)) cut(first);
+        if (M > c) cut(split);
+        else if (four) cut(second);
+        if (n && M - end[n - 1] >= 2 * fine && before_last - end[n - 1] >= fine) cut(before_last);
+        end[n] = M;
+    }
+
+    // Rows of chunk number `chunk`, which begins at row m0.
+    int64_t rows(int64_t m0, int64_t chunk) const {
+        const int64_t r = flat ? end[chunk] - m0 : !ramp || chunk >= 4 ? c : chunk < 2 ? c / 8 : chunk == 2 ? c / 4 : c / 2;
+        return r < M - m0 ? r : M - m0;
+    }
+};
 } // namespace
 
 int64_t pplb200_i8i8_linear_host_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t epilogue_mode, int64_t chunk_rows) {
@@ -442,42 +491,14 @@ int32_t pplb200_i8i8_linear_fp16_host(pplb200_stream_t stream_, const void* x_ho
     PPLB200_CU(cudaEventRecord(h->start, stream));
     PPLB200_CU(cudaStreamWaitEvent(h->in, h->start, 0));
     PPLB200_CU(cudaStreamWaitEvent(h->out, h->start, 0));
-    // Chunk sizes: the copy-out of the results is the longest of the three pipelines (PCIe, fp16 [rows, N]), and it can
-    // only start once the first chunk has been copied in and computed.  So the first full chunk is fed in as c/8, c/8,
-    // c/4, c/2 rows (each step's copy-in + compute still fits under the previous step's copy-out), which starts the
-    // copy-out after an eighth of the fill time.
-    const bool ramp = c >= 1024 && M >= 2 * c;
-    // A batch below two chunks fits the two staging buffers as a whole: no part of them is used twice.  Its chunks are few: while
-    // results leave, the end of a copy in is seen some 15 us late, by the kernel that waits for it and by the next copy.  Up to
-    // 12 MB a quarter, a half and a quarter, beyond 15, 30 .. 35 and 20 % (us per call, with chunks of 128 and 256 rows / now:
-    // 1024 x 4096 x 4096 308 / 286, 1000 x 8192 x 1024 re-quantized 414 / 375, 1999 x 4096 x 5120 re-quantized 777 / 750; even shares
-    // 300 at the first).  A first and last chunk no shorter than `fine` rows, which take as long on the wire as their linear does
-    // (the weights at about 5 TB/s plus 10 us of launches, against 55 GB/s of PCIe); less than two such chunks are not cut at all.
-    const bool flat = M < 2 * c;
-    const int64_t row_bytes = 2 * (K > N ? K : N);
-    int64_t fine = (N * K / 5000 + 10000) * 55 / row_bytes; // ns x bytes per ns / bytes per row
-    fine = fine < 128 ? 128 : round_up(fine, 128);          // 0 where a row alone takes longer than the launches (K 16, N 524288)
+    const HostCut cut(M, N, K, c);
+    const bool flat = cut.flat;
     int64_t chunk = 0, rows = 0;
     int last = 0;
     for (int64_t m0 = 0; m0 < M; m0 += rows, ++chunk) {
-        const int b = flat ? (m0 < c ? 0 : 1) : (int)(chunk & 1);
-        const int64_t r0 = flat ? m0 - b * c : 0; // first row inside the staging buffer
-        if (flat) {
-            const int64_t left = M - m0;
-            const bool wide = M * row_bytes > (12 << 20);
-            const auto share = [&](int64_t percent) { const int64_t r = round_up(M * percent / 100, 8); return r > fine ? r : fine; };
-            const int64_t last_rows = share(wide ? 20 : 25);
-            if (left < 2 * fine) rows = left;
-            else if (chunk == 0) rows = share(wide ? 15 : 25);
-            else if (M > c && m0 < c) rows = c - m0; // the rest of the first staging buffer
-            else if (wide && M <= c && chunk == 1 && left - share(30) >= last_rows + fine) rows = share(30);
-            else rows = left - last_rows >= fine ? left - last_rows : left;
-            if (rows > left) rows = left;
-            if (rows > c - r0) rows = c - r0;
-        } else {
-            rows = !ramp || chunk >= 4 ? c : chunk < 2 ? c / 8 : chunk == 2 ? c / 4 : c / 2;
-        }
-        if (rows > M - m0) rows = M - m0;
+        rows = cut.rows(m0, chunk);
+        const int b = flat ? (m0 < cut.split ? 0 : 1) : (int)(chunk & 1);
+        const int64_t r0 = flat ? m0 - b * cut.split : 0; // first row inside the staging buffer
         char* const xc = xd[b] + r0 * K * 2;
         char* const yc = yd[b] + r0 * N * 2;
         char* const yqc = requant ? yqd[b] + r0 * N : nullptr;
@@ -518,6 +539,15 @@ int32_t pplb200_debug_gemm_plan(int64_t M, int64_t N, int64_t K, int32_t swiglu,
 int32_t pplb200_debug_gemm_on_pairs(int64_t M, int64_t N, int64_t K, int32_t swiglu) {
     if (M <= 0 || N <= 0 || K <= 0) return fail(RC_INVALID_VALUE, "bad extents"), -1;
     return gemm_decode_on_pairs(M, N, K, swiglu != 0);
+}
+int32_t pplb200_debug_host_cut(int64_t M, int64_t N, int64_t K, int64_t chunk_rows, int64_t* ends, int64_t* split) {
+    if (!ends || !split || M <= 0 || N <= 0 || K <= 0) return fail(RC_INVALID_VALUE, "bad extents or null pointer"), -1;
+    const HostCut cut(M, N, K, host_chunk_rows(M, chunk_rows));
+    if (!cut.flat) return 0;
+    int32_t n = 0;
+    do ends[n] = cut.end[n]; while (cut.end[n++] < M);
+    *split = cut.split;
+    return n;
 }
 void pplb200_debug_gemm_tail_split(int32_t enabled) { set_tail_split(enabled < 0 ? 0 : enabled > 2 ? 2 : enabled); }
 

@@ -42,7 +42,7 @@ EXPORTS = [
     "pplb200_i8i8_row_parallel_p2p_bytes", "pplb200_p2p_create", "pplb200_p2p_export", "pplb200_p2p_connect",
     "pplb200_p2p_connect_local", "pplb200_p2p_destroy", "pplb200_p2p_status", "pplb200_i8i8_row_parallel_linear_p2p",
     "pplb200_i8i8_minmax_quantize_fp16_p2p",
-    "pplb200_probe_tensor_peak", "pplb200_probe_stream_read", "pplb200_i8i8_gemm_i32", "pplb200_debug_gemm_stall_counters", "pplb200_debug_gemm_tail_split", "pplb200_debug_gemm_plan", "pplb200_debug_gemm_on_pairs", "pplb200_i8i8_relayout", "pplb200_i8i8_column_parallel_linear_p2p", "pplb200_i8i8_linear_host_workspace_bytes", "pplb200_i8i8_linear_fp16_host",
+    "pplb200_probe_tensor_peak", "pplb200_probe_stream_read", "pplb200_i8i8_gemm_i32", "pplb200_debug_gemm_stall_counters", "pplb200_debug_gemm_tail_split", "pplb200_debug_gemm_plan", "pplb200_debug_gemm_on_pairs", "pplb200_debug_host_cut", "pplb200_i8i8_relayout", "pplb200_i8i8_column_parallel_linear_p2p", "pplb200_i8i8_linear_host_workspace_bytes", "pplb200_i8i8_linear_fp16_host",
 ]
 STATIC_SCRATCH_MAX_ROWS = 16384
 
@@ -104,6 +104,7 @@ def _load():
     lib.pplb200_debug_gemm_tail_split.restype = None
     lib.pplb200_debug_gemm_plan.argtypes = [i64, i64, i64, i32, vp]
     lib.pplb200_debug_gemm_on_pairs.argtypes = [i64, i64, i64, i32]
+    lib.pplb200_debug_host_cut.argtypes = [i64, i64, i64, i64, vp, vp]
     lib.pplb200_probe_stream_read.argtypes = [vp, vp, i64, vp]
     lib.pplb200_nccl_get_unique_id.argtypes = [vp]
     lib.pplb200_nccl_comm_init.argtypes = [vp, i32, i32, ctypes.POINTER(vp)]
@@ -591,6 +592,15 @@ def gemm_plan(M, N, K, swiglu=False):
     _check(lib.pplb200_debug_gemm_plan(M, N, K, int(swiglu), plan))
     return dict(zip(("tokens", "token_tiles", "rows", "row_tiles", "split", "parts", "fold", "early_weights"), plan),
                 pairs=lib.pplb200_debug_gemm_on_pairs(M, N, K, int(swiglu)) == 1)
+
+
+def host_cut(M, N, K, chunk_rows=0):
+    """Diagnostics: (rows of each chunk, first row in the second staging buffer) of the linear on host buffers; None from two chunk_rows up."""
+    ends, split = (ctypes.c_int64 * 5)(), ctypes.c_int64()
+    n = lib.pplb200_debug_host_cut(M, N, K, chunk_rows, ends, ctypes.byref(split))
+    if n < 0:
+        _check(RC_INVALID_VALUE)
+    return ([b - a for a, b in zip([0] + ends[:n], ends[:n])], split.value) if n else None
 
 
 def gemm_stall_profile(fn):

@@ -223,3 +223,20 @@ int main() {
     cmd = ["g++", "-std=c++17", "-Wall", "-c", "-I" + os.path.join(ROOT, "include"), "-I" + os.path.join(REFERENCE_DIR, "include"),
            "-I" + os.path.join(ROOT, "include", "compat"), "-I/usr/local/cuda/include", str(src), "-o", str(obj)]
     subprocess.run(cmd, check=True)
+
+
+@pytest.mark.parametrize("N,K,chunk", [(4096, 4096, 0), (1024, 11008, 0), (11008, 4096, 0), (272, 512, 0), (528, 1040, 256), (16384, 28672, 1001), (524288, 16, 0), (80, 576, 1000)])
+def test_host_linear_cut(N, K, chunk):
+    """Chunks of the linear on host buffers below two of chunk_rows: they cover the batch in order, each lies in one of two staging buffers of
+    chunk_rows rows, none of a batch that is cut into pieces worth their copies is a few rows long, none is nearly the whole batch."""
+    import pplb200
+    c0 = chunk or 1024
+    assert pplb200.host_cut(2 * c0, N, K, chunk) is None
+    for M in sorted(set(range(1, 2 * c0, 13)) | set(range(c0 - 3, c0 + 40)) | {c0 * 4 // 3, c0 * 9 // 5, 2 * c0 - 1}):
+        rows, split = pplb200.host_cut(M, N, K, chunk)
+        ends = [sum(rows[:i + 1]) for i in range(len(rows))]
+        c = min(c0, M)
+        assert min(rows) > 0 and ends[-1] == M and len(rows) <= 5
+        assert (split == M) if M <= c0 else (split in ends and split <= c and M - split <= c)
+        if c0 >= 1000 and M > c0:
+            assert min(rows) >= min(128, M // 8) and max(rows) <= max(M * 2 // 3, 2 * min(rows)), (M, rows)
