@@ -668,8 +668,8 @@ gemm_i8_fold_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_con
     pdl_launch_dependents();
     const unsigned long long t_main = p.stamps ? globaltimer_ns() : 0ull;
 
-    const unsigned long long t_exchange = fold_epilogue<BT, F, F * BT, C::NUM_THREADS, false, false>(p, tmem_base, ring, x_ring, per_part < 2 ? per_part : 2, acc_ready,
-                                                                                       nl, n, n_ok, sn, bias_h, token_scale);
+    const unsigned long long t_exchange = fold_epilogue<BT, F, F * BT, C::NUM_THREADS, false>(p, tmem_base, ring, x_ring, per_part < 2 ? per_part : 2, acc_ready,
+                                                                                       nl, n, n_ok, sn, bias_h, token_scale, [] {});
     if (warp == 1) {
         __syncwarp();
         ptx::tc_fence_after();

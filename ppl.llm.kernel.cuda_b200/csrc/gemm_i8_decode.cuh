@@ -291,11 +291,11 @@ __device__ __forceinline__ void tile_epilogue(const DecodeParams& p, uint32_t ta
 // f * (DENSE ? tile_rows : 128 / F) .., columns f * tile_tokens ..; two accumulator tiles ACC_STRIDE columns apart, `valid` of them used) meet in shared
 // memory at `blocks`, [part][token][row] with BT >= tokens, and leave summed; a warp handles 32 rows of one token at a time.
 // Row maxima for the re-quantizer are gathered at `maxima`.  nl / n: this thread's row in the tile and output column, sn / bias its
-// constants.  PAIR: every thread arrives at the cluster barrier once tensor memory has been read; the caller waits there.  Called by
+// constants.  after_reads() is called once this warp has read tensor memory.  Called by
 // every thread; returns the time stamp between the two halves.
-template <int BT, int F, int ACC_STRIDE, int THREADS, bool DENSE, bool PAIR>
+template <int BT, int F, int ACC_STRIDE, int THREADS, bool DENSE, typename Done>
 __device__ __forceinline__ unsigned long long fold_epilogue(const DecodeParams& p, uint32_t tmem_base, uint32_t blocks, uint32_t maxima, int valid,
-                                                            bool acc_ready, int nl, int n, bool n_ok, float sn, half bias_h, const float* token_scale) {
+                                                            bool acc_ready, int nl, int n, bool n_ok, float sn, half bias_h, const float* token_scale, Done after_reads) {
     constexpr int ROWS = BW / F, ROW_WARPS = ROWS / 32, GROUPS = THREADS / 128;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     {
@@ -326,8 +326,8 @@ __device__ __forceinline__ unsigned long long fold_epilogue(const DecodeParams& 
         }
     }
     ptx::tc_fence_before();
+    after_reads();
     __syncthreads();
-    if (PAIR) cluster_arrive();
     const unsigned long long t_exchange = p.stamps ? globaltimer_ns() : 0ull;
 
     // ---- sums and epilogue: a warp handles 32 rows of one token at a time

@@ -29,6 +29,12 @@ struct TPCfg {
     static constexpr int ACC_STRIDE = 256;
 };
 
+// Waits for the boxes of the last `depth` of the `issued` stages: for a CTA that gives up, so that none is under way when it leaves.
+__device__ __noinline__ void wait_for_boxes(uint32_t full0, int issued, int depth, unsigned int* status) {
+    for (int u = issued > depth ? issued - depth : 0; u < issued; ++u)
+        if (!ptx::mbar_wait(full0 + (uint32_t)(u % depth) * 8u, (uint32_t)(u / depth) & 1u, status, ST_DEC_PRODUCER)) break;
+}
+
 // grid = (2, row pairs, token tiles), cluster = (2, 1, 1).  A stage is one slot of [weights | activations] in each CTA; the leader's
 // full barrier counts the bytes of both CTAs, one multicast commit (a signal, not a load) frees the slot in both.
 template <int F, bool SWIGLU>
@@ -41,10 +47,12 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     __shared__ __align__(8) uint64_t full_bar[C::MAX_STAGES]; // used in the leader: both CTAs' boxes have landed
     __shared__ __align__(8) uint64_t empty_bar[C::MAX_STAGES];
     __shared__ __align__(8) uint64_t acc_full_bar;
+    __shared__ __align__(8) uint64_t tmem_read_bar; // both CTAs' warps have read their accumulators
     __shared__ uint32_t tmem_base_slot;
     __shared__ __align__(16) float token_scale[256];
     __shared__ uint32_t token_absmax[SWIGLU ? 256 : 1];
     __shared__ int loads_started;
+    __shared__ int issued; // stages that the producer has requested
 
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
@@ -68,6 +76,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
             ptx::prefetch_tensormap(&tmap_w);
             ptx::prefetch_tensormap(&tmap_x);
             ptx::mbar_init(ptx::smem_addr(&acc_full_bar), 2);
+            ptx::mbar_init(ptx::smem_addr(&tmem_read_bar), 2 * (C::NUM_THREADS / 32));
             loads_started = 0;
         }
         if (lane < C::MAX_STAGES) {
@@ -88,7 +97,6 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     const unsigned long long t_setup = p.stamps ? globaltimer_ns() : 0ull;
 
     bool ok = true;
-    int issued = 0; // the producer thread: stages requested so far
     const uint32_t full0 = ptx::smem_addr(&full_bar[0]), empty0 = ptx::smem_addr(&empty_bar[0]);
     if (warp == 0 && lane == 0) {
         // ---- TMA producer of this CTA's half of every stage.  Weights ahead of the dependency wait only where nothing still
@@ -129,19 +137,19 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
             load_weights(i, (uint32_t)i);
             if (!p.early_weights) load_tokens(i, (uint32_t)i);
         }
-        issued = pre;
         if (p.early_weights) {
             pdl_wait_before_tma(); // quantized activations are written by the preceding kernel
             for (int i = 0; i < pre; ++i) load_tokens(i, (uint32_t)i);
         }
         uint32_t s = 0, phase = 0; // phase of the release that the next use of slot s waits for
-        for (int i = pre; i < stages; ++i) {
+        int i = pre;
+        for (; i < stages; ++i) {
             if (!ptx::mbar_wait(empty0 + s * 8u, phase, p.status, ST_DEC_PRODUCER)) { ok = false; break; }
             load_weights(i, s);
             load_tokens(i, s);
-            issued = i + 1;
             if (++s == depth) { s = 0; phase ^= 1u; }
         }
+        *static_cast<volatile int*>(&issued) = i;
     } else if (warp == 4 && lane == 0) {
         if (!p.early_weights)
             prefetch_weights(stages, &loads_started, [&](int i) {
@@ -207,23 +215,27 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
     }
 
     const bool acc_ready = ptx::mbar_wait(ptx::smem_addr(&acc_full_bar), 0, p.status, ST_DEC_EPI);
-    // A wait has run out: no MMA waits for the boxes still under way, so the thread that counts them does (both CTAs' are counted in
-    // the leader, and the partner stays until this warp has arrived at the cluster barrier below).
-    if (!acc_ready && warp == 0 && lane == 0 && rank == 0)
-        for (int u = issued > (int)depth ? issued - (int)depth : 0; u < issued; ++u)
-            if (!ptx::mbar_wait(full0 + (uint32_t)(u % (int)depth) * 8u, (uint32_t)(u / (int)depth) & 1u, p.status, ST_DEC_PRODUCER)) break;
-    __syncwarp();
     ptx::tc_fence_after();
     pdl_launch_dependents();
     const unsigned long long t_main = p.stamps ? globaltimer_ns() : 0ull;
     unsigned long long t_exchange = t_main;
     __syncthreads(); // token_scale visible
     const int valid = stages < 2 ? stages : 2;
+    // This warp's tcgen05.ld's are complete (behind tc_fence_before): told to both CTAs, see the end.  Where a wait has run out no MMA waits for
+    // the boxes still under way, so the thread that counts them, both CTAs' in the leader, does it first.  (Here and not at the wait for
+    // the accumulators: there the branch, although nobody takes it, cost 333 x 4096 x 4096 16.7 instead of 15.6 us per call, 128 x 12288 x 4096
+    // re-quantized 20.7 instead of 19.9.)
+    auto reads_done = [&] {
+        if (!acc_ready && warp == 0 && lane == 0 && rank == 0) wait_for_boxes(full0, *static_cast<volatile int*>(&issued), (int)depth, p.status);
+        __syncwarp();
+        if (lane < 2) ptx::mbar_arrive_cluster_relaxed(ptx::map_to_cta(ptx::smem_addr(&tmem_read_bar), (uint32_t)lane));
+        __syncwarp();
+    };
 
     if constexpr (F > 1) {
         // the blocks take F * (256 / F) * ROWS * 4 bytes of the dead ring, the maxima the next KB
-        t_exchange = fold_epilogue<256 / F, F, C::ACC_STRIDE, C::NUM_THREADS, true, true>(p, tmem_base, ring, ring + 256 * ROWS * 4, valid, acc_ready, nl, n, n_ok, sn,
-                                                                              bias_h, token_scale);
+        t_exchange = fold_epilogue<256 / F, F, C::ACC_STRIDE, C::NUM_THREADS, true>(p, tmem_base, ring, ring + 256 * ROWS * 4, valid, acc_ready, nl, n, n_ok, sn,
+                                                                              bias_h, token_scale, reads_done);
     } else if constexpr (SWIGLU) {
         // accumulators into the dead ring, [token][x rows, gate rows]; then a warp finishes 32 channels of four tokens at a time
         const int pitch = 2 * p.tile_rows, lane_row = q * 32 + lane;
@@ -252,8 +264,8 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
             }
         }
         ptx::tc_fence_before();
+        reads_done();
         __syncthreads();
-        cluster_arrive(); // see the end
         t_exchange = p.stamps ? globaltimer_ns() : 0ull;
         constexpr int NV = 4;
 #pragma unroll 1
@@ -289,8 +301,7 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         tile_epilogue<C::ACC_STRIDE, C::NUM_THREADS / 128>(p, tmem_base + ((uint32_t)(q * 32) << 16), valid, acc_ready, ring, p.tile_rows, nl, nl < p.tile_rows, n,
                                                            sn, bias_h, token_scale, token0, M, grp);
         ptx::tc_fence_before();
-        __syncwarp();
-        cluster_arrive(); // see the end
+        reads_done();
         if (staged) {
             ptx::fence_proxy_async_smem(); // the tile is read by the TMA unit
             __syncthreads();
@@ -306,12 +317,12 @@ gemm_i8_token_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __gr
         }
     }
 
-    // Tensor memory was allocated by both CTAs together and is given back by both: each thread has arrived at the cluster barrier
-    // once its own tcgen05.ld's were complete, so nobody reads it any more when the wait returns, and neither CTA leaves while boxes
-    // of its partner are still counted on its barriers.  The arrival lies before the second half of the epilogue, which hides the wait.
-    __syncwarp();
-    cluster_wait();
+    // Tensor memory was allocated by both CTAs together and is given back by both, when all 32 warps have read their accumulators.  One warp of
+    // each CTA waits for that; as its CTA lives as long, nothing that the partner signals -- these arrivals, and before them the boxes
+    // counted in the leader -- comes too late.  Four limits: the partner may have used up several, one wait after another, before it arrives.
     if (warp == 1) {
+        for (int i = 0; i < 4 && !ptx::mbar_wait(ptx::smem_addr(&tmem_read_bar), 0, p.status, ST_DEC_EPI); ++i) {}
+        __syncwarp();
         ptx::tc_fence_after();
         ptx::tmem_dealloc_pair(tmem_base, C::TMEM_COLS);
     }
