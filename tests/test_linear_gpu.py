@@ -171,6 +171,15 @@ def test_linear_on_host_buffers_below_two_chunks(cuda, oracle, M, K, N, chunk, r
     test_linear_on_host_buffers_matches_device_path(cuda, oracle, M, K, N, chunk, requant)
 
 
+# Three and four chunks, the second staging buffer from a chunk's end on, not only from where the first one is full
+@pytest.mark.parametrize("M,K,N,requant,chunks", [(1000, 8192, 1024, True, 4), (1025, 2048, 2064, False, 3), (1100, 1024, 8192, True, 4),
+                                                  (1040, 8192, 520, False, 4), (1999, 4096, 1040, True, 4), (1500, 1024, 1032, False, 3)])
+def test_linear_on_host_buffers_in_three_and_four_chunks(cuda, oracle, M, K, N, requant, chunks):
+    import pplb200
+    assert len(pplb200.host_cut(M, N, K)[0]) == chunks
+    test_linear_on_host_buffers_matches_device_path(cuda, oracle, M, K, N, 0, requant)
+
+
 # A row takes longer on the wire than the launches of its linear: chunks stay at 128 rows (two and a part; one)
 @pytest.mark.parametrize("M,K,N", [(300, 16, 524288), (40, 600000, 16)])
 def test_linear_on_host_buffers_very_wide_rows(cuda, oracle, M, K, N):
