@@ -214,6 +214,15 @@ def test_linear_sees_weights_written_right_before(cuda, M, K, N):
         assert cuda.equal(y.view(cuda.int16), want.view(cuda.int16))
 
 
+# Pairs with K folded in four: both CTAs' boxes of weights counted before either CTA's activations are requested
+@pytest.mark.parametrize("M,K,N", [(48, 8208, 1024), (37, 11008, 4096), (20, 6144, 3008)])
+def test_linear_on_pairs_sees_weights_written_right_before(cuda, M, K, N):
+    import pplb200
+    plan = pplb200.gemm_plan(M, N, K)
+    assert plan["pairs"] and plan["fold"] == 4 and plan["early_weights"] == 1, plan
+    test_linear_sees_weights_written_right_before(cuda, M, K, N)
+
+
 # The first two: K shared by a cluster, weights requested ahead of the dependency wait; then token tiles, CTA pairs, K folded
 @pytest.mark.parametrize("M,K,N", [(14, 8192, 1056), (68, 15792, 2080), (300, 1024, 2048), (2400, 512, 2048), (24, 2048, 1040)])
 def test_linear_sees_scales_and_bias_written_right_before(cuda, M, K, N):
