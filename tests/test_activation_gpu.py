@@ -288,3 +288,27 @@ def test_fused_swiglu_quotient_by_all_ones(cuda, M, D, K, form):
         for a, b in zip(fused, two_step):
             assert cuda.equal(a.view(cuda.int8), b.view(cuda.int8)), t
     assert hit and pplb200.gemm_status() == 0
+
+
+# Token tiles that stay on single CTAs with K whole: x and gate on the two halves of the lanes, two row parts
+@pytest.mark.parametrize("M,D,K,parts", [(322, 3104, 32, 1), (341, 3120, 32, 1), (129, 2416, 14560, 1), (162, 4864, 16, 2), (415, 4160, 32, 2)])
+def test_medium_batch_gate_up_swiglu_on_single_ctas(cuda, oracle, M, D, K, parts):
+    import pplb200
+    plan = pplb200.gemm_plan(M, D, K, swiglu=True)
+    assert not plan["pairs"] and plan["split"] == 1 and plan["parts"] == parts and plan["token_tiles"] > 1, plan
+    test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K)
+
+
+@pytest.mark.parametrize("M,D,K,pairs", [(64, 2800, 144, True), (200, 2384, 1040, True), (33, 2688, 8192, False), (40, 11008, 272, False)])
+def test_gate_up_swiglu_of_strided_activations(cuda, M, D, K, pairs):
+    import pplb200
+    assert pplb200.gemm_plan(M, D, K, swiglu=True)["pairs"] == pairs
+    g = cuda.Generator(device="cuda").manual_seed(M + D + K)
+    xq = cuda.randint(-127, 128, (M, K + 64), generator=g, device="cuda", dtype=cuda.int8)[:, 32:32 + K]
+    w = cuda.randint(-127, 128, (2 * D, K), generator=g, device="cuda", dtype=cuda.int8)
+    sm, sn = ((cuda.rand((r,), generator=g, device="cuda") * 4 + 0.5).half() for r in (M, 2 * D))
+    got = pplb200.gate_up_swiglu_requant(xq, w, sm, sn)
+    want = pplb200.minmax_requantize_swiglu_fp16((xq.double() @ w.double().T).to(cuda.int32), sm, sn)  # int32 sums are exact in fp64
+    for a, b in zip(got, want):
+        assert cuda.equal(a.view(cuda.int8), b.view(cuda.int8))
+    assert pplb200.gemm_status() == 0

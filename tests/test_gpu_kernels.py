@@ -617,3 +617,73 @@ def test_pair_gemm_with_an_idle_partner_between_others(cuda, M, N, K, fold):
             pplb200.gemm_i8i8(a, b, out=out)
             wrong += (out != want).sum()
     assert int(wrong) == 0 and pplb200.gemm_status() == 0
+
+
+# Batches beyond 128 tokens that stay on single CTAs with K whole: one row part, two row parts; wide and few K blocks, ragged last tiles
+@pytest.mark.parametrize("M,N,K,parts", [(336, 6176, 32, 1), (367, 6256, 32, 1), (141, 5344, 15456, 1), (987, 1040, 8336, 1), (169, 9536, 16, 2), (923, 4312, 160, 2), (975, 3344, 32, 2)])
+def test_medium_batch_gemm_on_single_ctas(cuda, oracle, M, N, K, parts):
+    import pplb200
+    plan = pplb200.gemm_plan(M, N, K)
+    assert not plan["pairs"] and plan["split"] == 1 and plan["parts"] == parts and plan["token_tiles"] > 1, plan
+    if N % 16 == 0 and K < 1000:
+        test_decode_gemm_all_modes(cuda, oracle, M, N, K)
+    test_gemm_i32_alpha_beta_bias(cuda, M, N, K, 1, 0, False)
+    test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
+
+
+# Parts of K that share a quarter of the TMEM lanes, in every epilogue
+@pytest.mark.parametrize("M,N,K,fold", [(33, 896, 8192, 4), (20, 3008, 6160, 4), (64, 1808, 7744, 4), (128, 5008, 4112, 2), (81, 1296, 4096, 2)])
+def test_pair_gemm_of_densely_packed_parts(cuda, oracle, M, N, K, fold):
+    import pplb200
+    plan = pplb200.gemm_plan(M, N, K)
+    assert plan["pairs"] and plan["fold"] == fold and -(-N // 148) < 128 // fold - 8, plan
+    test_decode_gemm_all_modes(cuda, oracle, M, N, K)
+
+
+# Pairs: K folded in four and two with one box per operand and with a box per part, whole K, token tiles; columns that are 8 modulo 16
+@pytest.mark.parametrize("M,N,K,fold", [(48, 1032, 8208, 4), (33, 4728, 8192, 4), (100, 7000, 3360, 2), (128, 5000, 4112, 2), (17, 9480, 128, 0), (96, 12296, 1040, 0), (200, 4104, 528, 0)])
+def test_pair_gemm_of_strided_operands(cuda, M, N, K, fold):
+    """Rows further apart than K in both operands; int32, and fp16 against the dequantizer."""
+    import pplb200
+    plan = pplb200.gemm_plan(M, N, K)
+    assert plan["pairs"] and plan["fold"] == fold, plan
+    g = cuda.Generator(device="cuda").manual_seed(M + N + K)
+    a, b = (cuda.randint(-127, 128, (r, K + 48), generator=g, device="cuda", dtype=cuda.int8)[:, 32:32 + K] for r in (M, N))
+    sm, sn = ((cuda.rand((r,), generator=g, device="cuda") * 30 + 1).half() for r in (M, N))
+    bias = cuda.randn((N,), generator=g, device="cuda").half()
+    exact = _exact_gemm(cuda, a, b)
+    assert cuda.equal(pplb200.gemm_i8i8(a, b), exact)
+    y = pplb200.gemm_i8i8(a, b, mode=pplb200.EPI_DEQUANT_F16, scale_m=sm, scale_n=sn, bias=bias)
+    assert cuda.equal(y.view(cuda.int16), pplb200.minmax_dequantize_fp16(exact, sm, sn, bias).view(cuda.int16))
+    assert pplb200.gemm_status() == 0
+
+
+# Row maxima: of a staged tile (pairs; one CTA, one and two row parts), of folded parts (pairs, one CTA), of K partials
+@pytest.mark.parametrize("M,N,K", [(100, 12288, 256), (300, 4096, 512), (336, 6176, 32), (40, 19072, 144), (96, 8192, 4112), (37, 4096, 11008), (16, 4096, 512), (60, 2592, 7744)])
+def test_requant_epilogue_of_infinities_and_nans(cuda, M, N, K):
+    """Scales that make single results, whole rows and whole columns infinite or NaN: re-quantized as the quantizer does it from the fp16 results."""
+    import pplb200
+    g = cuda.Generator(device="cuda").manual_seed(M + N + K)
+    a, b = (cuda.randint(-127, 128, (r, K), generator=g, device="cuda", dtype=cuda.int8) for r in (M, N))
+    a[M // 2] = 0
+    b[N // 3] = 0
+    sm, sn = ((cuda.rand((r,), generator=g, device="cuda") * 30 + 1).half() for r in (M, N))
+    bias = cuda.randn((N,), generator=g, device="cuda").half()
+    for special in (float("inf"), float("nan")):
+        for where in ("column", "row", "bias", "most"):
+            m, n, c = sm.clone(), sn.clone(), bias.clone()
+            if where == "column":
+                n[N // 3], n[N - 1] = special, special
+            elif where == "row":
+                m[M // 2], m[M - 1] = special, special
+            elif where == "bias":
+                c[N - 2] = special
+            else:
+                n[1:] = special
+            y, q, s = pplb200.gemm_i8i8(a, b, mode=pplb200.EPI_DEQUANT_F16_REQUANT_I8, scale_m=m, scale_n=n, bias=c)
+            want = pplb200.minmax_dequantize_fp16(_exact_gemm(cuda, a, b), m, n, c)
+            nan = want.isnan()
+            assert cuda.equal(y.isnan(), nan) and cuda.equal(y[~nan].view(cuda.int16), want[~nan].view(cuda.int16)), (special, where)
+            wq, ws = pplb200.minmax_quantize_fp16(want)
+            assert cuda.equal(q, wq) and cuda.equal(s.isnan(), ws.isnan()) and cuda.equal(s[~s.isnan()].view(cuda.int16), ws[~ws.isnan()].view(cuda.int16)), (special, where)
+    assert pplb200.gemm_status() == 0
