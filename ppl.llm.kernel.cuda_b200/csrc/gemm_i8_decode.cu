@@ -62,7 +62,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const int lane = threadIdx.x & 31;
     const uint32_t ring = (ptx::smem_addr(smem_raw) + 1023u) & ~1023u;
     const uint32_t S = cluster_nctarank();
-    const uint32_t rank = cluster_ctarank();
+    const uint32_t rank = ptx::cluster_ctarank();
     const int n_tile = blockIdx.y;
     const unsigned long long t_start = p.stamps ? globaltimer_ns() : 0ull;
     const int SW = p.w_stages;
@@ -117,8 +117,9 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     const int q = warp & 3;    // TMEM lane quarter this warp may read
     const int grp = warp >> 2; // which groups of eight token columns it handles
     // Where K is shared or x and gate rows meet, the accumulators pass through shared memory and a warp finishes 32 rows of
-    // one token at a time; else it finishes what it reads from its lanes.
-    const bool exchanged = pack || S > 1;
+    // one token at a time; else it finishes what it reads from its lanes: two row parts, or one beyond 128 tokens (up to 128 tokens a whole K in
+    // one row part is gemm_i8_token_pair_kernel's).
+    const bool exchanged = !DUAL && (SWIGLU || BT < 128 || S > 1);
     const int row_warps = p.tile_rows > 64 ? 4 : p.tile_rows > 32 ? 2 : 1; // warps side by side in that last pass
     // per-thread output column (= weight row, one per part) and its constants
     // A tile holds tile_rows <= 128 weight rows; the MMA still spans 128 TMEM lanes, the upper ones compute on
@@ -339,31 +340,27 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         }
         {
             uint32_t a[8], b[8];
+            const int lane_row = pack ? (q & 1) * 32 + lane : q * 32 + lane;
+            const int row = lane_row + (pack ? (q >> 1) * p.tile_rows : 0);
+            auto fetch = [&](int c) {
+                TmemLd<8>::run(taddr_row + c * PIECE_COLS, a);
+                if (valid > 1) TmemLd<8>::run(taddr_row + BT + c * PIECE_COLS, b);
+            };
 #pragma unroll
-            for (int part = 0; part < NPART; ++part) { // two parts: S is 1 and nothing is exchanged
-                const int lane_row = pack ? (q & 1) * 32 + lane : q * 32 + lane;
-                const int row = lane_row + (pack ? (q >> 1) : part) * p.tile_rows;
-                const uint32_t taddr = taddr_row + part * BT;
-                auto fetch = [&](int c) {
-                    TmemLd<8>::run(taddr + c * PIECE_COLS, a);
-                    if (valid > 1) TmemLd<8>::run(taddr + NPART * BT + c * PIECE_COLS, b);
-                };
-#pragma unroll
-                for (int j = 0; j < 8; ++j) { a[j] = 0u; b[j] = 0u; }
-                int c = grp;
-                if (c < groups && have_acc) fetch(c);
+            for (int j = 0; j < 8; ++j) { a[j] = 0u; b[j] = 0u; }
+            int c = grp;
+            if (c < groups && have_acc) fetch(c);
 #pragma unroll 1
-                for (; c < groups; c += C::GROUPS) {
-                    uint32_t v[8];
-                    tmem_ld_wait8x2(a, b);
+            for (; c < groups; c += C::GROUPS) {
+                uint32_t v[8];
+                tmem_ld_wait8x2(a, b);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) v[j] = a[j] + b[j];
-                    if (c + C::GROUPS < groups && have_acc) fetch(c + C::GROUPS);
-                    if (lane_row < p.tile_rows) {
-                        const uint32_t dst = ring + (S == 1 ? (uint32_t)c * group_bytes : (uint32_t)c % S * block_bytes + (uint32_t)c / S * group_bytes) + (uint32_t)row * 4u;
+                for (int j = 0; j < 8; ++j) v[j] = a[j] + b[j];
+                if (c + C::GROUPS < groups && have_acc) fetch(c + C::GROUPS);
+                if (lane_row < p.tile_rows) {
+                    const uint32_t dst = ring + (S == 1 ? (uint32_t)c * group_bytes : (uint32_t)c % S * block_bytes + (uint32_t)c / S * group_bytes) + (uint32_t)row * 4u;
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (uint32_t)(j * pitch) * 4u), "r"(v[j]) : "memory");
-                    }
+                    for (int j = 0; j < 8; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst + (uint32_t)(j * pitch) * 4u), "r"(v[j]) : "memory");
                 }
             }
         }
@@ -379,7 +376,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                 const uint32_t to = (uint32_t)lane; // one lane per owner
                 const uint32_t bytes = groups > lane ? (uint32_t)((groups - lane + (int)S - 1) / (int)S) * group_bytes : 0u;
                 if (to < S && to != rank && bytes != 0u)
-                    ptx::bulk_copy_to_cta(map_to_cta(recv + (rank < to ? rank : rank - 1) * block_bytes, to), ring + to * block_bytes, bytes, map_to_cta(bar, to));
+                    ptx::bulk_copy_to_cta(ptx::map_to_cta(recv + (rank < to ? rank : rank - 1) * block_bytes, to), ring + to * block_bytes, bytes, ptx::map_to_cta(bar, to));
                 __syncwarp();
             }
             ok = ptx::mbar_wait(ptx::smem_addr(&recv_bar), 0, p.status, ST_DEC_EPI);
@@ -723,6 +720,7 @@ const DecDeviceInfo* dec_device_info() {
     DecDeviceInfo& d = g_dev[dev];
     if (!d.ready) {
         if (cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return nullptr;
+        d.sms &= ~1; // an SM without a partner takes no part: every whole K of up to 128 tokens in one row part runs on pairs
         if (!set_attr<16>(d.max_clusters[0]) || !set_attr<32>(d.max_clusters[1]) || !set_attr<64>(d.max_clusters[2]) ||
             !set_attr<128>(d.max_clusters[3]))
             return nullptr;

@@ -687,3 +687,14 @@ def test_requant_epilogue_of_infinities_and_nans(cuda, M, N, K):
             wq, ws = pplb200.minmax_quantize_fp16(want)
             assert cuda.equal(q, wq) and cuda.equal(s.isnan(), ws.isnan()) and cuda.equal(s[~s.isnan()].view(cuda.int16), ws[~ws.isnan()].view(cuda.int16)), (special, where)
     assert pplb200.gemm_status() == 0
+
+
+def test_whole_k_of_small_batches_in_one_row_part_runs_on_pairs(cuda):
+    """Up to 128 tokens gemm_i8_decode_kernel has no epilogue for a tile that one CTA owns in one row part: no shape may be cut that way."""
+    import pplb200
+    rng = np.random.default_rng(9)
+    for _ in range(4000):
+        M, N, K = int(rng.integers(1, 129)), int(2 ** rng.uniform(3, 15.5)) // 8 * 8, int(2 ** rng.uniform(4, 15)) // 16 * 16
+        for swiglu in (False, True):
+            plan = pplb200.gemm_plan(M, N, K, swiglu)
+            assert plan["pairs"] or plan["fold"] or plan["split"] > 1 or plan["parts"] == 2, (M, N, K, swiglu, plan)
