@@ -329,15 +329,14 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         // [owner][its groups][token][row], into its own dead ring, and one bulk copy per owner takes a block over into a
         // receive area there, counted by the owner's barrier; the owner sums S blocks.  Copies, because stores of the
         // accumulators into the other CTAs' memory, 16 bytes per lane, moved about 10 bytes per cycle: 96 x 1280 x 8192 with K
-        // shared by eight 4.4 us until the partial sums had arrived and 2.3 for the epilogue, now 3.2 and 0.8.
+        // shared by eight 4.4 us until the partial sums had arrived and 2.3 for the epilogue, now 3.1 and 0.8.  No __syncwarp in front of the cluster
+        // barriers: a warp comes out of the waits above as one, and each cost some 0.2 us (quantizer + GEMM in a graph, with / without: 4 x 5496 x 14480
+        // 19.4 / 18.6, 24 x 4752 x 8048 13.8 / 12.9, 96 x 1280 x 8192 12.8 / 11.9; by stores, before: 19.0, 13.5, 14.6).
         const int pitch = p.tile_rows * (SWIGLU ? 2 : 1); // rows of a token: x rows, then gate rows
         const int groups = (M + PIECE_COLS - 1) / PIECE_COLS, per_owner = (groups + (int)S - 1) / (int)S;
         const uint32_t group_bytes = (uint32_t)(PIECE_COLS * pitch) * 4u, block_bytes = (uint32_t)per_owner * group_bytes;
         const uint32_t recv = ring + S * block_bytes;
-        if (S > 1) {
-            __syncwarp();
-            cluster_arrive(); // this CTA's ring may be written from now on
-        }
+        if (S > 1) cluster_arrive(); // this CTA's ring may be written from now on
         {
             uint32_t a[8], b[8];
             const int lane_row = pack ? (q & 1) * 32 + lane : q * 32 + lane;
@@ -380,7 +379,6 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                 __syncwarp();
             }
             ok = ptx::mbar_wait(ptx::smem_addr(&recv_bar), 0, p.status, ST_DEC_EPI);
-            __syncwarp();
             cluster_arrive(); // received: the others' copies out of their rings to this CTA are done
         } else {
             ptx::tc_fence_before();
@@ -472,10 +470,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                 else if (token_absmax[m] != 0u) atomicMax(p.row_absmax_bits + token0 + m, token_absmax[m]);
             }
         }
-        if (S > 1) {
-            __syncwarp();
-            cluster_wait(); // nobody reads this CTA's ring any more
-        }
+        if (S > 1) cluster_wait(); // nobody reads this CTA's ring any more
     }
 #undef PPLB200_KB
     (void)ok;

@@ -312,3 +312,12 @@ def test_gate_up_swiglu_of_strided_activations(cuda, M, D, K, pairs):
     for a, b in zip(got, want):
         assert cuda.equal(a.view(cuda.int8), b.view(cuda.int8))
     assert pplb200.gemm_status() == 0
+
+
+# K shared by two or three CTAs and few groups of eight tokens
+@pytest.mark.parametrize("M,D,K", [(1, 2864, 4144), (23, 3616, 4128), (6, 2576, 1872), (8, 2688, 8192), (25, 2496, 2272)])
+def test_gate_up_swiglu_k_partials_of_few_tokens(cuda, oracle, M, D, K):
+    import pplb200
+    plan = pplb200.gemm_plan(M, D, K, swiglu=True)
+    assert plan["split"] > 1 and not plan["pairs"] and plan["rows"] > 32, plan
+    test_fused_gate_up_swiglu_matches_two_step(cuda, oracle, M, D, K)

@@ -698,3 +698,14 @@ def test_whole_k_of_small_batches_in_one_row_part_runs_on_pairs(cuda):
         for swiglu in (False, True):
             plan = pplb200.gemm_plan(M, N, K, swiglu)
             assert plan["pairs"] or plan["fold"] or plan["split"] > 1 or plan["parts"] == 2, (M, N, K, swiglu, plan)
+
+
+# K shared by three to eight CTAs and few groups of eight tokens: CTAs that own none, one or two; tiles of 40 to 128 rows
+@pytest.mark.parametrize("M,N,K", [(3, 4896, 6416), (8, 5504, 14480), (10, 4944, 7200), (31, 4784, 8752), (3, 2576, 10864), (1, 1680, 8224), (13, 1680, 9888), (17, 1984, 9808),
+                                   (65, 1680, 5952), (76, 672, 6192), (6, 448, 6816), (9, 432, 7952), (17, 1280, 7808), (86, 1264, 5504)])
+def test_decode_gemm_k_partials_of_few_tokens(cuda, oracle, M, N, K):
+    import pplb200
+    plan = pplb200.gemm_plan(M, N, K)
+    assert plan["split"] > 2 and plan["fold"] == 0 and not plan["pairs"] and plan["rows"] > 32, plan
+    test_decode_gemm_all_modes(cuda, oracle, M, N, K)
+    test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
