@@ -379,7 +379,6 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                 __syncwarp();
             }
             ok = ptx::mbar_wait(ptx::smem_addr(&recv_bar), 0, p.status, ST_DEC_EPI);
-            cluster_arrive(); // received: the others' copies out of their rings to this CTA are done
         } else {
             ptx::tc_fence_before();
             __syncthreads();
@@ -470,7 +469,14 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                 else if (token_absmax[m] != 0u) atomicMax(p.row_absmax_bits + token0 + m, token_absmax[m]);
             }
         }
-        if (S > 1) cluster_wait(); // nobody reads this CTA's ring any more
+        // Nobody reads this CTA's ring any more once all have received; but they leave together, when all are done.  Where CTAs that own nothing left
+        // first, the next launch's clusters started one by one on their SMs and prefetched against what this launch's slow ones were still
+        // waiting for: back to back in a graph, us, first / together, 1 x 5120 x 14336 16.2 / 14.6, 2 x 5120 x 8192 11.9 / 10.2 (17 x 1280 x 7808 6.3 / 6.6;
+        // with the quantizer between level).
+        if (S > 1) {
+            cluster_arrive();
+            cluster_wait();
+        }
     }
 #undef PPLB200_KB
     (void)ok;
