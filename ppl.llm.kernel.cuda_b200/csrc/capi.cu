@@ -210,10 +210,11 @@ namespace {
 // The fused form needs the CTA-pair kernel: enough 256-row x 128-channel tiles for every pair, and
 // the x / gate halves of the weight matrix aligned to the 128-row tiles.
 bool swiglu_fusable(int64_t M, int64_t D) { return M > 128 && D % 128 == 0 && ((M + 255) / 256) * (D / 128) >= kCtaPairs; }
-// Fused on single CTAs: batches for which the plain GEMM does not use CTA pairs either, from 16 channels per SM up.  With fewer the raw GEMM
-// (narrow enough to fold K) and the stand-alone kernel are faster: us fused / in two steps, tokens x channels x K: 38 x 304 x 2048
-// 12.2 / 8.2, 89 x 576 x 4096 15.9 / 12.0, 47 x 2000 x 5120 12.3 / 10.3; up to 4736 channels the two are close, beyond
-// fusing wins (83 x 8608 x 2048 15.1 / 21.2).
+// Fused in the small-batch GEMMs: batches for which the plain GEMM has no 256 x 256 tile for every CTA pair either, from 16 channels per SM up;
+// with fewer, the raw GEMM (narrow enough to fold K) and the stand-alone kernel.  The line was drawn when fused tiles had a CTA of their own
+// each and K partials met by scattered stores (38 x 304 x 2048 12.2 us fused, 8.2 in two steps).  With pairs and bulk copies fusing is the faster
+// one on both sides of it: two steps / fused, median over 129 random shapes, weights from HBM: below 600 channels 1.15 (4 of 44 shapes below
+// 1), up to 2368 1.19, up to 4736 1.15, beyond 1.23; by 1.05 .. 1.15 with more than 128 tokens.
 bool swiglu_single(int64_t M, int64_t D) { return D >= 16 * 2 * kCtaPairs && (M <= 128 || ((M + 255) / 256) * ((2 * D + 255) / 256) < kCtaPairs); }
 }
 
@@ -252,7 +253,7 @@ int32_t pplb200_i8i8_gate_up_swiglu_requant(pplb200_stream_t stream_, const void
                           activated, out_q, out_q_scale);
     }
 
-    // The single-CTA kernel writes its CTAs' partial maxima, at most 2 D per row: the [M, 2 D] int32 that the workspace
+    // The small-batch kernels write their CTAs' partial maxima, at most 2 D per row: the [M, 2 D] int32 that the workspace
     // holds for such a batch.
     int32_t parts = 1;
     if (pairs && cudaMemsetAsync(maxima, 0, (size_t)M * 4, stream) != cudaSuccess) return fail(RC_DEVICE_RUNTIME_ERROR, "memset failed");

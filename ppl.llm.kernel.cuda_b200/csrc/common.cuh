@@ -166,7 +166,7 @@ struct GemmArgs {
     // this kernel starts.
     bool after_quantizer = false;
     float beta = 1.0f;         // EPI_SWIGLU_F16
-    // EPI_SWIGLU_F16, M <= 128: the row maxima are written as *row_absmax_parts partial maxima per row, [M][parts] (at
+    // EPI_SWIGLU_F16 in a small-batch GEMM: the row maxima are written as *row_absmax_parts partial maxima per row, [M][parts] (at
     // most N values per row), instead of one cleared word; the launcher returns the number here.
     int32_t* row_absmax_parts = nullptr;
     // EPI_RAW_I32 only: out = raw_alpha * acc + raw_beta * out + raw_bias[n] in wrapping int32 (the scaling and

@@ -329,7 +329,7 @@ gemm_i8_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         // [owner][its groups][token][row], into its own dead ring, and one bulk copy per owner takes a block over into a
         // receive area there, counted by the owner's barrier; the owner sums S blocks.  Copies, because stores of the
         // accumulators into the other CTAs' memory, 16 bytes per lane, moved about 10 bytes per cycle: 96 x 1280 x 8192 with K
-        // shared by eight 4.4 us until the partial sums had arrived and 2.3 for the epilogue, now 3.1 and 0.8.  No __syncwarp in front of the cluster
+        // shared by eight 4.4 us until the partial sums had arrived and 2.3 for the epilogue, now 3.0 and 1.1.  No __syncwarp in front of the cluster
         // barriers: a warp comes out of the waits above as one, and each cost some 0.2 us (quantizer + GEMM in a graph, with / without: 4 x 5496 x 14480
         // 19.4 / 18.6, 24 x 4752 x 8048 13.8 / 12.9, 96 x 1280 x 8192 12.8 / 11.9; by stores, before: 19.0, 13.5, 14.6).
         const int pitch = p.tile_rows * (SWIGLU ? 2 : 1); // rows of a token: x rows, then gate rows
@@ -776,9 +776,10 @@ void plan_pair_swiglu(const DecDeviceInfo& dev, int64_t M, int64_t columns, int6
 // folded onto the lanes of one CTA (gemm_i8_fold_kernel).  All forms that run as one wave are modelled in SM cycles per CTA: a
 // stage costs the larger of its operands' way from L2 (60 bytes per cycle) and the issuing threads' bookkeeping (415; 425 and 500
 // with two and four boxes per operand), all weights arrive at 4500 bytes per cycle (between HBM's 3400 and the rate of what is
-// still in L2), and sharing K inside a cluster adds 3800 and 45 per token (exchange, scattered stores).  Fitted to 420 shapes of
-// 1024 .. 9472 columns, every form timed; on 520 others on average 1.3 % behind the fastest form, with SwiGLU (160 shapes) 3.1 %.  (16 x 2560 x 17424: 12.8 us
-// with clusters of six, 21.1 of seven, which need a second wave, 15.6 folded in four.)
+// still in L2), and sharing K inside a cluster adds 3800 and 45 per token (the exchange).  Fitted to 420 shapes of
+// 1024 .. 9472 columns, every form timed, when K partials still met by scattered stores; with bulk copies and pairs, on 168 random shapes of 1 .. 128
+// tokens, 1024 .. 18432 columns and K 512 .. 16384, on average 1.0 % behind the fastest form, 18 of them more than 3 % (the worst 48 x 1104 x 6304: pairs folded
+// in four 11.3 us, clusters of seven 9.6), with SwiGLU (121 shapes) 0.6 %.
 DecodePlan plan_small(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t K, bool swiglu) {
     DecodePlan best = {};
     best.tokens = (int)((M + 15) / 16 * 16);
@@ -835,7 +836,7 @@ DecodePlan plan_small(const DecDeviceInfo& dev, int64_t M, int64_t columns, int6
 // More than 128 tokens, too few for the CTA pairs' 256 x 256 tiles: the cheapest cut by a model of one CTA's time in SM
 // cycles.  A K block costs the larger of its operands' way from L2 (60 bytes per cycle and SM), its four MMAs per part
 // (half a cycle per token, 53 at least) and the issuing threads' bookkeeping (390); a launch 3000, an
-// exchange of K partials 12000 (clusters also start and end together).
+// exchange of K partials 12000 (clusters also start and end together; fitted to scattered stores).
 DecodePlan plan_medium(const DecDeviceInfo& dev, int64_t M, int64_t columns, int num_k_blocks, bool swiglu) {
     DecodePlan best = {};
     double best_cost = 1e30;
@@ -996,7 +997,8 @@ bool gemm_preloads_weights(int64_t M, int64_t N, int64_t K) {
     // only once the quantizer has ended.  Early -> late, us, tokens x N x K, weights from L2 (warm) or HBM (cold):
     // one wide MMA (fold * M columns) or a short K: 83 x 7168 x 4096 cold 13.2 -> 14.4, 2 x 5120 x 1024 cold 5.3 -> 5.5; else 1 x 8192 x 4096 warm 8.8 -> 8.4, 16 x 9216 x 4784 cold 13.3 -> 12.6
     // On pairs (2275 shapes, cold; median early / late): folded in four late, 1.02; folded in two early, 0.98 below K 6144 and 1.00 beyond; whole K early,
-    // 0.90 .. 0.96 below K 6144 -- but for the widest tiles, where graph replays are 2 % faster early and eager calls 1 % late.
+    // 0.90 .. 0.96 below K 6144.  The exception of the widest tiles is older than pairs and no longer earns its keep below K 8192.  Late / early at 112 .. 128
+    // tokens, 9728 .. 18944 columns: K 2560 1.02 .. 1.10 in graphs, 1.00 .. 1.05 eager; 4096 1.01 .. 1.06, 0.99 .. 1.04; 6144 1.00 .. 1.03, 0.97 .. 1.02; 8192 0.98 .. 1.02, 0.97 .. 1.01.
     if (plan.pair) return plan.fold == 4 || (plan.fold == 0 && M > 112 && M * K >= 320 * 1024);
     if (plan.fold) return plan.fold * M <= 128 && K >= 2048;
     // 16 x 5120 x 14336 warm 15.0 -> 14.3, 48 x 1024 x 11008 cold 12.5 -> 12.1

@@ -896,8 +896,8 @@ int32_t launch_gemm(cudaStream_t stream, const GemmArgs& a) {
     if (((a.M + 255) / 256) * ((a.N + 255) / 256) >= kCtaPairs)
         return launch_pair(stream, a, *dev);
 
-    // In between: one wave of smaller tiles on single CTAs.  (M333 K4096 N4096, linear: 16.4 us; the same on persistent
-    // 128 x 64 tiles, 192 of them in two waves, 26.4.)
+    // In between: one wave of smaller tiles, on CTA pairs that share the activations or on single CTAs.  (M333 K4096 N4096, linear: 15.6 us; on
+    // persistent 128 x 64 tiles, 192 of them in two waves, 26.4.)
     return launch_gemm_decode(stream, a, dev->status, a.pdl);
 }
 
