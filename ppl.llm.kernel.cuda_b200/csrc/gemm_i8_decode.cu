@@ -741,6 +741,7 @@ int variant_of(int64_t M) { return M <= 16 ? 0 : M <= 32 ? 1 : M <= 64 ? 2 : 3; 
 // pair at least 60 cycles for up to 120 columns, 2 per 4 columns beyond.  So they pay where there are stages enough to earn
 // the fixed part back.  Median time of quantizer + GEMM, single CTAs / pairs, over 4302 random shapes of 1 .. 128 tokens:
 //   folded in four: 32 tokens 0.91 up to 7 stages, 1.00 up to 15, 1.11 from 16; 48 tokens 0.93, 1.03, 1.11; 64 tokens 0.91, 0.99, 1.06
+//   (17 .. 32 tokens again, 18 shapes per number of stages, the quantizer's trigger early: 0.95 at 12, 1.01 at 13, 1.03 at 14, 1.04 at 15)
 //   folded in two:  80 tokens 0.99 up to 7 stages, 1.08 up to 15, 1.15 .. 1.25 from 16; 128 tokens 0.97, 1.01, 1.06 .. 1.19; 64 tokens 1.00 throughout
 //   whole K: 1.14 up to 15 stages, 1.12 up to 31, 1.04 .. 1.10 beyond
 void plan_pair(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t kb, DecodePlan& best) {
@@ -748,7 +749,7 @@ void plan_pair(const DecDeviceInfo& dev, int64_t M, int64_t columns, int64_t kb,
     const int ctas = dev.sms / 2 * 2;
     const int t16 = (int)((M + 15) / 16 * 16), t32 = (int)((M + 31) / 32 * 32);
     int F = 0;
-    if (best.fold == 4 && t16 >= 32 && (kb + 3) / 4 >= 12) F = 4;
+    if (best.fold == 4 && t16 >= 32 && (kb + 3) / 4 >= (t16 > 32 ? 12 : 13)) F = 4;
     else if (best.fold != 4 && t16 >= 80 && columns <= (int64_t)ctas * (BW / 2) && (kb + 1) / 2 * 10 >= t16) F = 2;
     else if (!best.fold && columns <= (int64_t)ctas * BW) F = 1;
     if (F == 0) return;
@@ -999,7 +1000,9 @@ bool gemm_preloads_weights(int64_t M, int64_t N, int64_t K) {
     // On pairs (2275 shapes, cold; median early / late): folded in four late, 1.02; folded in two early, 0.98 below K 6144 and 1.00 beyond; whole K early,
     // 0.90 .. 0.96 below K 6144.  The exception of the widest tiles is older than pairs and no longer earns its keep below K 8192.  Late / early at 112 .. 128
     // tokens, 9728 .. 18944 columns: K 2560 1.02 .. 1.10 in graphs, 1.00 .. 1.05 eager; 4096 1.01 .. 1.06, 0.99 .. 1.04; 6144 1.00 .. 1.03, 0.97 .. 1.02; 8192 0.98 .. 1.02, 0.97 .. 1.01.
-    if (plan.pair) return plan.fold == 4 || (plan.fold == 0 && M > 112 && M * K >= 320 * 1024);
+    // Folded in four with up to 32 tokens early all the same: late / early in graphs, three batches each, 3008 columns 1.05 at 13 stages, 1.06 at 20, 1.02 at 28,
+    // 4096 columns 1.05, 1.05, 1.02, 1.01 at 36 (early, they are no slower than single CTAs at any of them; late they were, by up to 5 %).
+    if (plan.pair) return (plan.fold == 4 && M > 32) || (plan.fold == 0 && M > 112 && M * K >= 320 * 1024);
     if (plan.fold) return plan.fold * M <= 128 && K >= 2048;
     // 16 x 5120 x 14336 warm 15.0 -> 14.3, 48 x 1024 x 11008 cold 12.5 -> 12.1
     if (plan.S > 1) return true;

@@ -709,3 +709,12 @@ def test_decode_gemm_k_partials_of_few_tokens(cuda, oracle, M, N, K):
     assert plan["split"] > 2 and plan["fold"] == 0 and not plan["pairs"] and plan["rows"] > 32, plan
     test_decode_gemm_all_modes(cuda, oracle, M, N, K)
     test_gemm_i32_alpha_beta_bias(cuda, M, N, K, -2, 5, True)
+
+
+# 17 .. 32 tokens, K folded in four: single CTAs up to twelve stages, weights ahead of the wait; pairs from thirteen on, behind it
+@pytest.mark.parametrize("M,N,K,pairs,early", [(32, 4096, 5760, False, 1), (17, 1184, 6144, False, 1), (20, 3008, 6160, True, 0), (32, 1536, 7680, True, 0), (24, 2368, 7696, True, 0)])
+def test_folded_gemm_of_17_to_32_tokens(cuda, oracle, M, N, K, pairs, early):
+    import pplb200
+    plan = pplb200.gemm_plan(M, N, K)
+    assert plan["fold"] == 4 and plan["pairs"] == pairs and plan["early_weights"] == early, plan
+    test_decode_gemm_all_modes(cuda, oracle, M, N, K)
