@@ -426,14 +426,19 @@ struct HostCut {
         const int64_t row_bytes = 2 * (K > N ? K : N);
         int64_t fine = (N * K / 5000 + 10000) * 55 / row_bytes; // ns x bytes per ns / bytes per row
         fine = fine < 128 ? 128 : round_up(fine, 128);          // 0 where a row alone takes longer than the launches (K 16, N 524288)
-        const auto share = [&](int64_t percent) { const int64_t r = round_up(M * percent / 100, 8); return r > fine ? r : fine; };
+        // rows up to a percentage of the batch, in whole 128s: a few rows more cost the GEMM a further row of tiles (538 x 19888 x 19384 cut into
+        // 128, 282 and 128 rows 810 us, into 128, 128, 128 and 154 670 .. 746; 647 x 19056 x 12136 687, 656 .. 674; 851 x 3792 x 9552 398, 390)
+        const auto part = [&](int64_t percent) { return (M * percent / 100 + 64) / 128 * 128; };
+        const auto at_least = [&](int64_t rows) { return rows > fine ? rows : fine; };
         const bool large = M * row_bytes > (12 << 20);
-        const int64_t first = share(large ? 15 : 25), second = first + share(30), before_last = M - share(large ? 20 : 25);
+        const int64_t first = at_least(part(large ? 15 : 25)), second = first + at_least(part(30));
+        int64_t before_last = part(large ? 80 : 75);
+        if (M - before_last < fine) before_last = (M - fine) / 128 * 128;
         const bool four = large && before_last - second >= fine;
         if (M > c) { // both sides of the split hold at most c rows
             split = four ? second : M >= 2 * fine ? before_last : round_up(M / 2, 8);
+            if (split < M - c) split = round_up(M - c, 128);
             if (split > c) split = c;
-            if (split < M - c) split = M - c;
         }
         int n = 0;
         const auto cut = [&](int64_t at) { if (at > (n ? end[n - 1] : 0) && at < M) end[n++] = at; };
